@@ -760,7 +760,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
       rc = want_records(direct_stat_records(npts));
       if (rc) return rc;
       if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
-      SCARF_CUDA(launch_direct_structured(s, t_ctx->obj.fs, n, p.ds, d_table, nh, d_field, d_status, st, d_rec));
+      SCARF_CUDA(launch_direct_structured(s, t_ctx->obj.fs, n, p.ds, d_table, nh, d_field, st, d_rec));
       if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
     } else {
       SCARF_CUDA(cudaMemsetAsync(d_field, 0, sizeof(float) * npts, st));
@@ -777,7 +777,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
       rc = want_records(direct_stat_records(npts));
       if (rc) return rc;
       if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
-      SCARF_CUDA(launch_direct_points(s, dx, dy, dz, npts, d_table, nh, d_field, d_status, st, d_rec));
+      SCARF_CUDA(launch_direct_points(s, dx, dy, dz, npts, d_table, nh, d_field, st, d_rec));
       if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
     } else {
       SCARF_CUDA(cudaMemsetAsync(d_field, 0, sizeof(float) * npts, st));
@@ -1289,18 +1289,16 @@ int scarf_srm_direct_structured(const scarf_srm_setup* s, const int fs[3], const
   int rc = ensure_resources();
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int* d_status = static_cast<int*>(t_ctx->res.status.p);
-  SCARF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   if (nh == 0) {
     SCARF_CUDA(cudaMemsetAsync(d_field, 0, sizeof(float) * n[0] * n[1] * n[2], st));
     return SCARF_OK;
   }
   if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
-  SCARF_CUDA(launch_direct_structured(*s, fs, n, ds, d_table, nh, d_field, d_status, st));
+  SCARF_CUDA(launch_direct_structured(*s, fs, n, ds, d_table, nh, d_field, st));
   if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
-  rc = check_device_status(d_status, st);
-  if (!rc) collect_kernel_time();
-  return rc;
+  SCARF_CUDA(cudaStreamSynchronize(st));
+  collect_kernel_time();
+  return SCARF_OK;
 }
 
 int scarf_srm_direct_points(const scarf_srm_setup* s, const float* d_x, const float* d_y, const float* d_z,
@@ -1311,18 +1309,16 @@ int scarf_srm_direct_points(const scarf_srm_setup* s, const float* d_x, const fl
   int rc = ensure_resources();
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int* d_status = static_cast<int*>(t_ctx->res.status.p);
-  SCARF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   if (nh == 0) {
     SCARF_CUDA(cudaMemsetAsync(d_field, 0, sizeof(float) * npts, st));
     return SCARF_OK;
   }
   if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
-  SCARF_CUDA(launch_direct_points(*s, d_x, d_y, d_z, npts, d_table, nh, d_field, d_status, st));
+  SCARF_CUDA(launch_direct_points(*s, d_x, d_y, d_z, npts, d_table, nh, d_field, st));
   if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
-  rc = check_device_status(d_status, st);
-  if (!rc) collect_kernel_time();
-  return rc;
+  SCARF_CUDA(cudaStreamSynchronize(st));
+  collect_kernel_time();
+  return SCARF_OK;
 }
 
 // Device-field entry points let the longest axis be the column axis

@@ -30,10 +30,10 @@ int direct_get_sincos();
 // d_stats (optional): direct_stat_records(npts) records.
 long long direct_stat_records(long long npts);
 cudaError_t launch_direct_structured(const scarf_srm_setup& s, const int fs[3], const int n[3], float ds,
-                                     const float* d_table, int nh, float* d_field, int* d_status,
+                                     const float* d_table, int nh, float* d_field,
                                      cudaStream_t stream, StatRecord* d_stats = nullptr);
 cudaError_t launch_direct_points(const scarf_srm_setup& s, const float* d_x, const float* d_y, const float* d_z,
-                                 long long npts, const float* d_table, int nh, float* d_field, int* d_status,
+                                 long long npts, const float* d_table, int nh, float* d_field,
                                  cudaStream_t stream, StatRecord* d_stats = nullptr);
 
 // ---- factorised tensor-core form (srm_tc.cu) ----

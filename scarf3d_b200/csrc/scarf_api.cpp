@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <sstream>
@@ -185,6 +186,7 @@ struct Resources {
   DeviceBuf status, stats, table, field, coords, work, slab_cnt, statrec, poi;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr, evs = nullptr;
   cudaEvent_t evp = nullptr;  // the coordinates' upload on the copy stream
+  std::vector<cudaEvent_t> pass_ev;    // end of each pass of the gridded form
   cudaStream_t copy_stream = nullptr;  // non-blocking: runs beside the legacy stream too
   int* slab_flags = nullptr;           // host-mapped, written by the kernel
   int* slab_flags_dev = nullptr;
@@ -211,6 +213,8 @@ struct Resources {
     evs = nullptr;
     if (evp) cudaEventDestroy(evp);
     evp = nullptr;
+    for (cudaEvent_t e : pass_ev) cudaEventDestroy(e);
+    pass_ev.clear();
     if (evk0) cudaEventDestroy(evk0);
     if (evk1) cudaEventDestroy(evk1);
     evk0 = evk1 = nullptr;
@@ -463,6 +467,50 @@ int copy_slabs_out(const TcPlan& plan, const TcSlabSignal& sig, const float* d_f
     }
     SCARF_CUDA(cudaMemcpy2DAsync(field + off, plane * sizeof(float), d_field + off, plane * sizeof(float), width,
                                  e.z1 - e.z0, cudaMemcpyDeviceToHost, t_ctx->res.copy_stream));
+  }
+  return bc.finish();
+}
+
+// The copy stream, its join event and one event per pass of the gridded form.
+int ensure_pass_resources(int passes) {
+  if (!t_ctx->res.copy_stream) SCARF_CUDA(cudaStreamCreateWithFlags(&t_ctx->res.copy_stream, cudaStreamNonBlocking));
+  if (!t_ctx->res.evs) SCARF_CUDA(cudaEventCreateWithFlags(&t_ctx->res.evs, cudaEventDisableTiming));
+  while (static_cast<int>(t_ctx->res.pass_ev.size()) < passes) {
+    cudaEvent_t e = nullptr;
+    SCARF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    t_ctx->res.pass_ev.push_back(e);
+  }
+  return SCARF_OK;
+}
+
+// Copies the planes of each pass of the gridded form to the host field on
+// the copy stream, behind the pass's event, while later passes compute.
+int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
+  const bool bounce = is_pageable(field);
+  const size_t plane = sizeof(float) * static_cast<size_t>(plan.nx) * plan.ny;
+  if (bounce) {
+    const int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(plane * plan.zc / 2, 1 << 20)));
+    if (rc) return rc;
+  }
+  cudaStream_t cs = t_ctx->res.copy_stream;
+  BounceCopier bc(cs);
+  for (int pass = 0; pass < grid_passes(plan); ++pass) {
+    int z0, z1;
+    grid_pass_planes(plan, pass, &z0, &z1);
+    SCARF_CUDA(cudaStreamWaitEvent(cs, t_ctx->res.pass_ev[pass], 0));
+    char* dst = reinterpret_cast<char*>(field) + plane * z0;
+    const char* src = reinterpret_cast<const char*>(d_field) + plane * z0;
+    const size_t bytes = plane * (z1 - z0);
+    if (!bounce) {
+      SCARF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, cs));
+      continue;
+    }
+    const size_t row = t_ctx->res.bounce_slot;
+    const size_t rows = bytes / row, rest = bytes - rows * row;
+    int rc = SCARF_OK;
+    if (rows) rc = bc.issue(dst, row, src, row, row, rows);
+    if (!rc && rest) rc = bc.issue(dst + rows * row, rest, src + rows * row, rest, rest, 1);
+    if (rc) return rc;
   }
   return bc.finish();
 }
@@ -730,9 +778,39 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     TcPlan plan{};
     TcChoice tuned{};
     const bool have_tuned = use_tc && nh > 0 && tc_tuned_choice(s.ndim, n, true, &tuned);
+    // The automatic form: the gridded sum where it takes the grid and its
+    // workspace fits (also within the device-memory cap), unless a tensor-core
+    // plan was tuned for this grid.
+    GridPlan grid{};
+    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned && grid_make_plan(s.ndim, n, nh, &grid);
+    if (use_grid && t_ctx->res.work.ensure(grid.bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      (void)scarf::take_device_alloc_failure();
+      use_grid = false;
+    }
     const bool planned = have_tuned ? tc_make_plan(s.ndim, n, nh, &plan, tuned.tile_j, false, tuned.variant)
                                     : tc_make_plan(s.ndim, n, nh, &plan);
-    if (use_tc && nh > 0 && planned) {
+    if (use_grid) {
+      const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
+      if (overlap) {
+        rc = ensure_pass_resources(grid_passes(grid));
+        if (rc) return rc;
+      }
+      rc = want_records(grid_stat_records(grid));
+      if (rc) return rc;
+      if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
+      std::function<cudaError_t(int)> pass_done;
+      if (overlap) pass_done = [&](int pass) { return cudaEventRecord(t_ctx->res.pass_ev[pass], st); };
+      SCARF_CUDA(launch_grid_structured(s, t_ctx->obj.fs, p.ds, d_table, d_field, t_ctx->res.work.p, grid, st, d_rec,
+                                        pass_done));
+      if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
+      if (overlap) {
+        copy_join.active = true;
+        rc = copy_passes_out(grid, d_field, field);
+        if (rc) return rc;
+        copied_out = true;
+      }
+    } else if (use_tc && nh > 0 && planned) {
       SCARF_CUDA(t_ctx->res.work.ensure(plan.bytes));
       // Without rescale or taper the field is final when the kernel stores
       // it: copy it out slab by slab while the kernel still runs.

@@ -1,0 +1,992 @@
+// Structured SRM sums through a non-uniform Fourier transform.
+//
+// On a regular grid the sum over harmonics (scarflib_srm.f90:794-809) is a
+// Fourier sum at arbitrary wavenumbers: with i', j' the indices about the
+// grid's middle,
+//   field(i, j, k) = scaling Re sum_h E_h(k) e^{2 pi i (wx_h i' + wy_h j')},
+//   E_h(k) = (b - i a) e^{i (kx x_mid + ky y_mid + kz z_k + v . bar)},
+// and e^{2 pi i w n} for |n| <= N/2 is, to ~2e-7, a weighted sum of the nine
+// nearest waves of period M >= 1.5 N (Dutt & Rokhlin 1993; Kaiser-Bessel
+// weights, whose Fourier transform is known in closed form). So
+//   1. every harmonic adds E_h(k) to 9 x 9 cells (cx, cy) of a wavenumber
+//      grid, for every k (the z dependence stays exact): T1[cx][cy][k];
+//   2. an inverse FFT of length My along cy gives T2[cx][j][k];
+//   3. an inverse real FFT of length Mx along cx gives the field.
+// Wavenumbers with wx < 0 are taken as their conjugates (the field is a real
+// part), so only cx in [0, Mx/2] is kept; the parts of a harmonic's cells
+// outside that range fold back as the cells of a mirror entry (-w, conj E).
+// The work is ~1.5 x 2.25 cells per point through two FFT passes plus 81
+// multiply-adds per harmonic and plane, where the factorised contraction
+// (srm_tc.cu) takes 12 tensor operations per point and harmonic.
+//
+// Precision: phases in FP64, E, weights and FFTs in FP32; ~4e-7 of the
+// field's standard deviation against FP64 where the split-BF16 contraction
+// has ~5e-6. Summation order is fixed (sorted entries, fixed partial sums),
+// so a field is reproducible bit for bit.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
+#include "common.cuh"
+#include "srm_kernels.h"
+
+namespace scarf {
+namespace {
+
+constexpr int kW = 9;             // cells per harmonic and gridded axis
+constexpr int kB = 4;             // cells per bin
+constexpr int kSpan = 3;          // bins that a harmonic's cells can touch
+constexpr int kMinM = 24;         // shortest transform (a harmonic's cells never wrap onto themselves)
+constexpr double kOversample = 1.5;
+constexpr int kSparse = 32;       // entries of a bin that one warp sums
+constexpr int kPart = 256;        // entries that one block sums (32 per warp)
+constexpr int kScanThreads = 1024;
+constexpr int kFftThreads = 256;
+static_assert((kSpan - 1) * kB + 1 == kW, "a cell bin is reached from exactly kSpan start bins");
+
+// -------------------------------------------------------------- FFT stages --
+using GridFft = GridPlan::Fft;
+
+struct GridArgs {
+  GridFft fx, fy;      // lengths mx / 2 and my
+  int mx, my, hx;      // transform lengths, hx = mx / 2
+  int nx, ny, nz;      // logical extents: x, gridded second axis (1: none), z
+  int sx, sy;          // index of the grid's middle: i' = i - sx, j' = j - sy
+  int nbx, nby, nkeys; // cell bins along x and y; start-bin keys
+  int nent;            // entries: a harmonic and possibly its mirror
+  int nh;
+  long long ez;        // z pitch of E
+  int maxtasks, maxslots;
+  double beta_x, beta_y, inv_i0_x, inv_i0_y;
+  double m[9], bar[3], ds;
+  int fs[3];           // first index (1-based) of the axes x, y, z of the caller
+  int ax_y, ax_z;      // physical axes of the logical second and third axes
+  float scaling;
+  long long plane;     // elements between consecutive z of the field
+  const float* table;
+  uint2* keys;         // per entry: start-bin key, order of arrival in its bin
+  int* members;        // entries by bin, in order of arrival
+  int* place;          // per entry: its place in bin and entry order
+  int* counts;         // entries per key
+  double4* par;        // per harmonic: phase (turns), wz (turns per index), a, b
+  double2* w;          // per harmonic: wx, wy (cells)
+  int* bin_start;
+  float* weights;      // per sorted entry: x weights of 3 bins, y weights of 3 bins
+  float2* e;           // [nent][ez]
+  float2* t1;          // [hx + 1][my][zc]
+  float2* t2;          // [hx + 1][ny][zc]
+  float2* partial;     // [slot][kB * kB][zc]
+  int* ntasks;         // three counters: tasks, slots, bins with several parts
+  int4* tasks;         // {bin, part, parts, slot} of the bins that blocks sum
+  int4* multi;         // {bin, parts, slot, -} of those with several parts
+  float2* twx;         // e^{2 pi i k / mx}
+  float2* twy;         // e^{2 pi i k / my}
+  int* revx;
+  int* revy;
+  float* dcx;          // 1 / window transform, times the field's scaling
+  float* dcy;
+};
+
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
+  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ float2 muli(float2 a) { return make_float2(-a.y, a.x); }
+
+// Inverse (e^{+i}) DFT of R values in registers, natural order.
+template <int R>
+struct Dft;
+template <>
+struct Dft<2> {
+  static __device__ __forceinline__ void run(float2* v) {
+    const float2 t = v[0];
+    v[0] = cadd(t, v[1]);
+    v[1] = csub(t, v[1]);
+  }
+};
+template <>
+struct Dft<3> {
+  static __device__ __forceinline__ void run(float2* v) {
+    const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+    const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
+    const float2 s = muli(make_float2(0.86602540378443864676f * d.x, 0.86602540378443864676f * d.y));
+    v[0] = cadd(v[0], t);
+    v[1] = cadd(m, s);
+    v[2] = csub(m, s);
+  }
+};
+template <>
+struct Dft<4> {
+  static __device__ __forceinline__ void run(float2* v) {
+    const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = muli(csub(v[1], v[3]));
+    v[0] = cadd(a, c);
+    v[1] = cadd(b, d);
+    v[2] = csub(a, c);
+    v[3] = csub(b, d);
+  }
+};
+template <>
+struct Dft<5> {
+  static __device__ __forceinline__ void run(float2* v) {
+    constexpr float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;  // cos(2 pi / 5), cos(4 pi / 5)
+    constexpr float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;   // sin
+    const float2 a = cadd(v[1], v[4]), b = cadd(v[2], v[3]), c = csub(v[1], v[4]), d = csub(v[2], v[3]);
+    const float2 m1 = make_float2(v[0].x + c1 * a.x + c2 * b.x, v[0].y + c1 * a.y + c2 * b.y);
+    const float2 m2 = make_float2(v[0].x + c2 * a.x + c1 * b.x, v[0].y + c2 * a.y + c1 * b.y);
+    const float2 n1 = muli(make_float2(s1 * c.x + s2 * d.x, s1 * c.y + s2 * d.y));
+    const float2 n2 = muli(make_float2(s2 * c.x - s1 * d.x, s2 * c.y - s1 * d.y));
+    v[0] = cadd(v[0], cadd(a, b));
+    v[1] = cadd(m1, n1);
+    v[2] = cadd(m2, n2);
+    v[3] = csub(m2, n2);
+    v[4] = csub(m1, n1);
+  }
+};
+template <>
+struct Dft<8> {
+  static __device__ __forceinline__ void run(float2* v) {
+    constexpr float r = 0.70710678118654752440f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    Dft<4>::run(e);
+    Dft<4>::run(o);
+    o[1] = make_float2(r * (o[1].x - o[1].y), r * (o[1].x + o[1].y));
+    o[2] = muli(o[2]);
+    o[3] = make_float2(-r * (o[3].x + o[3].y), r * (o[3].x - o[3].y));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = cadd(e[k], o[k]);
+      v[k + 4] = csub(e[k], o[k]);
+    }
+  }
+};
+template <>
+struct Dft<16> {
+  static __device__ __forceinline__ void run(float2* v) {
+    constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, r = 0.70710678118654752440f;
+    // e^{2 pi i b k / 16} for b, k in 1..3
+    const float2 w[3][3] = {{{c1, s1}, {r, r}, {s1, c1}}, {{r, r}, {0.0f, 1.0f}, {-r, r}}, {{s1, c1}, {-r, r}, {-c1, -s1}}};
+    float2 y[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      y[b][0] = v[b], y[b][1] = v[b + 4], y[b][2] = v[b + 8], y[b][3] = v[b + 12];
+      Dft<4>::run(y[b]);
+      if (b > 0) {
+#pragma unroll
+        for (int k = 1; k < 4; ++k) y[b][k] = cmulf(y[b][k], w[b - 1][k - 1]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 t[4] = {y[0][k], y[1][k], y[2][k], y[3][k]};
+      Dft<4>::run(t);
+      v[k] = t[0], v[k + 4] = t[1], v[k + 8] = t[2], v[k + 12] = t[3];
+    }
+  }
+};
+
+// One decimation-in-frequency stage of radix R over a tile of ZT transforms
+// in shared memory (element e of transform z at [e * ZT + z]): reads through
+// `in`, writes through `out`, both called with (element, z). In place when
+// both address the same array: a butterfly writes where it read.
+template <int R, int ZT, class In, class Out>
+__device__ __forceinline__ void fft_stage(const GridFft& f, int s, const float2* __restrict__ tw, int tw_step, In in,
+                                          Out out) {
+  const int m = f.m[s];       // distance between a butterfly's elements
+  const int len = m * R;      // sub-transform length of this stage
+  const float inv_m = f.inv_m[s];
+  const int step = f.n / len * tw_step;  // twiddle e^{2 pi i q t / len} is tw[q t step]
+  for (int it = threadIdx.x; it < f.n / R * ZT; it += kFftThreads) {
+    const int z = it & (ZT - 1), g = it / ZT;
+    const int blk = static_cast<int>((static_cast<float>(g) + 0.5f) * inv_m);
+    const int q = g - blk * m;
+    const int base = blk * len + q;
+    float2 v[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = in(base + t * m, z);
+    Dft<R>::run(v);
+    if (m > 1) {
+#pragma unroll
+      for (int t = 1; t < R; ++t) v[t] = cmulf(v[t], __ldg(tw + q * t * step));
+    }
+#pragma unroll
+    for (int t = 0; t < R; ++t) out(base + t * m, z, t, v[t]);
+  }
+}
+template <int ZT, class In, class Out>
+__device__ __forceinline__ void fft_stage_any(const GridFft& f, int s, const float2* tw, int tw_step, In in, Out out) {
+  switch (f.r[s]) {
+    case 16: fft_stage<16, ZT>(f, s, tw, tw_step, in, out); break;
+    case 8: fft_stage<8, ZT>(f, s, tw, tw_step, in, out); break;
+    case 5: fft_stage<5, ZT>(f, s, tw, tw_step, in, out); break;
+    case 4: fft_stage<4, ZT>(f, s, tw, tw_step, in, out); break;
+    case 3: fft_stage<3, ZT>(f, s, tw, tw_step, in, out); break;
+    default: fft_stage<2, ZT>(f, s, tw, tw_step, in, out); break;
+  }
+}
+
+// ------------------------------------------------------------- preparation --
+// Kaiser-Bessel weight at distance d (cells) from a harmonic's wavenumber.
+__device__ __forceinline__ float kb_weight(double d, double beta, double inv_i0) {
+  const double x = d * (2.0 / kW);
+  const double t = 1.0 - x * x;
+  return t <= 0.0 ? 0.0f : static_cast<float>(cyl_bessel_i0(beta * sqrt(t)) * inv_i0);
+}
+
+// One thread per item: every harmonic's wavenumber in cells, its phase at
+// the grid's middle and its entries' sort keys; then the twiddles, output
+// orders and window transforms of both axes.
+__device__ __forceinline__ int first_cell(double c) { return static_cast<int>(ceil(c - 0.5 * kW)); }
+__device__ __forceinline__ int floor_bin(int c) { return (c >= 0 ? c : c - (kB - 1)) / kB; }
+
+__device__ int output_order(const GridFft& f, int g) {
+  // Butterfly g of the last stage holds elements g R .. g R + R - 1 of the
+  // digit-reversed output; its first output index:
+  int k = 0, w = 1, pos = g * f.r[f.nst - 1], span = f.n;
+  for (int s = 0; s + 1 < f.nst; ++s) {
+    span /= f.r[s];
+    const int d = pos / span;
+    pos -= d * span;
+    k += d * w;
+    w *= f.r[s];
+  }
+  return k;
+}
+
+__device__ float window_inverse(int n, int m, double beta) {
+  const double pi = 3.14159265358979323846;
+  const double u = pi * kW * n / m;
+  const double r = sqrt(beta * beta - u * u);
+  return static_cast<float>(cyl_bessel_i0(beta) * r / (kW * sinh(r)));
+}
+
+__global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
+  long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const double two_pi = 6.28318530717958647692;
+  if (t < A.nh) {
+    const float* r = A.table + 5 * t;
+    const double v1 = r[0], v2 = r[1], v3 = r[2];
+    double k[3];
+    for (int c = 0; c < 3; ++c) k[c] = (v1 * A.m[c] + v2 * A.m[3 + c] + v3 * A.m[6 + c]) * A.ds / two_pi;
+    const double c = (v1 * A.bar[0] + v2 * A.bar[1] + v3 * A.bar[2]) / two_pi;
+    // Phase at the middle of x and y and at the first z; axes of one point
+    // other than these add their constant.
+    double ph = c;
+    int mid[3] = {A.sx, 0, 0};
+    if (A.ny > 1) mid[A.ax_y] = A.sy;
+    for (int ax = 0; ax < 3; ++ax) ph += k[ax] * static_cast<double>(A.fs[ax] - 1 + mid[ax]);
+    double wx = k[0] - rint(k[0]), wy = A.ny > 1 ? k[A.ax_y] - rint(k[A.ax_y]) : 0.0, wz = k[A.ax_z];
+    double a = r[3], b = r[4];
+    if (wx < 0.0) {  // the conjugate: (b - i a) e^{i p} -> (b + i a) e^{-i p}
+      wx = -wx;
+      wy = -wy;
+      wz = -wz;
+      ph = -ph;
+      a = -a;
+    }
+    if (wy < 0.0) wy += 1.0;
+    const double cx = wx * A.mx, cy = wy * A.my;
+    A.par[t] = make_double4(ph - rint(ph), wz, a, b);
+    A.w[t] = make_double2(cx, cy);
+    auto key = [&](double x, double y) {
+      const int bx = floor_bin(first_cell(x)) + kSpan;  // -kSpan .. nbx - 1, shifted
+      if (A.ny == 1) return static_cast<uint32_t>(bx);
+      int s = first_cell(y);
+      s += s < 0 ? A.my : 0;
+      s -= s >= A.my ? A.my : 0;
+      return static_cast<uint32_t>(bx * A.nby + s / kB);
+    };
+    auto arrive = [&](uint32_t k) {
+      const bool none = static_cast<int>(k) >= A.nkeys;
+      return make_uint2(k, none ? 0u : static_cast<uint32_t>(atomicAdd(A.counts + k, 1)));
+    };
+    A.keys[t] = arrive(key(cx, cy));
+    // Mirror entry: cells below 0 or above hx, folded back.
+    uint32_t mk = static_cast<uint32_t>(A.nkeys);  // none
+    const int s0 = first_cell(cx);
+    const double my_y = cy > 0.0 ? A.my - cy : 0.0;
+    if (s0 < 0)
+      mk = key(-cx, my_y);
+    else if (s0 + kW - 1 > A.hx)
+      mk = key(A.mx - cx, my_y);
+    A.keys[A.nh + t] = arrive(mk);
+    return;
+  }
+  t -= A.nh;
+  if (t < A.mx) {
+    double s, c;
+    sincospi(2.0 * static_cast<double>(t) / A.mx, &s, &c);
+    A.twx[t] = make_float2(static_cast<float>(c), static_cast<float>(s));
+    return;
+  }
+  t -= A.mx;
+  if (t < A.my) {
+    double s, c;
+    sincospi(2.0 * static_cast<double>(t) / A.my, &s, &c);
+    A.twy[t] = make_float2(static_cast<float>(c), static_cast<float>(s));
+    return;
+  }
+  t -= A.my;
+  if (t < A.nx) {
+    A.dcx[t] = window_inverse(static_cast<int>(t) - A.sx, A.mx, A.beta_x) * A.scaling;
+    return;
+  }
+  t -= A.nx;
+  if (t < A.ny) {
+    A.dcy[t] = A.ny > 1 ? window_inverse(static_cast<int>(t) - A.sy, A.my, A.beta_y) : 1.0f;
+    return;
+  }
+  t -= A.ny;
+  const int gx = A.fx.n / A.fx.r[A.fx.nst - 1];
+  if (t < gx) {
+    A.revx[t] = output_order(A.fx, static_cast<int>(t));
+    return;
+  }
+  t -= gx;
+  if (A.ny > 1 && t < A.fy.n / A.fy.r[A.fy.nst - 1]) A.revy[t] = output_order(A.fy, static_cast<int>(t));
+}
+
+// Exclusive scan of the entry counts per key (one block).
+__global__ void __launch_bounds__(kScanThreads) grid_scan_kernel(const GridArgs A) {
+  __shared__ int s_warp[kScanThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int carry = 0;
+  for (int base = 0; base <= A.nkeys; base += 4 * kScanThreads) {
+    int v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = base + 4 * t + u;
+      v[u] = k < A.nkeys ? A.counts[k] : 0;
+    }
+    const int mine = v[0] + v[1] + v[2] + v[3];
+    int x = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    int w = s_warp[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    const int before_warp = warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0;
+    const int all = __shfl_sync(0xffffffffu, w, 31);
+    int at = carry + before_warp + x - mine;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = base + 4 * t + u;
+      if (k <= A.nkeys) A.bin_start[k] = at;
+      at += v[u];
+    }
+    carry += all;
+    __syncthreads();
+  }
+}
+
+// The kSpan x kSpan start bins whose entries reach cell bin (bx, by): lane
+// l < 9 holds bin l's entry range.
+__device__ __forceinline__ void bin_ranges(const GridArgs& A, int bin, int lane, int* lo, int* hi) {
+  const int bx = bin / A.nby, by = bin - bx * A.nby;
+  *lo = *hi = 0;
+  const int dx = lane / kSpan, dy = lane - dx * kSpan;
+  if (lane < kSpan * kSpan && (A.ny > 1 || dy == 0)) {
+    int sy = by - dy;
+    sy += sy < 0 ? A.nby : 0;
+    const int key = (bx - dx + kSpan) * A.nby + sy;
+    *lo = A.bin_start[key];
+    *hi = A.bin_start[key + 1];
+  }
+}
+
+// Entries into their bins, in order of arrival; the blocks after them list
+// the tasks of bins with more than kSparse entries (one warp per bin): one
+// block per kPart entries, whose partial sum gets a slot when the bin has
+// several. Task and slot numbers depend on the order of arrival, sums do not.
+__global__ void __launch_bounds__(256) grid_bins_kernel(const GridArgs A, int scatter_blocks) {
+  if (static_cast<int>(blockIdx.x) < scatter_blocks) {
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= A.nent) return;
+    const uint2 k = A.keys[e];
+    if (static_cast<int>(k.x) < A.nkeys) A.members[A.bin_start[k.x] + k.y] = e;
+    return;
+  }
+  const int bin = (blockIdx.x - scatter_blocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (bin >= A.nbx * A.nby) return;
+  int lo, hi;
+  bin_ranges(A, bin, lane, &lo, &hi);
+  const int total = __reduce_add_sync(0xffffffffu, hi - lo);
+  if (total <= kSparse) return;
+  const int parts = (total + kPart - 1) / kPart;
+  int task = 0, slot = 0;
+  if (lane == 0) {
+    task = atomicAdd(A.ntasks, parts);
+    if (parts > 1) {
+      slot = atomicAdd(A.ntasks + 1, parts);
+      A.multi[atomicAdd(A.ntasks + 2, 1)] = make_int4(bin, parts, slot, 0);
+    }
+  }
+  task = __shfl_sync(0xffffffffu, task, 0);
+  slot = __shfl_sync(0xffffffffu, slot, 0);
+  for (int p = lane; p < parts; p += 32) A.tasks[task + p] = make_int4(bin, p, parts, slot);
+}
+
+// One warp per entry: its place among its bin's entries (ordered by entry
+// number: a fixed order makes every sum over a bin reproducible), its weights
+// aligned to bins, and E along z: FP64 phases, stepped by 32 planes with one
+// complex product.
+__global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z0, int nzc, int first) {
+  const int e = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (e >= A.nent) return;
+  const int key = static_cast<int>(A.keys[e].x);
+  if (key >= A.nkeys) return;  // no mirror
+  int i;
+  if (first) {
+    const int lo = A.bin_start[key], hi = A.bin_start[key + 1];
+    int before = 0;
+    for (int k = lo + lane; k < hi; k += 32) before += A.members[k] < e ? 1 : 0;
+    i = lo + __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) A.place[e] = i;
+  } else {
+    i = A.place[e];
+  }
+  const bool mirror = e >= A.nh;
+  const int h = mirror ? e - A.nh : e;
+  double4 p = A.par[h];
+  if (mirror) {
+    p.x = -p.x;
+    p.y = -p.y;
+    p.z = -p.z;
+  }
+  if (first && lane < 2 * kSpan * kB) {
+    const double2 c = A.w[h];
+    float v;
+    if (lane < kSpan * kB) {
+      const bool low = first_cell(c.x) < 0;
+      const double x = !mirror ? c.x : (low ? -c.x : A.mx - c.x);
+      const int cell = floor_bin(first_cell(x)) * kB + lane;
+      v = kb_weight(cell - x, A.beta_x, A.inv_i0_x);
+      // A cell belongs to the primary entry inside [0, hx], and outside it,
+      // folded, to the mirror.
+      if (!mirror ? (cell < 0 || cell > A.hx) : (low ? cell < 1 : cell > A.hx - 1)) v = 0.0f;
+    } else if (A.ny > 1) {
+      const double y = !mirror ? c.y : (c.y > 0.0 ? A.my - c.y : 0.0);
+      const int cell = floor_bin(first_cell(y)) * kB + (lane - kSpan * kB);
+      v = kb_weight(cell - y, A.beta_y, A.inv_i0_y);
+    } else {
+      v = lane == kSpan * kB ? 1.0f : 0.0f;
+    }
+    A.weights[static_cast<size_t>(i) * (2 * kSpan * kB) + lane] = v;
+  }
+  // E(z) = (b - i a) e^{2 pi i (phase + wz z)} for z = z0 + lane, + 32, ...
+  double s, c, ds, dc;
+  const double turns = p.x + p.y * static_cast<double>(z0 + lane), step = p.y * 32.0;
+  sincospi(2.0 * (turns - rint(turns)), &s, &c);
+  sincospi(2.0 * (step - rint(step)), &ds, &dc);
+  float2* out = A.e + static_cast<size_t>(i) * A.ez;
+  for (int z = lane; z < nzc; z += 32) {
+    out[z] = make_float2(static_cast<float>(p.w * c + p.z * s), static_cast<float>(p.w * s - p.z * c));
+    const double n = c * dc - s * ds;
+    s = c * ds + s * dc;
+    c = n;
+  }
+}
+
+// Step 1. A warp sums up to 32 entries of one 4 x 4-cell bin over 32 planes:
+// lanes are planes, the 16 cells are registers. Bins of up to kSparse entries
+// are one warp's; the first blocks take the listed tasks, 8 warps each whose
+// sums are added in order through shared memory. Bound: load latency (256
+// bytes of E and two weight vectors per entry), hence four entries in flight;
+// FP32 issue (40 multiply-adds per entry and warp) where bins are dense.
+struct BinSum {
+  float2 acc[kB][kB];
+};
+__device__ __forceinline__ void sum_entries(const GridArgs& A, int lane, int lo, int hi, int beg, int end,
+                                            const float2* ez, BinSum& S) {
+#pragma unroll
+  for (int i = 0; i < kB; ++i)
+#pragma unroll
+    for (int j = 0; j < kB; ++j) S.acc[i][j] = make_float2(0.0f, 0.0f);
+  if (beg >= end) return;
+  // Inclusive prefix of the range lengths; lane l resolves visit beg + l to an
+  // entry and its bin offset.
+  int pre = hi - lo;
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, pre, o);
+    if (lane >= o) pre += y;
+  }
+  int r = 0;
+#pragma unroll
+  for (int q = 0; q < kSpan * kSpan; ++q) r += __shfl_sync(0xffffffffu, pre, q) <= beg + lane ? 1 : 0;
+  const int rc = min(r, kSpan * kSpan - 1);
+  const int ent = __shfl_sync(0xffffffffu, hi, rc) - (__shfl_sync(0xffffffffu, pre, rc) - (beg + lane));
+  const int n = end - beg;
+  auto add = [&](const float4& wx, const float4& wy, const float2& e) {
+    const float x[4] = {wx.x, wx.y, wx.z, wx.w}, y[4] = {wy.x, wy.y, wy.z, wy.w};
+#pragma unroll
+    for (int i = 0; i < kB; ++i) {
+      const float2 t = make_float2(x[i] * e.x, x[i] * e.y);
+#pragma unroll
+      for (int j = 0; j < kB; ++j) {
+        S.acc[i][j].x = fmaf(y[j], t.x, S.acc[i][j].x);
+        S.acc[i][j].y = fmaf(y[j], t.y, S.acc[i][j].y);
+      }
+    }
+  };
+  int u = 0;
+  for (; u + 4 <= n; u += 4) {
+    float4 wx[4], wy[4];
+    float2 e[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int en = __shfl_sync(0xffffffffu, ent, u + g), rr = __shfl_sync(0xffffffffu, rc, u + g);
+      const float4* w = reinterpret_cast<const float4*>(A.weights) + static_cast<size_t>(en) * (2 * kSpan);
+      wx[g] = __ldg(w + rr / kSpan);
+      wy[g] = __ldg(w + kSpan + rr % kSpan);
+      e[g] = __ldg(ez + static_cast<size_t>(en) * A.ez);
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) add(wx[g], wy[g], e[g]);
+  }
+  for (; u < n; ++u) {
+    const int en = __shfl_sync(0xffffffffu, ent, u), rr = __shfl_sync(0xffffffffu, rc, u);
+    const float4* w = reinterpret_cast<const float4*>(A.weights) + static_cast<size_t>(en) * (2 * kSpan);
+    add(__ldg(w + rr / kSpan), __ldg(w + kSpan + rr % kSpan), __ldg(ez + static_cast<size_t>(en) * A.ez));
+  }
+}
+
+__global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int task_blocks, int zoff, int zc) {
+  __shared__ float2 part[8][kB * kB][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int zb = blockIdx.y * 32, z = zb + lane;
+  const float2* ez = A.e + zoff + z;
+  BinSum S;
+  int lo, hi;
+  if (static_cast<int>(blockIdx.x) < task_blocks) {
+    const int n = *A.ntasks;
+    for (int task = blockIdx.x; task < n; task += task_blocks) {
+      const int4 T = A.tasks[task];
+      bin_ranges(A, T.x, lane, &lo, &hi);
+      const int total = __reduce_add_sync(0xffffffffu, hi - lo);
+      const int beg = min(total, T.y * kPart + warp * 32);
+      sum_entries(A, lane, lo, hi, beg, min(total, beg + 32), ez, S);
+#pragma unroll
+      for (int c = 0; c < kB * kB; ++c) part[warp][c][lane] = S.acc[c / kB][c % kB];
+      __syncthreads();
+      const int bx = T.x / A.nby, by = T.x - bx * A.nby;
+#pragma unroll
+      for (int q = 0; q < kB * kB / 8; ++q) {
+        const int c = warp + 8 * q;
+        float2 v = part[0][c][lane];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) v = cadd(v, part[w][c][lane]);
+        const int cx = bx * kB + c / kB, cy = by * kB + c % kB;
+        if (T.z > 1)
+          A.partial[(static_cast<size_t>(T.w + T.y) * (kB * kB) + c) * zc + z] = v;
+        else if (cx <= A.hx && cy < A.my)
+          A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = v;
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const int bin = (blockIdx.x - task_blocks) * 8 + warp;
+  if (bin >= A.nbx * A.nby) return;
+  bin_ranges(A, bin, lane, &lo, &hi);
+  const int total = __reduce_add_sync(0xffffffffu, hi - lo);
+  if (total > kSparse) return;
+  sum_entries(A, lane, lo, hi, 0, total, ez, S);
+  const int bx = bin / A.nby, by = bin - bx * A.nby;
+#pragma unroll
+  for (int i = 0; i < kB; ++i) {
+    const int cx = bx * kB + i;
+    if (cx > A.hx) break;
+#pragma unroll
+    for (int j = 0; j < kB; ++j) {
+      const int cy = by * kB + j;
+      if (cy < A.my) A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = S.acc[i][j];
+    }
+  }
+}
+
+// The parts of each bin with several, added in order: one block per bin and
+// 32 planes at a time.
+__global__ void __launch_bounds__(512) grid_parts_kernel(const GridArgs A, int zc) {
+  const int n = A.ntasks[2], cell = threadIdx.x >> 5, z = blockIdx.y * 32 + (threadIdx.x & 31);
+  for (int m = blockIdx.x; m < n; m += gridDim.x) {
+    const int4 T = A.multi[m];
+    const int bx = T.x / A.nby, by = T.x - bx * A.nby;
+    const size_t hop = static_cast<size_t>(kB * kB) * zc;
+    const float2* p = A.partial + (static_cast<size_t>(T.z) * (kB * kB) + cell) * zc + z;
+    float2 v = make_float2(0.0f, 0.0f);
+    int q = 0;
+    for (; q + 8 <= T.y; q += 8) {
+      float2 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = p[(q + u) * hop];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v = cadd(v, x[u]);
+    }
+    for (; q < T.y; ++q) v = cadd(v, p[q * hop]);
+    const int cx = bx * kB + cell / kB, cy = by * kB + cell % kB;
+    if (cx <= A.hx && cy < A.my) A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = v;
+  }
+}
+
+// Step 2: inverse FFT along cy of ZT planes of one cx, the ny outputs kept
+// and divided by the window's transform.
+template <int ZT>
+__global__ void __launch_bounds__(kFftThreads) grid_fft_y_kernel(const GridArgs A, int zc) {
+  extern __shared__ float2 sh[];
+  const int cx = blockIdx.y, z0 = blockIdx.x * ZT;
+  const float2* src = A.t1 + static_cast<size_t>(cx) * A.my * zc + z0;
+  float2* dst = A.t2 + static_cast<size_t>(cx) * A.ny * zc + z0;
+  const GridFft& f = A.fy;
+  auto gin = [&](int e, int z) { return __ldg(src + static_cast<size_t>(e) * zc + z); };
+  auto sin = [&](int e, int z) { return sh[e * ZT + z]; };
+  auto sout = [&](int e, int z, int, float2 v) { sh[e * ZT + z] = v; };
+  const int rl = f.r[f.nst - 1], hop = f.n / rl;
+  auto gout = [&](int e, int z, int t, float2 v) {
+    // element e = g R + t; output index rev[g] + t hop, about the middle
+    int j = __ldg(A.revy + (e - t) / rl) + t * hop + A.sy;
+    j -= j >= A.my ? A.my : 0;
+    if (j < A.ny) {
+      const float d = __ldg(A.dcy + j);
+      dst[static_cast<size_t>(j) * zc + z] = make_float2(v.x * d, v.y * d);
+    }
+  };
+  fft_stage_any<ZT>(f, 0, A.twy, 1, gin, sout);
+  for (int s = 1; s + 1 < f.nst; ++s) {
+    __syncthreads();
+    fft_stage_any<ZT>(f, s, A.twy, 1, sin, sout);
+  }
+  __syncthreads();
+  fft_stage_any<ZT>(f, f.nst - 1, A.twy, 1, sin, gout);
+}
+
+// Step 3: inverse real FFT along cx of ZT planes of one j: the hx + 1 inputs
+// (real parts only at 0 and hx) as one complex transform of length hx whose
+// output m is (x[2 m], x[2 m + 1]); x rows leave through shared memory.
+template <int ZT>
+__global__ void __launch_bounds__(kFftThreads) grid_fft_x_kernel(const GridArgs A, float* field, int zbeg, int zc,
+                                                                 int nzc, Moments* stats) {
+  extern __shared__ float2 sh[];
+  const GridFft& f = A.fx;
+  const int j = blockIdx.y, z0 = blockIdx.x * ZT;
+  if (z0 >= nzc) {  // a tile past the last plane
+    if (stats && threadIdx.x == 0)
+      stats[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = Moments{0.0, 0.0, 0.0};
+    return;
+  }
+  int pitch = (A.nx + 2) / 2 * 2;  // even for the paired stores; half of it odd: no bank conflicts
+  if (pitch / 2 % 2 == 0) pitch += 2;
+  float* rows = reinterpret_cast<float*>(sh + static_cast<size_t>(f.n) * ZT);
+  const float2* src = A.t2 + static_cast<size_t>(j) * zc + z0;
+  const size_t hop_in = static_cast<size_t>(A.ny) * zc;
+  const int half = f.n / 2;
+  for (int it = threadIdx.x; it < (half + 1) * ZT; it += kFftThreads) {
+    const int z = it & (ZT - 1), k = it / ZT;
+    const float2 a = __ldg(src + k * hop_in + z), b = __ldg(src + (f.n - k) * hop_in + z);
+    if (k == 0) {
+      sh[z] = make_float2(a.x + b.x, a.x - b.x);
+    } else {
+      // P = A_k / 2, Q = conj(A_{n-k}) / 2: (P + Q) + i e^{2 pi i k / mx} (P - Q)
+      const float2 w = __ldg(A.twx + k);
+      const float2 s = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+      const float2 d = make_float2(0.5f * (a.x - b.x), 0.5f * (a.y + b.y));
+      const float2 u = muli(cmulf(w, d));
+      sh[k * ZT + z] = cadd(s, u);
+      // index n - k: conj(s) + i conj(w) ... = conj(s - u)
+      if (2 * k != f.n) sh[(f.n - k) * ZT + z] = make_float2(s.x - u.x, -(s.y - u.y));
+    }
+  }
+  auto sin = [&](int e, int z) { return sh[e * ZT + z]; };
+  auto sout = [&](int e, int z, int, float2 v) { sh[e * ZT + z] = v; };
+  const int rl = f.r[f.nst - 1], hop = f.n / rl;
+  auto rout = [&](int e, int z, int t, float2 v) {
+    int i = 2 * (__ldg(A.revx + (e - t) / rl) + t * hop) + A.sx;
+    i -= i >= A.mx ? A.mx : 0;
+    if (i < A.nx) *reinterpret_cast<float2*>(rows + z * pitch + i) = v;
+  };
+  for (int s = 0; s + 1 < f.nst; ++s) {
+    __syncthreads();
+    fft_stage_any<ZT>(f, s, A.twx, 2, sin, sout);
+  }
+  __syncthreads();
+  fft_stage_any<ZT>(f, f.nst - 1, A.twx, 2, sin, rout);
+  __syncthreads();
+  // Rows of x: one warp per plane at a time.
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s1 = 0.0, s2 = 0.0, cnt = 0.0, shift = 0.0;
+  bool have = false;
+  for (int z = warp; z < ZT && z0 + z < nzc; z += kFftThreads / 32) {
+    float* out = field + static_cast<size_t>(zbeg + z0 + z) * A.plane + static_cast<size_t>(j) * A.nx;
+    for (int i = lane; i < A.nx; i += 32) {
+      const float v = rows[z * pitch + i] * __ldg(A.dcx + i);
+      out[i] = v;
+      if (stats) {
+        if (!have) {
+          shift = v;
+          have = true;
+        }
+        const double d = static_cast<double>(v) - shift;
+        s1 += d;
+        s2 = fma(d, d, s2);
+        cnt += 1.0;
+      }
+    }
+  }
+  if (stats) {
+    __shared__ Moments s_warp[kFftThreads / 32];
+    const Moments m = warp_moments(moments_from_shifted(cnt, shift, s1, s2));
+    if (lane == 0) s_warp[warp] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      Moments b = s_warp[0];
+      for (int w = 1; w < kFftThreads / 32; ++w) b = moments_merge(b, s_warp[w]);
+      stats[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = b;
+    }
+  }
+}
+
+// ------------------------------------------------------------------- plans --
+// Stages of an FFT of length n (2, 3, 5-smooth); large radices first.
+bool fft_plan(int n, GridFft* f) {
+  f->n = n;
+  f->nst = 0;
+  int rest = n;
+  for (int r : {16, 8, 5, 4, 3, 2})
+    while (rest % r == 0 && rest > 1) {
+      if (f->nst == GridFft::kMaxStages) return false;
+      f->r[f->nst++] = r;
+      rest /= r;
+    }
+  if (rest != 1 || f->nst < 2) return false;
+  int len = n;
+  for (int s = 0; s < f->nst; ++s) {
+    len /= f->r[s];
+    f->m[s] = len;
+    f->inv_m[s] = 1.0f / static_cast<float>(len);
+  }
+  return true;
+}
+
+// Transform length for n outputs: at least 1.5 n, a multiple of 4, with the
+// least length x (stages + 2) among lengths up to 15 % longer. `half`: the
+// complex transform has half the length (the real axis).
+int fft_length(int n, bool half, GridFft* f) {
+  const int lo = std::max(kMinM, static_cast<int>(std::ceil(kOversample * n)));
+  int best = 0;
+  double best_cost = 0.0;
+  for (int m = (lo + 3) / 4 * 4; m <= std::max(lo * 23 / 20, lo + 16); m += 4) {
+    GridFft g;
+    if (!fft_plan(half ? m / 2 : m, &g)) continue;
+    const double cost = static_cast<double>(m) * (g.nst + 2);
+    if (!best || cost < best_cost) {
+      best = m;
+      best_cost = cost;
+      *f = g;
+    }
+  }
+  return best;
+}
+
+size_t align256(size_t v) { return (v + 255) / 256 * 256; }
+
+constexpr size_t kSmemMax = 224 * 1024;  // dynamic; the kernels keep a little static shared memory
+size_t smem_y(const GridPlan& p, int zt) { return sizeof(float2) * static_cast<size_t>(p.my) * zt; }
+size_t smem_x(const GridPlan& p, int zt) {
+  return sizeof(float2) * static_cast<size_t>(p.mx / 2) * zt + sizeof(float) * static_cast<size_t>(p.nx + 4) * zt;
+}
+
+double window_beta(int n, int m) {
+  // Shape parameter of the Kaiser-Bessel window for this oversampling
+  // (Beatty, Nishimura & Pauly 2005), 2 % below: the least error measured
+  // with FP32 weights at 1.5.
+  const double sigma = static_cast<double>(m) / n;
+  return 0.98 * 3.14159265358979323846 * kW * (1.0 - 0.5 / sigma);
+}
+
+}  // namespace
+
+bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
+  GridPlan p{};
+  if (nh <= 0 || nh > kGridMaxHarmonics || n[0] <= 0 || n[1] <= 0 || n[2] <= 0) return false;
+  p.ndim = ndim;
+  p.nh = nh;
+  p.nx = n[0];
+  // The second axis is transformed, the third summed exactly; a single plane
+  // leaves (x, y) as x and the third.
+  if (n[2] == 1) {
+    p.ny = 1, p.nz = n[1], p.ax_y = 2, p.ax_z = 1;
+  } else {
+    p.ny = n[1], p.nz = n[2], p.ax_y = 1, p.ax_z = 2;
+  }
+  p.mx = fft_length(p.nx, true, &p.fx);
+  if (!p.mx) return false;
+  p.my = 1;
+  if (p.ny > 1 && !(p.my = fft_length(p.ny, false, &p.fy))) return false;
+  p.zt = 0;
+  for (int zt : {16, 8})
+    if (!p.zt && (p.ny == 1 || smem_y(p, zt) <= kSmemMax) && smem_x(p, zt) <= kSmemMax) p.zt = zt;
+  if (!p.zt) return false;
+  p.nbx = (p.mx / 2 + kB) / kB;
+  p.nby = p.ny > 1 ? p.my / kB : 1;
+  p.nkeys = (p.nbx + kSpan) * p.nby;
+  p.nent = 2 * nh;
+  const int nzp = (p.nz + 31) / 32 * 32;
+  // Planes per pass: T1 and T2 of a pass stay in L2 between the kernels.
+  const size_t per_z = sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * (p.my + (p.ny > 1 ? p.ny : 0));
+  int zc = static_cast<int>(std::max<size_t>(1, kGridPassBytes / (per_z * 32))) * 32;
+  p.zc = std::min(zc, nzp);
+  // E for as many passes as fit a bounded buffer.
+  const size_t e_pass = sizeof(float2) * static_cast<size_t>(p.nent) * p.zc;
+  const int passes = static_cast<int>(std::max<size_t>(1, kGridEBytes / e_pass));
+  p.ez = static_cast<int>(std::min<long long>(static_cast<long long>(passes) * p.zc, (nzp + p.zc - 1) / p.zc * p.zc));
+  // At most 9 visits of bins by a primary and 6 by a mirror entry.
+  const long long visits = 15ll * nh;
+  p.maxtasks = static_cast<int>(visits / kSparse + visits / kPart) + 1;
+  p.maxslots = static_cast<int>(2 * (visits / kPart)) + 2;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off = align256(off + bytes);
+    return at;
+  };
+  p.off_counts = take(sizeof(int) * (p.nkeys + 3));
+  p.off_keys = take(sizeof(uint2) * p.nent);
+  p.off_members = take(2 * sizeof(int) * p.nent);
+  p.off_par = take(sizeof(double4) * nh);
+  p.off_w = take(sizeof(double2) * nh);
+  p.off_bins = take(sizeof(int) * (p.nkeys + 2));
+  p.off_weights = take(sizeof(float) * 2 * kSpan * kB * static_cast<size_t>(p.nent));
+  p.off_e = take(sizeof(float2) * static_cast<size_t>(p.nent) * p.ez);
+  p.off_t1 = take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.my * p.zc);
+  p.off_t2 = p.ny > 1 ? take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.ny * p.zc) : p.off_t1;
+  p.off_partial = take(sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * kB * p.zc);
+  p.off_tasks = take(sizeof(int4) * (p.maxtasks + p.maxslots));
+  p.off_tables = take(sizeof(float2) * (p.mx + p.my) + sizeof(int) * (p.mx + p.my) + sizeof(float) * (p.nx + p.ny));
+  p.bytes = off;
+  *P = p;
+  return true;
+}
+
+int grid_passes(const GridPlan& p) { return (p.nz + p.zc - 1) / p.zc; }
+void grid_pass_planes(const GridPlan& p, int pass, int* z0, int* z1) {
+  *z0 = pass * p.zc;
+  *z1 = std::min(p.nz, *z0 + p.zc);
+}
+long long grid_stat_records(const GridPlan& p) {
+  return static_cast<long long>(grid_passes(p)) * p.ny * (p.zc / p.zt);
+}
+
+namespace {
+// Dynamic shared-memory limits, raised once per device.
+cudaError_t ensure_grid_attributes() {
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  const int most = static_cast<int>(kSmemMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_y_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_y_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  return e;
+}
+}  // namespace
+
+cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], float ds, const float* d_table,
+                                   float* d_field, void* d_work, const GridPlan& p, cudaStream_t stream,
+                                   StatRecord* d_stats, const std::function<cudaError_t(int)>& pass_done) {
+  cudaError_t e = ensure_grid_attributes();
+  if (e != cudaSuccess) return e;
+  uint8_t* w = static_cast<uint8_t*>(d_work);
+  GridArgs A{};
+  A.fx = p.fx, A.fy = p.fy;
+  A.mx = p.mx, A.my = p.my, A.hx = p.mx / 2;
+  A.nx = p.nx, A.ny = p.ny, A.nz = p.nz;
+  A.sx = p.nx / 4 * 2;  // even: outputs come in pairs
+  A.sy = p.ny / 2;
+  A.nbx = p.nbx, A.nby = p.nby, A.nkeys = p.nkeys;
+  A.nent = p.nent, A.nh = p.nh;
+  A.ez = p.ez;
+  A.maxtasks = p.maxtasks;
+  A.maxslots = p.maxslots;
+  A.beta_x = window_beta(p.nx, p.mx);
+  A.beta_y = window_beta(p.ny, p.my);
+  A.inv_i0_x = 1.0 / std::cyl_bessel_i(0.0, A.beta_x);
+  A.inv_i0_y = 1.0 / std::cyl_bessel_i(0.0, A.beta_y);
+  for (int i = 0; i < 9; ++i) A.m[i] = s.m[i];
+  for (int i = 0; i < 3; ++i) A.bar[i] = s.bar[i], A.fs[i] = fs[i];
+  A.ds = ds;
+  A.ax_y = p.ax_y, A.ax_z = p.ax_z;
+  A.scaling = s.scaling;
+  A.plane = static_cast<long long>(p.nx) * p.ny;
+  A.table = d_table;
+  A.counts = reinterpret_cast<int*>(w + p.off_counts);
+  A.ntasks = A.counts + p.nkeys;
+  A.keys = reinterpret_cast<uint2*>(w + p.off_keys);
+  A.members = reinterpret_cast<int*>(w + p.off_members);
+  A.place = A.members + p.nent;
+  A.par = reinterpret_cast<double4*>(w + p.off_par);
+  A.w = reinterpret_cast<double2*>(w + p.off_w);
+  A.bin_start = reinterpret_cast<int*>(w + p.off_bins);
+  A.weights = reinterpret_cast<float*>(w + p.off_weights);
+  A.e = reinterpret_cast<float2*>(w + p.off_e);
+  A.t1 = reinterpret_cast<float2*>(w + p.off_t1);
+  A.t2 = reinterpret_cast<float2*>(w + p.off_t2);
+  A.partial = reinterpret_cast<float2*>(w + p.off_partial);
+  A.tasks = reinterpret_cast<int4*>(w + p.off_tasks);
+  A.multi = A.tasks + p.maxtasks;
+  A.twx = reinterpret_cast<float2*>(w + p.off_tables);
+  A.twy = A.twx + p.mx;
+  A.revx = reinterpret_cast<int*>(A.twy + p.my);
+  A.revy = A.revx + p.mx;
+  A.dcx = reinterpret_cast<float*>(A.revy + p.my);
+  A.dcy = A.dcx + p.nx;
+
+  const long long items = static_cast<long long>(p.nh) + 2 * (p.mx + p.my) + p.nx + p.ny;
+  // Entry counts and the task counters behind them.
+  if ((e = cudaMemsetAsync(A.counts, 0, sizeof(int) * (p.nkeys + 3), stream)) != cudaSuccess) return e;
+  grid_prep_kernel<<<static_cast<unsigned>((items + 127) / 128), 128, 0, stream>>>(A);
+  grid_scan_kernel<<<1, kScanThreads, 0, stream>>>(A);
+  const int nbins = p.nbx * p.nby;
+  const int scatter = (p.nent + 255) / 256;
+  grid_bins_kernel<<<scatter + (nbins + 7) / 8, 256, 0, stream>>>(A, scatter);
+  const int task_blocks = std::min(p.maxtasks, 148 * 4);
+  const int tiles = p.zc / p.zt;
+  for (int pass = 0; pass < grid_passes(p); ++pass) {
+    int z0, z1;
+    grid_pass_planes(p, pass, &z0, &z1);
+    const int zoff = z0 % p.ez;
+    if (zoff == 0) {
+      const int nze = (std::min(p.nz - z0, p.ez) + 31) / 32 * 32;
+      grid_entry_kernel<<<(p.nent + 3) / 4, 128, 0, stream>>>(A, z0, nze, pass == 0);
+    }
+    const int planes = (z1 - z0 + 31) / 32 * 32;
+    grid_spread_kernel<<<dim3(task_blocks + (nbins + 7) / 8, planes / 32), 256, 0, stream>>>(A, task_blocks, zoff, p.zc);
+    grid_parts_kernel<<<dim3(std::min(p.maxslots, 148), planes / 32), 512, 0, stream>>>(A, p.zc);
+    const dim3 gy(static_cast<unsigned>(planes / p.zt), static_cast<unsigned>(p.mx / 2 + 1));
+    const dim3 gx(static_cast<unsigned>(tiles), static_cast<unsigned>(p.ny));
+    StatRecord* rec = d_stats ? d_stats + static_cast<size_t>(pass) * p.ny * tiles : nullptr;
+    if (p.zt == 16) {
+      if (p.ny > 1) grid_fft_y_kernel<16><<<gy, kFftThreads, smem_y(p, 16), stream>>>(A, p.zc);
+      grid_fft_x_kernel<16><<<gx, kFftThreads, smem_x(p, 16), stream>>>(A, d_field, z0, p.zc, z1 - z0, rec);
+    } else {
+      if (p.ny > 1) grid_fft_y_kernel<8><<<gy, kFftThreads, smem_y(p, 8), stream>>>(A, p.zc);
+      grid_fft_x_kernel<8><<<gx, kFftThreads, smem_x(p, 8), stream>>>(A, d_field, z0, p.zc, z1 - z0, rec);
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (pass_done && (e = pass_done(pass)) != cudaSuccess) return e;
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace scarf

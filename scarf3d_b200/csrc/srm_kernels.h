@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstddef>
+#include <functional>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -167,6 +168,40 @@ struct BuilderFork {
 cudaError_t tc_batch_launch(const TcBatchPlan& plan, void* d_work, cudaStream_t stream,
                             cudaEvent_t ev_main0 = nullptr, cudaEvent_t ev_main1 = nullptr,
                             const BuilderFork* fork = nullptr);
+
+// ---- gridded Fourier form of structured sums (srm_grid.cu) ----
+constexpr int kGridMaxHarmonics = 1 << 20;
+constexpr size_t kGridPassBytes = size_t(96) << 20;  // T1 and T2 of one pass
+constexpr size_t kGridEBytes = size_t(1) << 30;      // E of as many passes as fit
+struct GridPlan {
+  struct Fft {
+    static constexpr int kMaxStages = 8;
+    int n, nst;
+    int r[kMaxStages], m[kMaxStages];  // radix and element distance of each stage
+    float inv_m[kMaxStages];
+  };
+  int ndim, nh, nent;
+  int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly
+  int ax_y, ax_z;      // their physical axes
+  int mx, my;          // transform lengths
+  Fft fx, fy;          // of length mx / 2 and my
+  int nbx, nby, nkeys, maxtasks, maxslots;
+  int zt, zc, ez;      // planes per transform tile, per pass, per build of E
+  size_t off_counts, off_keys, off_members, off_par, off_w, off_bins, off_weights, off_e, off_t1, off_t2, off_partial,
+      off_tasks, off_tables, bytes;
+};
+// False when the form does not take the grid (an axis too long for a
+// transform in shared memory, no or too many harmonics).
+bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* plan);
+int grid_passes(const GridPlan& p);
+// Planes [z0, z1) that a pass completes; whole contiguous pieces of the field.
+void grid_pass_planes(const GridPlan& p, int pass, int* z0, int* z1);
+long long grid_stat_records(const GridPlan& p);
+// Enqueues the whole sum. pass_done(pass), when set, is called once the
+// launches that complete a pass's planes are enqueued.
+cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], float ds, const float* d_table,
+                                   float* d_field, void* d_work, const GridPlan& plan, cudaStream_t stream,
+                                   StatRecord* d_stats, const std::function<cudaError_t(int)>& pass_done);
 
 // ---- device side of the harmonic sampler (srm_sampler.cu) ----
 struct SampleEntry {

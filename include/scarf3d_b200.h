@@ -31,7 +31,8 @@ extern "C" {
 #define SCARF_ERR_NOMEM (-6)       /* host or device allocation failed           */
 
 /* Summation form used by scarf_execute / scarf_execute_ex. */
-#define SCARF_FORM_AUTO 0   /* tensor-core form for structured grids, else direct */
+#define SCARF_FORM_AUTO 0   /* structured grids: the faster of the gridded Fourier sum
+                             * and the tensor-core form; point sets: direct        */
 #define SCARF_FORM_DIRECT 1 /* FP32 direct sum (any point set)                    */
 #define SCARF_FORM_TC 2     /* factorised tcgen05 split-16-bit form (structured)   */
 
@@ -110,8 +111,10 @@ int scarf_selftest_wait_limit(int blocks, int *device_status, double *waited_s);
  * does not round to nearest, so its error grows with this length. */
 int scarf_set_tc_chunk(int harmonics);
 
-/* Host-field output of scarf_execute on a structured mesh with the
- * tensor-core form, no rescale and no taper: the field is copied to the host
+/* Host-field output of scarf_execute on a structured mesh, no rescale and no
+ * taper. With the gridded sum the planes of each pass are copied to the host
+ * while later passes compute (0 = copy the whole field afterwards). With the
+ * tensor-core form the field is copied
  * in slabs (a column tile x a run of row blocks, about items_per_slab work
  * items of 128 x <=256 points each) while the kernel computes the rest.
  * 1 = default slab size (64 items), >= 2 = that size, 0 = copy the whole

@@ -319,6 +319,9 @@ inline void cpu_relax() {
 // while the next slots are in flight.
 constexpr int kBounceSlots = 4;
 constexpr size_t kBounceSlotCap = size_t(16) << 20;
+// Slots of the gridded form's copies: page-locking costs ~0.8 ms per MB, once per
+// context, and slots of this size keep the copy engine busy.
+constexpr size_t kPassSlotCap = size_t(6) << 20;
 
 bool is_pageable(const void* p) {
   cudaPointerAttributes a{};
@@ -415,7 +418,7 @@ class BounceCopier {
     q.busy = false;
     SCARF_CUDA(cudaEventSynchronize(t_ctx->res.bounce_ev[slot]));
     const char* buf = t_ctx->res.bounce + static_cast<size_t>(slot) * t_ctx->res.bounce_slot;
-    constexpr size_t kPiece = size_t(1) << 20;
+    constexpr size_t kPiece = size_t(256) << 10;
     const size_t per_row = (q.width + kPiece - 1) / kPiece;
     const Pending w = q;
     parallel_tasks(static_cast<int>(per_row * w.height), host_threads(), [&](int t) {
@@ -489,7 +492,7 @@ int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
   const bool bounce = is_pageable(field);
   const size_t plane = sizeof(float) * static_cast<size_t>(plan.nx) * plan.ny;
   if (bounce) {
-    const int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(plane * plan.zc / 2, 1 << 20)));
+    const int rc = ensure_bounce(std::min<size_t>(kPassSlotCap, std::max<size_t>(plane * plan.zc, 1 << 20)));
     if (rc) return rc;
   }
   cudaStream_t cs = t_ctx->res.copy_stream;
@@ -778,31 +781,31 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     TcPlan plan{};
     TcChoice tuned{};
     const bool have_tuned = use_tc && nh > 0 && tc_tuned_choice(s.ndim, n, true, &tuned);
-    // The automatic form: the gridded sum where it takes the grid and its
+    const bool planned = have_tuned ? tc_make_plan(s.ndim, n, nh, &plan, tuned.tile_j, false, tuned.variant)
+                                    : tc_make_plan(s.ndim, n, nh, &plan);
+    // The automatic form: the gridded sum where it is the faster and its
     // workspace fits (also within the device-memory cap), unless a tensor-core
     // plan was tuned for this grid.
     GridPlan grid{};
-    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned && grid_make_plan(s.ndim, n, nh, &grid);
-    if (use_grid && t_ctx->res.work.ensure(grid.bytes) != cudaSuccess) {
+    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned && grid_make_plan(s.ndim, n, nh, &grid) &&
+                    (!planned || grid_pays(grid, plan));
+    if (use_grid && (want_records(grid_stat_records(grid)) != SCARF_OK ||
+                     t_ctx->res.work.ensure(grid.bytes) != cudaSuccess)) {
       (void)cudaGetLastError();
       (void)scarf::take_device_alloc_failure();
       use_grid = false;
     }
-    const bool planned = have_tuned ? tc_make_plan(s.ndim, n, nh, &plan, tuned.tile_j, false, tuned.variant)
-                                    : tc_make_plan(s.ndim, n, nh, &plan);
     if (use_grid) {
       const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
       if (overlap) {
         rc = ensure_pass_resources(grid_passes(grid));
         if (rc) return rc;
       }
-      rc = want_records(grid_stat_records(grid));
-      if (rc) return rc;
       if (kernel_ev0()) SCARF_CUDA(cudaEventRecord(kernel_ev0(), st));
       std::function<cudaError_t(int)> pass_done;
       if (overlap) pass_done = [&](int pass) { return cudaEventRecord(t_ctx->res.pass_ev[pass], st); };
-      SCARF_CUDA(launch_grid_structured(s, t_ctx->obj.fs, p.ds, d_table, d_field, t_ctx->res.work.p, grid, st, d_rec,
-                                        pass_done));
+      SCARF_CUDA(launch_grid_structured(s, t_ctx->obj.fs, p.ds, d_table, d_field, t_ctx->res.work.p, grid, d_status, st,
+                                        d_rec, pass_done));
       if (kernel_ev1()) SCARF_CUDA(cudaEventRecord(kernel_ev1(), st));
       if (overlap) {
         copy_join.active = true;

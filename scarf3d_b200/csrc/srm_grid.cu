@@ -30,6 +30,7 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "fft_tile.cuh"
 #include "srm_kernels.h"
 
 namespace scarf {
@@ -43,14 +44,13 @@ constexpr double kOversample = 1.5;
 constexpr int kSparse = 32;       // entries of a bin that one warp sums
 constexpr int kPart = 256;        // entries that one block sums (32 per warp)
 constexpr int kScanThreads = 1024;
-constexpr int kFftThreads = 256;
+constexpr int kZT = 8;            // planes of a transform tile
+constexpr int kPairs = kZT / 2;
+constexpr int kFftMaxThreads = 512;
 static_assert((kSpan - 1) * kB + 1 == kW, "a cell bin is reached from exactly kSpan start bins");
 
-// -------------------------------------------------------------- FFT stages --
-using GridFft = GridPlan::Fft;
-
 struct GridArgs {
-  GridFft fx, fy;      // lengths mx / 2 and my
+  FftPlan fx, fy;      // lengths mx / 2 and my
   int mx, my, hx;      // transform lengths, hx = mx / 2
   int nx, ny, nz;      // logical extents: x, gridded second axis (1: none), z
   int sx, sy;          // index of the grid's middle: i' = i - sx, j' = j - sy
@@ -74,158 +74,30 @@ struct GridArgs {
   double2* w;          // per harmonic: wx, wy (cells)
   int* bin_start;
   float* weights;      // per sorted entry: x weights of 3 bins, y weights of 3 bins
+  // Complex grids, planes in pairs: {re, re', im, im'} of planes 2 q, 2 q + 1.
+  // The sums of step 1 have real weights, so its lanes take 8 bytes each,
+  // whichever parts these are.
   float2* e;           // [nent][ez]
-  float2* t1;          // [hx + 1][my][zc]
-  float2* t2;          // [hx + 1][ny][zc]
+  // A transform's tile (kZT planes) is one contiguous piece.
+  float2* t1;          // [zc / kZT][hx + 1][my][kZT]
+  float2* t2;          // [zc / kZT][ny][hx + 1][kZT]
   float2* partial;     // [slot][kB * kB][zc]
   int* ntasks;         // three counters: tasks, slots, bins with several parts
   int4* tasks;         // {bin, part, parts, slot} of the bins that blocks sum
   int4* multi;         // {bin, parts, slot, -} of those with several parts
-  float2* twx;         // e^{2 pi i k / mx}
-  float2* twy;         // e^{2 pi i k / my}
+  // Twiddles as {cos, cos, sin, sin}: of the plans fx and fy, and
+  // e^{2 pi i k / mx} for k <= hx / 2.
+  float4* twx;
+  float4* twy;
+  float4* twr;
   int* revx;
   int* revy;
+  int* status;         // error word of the bounded waits
   float* dcx;          // 1 / window transform, times the field's scaling
   float* dcy;
 };
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 muli(float2 a) { return make_float2(-a.y, a.x); }
-
-// Inverse (e^{+i}) DFT of R values in registers, natural order.
-template <int R>
-struct Dft;
-template <>
-struct Dft<2> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float2 t = v[0];
-    v[0] = cadd(t, v[1]);
-    v[1] = csub(t, v[1]);
-  }
-};
-template <>
-struct Dft<3> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
-    const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
-    const float2 s = muli(make_float2(0.86602540378443864676f * d.x, 0.86602540378443864676f * d.y));
-    v[0] = cadd(v[0], t);
-    v[1] = cadd(m, s);
-    v[2] = csub(m, s);
-  }
-};
-template <>
-struct Dft<4> {
-  static __device__ __forceinline__ void run(float2* v) {
-    const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = muli(csub(v[1], v[3]));
-    v[0] = cadd(a, c);
-    v[1] = cadd(b, d);
-    v[2] = csub(a, c);
-    v[3] = csub(b, d);
-  }
-};
-template <>
-struct Dft<5> {
-  static __device__ __forceinline__ void run(float2* v) {
-    constexpr float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;  // cos(2 pi / 5), cos(4 pi / 5)
-    constexpr float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;   // sin
-    const float2 a = cadd(v[1], v[4]), b = cadd(v[2], v[3]), c = csub(v[1], v[4]), d = csub(v[2], v[3]);
-    const float2 m1 = make_float2(v[0].x + c1 * a.x + c2 * b.x, v[0].y + c1 * a.y + c2 * b.y);
-    const float2 m2 = make_float2(v[0].x + c2 * a.x + c1 * b.x, v[0].y + c2 * a.y + c1 * b.y);
-    const float2 n1 = muli(make_float2(s1 * c.x + s2 * d.x, s1 * c.y + s2 * d.y));
-    const float2 n2 = muli(make_float2(s2 * c.x - s1 * d.x, s2 * c.y - s1 * d.y));
-    v[0] = cadd(v[0], cadd(a, b));
-    v[1] = cadd(m1, n1);
-    v[2] = cadd(m2, n2);
-    v[3] = csub(m2, n2);
-    v[4] = csub(m1, n1);
-  }
-};
-template <>
-struct Dft<8> {
-  static __device__ __forceinline__ void run(float2* v) {
-    constexpr float r = 0.70710678118654752440f;
-    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4>::run(e);
-    Dft<4>::run(o);
-    o[1] = make_float2(r * (o[1].x - o[1].y), r * (o[1].x + o[1].y));
-    o[2] = muli(o[2]);
-    o[3] = make_float2(-r * (o[3].x + o[3].y), r * (o[3].x - o[3].y));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = cadd(e[k], o[k]);
-      v[k + 4] = csub(e[k], o[k]);
-    }
-  }
-};
-template <>
-struct Dft<16> {
-  static __device__ __forceinline__ void run(float2* v) {
-    constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, r = 0.70710678118654752440f;
-    // e^{2 pi i b k / 16} for b, k in 1..3
-    const float2 w[3][3] = {{{c1, s1}, {r, r}, {s1, c1}}, {{r, r}, {0.0f, 1.0f}, {-r, r}}, {{s1, c1}, {-r, r}, {-c1, -s1}}};
-    float2 y[4][4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      y[b][0] = v[b], y[b][1] = v[b + 4], y[b][2] = v[b + 8], y[b][3] = v[b + 12];
-      Dft<4>::run(y[b]);
-      if (b > 0) {
-#pragma unroll
-        for (int k = 1; k < 4; ++k) y[b][k] = cmulf(y[b][k], w[b - 1][k - 1]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float2 t[4] = {y[0][k], y[1][k], y[2][k], y[3][k]};
-      Dft<4>::run(t);
-      v[k] = t[0], v[k + 4] = t[1], v[k + 8] = t[2], v[k + 12] = t[3];
-    }
-  }
-};
-
-// One decimation-in-frequency stage of radix R over a tile of ZT transforms
-// in shared memory (element e of transform z at [e * ZT + z]): reads through
-// `in`, writes through `out`, both called with (element, z). In place when
-// both address the same array: a butterfly writes where it read.
-template <int R, int ZT, class In, class Out>
-__device__ __forceinline__ void fft_stage(const GridFft& f, int s, const float2* __restrict__ tw, int tw_step, In in,
-                                          Out out) {
-  const int m = f.m[s];       // distance between a butterfly's elements
-  const int len = m * R;      // sub-transform length of this stage
-  const float inv_m = f.inv_m[s];
-  const int step = f.n / len * tw_step;  // twiddle e^{2 pi i q t / len} is tw[q t step]
-  for (int it = threadIdx.x; it < f.n / R * ZT; it += kFftThreads) {
-    const int z = it & (ZT - 1), g = it / ZT;
-    const int blk = static_cast<int>((static_cast<float>(g) + 0.5f) * inv_m);
-    const int q = g - blk * m;
-    const int base = blk * len + q;
-    float2 v[R];
-#pragma unroll
-    for (int t = 0; t < R; ++t) v[t] = in(base + t * m, z);
-    Dft<R>::run(v);
-    if (m > 1) {
-#pragma unroll
-      for (int t = 1; t < R; ++t) v[t] = cmulf(v[t], __ldg(tw + q * t * step));
-    }
-#pragma unroll
-    for (int t = 0; t < R; ++t) out(base + t * m, z, t, v[t]);
-  }
-}
-template <int ZT, class In, class Out>
-__device__ __forceinline__ void fft_stage_any(const GridFft& f, int s, const float2* tw, int tw_step, In in, Out out) {
-  switch (f.r[s]) {
-    case 16: fft_stage<16, ZT>(f, s, tw, tw_step, in, out); break;
-    case 8: fft_stage<8, ZT>(f, s, tw, tw_step, in, out); break;
-    case 5: fft_stage<5, ZT>(f, s, tw, tw_step, in, out); break;
-    case 4: fft_stage<4, ZT>(f, s, tw, tw_step, in, out); break;
-    case 3: fft_stage<3, ZT>(f, s, tw, tw_step, in, out); break;
-    default: fft_stage<2, ZT>(f, s, tw, tw_step, in, out); break;
-  }
-}
 
 // ------------------------------------------------------------- preparation --
 // Kaiser-Bessel weight at distance d (cells) from a harmonic's wavenumber.
@@ -240,20 +112,6 @@ __device__ __forceinline__ float kb_weight(double d, double beta, double inv_i0)
 // orders and window transforms of both axes.
 __device__ __forceinline__ int first_cell(double c) { return static_cast<int>(ceil(c - 0.5 * kW)); }
 __device__ __forceinline__ int floor_bin(int c) { return (c >= 0 ? c : c - (kB - 1)) / kB; }
-
-__device__ int output_order(const GridFft& f, int g) {
-  // Butterfly g of the last stage holds elements g R .. g R + R - 1 of the
-  // digit-reversed output; its first output index:
-  int k = 0, w = 1, pos = g * f.r[f.nst - 1], span = f.n;
-  for (int s = 0; s + 1 < f.nst; ++s) {
-    span /= f.r[s];
-    const int d = pos / span;
-    pos -= d * span;
-    k += d * w;
-    w *= f.r[s];
-  }
-  return k;
-}
 
 __device__ float window_inverse(int n, int m, double beta) {
   const double pi = 3.14159265358979323846;
@@ -315,17 +173,23 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
     return;
   }
   t -= A.nh;
-  if (t < A.mx) {
+  auto root = [&](double turns) {
     double s, c;
-    sincospi(2.0 * static_cast<double>(t) / A.mx, &s, &c);
-    A.twx[t] = make_float2(static_cast<float>(c), static_cast<float>(s));
+    sincospi(2.0 * turns, &s, &c);
+    return make_float4(static_cast<float>(c), static_cast<float>(c), static_cast<float>(s), static_cast<float>(s));
+  };
+  if (t < A.hx) {
+    A.twx[t] = root(fft::twiddle_entry(A.fx, static_cast<int>(t)));
     return;
   }
-  t -= A.mx;
+  t -= A.hx;
+  if (t <= A.hx / 2) {
+    A.twr[t] = root(static_cast<double>(t) / A.mx);
+    return;
+  }
+  t -= A.hx / 2 + 1;
   if (t < A.my) {
-    double s, c;
-    sincospi(2.0 * static_cast<double>(t) / A.my, &s, &c);
-    A.twy[t] = make_float2(static_cast<float>(c), static_cast<float>(s));
+    if (A.ny > 1) A.twy[t] = root(fft::twiddle_entry(A.fy, static_cast<int>(t)));
     return;
   }
   t -= A.my;
@@ -341,11 +205,11 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
   t -= A.ny;
   const int gx = A.fx.n / A.fx.r[A.fx.nst - 1];
   if (t < gx) {
-    A.revx[t] = output_order(A.fx, static_cast<int>(t));
+    A.revx[t * A.fx.r[A.fx.nst - 1]] = fft::output_order(A.fx, static_cast<int>(t));
     return;
   }
   t -= gx;
-  if (A.ny > 1 && t < A.fy.n / A.fy.r[A.fy.nst - 1]) A.revy[t] = output_order(A.fy, static_cast<int>(t));
+  if (A.ny > 1 && t < A.fy.n / A.fy.r[A.fy.nst - 1]) A.revy[t * A.fy.r[A.fy.nst - 1]] = fft::output_order(A.fy, static_cast<int>(t));
 }
 
 // Exclusive scan of the entry counts per key (one block).
@@ -488,11 +352,23 @@ __global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z
   sincospi(2.0 * (step - rint(step)), &ds, &dc);
   float2* out = A.e + static_cast<size_t>(i) * A.ez;
   for (int z = lane; z < nzc; z += 32) {
-    out[z] = make_float2(static_cast<float>(p.w * c + p.z * s), static_cast<float>(p.w * s - p.z * c));
+    const float re = static_cast<float>(p.w * c + p.z * s), im = static_cast<float>(p.w * s - p.z * c);
+    // Even lanes store both real parts of a pair of planes, odd lanes both
+    // imaginary parts.
+    const bool odd = lane & 1;
+    const float other = __shfl_xor_sync(0xffffffffu, odd ? re : im, 1);
+    out[z] = odd ? make_float2(other, im) : make_float2(re, other);
     const double n = c * dc - s * ds;
     s = c * ds + s * dc;
     c = n;
   }
+}
+
+// T1 cell (cx, cy), plane z of the pass.
+__device__ __forceinline__ size_t t1_index(const GridArgs& A, int cx, int cy, int z) {
+  const int g = z / kZT;
+  // A single gridded axis goes straight to step 3, as [zc / kZT][ny = 1][hx + 1][kZT].
+  return ((static_cast<size_t>(g) * (A.hx + 1) + cx) * A.my + cy) * kZT + z % kZT;
 }
 
 // Step 1. A warp sums up to 32 entries of one 4 x 4-cell bin over 32 planes:
@@ -588,7 +464,7 @@ __global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int 
         if (T.z > 1)
           A.partial[(static_cast<size_t>(T.w + T.y) * (kB * kB) + c) * zc + z] = v;
         else if (cx <= A.hx && cy < A.my)
-          A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = v;
+          A.t1[t1_index(A, cx, cy, z)] = v;
       }
       __syncthreads();
     }
@@ -608,7 +484,7 @@ __global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int 
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
       const int cy = by * kB + j;
-      if (cy < A.my) A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = S.acc[i][j];
+      if (cy < A.my) A.t1[t1_index(A, cx, cy, z)] = S.acc[i][j];
     }
   }
 }
@@ -633,139 +509,249 @@ __global__ void __launch_bounds__(512) grid_parts_kernel(const GridArgs A, int z
     }
     for (; q < T.y; ++q) v = cadd(v, p[q * hop]);
     const int cx = bx * kB + cell / kB, cy = by * kB + cell % kB;
-    if (cx <= A.hx && cy < A.my) A.t1[(static_cast<size_t>(cx) * A.my + cy) * zc + z] = v;
+    if (cx <= A.hx && cy < A.my) A.t1[t1_index(A, cx, cy, z)] = v;
   }
 }
 
-// Step 2: inverse FFT along cy of ZT planes of one cx, the ny outputs kept
-// and divided by the window's transform.
-template <int ZT>
-__global__ void __launch_bounds__(kFftThreads) grid_fft_y_kernel(const GridArgs A, int zc) {
-  extern __shared__ float2 sh[];
-  const int cx = blockIdx.y, z0 = blockIdx.x * ZT;
-  const float2* src = A.t1 + static_cast<size_t>(cx) * A.my * zc + z0;
-  float2* dst = A.t2 + static_cast<size_t>(cx) * A.ny * zc + z0;
-  const GridFft& f = A.fy;
-  auto gin = [&](int e, int z) { return __ldg(src + static_cast<size_t>(e) * zc + z); };
-  auto sin = [&](int e, int z) { return sh[e * ZT + z]; };
-  auto sout = [&](int e, int z, int, float2 v) { sh[e * ZT + z] = v; };
-  const int rl = f.r[f.nst - 1], hop = f.n / rl;
-  auto gout = [&](int e, int z, int t, float2 v) {
-    // element e = g R + t; output index rev[g] + t hop, about the middle
-    int j = __ldg(A.revy + (e - t) / rl) + t * hop + A.sy;
-    j -= j >= A.my ? A.my : 0;
-    if (j < A.ny) {
-      const float d = __ldg(A.dcy + j);
-      dst[static_cast<size_t>(j) * zc + z] = make_float2(v.x * d, v.y * d);
+// The transforms' blocks are persistent: a block takes tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ... and has the next tile on its way (one bulk copy
+// into the other buffer) while it transforms the current one. Loaded by the
+// threads themselves, a tile's latency was 40 % of its time.
+struct TileRing {
+  unsigned char* buf;
+  uint64_t* bar;
+  uint32_t bytes;  // one tile
+  uint32_t pitch;  // between buffers
+  int nbuf;
+};
+__device__ __forceinline__ void tile_issue(const TileRing& R, int slot, const void* src) {
+  mbar_arrive_expect_tx(R.bar + slot, R.bytes);
+  bulk_g2s(R.buf + static_cast<size_t>(slot) * R.pitch, src, R.bytes, R.bar + slot);
+}
+
+// Step 2: inverse FFT along cy of the planes of a tile (one cx), the ny
+// outputs kept.
+__global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridArgs A, int tiles, int nbuf) {
+  using namespace fft;
+  constexpr int NP = kPairs;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_full[2];
+  const FftPlan& f = A.fy;
+  const uint32_t bytes = static_cast<uint32_t>(A.my) * NP * 16;
+  const TileRing R{smem, s_full, bytes, bytes, nbuf};
+  const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < nbuf; ++i) mbar_init(&s_full[i], 1);
+    fence_mbar_init();
+    for (int i = 0; i < nbuf; ++i) {
+      const long long t = blockIdx.x + static_cast<long long>(i) * gridDim.x;
+      if (t < tiles) tile_issue(R, i, base + static_cast<size_t>(t) * bytes);
     }
-  };
-  fft_stage_any<ZT>(f, 0, A.twy, 1, gin, sout);
-  for (int s = 1; s + 1 < f.nst; ++s) {
-    __syncthreads();
-    fft_stage_any<ZT>(f, s, A.twy, 1, sin, sout);
   }
   __syncthreads();
-  fft_stage_any<ZT>(f, f.nst - 1, A.twy, 1, sin, gout);
+  const int rl = f.r[f.nst - 1], hop = f.n / rl, row = (A.hx + 1) * NP;
+  int n = 0;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
+    const int slot = n % nbuf;
+    const bool ok = mbar_wait_bounded(&s_full[slot], (n / nbuf) & 1, A.status);
+    if (!__syncthreads_and(ok)) {
+      // Unwind: the copies in flight land before the block exits.
+      if (threadIdx.x == 0)
+        for (int i = 0; i < nbuf; ++i)
+          if (t + static_cast<long long>(i) * gridDim.x < tiles)
+            mbar_wait_drain(&s_full[(n + i) % nbuf], ((n + i) / nbuf) & 1);
+      return;
+    }
+    ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem + static_cast<size_t>(slot) * bytes);
+    const int g = t / (A.hx + 1), cx = t - g * (A.hx + 1);
+    ulonglong2* dst = reinterpret_cast<ulonglong2*>(A.t2) + static_cast<size_t>(g) * A.ny * row + cx * NP;
+    auto in = [&](int e, int p) {
+      const ulonglong2 v = sh[e * NP + p];
+      return C2{v.x, v.y};
+    };
+    auto out = [&](int e, int p, int, C2 v) { sh[e * NP + p] = make_ulonglong2(v.re, v.im); };
+    auto gout = [&](int e, int p, int u, C2 v) {
+      // element e = g R + u; output index rev[g] + u hop, about the middle
+      int j = __ldg(A.revy + e - u) + u * hop + A.sy;
+      j -= j >= A.my ? A.my : 0;
+      if (j < A.ny) dst[static_cast<uint32_t>(j * row + p)] = make_ulonglong2(v.re, v.im);
+    };
+    for (int s = 0; s + 1 < f.nst; ++s) {
+      stage_any<NP>(f, s, A.twy, in, out);
+      __syncthreads();
+    }
+    stage_any<NP>(f, f.nst - 1, A.twy, in, gout);
+    __syncthreads();
+    const long long next = t + static_cast<long long>(nbuf) * gridDim.x;
+    if (threadIdx.x == 0 && next < tiles) {
+      fence_proxy_async_smem();
+      tile_issue(R, slot, base + static_cast<size_t>(next) * bytes);
+    }
+  }
 }
 
-// Step 3: inverse real FFT along cx of ZT planes of one j: the hx + 1 inputs
-// (real parts only at 0 and hx) as one complex transform of length hx whose
-// output m is (x[2 m], x[2 m + 1]); x rows leave through shared memory.
-template <int ZT>
-__global__ void __launch_bounds__(kFftThreads) grid_fft_x_kernel(const GridArgs A, float* field, int zbeg, int zc,
-                                                                 int nzc, Moments* stats) {
-  extern __shared__ float2 sh[];
-  const GridFft& f = A.fx;
-  const int j = blockIdx.y, z0 = blockIdx.x * ZT;
-  if (z0 >= nzc) {  // a tile past the last plane
-    if (stats && threadIdx.x == 0)
-      stats[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = Moments{0.0, 0.0, 0.0};
-    return;
+// Step 3: inverse real FFT along cx of the planes of a tile (one j): the
+// hx + 1 inputs (real parts only at 0 and hx) as one complex transform of
+// length hx whose output m is (x[2 m], x[2 m + 1]); x rows leave through
+// shared memory, divided by both axes' window transforms.
+__global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridArgs A, float* field, int zbeg, int nzc,
+                                                                    int tiles, int nbuf, Moments* stats) {
+  using namespace fft;
+  constexpr int NP = kPairs;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_full[2];
+  __shared__ Moments s_warp[kFftMaxThreads / 32];
+  const FftPlan& f = A.fx;
+  const uint32_t bytes = static_cast<uint32_t>(A.hx + 1) * NP * 16;
+  const TileRing R{smem, s_full, bytes, bytes, nbuf};
+  const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t2);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < nbuf; ++i) mbar_init(&s_full[i], 1);
+    fence_mbar_init();
+    for (int i = 0; i < nbuf; ++i) {
+      const long long t = blockIdx.x + static_cast<long long>(i) * gridDim.x;
+      if (t < tiles) tile_issue(R, i, base + static_cast<size_t>(t) * bytes);
+    }
   }
+  __syncthreads();
   int pitch = (A.nx + 2) / 2 * 2;  // even for the paired stores; half of it odd: no bank conflicts
   if (pitch / 2 % 2 == 0) pitch += 2;
-  float* rows = reinterpret_cast<float*>(sh + static_cast<size_t>(f.n) * ZT);
-  const float2* src = A.t2 + static_cast<size_t>(j) * zc + z0;
-  const size_t hop_in = static_cast<size_t>(A.ny) * zc;
+  float* rows = reinterpret_cast<float*>(smem + static_cast<size_t>(nbuf) * bytes);
   const int half = f.n / 2;
-  for (int it = threadIdx.x; it < (half + 1) * ZT; it += kFftThreads) {
-    const int z = it & (ZT - 1), k = it / ZT;
-    const float2 a = __ldg(src + k * hop_in + z), b = __ldg(src + (f.n - k) * hop_in + z);
-    if (k == 0) {
-      sh[z] = make_float2(a.x + b.x, a.x - b.x);
-    } else {
-      // P = A_k / 2, Q = conj(A_{n-k}) / 2: (P + Q) + i e^{2 pi i k / mx} (P - Q)
-      const float2 w = __ldg(A.twx + k);
-      const float2 s = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-      const float2 d = make_float2(0.5f * (a.x - b.x), 0.5f * (a.y + b.y));
-      const float2 u = muli(cmulf(w, d));
-      sh[k * ZT + z] = cadd(s, u);
-      // index n - k: conj(s) + i conj(w) ... = conj(s - u)
-      if (2 * k != f.n) sh[(f.n - k) * ZT + z] = make_float2(s.x - u.x, -(s.y - u.y));
-    }
-  }
-  auto sin = [&](int e, int z) { return sh[e * ZT + z]; };
-  auto sout = [&](int e, int z, int, float2 v) { sh[e * ZT + z] = v; };
   const int rl = f.r[f.nst - 1], hop = f.n / rl;
-  auto rout = [&](int e, int z, int t, float2 v) {
-    int i = 2 * (__ldg(A.revx + (e - t) / rl) + t * hop) + A.sx;
-    i -= i >= A.mx ? A.mx : 0;
-    if (i < A.nx) *reinterpret_cast<float2*>(rows + z * pitch + i) = v;
-  };
-  for (int s = 0; s + 1 < f.nst; ++s) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const bool paired = (A.nx & 1) == 0 && (reinterpret_cast<uintptr_t>(field) & 7u) == 0;
+  double s1[2] = {0.0, 0.0}, s2[2] = {0.0, 0.0}, shift = 0.0;
+  int count = 0, n = 0;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
+    const int slot = n % nbuf;
+    const bool ok = mbar_wait_bounded(&s_full[slot], (n / nbuf) & 1, A.status);
+    if (!__syncthreads_and(ok)) {
+      if (threadIdx.x == 0)
+        for (int i = 0; i < nbuf; ++i)
+          if (t + static_cast<long long>(i) * gridDim.x < tiles)
+            mbar_wait_drain(&s_full[(n + i) % nbuf], ((n + i) / nbuf) & 1);
+      return;
+    }
+    ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem + static_cast<size_t>(slot) * bytes);
+    const int g = t / A.ny, j = t - g * A.ny, z0 = g * kZT;
+    for (int it = threadIdx.x; it < (half + 1) * NP; it += blockDim.x) {
+      const int p = it & (NP - 1), k = it / NP;
+      const ulonglong2 a = sh[k * NP + p], b = sh[(f.n - k) * NP + p];
+      if (k == 0) {
+        sh[p] = make_ulonglong2(add(a.x, b.x), sub(a.x, b.x));
+      } else {
+        // P = A_k / 2, Q = conj(A_{n-k}) / 2: (P + Q) + i e^{2 pi i k / mx} (P - Q)
+        const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(A.twr + k));
+        const C2 s = scale(C2{add(a.x, b.x), sub(a.y, b.y)}, dup(0.5f));
+        const C2 u = cmul(scale(C2{sub(a.x, b.x), add(a.y, b.y)}, dup(0.5f)), w.x, w.y);
+        const C2 z = add_i(s, u);
+        sh[k * NP + p] = make_ulonglong2(z.re, z.im);
+        // index n - k: the conjugate of s - i u
+        if (2 * k != f.n) sh[(f.n - k) * NP + p] = make_ulonglong2(add(s.re, u.im), sub(u.re, s.im));
+      }
+    }
+    auto in = [&](int e, int p) {
+      const ulonglong2 v = sh[e * NP + p];
+      return C2{v.x, v.y};
+    };
+    auto out = [&](int e, int p, int, C2 v) { sh[e * NP + p] = make_ulonglong2(v.re, v.im); };
+    auto rout = [&](int e, int p, int u, C2 v) {
+      int i = 2 * (__ldg(A.revx + e - u) + u * hop) + A.sx;
+      i -= i >= A.mx ? A.mx : 0;
+      if (i < A.nx) {
+        *reinterpret_cast<float2*>(rows + 2 * p * pitch + i) = make_float2(lo(v.re), lo(v.im));
+        *reinterpret_cast<float2*>(rows + (2 * p + 1) * pitch + i) = make_float2(hi(v.re), hi(v.im));
+      }
+    };
+    for (int s = 0; s + 1 < f.nst; ++s) {
+      __syncthreads();
+      stage_any<NP>(f, s, A.twx, in, out);
+    }
     __syncthreads();
-    fft_stage_any<ZT>(f, s, A.twx, 2, sin, sout);
-  }
-  __syncthreads();
-  fft_stage_any<ZT>(f, f.nst - 1, A.twx, 2, sin, rout);
-  __syncthreads();
-  // Rows of x: one warp per plane at a time.
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double s1 = 0.0, s2 = 0.0, cnt = 0.0, shift = 0.0;
-  bool have = false;
-  for (int z = warp; z < ZT && z0 + z < nzc; z += kFftThreads / 32) {
-    float* out = field + static_cast<size_t>(zbeg + z0 + z) * A.plane + static_cast<size_t>(j) * A.nx;
-    for (int i = lane; i < A.nx; i += 32) {
-      const float v = rows[z * pitch + i] * __ldg(A.dcx + i);
-      out[i] = v;
-      if (stats) {
-        if (!have) {
-          shift = v;
-          have = true;
+    stage_any<NP>(f, f.nst - 1, A.twx, in, rout);
+    __syncthreads();
+    const long long next = t + static_cast<long long>(nbuf) * gridDim.x;
+    if (threadIdx.x == 0 && next < tiles) {
+      fence_proxy_async_smem();
+      tile_issue(R, slot, base + static_cast<size_t>(next) * bytes);
+    }
+    // Rows of x: one warp per plane at a time, two values per lane where the
+    // field's rows are 8-byte aligned. The next tile's rows are written after
+    // at least one more barrier.
+    const float dy = __ldg(A.dcy + j);
+    if (n == 0) shift = rows[0] * (__ldg(A.dcx) * dy);  // any value of the field's size
+    auto take = [&](float v, int c) {
+      const double d = static_cast<double>(v) - shift;
+      s1[c] += d;
+      s2[c] = ::fma(d, d, s2[c]);
+    };
+    for (int z = warp; z < kZT && z0 + z < nzc; z += warps) {
+      float* dst = field + static_cast<size_t>(zbeg + z0 + z) * A.plane + static_cast<size_t>(j) * A.nx;
+      const float* row = rows + z * pitch;
+      if (paired) {
+#pragma unroll 4
+        for (int i = 2 * lane; i < A.nx; i += 64) {
+          float2 v = *reinterpret_cast<const float2*>(row + i);
+          const float2 d = __ldg(reinterpret_cast<const float2*>(A.dcx + i));
+          v.x *= d.x * dy;
+          v.y *= d.y * dy;
+          *reinterpret_cast<float2*>(dst + i) = v;
+          take(v.x, 0);
+          take(v.y, 1);
+          count += 2;
         }
-        const double d = static_cast<double>(v) - shift;
-        s1 += d;
-        s2 = fma(d, d, s2);
-        cnt += 1.0;
+      } else {
+#pragma unroll 4
+        for (int i = lane; i < A.nx; i += 32) {
+          const float v = row[i] * (__ldg(A.dcx + i) * dy);
+          dst[i] = v;
+          take(v, 0);
+          ++count;
+        }
       }
     }
   }
   if (stats) {
-    __shared__ Moments s_warp[kFftThreads / 32];
-    const Moments m = warp_moments(moments_from_shifted(cnt, shift, s1, s2));
+    const Moments m = warp_moments(moments_from_shifted(count, shift, s1[0] + s1[1], s2[0] + s2[1]));
     if (lane == 0) s_warp[warp] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
       Moments b = s_warp[0];
-      for (int w = 1; w < kFftThreads / 32; ++w) b = moments_merge(b, s_warp[w]);
-      stats[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = b;
+      for (int w = 1; w < warps; ++w) b = moments_merge(b, s_warp[w]);
+      stats[blockIdx.x] = b;
     }
   }
 }
 
 // ------------------------------------------------------------------- plans --
-// Stages of an FFT of length n (2, 3, 5-smooth); large radices first.
-bool fft_plan(int n, GridFft* f) {
-  f->n = n;
-  f->nst = 0;
-  int rest = n;
-  for (int r : {16, 8, 5, 4, 3, 2})
-    while (rest % r == 0 && rest > 1) {
-      if (f->nst == GridFft::kMaxStages) return false;
-      f->r[f->nst++] = r;
-      rest /= r;
+// Stages of an FFT of length n (2, 3, 5-smooth): the fewest, with the
+// smallest largest radix (registers) among those; descending radices.
+bool factor(int rest, int most, int depth, int* r, int* best, int* nbest) {
+  if (rest == 1) {
+    if (depth >= 2 && (!*nbest || depth < *nbest || (depth == *nbest && r[0] < best[0]))) {
+      std::copy(r, r + depth, best);
+      *nbest = depth;
     }
-  if (rest != 1 || f->nst < 2) return false;
+    return true;
+  }
+  if (depth == FftPlan::kMaxStages) return false;
+  for (int k : {12, 10, 9, 8, 6, 5, 4, 3, 2})
+    if (k <= most && rest % k == 0) {
+      r[depth] = k;
+      factor(rest / k, k, depth + 1, r, best, nbest);
+    }
+  return *nbest > 0;
+}
+bool fft_plan(int n, FftPlan* f) {
+  int rest = n;
+  for (int k : {2, 3, 5})
+    while (rest % k == 0) rest /= k;
+  if (rest != 1) return false;
+  int r[FftPlan::kMaxStages], nst = 0;
+  f->n = n;
+  if (!factor(n, n, 0, r, f->r, &nst)) return false;
+  f->nst = nst;
   int len = n;
   for (int s = 0; s < f->nst; ++s) {
     len /= f->r[s];
@@ -775,15 +761,47 @@ bool fft_plan(int n, GridFft* f) {
   return true;
 }
 
+constexpr size_t kSmemMax = 224 * 1024;  // dynamic; the kernels keep a little static shared memory
+
+// Launch shape of a transform kernel: two tile buffers where they fit, and
+// the block size that fills an SM's registers (kFftMaxThreads threads) with
+// the least idle threads in the stages' rounds.
+struct FftShape {
+  int threads, blocks, nbuf;
+  size_t smem;
+};
+FftShape fft_shape(const FftPlan& f, size_t tile, size_t extra, long long tiles) {
+  FftShape best{};
+  best.nbuf = 2 * tile + extra <= kSmemMax ? 2 : 1;
+  best.smem = best.nbuf * tile + extra;
+  double best_cost = 1e30;
+  for (int t = 64; t <= kFftMaxThreads; t += 32) {
+    const int per_sm = static_cast<int>(std::min<size_t>(std::min<size_t>(kSmemMax / best.smem, kFftMaxThreads / t), 8));
+    if (per_sm < 1) continue;
+    double work = 0.0;
+    for (int s = 0; s < f.nst; ++s) {
+      const int items = f.n / f.r[s] * kPairs;
+      work += static_cast<double>((items + t - 1) / t) * t / items;
+    }
+    const double cost = work / (per_sm * t);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best.threads = t;
+      best.blocks = static_cast<int>(std::min<long long>(tiles, 148ll * per_sm));
+    }
+  }
+  return best;
+}
+
 // Transform length for n outputs: at least 1.5 n, a multiple of 4, with the
 // least length x (stages + 2) among lengths up to 15 % longer. `half`: the
 // complex transform has half the length (the real axis).
-int fft_length(int n, bool half, GridFft* f) {
+int fft_length(int n, bool half, FftPlan* f) {
   const int lo = std::max(kMinM, static_cast<int>(std::ceil(kOversample * n)));
   int best = 0;
   double best_cost = 0.0;
   for (int m = (lo + 3) / 4 * 4; m <= std::max(lo * 23 / 20, lo + 16); m += 4) {
-    GridFft g;
+    FftPlan g;
     if (!fft_plan(half ? m / 2 : m, &g)) continue;
     const double cost = static_cast<double>(m) * (g.nst + 2);
     if (!best || cost < best_cost) {
@@ -797,11 +815,9 @@ int fft_length(int n, bool half, GridFft* f) {
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-constexpr size_t kSmemMax = 224 * 1024;  // dynamic; the kernels keep a little static shared memory
-size_t smem_y(const GridPlan& p, int zt) { return sizeof(float2) * static_cast<size_t>(p.my) * zt; }
-size_t smem_x(const GridPlan& p, int zt) {
-  return sizeof(float2) * static_cast<size_t>(p.mx / 2) * zt + sizeof(float) * static_cast<size_t>(p.nx + 4) * zt;
-}
+size_t tile_y(const GridPlan& p) { return sizeof(float2) * kZT * static_cast<size_t>(p.my); }
+size_t tile_x(const GridPlan& p) { return sizeof(float2) * kZT * static_cast<size_t>(p.mx / 2 + 1); }
+size_t rows_x(const GridPlan& p) { return sizeof(float) * kZT * static_cast<size_t>(p.nx + 4); }
 
 double window_beta(int n, int m) {
   // Shape parameter of the Kaiser-Bessel window for this oversampling
@@ -830,10 +846,7 @@ bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
   if (!p.mx) return false;
   p.my = 1;
   if (p.ny > 1 && !(p.my = fft_length(p.ny, false, &p.fy))) return false;
-  p.zt = 0;
-  for (int zt : {16, 8})
-    if (!p.zt && (p.ny == 1 || smem_y(p, zt) <= kSmemMax) && smem_x(p, zt) <= kSmemMax) p.zt = zt;
-  if (!p.zt) return false;
+  if ((p.ny > 1 && tile_y(p) > kSmemMax) || tile_x(p) + rows_x(p) > kSmemMax) return false;
   p.nbx = (p.mx / 2 + kB) / kB;
   p.nby = p.ny > 1 ? p.my / kB : 1;
   p.nkeys = (p.nbx + kSpan) * p.nby;
@@ -866,13 +879,25 @@ bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
   p.off_weights = take(sizeof(float) * 2 * kSpan * kB * static_cast<size_t>(p.nent));
   p.off_e = take(sizeof(float2) * static_cast<size_t>(p.nent) * p.ez);
   p.off_t1 = take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.my * p.zc);
-  p.off_t2 = p.ny > 1 ? take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.ny * p.zc) : p.off_t1;
-  p.off_partial = take(sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * kB * p.zc);
+  // T2 takes the place of the partial sums, which are in T1 by then; a single
+  // gridded axis has no T2.
+  const size_t partial = sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * kB * p.zc;
+  const size_t t2 = p.ny > 1 ? sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.ny * p.zc : 0;
+  p.off_partial = take(std::max(partial, t2));
+  p.off_t2 = p.ny > 1 ? p.off_partial : p.off_t1;
   p.off_tasks = take(sizeof(int4) * (p.maxtasks + p.maxslots));
-  p.off_tables = take(sizeof(float2) * (p.mx + p.my) + sizeof(int) * (p.mx + p.my) + sizeof(float) * (p.nx + p.ny));
+  p.off_dc = take(sizeof(float) * (p.nx + 2 + p.ny));
+  p.off_tables = take(sizeof(float4) * (p.mx + p.my) + sizeof(int) * (p.mx + p.my));
   p.bytes = off;
   *P = p;
   return true;
+}
+
+bool grid_pays(const GridPlan& p, const TcPlan& tc) {
+  const double cells = static_cast<double>(p.mx / 2) * p.my * p.nz, visits = p.ny > 1 ? 9.0 : 3.0;
+  const double grid = 90.0 + 1.35e-5 * cells + p.nh * (0.008 + 0.67e-5 * visits * p.nz);
+  const double waves = std::ceil(static_cast<double>(tc.bix) * tc.bjx * tc.bn / 148.0);
+  return grid < 50.0 + waves * (20.0 + 0.0435 * p.nh);
 }
 
 int grid_passes(const GridPlan& p) { return (p.nz + p.zc - 1) / p.zc; }
@@ -880,8 +905,20 @@ void grid_pass_planes(const GridPlan& p, int pass, int* z0, int* z1) {
   *z0 = pass * p.zc;
   *z1 = std::min(p.nz, *z0 + p.zc);
 }
-long long grid_stat_records(const GridPlan& p) {
-  return static_cast<long long>(grid_passes(p)) * p.ny * (p.zc / p.zt);
+namespace {
+// Step 3 of a pass: tiles past the last plane have nothing to store.
+int x_tiles(const GridPlan& p, int planes) { return (planes + kZT - 1) / kZT * p.ny; }
+FftShape x_shape(const GridPlan& p, int planes) { return fft_shape(p.fx, tile_x(p), rows_x(p), x_tiles(p, planes)); }
+}  // namespace
+
+long long grid_stat_records(const GridPlan& p) {  // one per block of every pass's step 3
+  long long n = 0;
+  for (int pass = 0; pass < grid_passes(p); ++pass) {
+    int z0, z1;
+    grid_pass_planes(p, pass, &z0, &z1);
+    n += x_shape(p, z1 - z0).blocks;
+  }
+  return n;
 }
 
 namespace {
@@ -893,17 +930,15 @@ cudaError_t ensure_grid_attributes() {
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
   const int most = static_cast<int>(kSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_y_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_y_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  e = cudaFuncSetAttribute(grid_fft_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
   return e;
 }
 }  // namespace
 
 cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], float ds, const float* d_table,
-                                   float* d_field, void* d_work, const GridPlan& p, cudaStream_t stream,
+                                   float* d_field, void* d_work, const GridPlan& p, int* d_status, cudaStream_t stream,
                                    StatRecord* d_stats, const std::function<cudaError_t(int)>& pass_done) {
   cudaError_t e = ensure_grid_attributes();
   if (e != cudaSuccess) return e;
@@ -930,6 +965,7 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.scaling = s.scaling;
   A.plane = static_cast<long long>(p.nx) * p.ny;
   A.table = d_table;
+  A.status = d_status;
   A.counts = reinterpret_cast<int*>(w + p.off_counts);
   A.ntasks = A.counts + p.nkeys;
   A.keys = reinterpret_cast<uint2*>(w + p.off_keys);
@@ -945,12 +981,13 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.partial = reinterpret_cast<float2*>(w + p.off_partial);
   A.tasks = reinterpret_cast<int4*>(w + p.off_tasks);
   A.multi = A.tasks + p.maxtasks;
-  A.twx = reinterpret_cast<float2*>(w + p.off_tables);
-  A.twy = A.twx + p.mx;
+  A.twx = reinterpret_cast<float4*>(w + p.off_tables);
+  A.twr = A.twx + p.mx / 2;
+  A.twy = A.twr + p.mx / 2;
   A.revx = reinterpret_cast<int*>(A.twy + p.my);
   A.revy = A.revx + p.mx;
-  A.dcx = reinterpret_cast<float*>(A.revy + p.my);
-  A.dcy = A.dcx + p.nx;
+  A.dcx = reinterpret_cast<float*>(w + p.off_dc);
+  A.dcy = A.dcx + p.nx + 1;
 
   const long long items = static_cast<long long>(p.nh) + 2 * (p.mx + p.my) + p.nx + p.ny;
   // Entry counts and the task counters behind them.
@@ -961,7 +998,6 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   const int scatter = (p.nent + 255) / 256;
   grid_bins_kernel<<<scatter + (nbins + 7) / 8, 256, 0, stream>>>(A, scatter);
   const int task_blocks = std::min(p.maxtasks, 148 * 4);
-  const int tiles = p.zc / p.zt;
   for (int pass = 0; pass < grid_passes(p); ++pass) {
     int z0, z1;
     grid_pass_planes(p, pass, &z0, &z1);
@@ -973,16 +1009,15 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
     const int planes = (z1 - z0 + 31) / 32 * 32;
     grid_spread_kernel<<<dim3(task_blocks + (nbins + 7) / 8, planes / 32), 256, 0, stream>>>(A, task_blocks, zoff, p.zc);
     grid_parts_kernel<<<dim3(std::min(p.maxslots, 148), planes / 32), 512, 0, stream>>>(A, p.zc);
-    const dim3 gy(static_cast<unsigned>(planes / p.zt), static_cast<unsigned>(p.mx / 2 + 1));
-    const dim3 gx(static_cast<unsigned>(tiles), static_cast<unsigned>(p.ny));
-    StatRecord* rec = d_stats ? d_stats + static_cast<size_t>(pass) * p.ny * tiles : nullptr;
-    if (p.zt == 16) {
-      if (p.ny > 1) grid_fft_y_kernel<16><<<gy, kFftThreads, smem_y(p, 16), stream>>>(A, p.zc);
-      grid_fft_x_kernel<16><<<gx, kFftThreads, smem_x(p, 16), stream>>>(A, d_field, z0, p.zc, z1 - z0, rec);
-    } else {
-      if (p.ny > 1) grid_fft_y_kernel<8><<<gy, kFftThreads, smem_y(p, 8), stream>>>(A, p.zc);
-      grid_fft_x_kernel<8><<<gx, kFftThreads, smem_x(p, 8), stream>>>(A, d_field, z0, p.zc, z1 - z0, rec);
+    const long long groups = planes / kZT;
+    if (p.ny > 1) {
+      const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * (p.mx / 2 + 1));
+      grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * (p.mx / 2 + 1)), y.nbuf);
     }
+    const FftShape x = x_shape(p, z1 - z0);
+    grid_fft_x_kernel<<<x.blocks, x.threads, x.smem, stream>>>(A, d_field, z0, z1 - z0, x_tiles(p, z1 - z0), x.nbuf,
+                                                               d_stats);
+    if (d_stats) d_stats += x.blocks;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (pass_done && (e = pass_done(pass)) != cudaSuccess) return e;
   }

@@ -171,28 +171,39 @@ cudaError_t tc_batch_launch(const TcBatchPlan& plan, void* d_work, cudaStream_t 
 
 // ---- gridded Fourier form of structured sums (srm_grid.cu) ----
 constexpr int kGridMaxHarmonics = 1 << 20;
-constexpr size_t kGridPassBytes = size_t(96) << 20;  // T1 and T2 of one pass
+constexpr size_t kGridPassBytes = size_t(48) << 20;  // T1 and T2 of one pass
 constexpr size_t kGridEBytes = size_t(1) << 30;      // E of as many passes as fit
+// Stages of an FFT of length n: radix, distance between a butterfly's
+// elements and its reciprocal.
+struct FftPlan {
+  static constexpr int kMaxStages = 8;
+  int n, nst;
+  int r[kMaxStages], m[kMaxStages];
+  float inv_m[kMaxStages];
+};
+
 struct GridPlan {
-  struct Fft {
-    static constexpr int kMaxStages = 8;
-    int n, nst;
-    int r[kMaxStages], m[kMaxStages];  // radix and element distance of each stage
-    float inv_m[kMaxStages];
-  };
   int ndim, nh, nent;
   int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly
   int ax_y, ax_z;      // their physical axes
   int mx, my;          // transform lengths
-  Fft fx, fy;          // of length mx / 2 and my
+  FftPlan fx, fy;      // of length mx / 2 and my
   int nbx, nby, nkeys, maxtasks, maxslots;
-  int zt, zc, ez;      // planes per transform tile, per pass, per build of E
+  int zc, ez;          // planes per pass, per build of E
   size_t off_counts, off_keys, off_members, off_par, off_w, off_bins, off_weights, off_e, off_t1, off_t2, off_partial,
-      off_tasks, off_tables, bytes;
+      off_tasks, off_dc, off_tables, bytes;
 };
 // False when the form does not take the grid (an axis too long for a
 // transform in shared memory, no or too many harmonics).
 bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* plan);
+// Whether the gridded sum is faster than a tensor-core plan, from fits (in us)
+// to measured device times. The contraction pays per wave of output tiles and
+// harmonic, the gridded sum per cell of its wavenumber grid, and per harmonic
+// and plane. Measured, gridded / tensor cores: 128^3 120 / 99 us at 500
+// harmonics, 127 / 126 at 1 000, 169 / 280 at 4 000; 400^3 1 104 / 926 at 1 000,
+// 1 160 / 1 582 at 2 000, 1 506 / 10 768 at 16 000; 24 x 24 x 1000 339 / 297 at
+// 4 000; 1 500 x 1 500 143 / 159 at 500, 573 / 1 250 at 16 000.
+bool grid_pays(const GridPlan& p, const TcPlan& tc);
 int grid_passes(const GridPlan& p);
 // Planes [z0, z1) that a pass completes; whole contiguous pieces of the field.
 void grid_pass_planes(const GridPlan& p, int pass, int* z0, int* z1);
@@ -200,7 +211,8 @@ long long grid_stat_records(const GridPlan& p);
 // Enqueues the whole sum. pass_done(pass), when set, is called once the
 // launches that complete a pass's planes are enqueued.
 cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], float ds, const float* d_table,
-                                   float* d_field, void* d_work, const GridPlan& plan, cudaStream_t stream,
+                                   float* d_field, void* d_work, const GridPlan& plan, int* d_status,
+                                   cudaStream_t stream,
                                    StatRecord* d_stats, const std::function<cudaError_t(int)>& pass_done);
 
 // ---- device side of the harmonic sampler (srm_sampler.cu) ----

@@ -1,8 +1,7 @@
-"""The gridded Fourier form that scarf_execute takes for structured meshes,
-against the FP64 sum over the same harmonics at every point: grids at the
+"""The gridded Fourier form that scarf_execute takes for structured meshes
+(of enough harmonics for it to be the faster), against the FP64 sum over the same harmonics at every point: grids at the
 edges of its plans (one-point and tiny axes, odd sizes, transform lengths of
-every radix, several passes over z, tiles past the last plane), few and many
-harmonics, rotation, offsets.
+every radix, several passes over z, tiles past the last plane), rotation, offsets.
 
 Tolerance: the window's interpolation error (nine cells at an oversampling of
 1.5: 1.8e-7 rms per transformed axis, up to 1.1e-6 at single wavenumbers) and
@@ -63,15 +62,15 @@ def _case(n, nharm, fs=None, acf=0, frac=0.1, angles=(0.0, 0.0, 0.0), ds=25.0, s
     (16, 16, 16), (17, 13, 31), (48, 40, 33), (64, 1, 64), (64, 64, 1), (1, 40, 50), (2, 3, 200), (100, 2, 5),
     (31, 97, 65), (200, 9, 3), (128, 81, 32), (333, 20, 40), (20, 251, 40)])
 def test_grids_match_fp64(n):
-    _case(n, 700)
+    _case(n, 1500)
 
 
 @pytest.mark.parametrize("n", [(100, 70), (1201, 40), (37, 801), (5, 300), (300, 1)])
 def test_2d_grids_match_fp64(n):
-    _case(n, 900, angles=(20.0, 0.0, 0.0))
+    _case(n, 1500, angles=(20.0, 0.0, 0.0))
 
 
-@pytest.mark.parametrize("nharm", [1, 2, 31, 257, 5000, 30000])
+@pytest.mark.parametrize("nharm", [1501, 5000, 30000])
 def test_harmonic_counts(nharm):
     _case((40, 36, 50), nharm, fs=[5, 3, -7], angles=(30.0, -10.0, 5.0))
 

@@ -713,12 +713,19 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   scarf_srm_setup s{};
   rc = srm_setup(p, &s);
   if (rc) return fail(rc, "invalid SRM parameters (acf %d, nharm %d)", p.acf, p.nharm);
-  std::vector<float> table(5 * static_cast<size_t>(p.nharm));
   const int threads = t_ctx->cfg.threads > 0 ? t_ctx->cfg.threads : host_threads();
   long long pairs = 0;
   const bool on_gpu = !t_ctx->cfg.src.srng && t_ctx->cfg.sampler != SCARF_SAMPLER_HOST;
-  const int nh = on_gpu ? srm_sample_device(p, s, table.data(), &pairs, st, nullptr)
-                        : srm_sample(p, s, &t_ctx->cfg.src, threads, table.data(), &pairs);
+  std::vector<float> table;
+  const float* rows = nullptr;  // in memory of the device sampler's, or the table
+  int nh;
+  if (on_gpu) {
+    nh = srm_sample_field(p, s, nullptr, &rows, &pairs, st, nullptr);
+  } else {
+    table.resize(5 * static_cast<size_t>(p.nharm));
+    nh = srm_sample(p, s, &t_ctx->cfg.src, threads, table.data(), &pairs);
+    rows = table.data();
+  }
   if (nh == -2) return sampler_fail("device sampler");
   if (nh < 0)
     return fail(SCARF_ERR_ARG,
@@ -749,7 +756,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   SCARF_CUDA(cudaEventRecord(t_ctx->res.ev0, st));
   SCARF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   if (nh > 0)
-    SCARF_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(float) * 5 * nh, cudaMemcpyHostToDevice, st));
+    SCARF_CUDA(cudaMemcpyAsync(d_table, rows, sizeof(float) * 5 * nh, cudaMemcpyHostToDevice, st));
 
   const float* dx = nullptr;
   const float* dy = nullptr;
@@ -1305,7 +1312,7 @@ int scarf_srm_sample_device(const scarf_srm_params* p, const scarf_srm_setup* s,
   if (!p || !s || !table) return fail(SCARF_ERR_ARG, "NULL argument");
   scarf::take_device_alloc_failure();
   long long used = 0, open = 0;
-  const int kept = srm_sample_device(*p, *s, table, &used, stream, &open);
+  const int kept = srm_sample_field(*p, *s, table, nullptr, &used, stream, &open);
   if (kept == -1)
     return fail(SCARF_ERR_ARG, "rejection sampling infeasible: acceptance rate %.3g < %.1g", acceptance_rate(*s),
                 kMinAcceptance);
@@ -1651,6 +1658,7 @@ int scarf_release_device_memory(void) {
     SCARF_CUDA(cudaSetDevice(dev));
   }
   scarf::release_sampler_device_memory();
+  scarf::release_field_sampler_memory();
   scarf::release_fim_plans();
   return SCARF_OK;
 }

@@ -495,6 +495,20 @@ int walk_parallel(const scarf_srm_params& p, const scarf_srm_setup& s, int threa
 
 }  // namespace
 
+bool sampler_host_accept(const scarf_srm_setup& s, int acf, float r1, float r2) {
+  float u;
+  return accept(r1, r2, s, acf, &u);
+}
+
+void sampler_row(float u, const float draws[6], int ndim, const float cl[3], float* row) {
+  Draws d{};
+  d.u = u;
+  d.ang[0] = draws[0], d.ang[1] = draws[1];
+  d.ra[0] = draws[2], d.ra[1] = draws[3];
+  d.rb[0] = draws[4], d.rb[1] = draws[5];
+  harmonic_row(d, ndim, cl, row);
+}
+
 double acceptance_rate(const scarf_srm_setup& s) {
   const double width = static_cast<double>(s.kmax) - static_cast<double>(s.kmin);
   if (!(width > 0.0)) return 0.0;
@@ -588,12 +602,6 @@ long long g_pass_pairs_cap = 0;  // 0: size passes from the acceptance rate
 // while the following groups scan.
 constexpr int kSamplerGroups = 8;
 
-// Host decision for a pair the device left open (glibc spectrum).
-bool host_accept(const scarf_srm_setup& s, int acf, float r1, float r2) {
-  float u;
-  return accept(r1, r2, s, acf, &u);
-}
-
 }  // namespace
 
 void sampler_reject_thresholds(const scarf_srm_setup& s, int acf, float margin, uint32_t* thr) {
@@ -635,6 +643,11 @@ void sampler_reject_thresholds(const scarf_srm_setup& s, int acf, float margin, 
     }
     thr[b] = t;
   }
+}
+
+long long device_sampler_pass_cap() {
+  std::lock_guard<std::mutex> lk(g_dev_sampler_mu);
+  return g_pass_pairs_cap;
 }
 
 void set_device_sampler_pass_cap(long long pairs) {
@@ -775,7 +788,7 @@ struct DeviceWalk {
         bool ok = e.flag == 1;
         if (e.flag == 2) {
           ++open;
-          ok = host_accept(*s, p->acf, e.r[0], e.r[1]);
+          ok = sampler_host_accept(*s, p->acf, e.r[0], e.r[1]);
         }
         if (!ok) {
           ++ei;

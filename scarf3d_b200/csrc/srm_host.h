@@ -86,6 +86,17 @@ double acceptance_rate(const scarf_srm_setup& s);
 // pairs decided on the host.
 int srm_sample_device(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
                       void* stream, long long* uncertain);
+// The same table (and counts) by the single-field form of the device scan
+// (srm_sample_field.cu); scarf_execute's sampler. With `staged`, table may be
+// null and the rows are wherever *staged says: memory of the sampler's own
+// (page-locked, usually), valid until its next call.
+int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, const float** staged,
+                     long long* pairs_used, void* stream, long long* uncertain);
+void release_field_sampler_memory();
+// Host decision for a pair the device left open (glibc spectrum), and a
+// harmonic's table row from u and the three pairs drawn after it.
+bool sampler_host_accept(const scarf_srm_setup& s, int acf, float r1, float r2);
+void sampler_row(float u, const float draws[6], int ndim, const float cl[3], float* row);
 // srm_sample_device for many fields at once: the first pass of every field
 // runs in one count launch and one write launch, then the host walks the
 // fields one by one (further passes per field only if needed). Tables are
@@ -111,6 +122,7 @@ constexpr float kSamplerMargin = 2e-5f;
 // Upper bound on the pairs tested per device pass (0 = sized from the
 // acceptance rate); smaller passes are chained until every harmonic is drawn.
 void set_device_sampler_pass_cap(long long pairs);
+long long device_sampler_pass_cap();
 
 int host_threads();
 

@@ -364,29 +364,43 @@ __global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z
   }
 }
 
-// T1 cell (cx, cy), plane z of the pass.
-__device__ __forceinline__ size_t t1_index(const GridArgs& A, int cx, int cy, int z) {
-  const int g = z / kZT;
-  // A single gridded axis goes straight to step 3, as [zc / kZT][ny = 1][hx + 1][kZT].
-  return ((static_cast<size_t>(g) * (A.hx + 1) + cx) * A.my + cy) * kZT + z % kZT;
-}
-
 // Step 1. A warp sums up to 32 entries of one 4 x 4-cell bin over 32 planes:
-// lanes are planes, the 16 cells are registers. Bins of up to kSparse entries
-// are one warp's; the first blocks take the listed tasks, 8 warps each whose
-// sums are added in order through shared memory. Bound: load latency (256
-// bytes of E and two weight vectors per entry), hence four entries in flight;
-// FP32 issue (40 multiply-adds per entry and warp) where bins are dense.
-struct BinSum {
-  float2 acc[kB][kB];
+// lanes are planes, the 16 cells are registers. The entries' E rows (256
+// bytes each) and weights come into shared memory by asynchronous copies, all
+// at once: with four entries in flight from registers the load latency of a
+// group was most of its time (512^3 x 20 000: 40 us a pass, 16 warps per SM).
+// Bins of up to kSparse entries are one warp's; the first blocks take the
+// listed tasks, 8 warps each whose sums are added in order through shared
+// memory. Bound: FP32 issue (40 multiply-adds per entry and warp).
+struct SpreadWarp {
+  float2 e[32][32];         // [entry][lane]
+  float w[32][2 * kB];      // x and y weights of the bin's cells
 };
-__device__ __forceinline__ void sum_entries(const GridArgs& A, int lane, int lo, int hi, int beg, int end,
-                                            const float2* ez, BinSum& S) {
+constexpr int kSpreadWarps = 8;
+static_assert(sizeof(SpreadWarp) >= sizeof(float2) * kB * kB * 32, "the partial sums take the entries' place");
+
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int KY>  // cells along y: kB, or 1 when only x is gridded
+struct BinSum {
+  float2 acc[kB][KY];
+};
+// Entries [beg, end) (at most 32) of the nine ranges lo, hi of lanes 0 .. 8.
+template <int KY>
+__device__ __forceinline__ void sum_entries(const GridArgs& A, SpreadWarp& W, int lane, int lo, int hi, int beg, int end,
+                                            const float2* ez, BinSum<KY>& S) {
 #pragma unroll
   for (int i = 0; i < kB; ++i)
 #pragma unroll
-    for (int j = 0; j < kB; ++j) S.acc[i][j] = make_float2(0.0f, 0.0f);
-  if (beg >= end) return;
+    for (int j = 0; j < KY; ++j) S.acc[i][j] = make_float2(0.0f, 0.0f);
+  const int n = end - beg;
+  if (n <= 0) return;
   // Inclusive prefix of the range lengths; lane l resolves visit beg + l to an
   // entry and its bin offset.
   int pre = hi - lo;
@@ -400,69 +414,74 @@ __device__ __forceinline__ void sum_entries(const GridArgs& A, int lane, int lo,
   for (int q = 0; q < kSpan * kSpan; ++q) r += __shfl_sync(0xffffffffu, pre, q) <= beg + lane ? 1 : 0;
   const int rc = min(r, kSpan * kSpan - 1);
   const int ent = __shfl_sync(0xffffffffu, hi, rc) - (__shfl_sync(0xffffffffu, pre, rc) - (beg + lane));
-  const int n = end - beg;
-  auto add = [&](const float4& wx, const float4& wy, const float2& e) {
+  if (lane < n) {
+    const float* w = A.weights + static_cast<size_t>(ent) * (2 * kSpan * kB);
+    cp_async16(&W.w[lane][0], w + rc / kSpan * kB);
+    cp_async16(&W.w[lane][kB], w + (kSpan + rc % kSpan) * kB);
+  }
+  for (int u = 0; u < n; ++u) {
+    const int en = __shfl_sync(0xffffffffu, ent, u);
+    cp_async8(&W.e[u][lane], ez + static_cast<size_t>(en) * A.ez);
+  }
+  cp_async_wait();
+  __syncwarp();
+#pragma unroll 2
+  for (int u = 0; u < n; ++u) {
+    const float4 wx = *reinterpret_cast<const float4*>(&W.w[u][0]), wy = *reinterpret_cast<const float4*>(&W.w[u][kB]);
+    const float2 e = W.e[u][lane];
     const float x[4] = {wx.x, wx.y, wx.z, wx.w}, y[4] = {wy.x, wy.y, wy.z, wy.w};
 #pragma unroll
     for (int i = 0; i < kB; ++i) {
       const float2 t = make_float2(x[i] * e.x, x[i] * e.y);
 #pragma unroll
-      for (int j = 0; j < kB; ++j) {
+      for (int j = 0; j < KY; ++j) {
         S.acc[i][j].x = fmaf(y[j], t.x, S.acc[i][j].x);
         S.acc[i][j].y = fmaf(y[j], t.y, S.acc[i][j].y);
       }
     }
-  };
-  int u = 0;
-  for (; u + 4 <= n; u += 4) {
-    float4 wx[4], wy[4];
-    float2 e[4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const int en = __shfl_sync(0xffffffffu, ent, u + g), rr = __shfl_sync(0xffffffffu, rc, u + g);
-      const float4* w = reinterpret_cast<const float4*>(A.weights) + static_cast<size_t>(en) * (2 * kSpan);
-      wx[g] = __ldg(w + rr / kSpan);
-      wy[g] = __ldg(w + kSpan + rr % kSpan);
-      e[g] = __ldg(ez + static_cast<size_t>(en) * A.ez);
-    }
-#pragma unroll
-    for (int g = 0; g < 4; ++g) add(wx[g], wy[g], e[g]);
-  }
-  for (; u < n; ++u) {
-    const int en = __shfl_sync(0xffffffffu, ent, u), rr = __shfl_sync(0xffffffffu, rc, u);
-    const float4* w = reinterpret_cast<const float4*>(A.weights) + static_cast<size_t>(en) * (2 * kSpan);
-    add(__ldg(w + rr / kSpan), __ldg(w + kSpan + rr % kSpan), __ldg(ez + static_cast<size_t>(en) * A.ez));
   }
 }
 
-__global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int task_blocks, int zoff, int zc) {
-  __shared__ float2 part[8][kB * kB][32];
+// T1 cell (cx, cy), plane z of the pass.
+__device__ __forceinline__ size_t t1_index(const GridArgs& A, int cx, int cy, int z) {
+  const int g = z / kZT;
+  // A single gridded axis goes straight to step 3, as [zc / kZT][ny = 1][hx + 1][kZT].
+  return ((static_cast<size_t>(g) * (A.hx + 1) + cx) * A.my + cy) * kZT + z % kZT;
+}
+
+template <int KY>
+__global__ void __launch_bounds__(32 * kSpreadWarps) grid_spread_kernel(const GridArgs A, int task_blocks, int zoff, int zc) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  SpreadWarp* warps = reinterpret_cast<SpreadWarp*>(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int zb = blockIdx.y * 32, z = zb + lane;
+  const int z = blockIdx.y * 32 + lane;
   const float2* ez = A.e + zoff + z;
-  BinSum S;
+  BinSum<KY> S;
   int lo, hi;
   if (static_cast<int>(blockIdx.x) < task_blocks) {
-    const int n = *A.ntasks;
+    const int n = A.ntasks[0];
     for (int task = blockIdx.x; task < n; task += task_blocks) {
       const int4 T = A.tasks[task];
       bin_ranges(A, T.x, lane, &lo, &hi);
       const int total = __reduce_add_sync(0xffffffffu, hi - lo);
       const int beg = min(total, T.y * kPart + warp * 32);
-      sum_entries(A, lane, lo, hi, beg, min(total, beg + 32), ez, S);
+      sum_entries(A, warps[warp], lane, lo, hi, beg, min(total, beg + 32), ez, S);
+      __syncwarp();  // the warp's entries are read
+      float2(*mine)[32] = reinterpret_cast<float2(*)[32]>(&warps[warp]);
 #pragma unroll
-      for (int c = 0; c < kB * kB; ++c) part[warp][c][lane] = S.acc[c / kB][c % kB];
+      for (int c = 0; c < kB * KY; ++c) mine[c][lane] = S.acc[c / KY][c % KY];
       __syncthreads();
       const int bx = T.x / A.nby, by = T.x - bx * A.nby;
 #pragma unroll
-      for (int q = 0; q < kB * kB / 8; ++q) {
-        const int c = warp + 8 * q;
-        float2 v = part[0][c][lane];
+      for (int q = 0; q < (kB * KY + kSpreadWarps - 1) / kSpreadWarps; ++q) {
+        const int c = warp + kSpreadWarps * q;
+        if (c >= kB * KY) break;
+        float2 v = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int w = 1; w < 8; ++w) v = cadd(v, part[w][c][lane]);
-        const int cx = bx * kB + c / kB, cy = by * kB + c % kB;
+        for (int w = 0; w < kSpreadWarps; ++w) v = cadd(v, reinterpret_cast<const float2(*)[32]>(&warps[w])[c][lane]);
+        const int cx = bx * kB + c / KY, cy = by * kB + c % KY;
         if (T.z > 1)
-          A.partial[(static_cast<size_t>(T.w + T.y) * (kB * kB) + c) * zc + z] = v;
+          A.partial[(static_cast<size_t>(T.w + T.y) * (kB * KY) + c) * zc + z] = v;
         else if (cx <= A.hx && cy < A.my)
           A.t1[t1_index(A, cx, cy, z)] = v;
       }
@@ -470,19 +489,19 @@ __global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int 
     }
     return;
   }
-  const int bin = (blockIdx.x - task_blocks) * 8 + warp;
+  const int bin = (blockIdx.x - task_blocks) * kSpreadWarps + warp;
   if (bin >= A.nbx * A.nby) return;
   bin_ranges(A, bin, lane, &lo, &hi);
   const int total = __reduce_add_sync(0xffffffffu, hi - lo);
   if (total > kSparse) return;
-  sum_entries(A, lane, lo, hi, 0, total, ez, S);
+  sum_entries(A, warps[warp], lane, lo, hi, 0, total, ez, S);
   const int bx = bin / A.nby, by = bin - bx * A.nby;
 #pragma unroll
   for (int i = 0; i < kB; ++i) {
     const int cx = bx * kB + i;
     if (cx > A.hx) break;
 #pragma unroll
-    for (int j = 0; j < kB; ++j) {
+    for (int j = 0; j < KY; ++j) {
       const int cy = by * kB + j;
       if (cy < A.my) A.t1[t1_index(A, cx, cy, z)] = S.acc[i][j];
     }
@@ -491,13 +510,14 @@ __global__ void __launch_bounds__(256) grid_spread_kernel(const GridArgs A, int 
 
 // The parts of each bin with several, added in order: one block per bin and
 // 32 planes at a time.
-__global__ void __launch_bounds__(512) grid_parts_kernel(const GridArgs A, int zc) {
+template <int KY>
+__global__ void __launch_bounds__(32 * kB * KY) grid_parts_kernel(const GridArgs A, int zc) {
   const int n = A.ntasks[2], cell = threadIdx.x >> 5, z = blockIdx.y * 32 + (threadIdx.x & 31);
   for (int m = blockIdx.x; m < n; m += gridDim.x) {
     const int4 T = A.multi[m];
     const int bx = T.x / A.nby, by = T.x - bx * A.nby;
-    const size_t hop = static_cast<size_t>(kB * kB) * zc;
-    const float2* p = A.partial + (static_cast<size_t>(T.z) * (kB * kB) + cell) * zc + z;
+    const size_t hop = static_cast<size_t>(kB * KY) * zc;
+    const float2* p = A.partial + (static_cast<size_t>(T.z) * (kB * KY) + cell) * zc + z;
     float2 v = make_float2(0.0f, 0.0f);
     int q = 0;
     for (; q + 8 <= T.y; q += 8) {
@@ -508,7 +528,7 @@ __global__ void __launch_bounds__(512) grid_parts_kernel(const GridArgs A, int z
       for (int u = 0; u < 8; ++u) v = cadd(v, x[u]);
     }
     for (; q < T.y; ++q) v = cadd(v, p[q * hop]);
-    const int cx = bx * kB + cell / kB, cy = by * kB + cell % kB;
+    const int cx = bx * kB + cell / KY, cy = by * kB + cell % KY;
     if (cx <= A.hx && cy < A.my) A.t1[t1_index(A, cx, cy, z)] = v;
   }
 }
@@ -881,7 +901,7 @@ bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
   p.off_t1 = take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.my * p.zc);
   // T2 takes the place of the partial sums, which are in T1 by then; a single
   // gridded axis has no T2.
-  const size_t partial = sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * kB * p.zc;
+  const size_t partial = sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * (p.ny > 1 ? kB : 1) * p.zc;
   const size_t t2 = p.ny > 1 ? sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.ny * p.zc : 0;
   p.off_partial = take(std::max(partial, t2));
   p.off_t2 = p.ny > 1 ? p.off_partial : p.off_t1;
@@ -930,6 +950,10 @@ cudaError_t ensure_grid_attributes() {
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
   const int most = static_cast<int>(kSmemMax);
+  const int spread = static_cast<int>(sizeof(SpreadWarp) * kSpreadWarps);
+  e = cudaFuncSetAttribute(grid_spread_kernel<kB>, cudaFuncAttributeMaxDynamicSharedMemorySize, spread);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_spread_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, spread);
+  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(grid_fft_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
@@ -1007,8 +1031,15 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
       grid_entry_kernel<<<(p.nent + 3) / 4, 128, 0, stream>>>(A, z0, nze, pass == 0);
     }
     const int planes = (z1 - z0 + 31) / 32 * 32;
-    grid_spread_kernel<<<dim3(task_blocks + (nbins + 7) / 8, planes / 32), 256, 0, stream>>>(A, task_blocks, zoff, p.zc);
-    grid_parts_kernel<<<dim3(std::min(p.maxslots, 148), planes / 32), 512, 0, stream>>>(A, p.zc);
+    const dim3 gs(task_blocks + (nbins + kSpreadWarps - 1) / kSpreadWarps, planes / 32);
+    const dim3 gp(std::min(p.maxslots, 148), planes / 32);
+    if (p.ny > 1) {
+      grid_spread_kernel<kB><<<gs, 32 * kSpreadWarps, sizeof(SpreadWarp) * kSpreadWarps, stream>>>(A, task_blocks, zoff, p.zc);
+      grid_parts_kernel<kB><<<gp, 32 * kB * kB, 0, stream>>>(A, p.zc);
+    } else {
+      grid_spread_kernel<1><<<gs, 32 * kSpreadWarps, sizeof(SpreadWarp) * kSpreadWarps, stream>>>(A, task_blocks, zoff, p.zc);
+      grid_parts_kernel<1><<<gp, 32 * kB, 0, stream>>>(A, p.zc);
+    }
     const long long groups = planes / kZT;
     if (p.ny > 1) {
       const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * (p.mx / 2 + 1));

@@ -18,9 +18,10 @@
 //      normalisation), then c2r along x, by cuFFT; the imaginary parts of the
 //      x bins 0 and n1/2, which a c2r transform does not use, are cleared
 //      before it so that every c2r implementation reads the same input.
-//   4. scaling by 1 / sqrt(n1 n2 n3 dh^n) (:1019), with per-block statistics
-//      records of the scaled values (the mean/variance of the internal grid,
-//      :1027-1036), merged in record order.
+//   4. per-block statistics records of the values scaled by
+//      1 / sqrt(n1 n2 n3 dh^n) (:1019; the mean/variance of the internal grid,
+//      :1027-1036), merged in record order; the scaling itself is applied by
+//      the next step that reads the values.
 //   5. rescale and taper on the internal grid (:1038-1070) in one pass.
 //   6. each external point takes the value of its nearest internal node
 //      (grid_mapping / order_points / interpolate, :1110-1699, 3086-3162),
@@ -56,24 +57,24 @@ constexpr int kRowsPerWarp = 8;
 __device__ uint32_t g_fim_pow[kPowWords];
 // c_jump[b] = A^(2^b), c_lane[l] = A^(l + 1), c_step = A^32; each row-major
 // {a, b, c, d} for [[a, b], [c, d]] acting on the state (r0, r1).
-__constant__ uint64_t c_jump[kJumpBits][4];
-__constant__ uint64_t c_lane[32][4];
-__constant__ uint64_t c_step[4];
+__constant__ uint32_t c_jump[kJumpBits][4];
+__constant__ uint32_t c_lane[32][4];
+__constant__ uint32_t c_step[4];
 
 struct State {
-  uint64_t r0, r1;
+  uint32_t r0, r1;
 };
 
-__device__ __forceinline__ State apply(const uint64_t* M, State s) {
-  return State{addmod(mulmod(M[0], s.r0), mulmod(M[1], s.r1)), addmod(mulmod(M[2], s.r0), mulmod(M[3], s.r1))};
+__device__ __forceinline__ State apply(const uint32_t* M, State s) {
+  return State{sub_m(mulmod32(M[0], s.r0) + mulmod32(M[1], s.r1)), sub_m(mulmod32(M[2], s.r0) + mulmod32(M[3], s.r1))};
 }
 
 struct SpecArgs {
   int n1, n2, n3, n1h;
   float dk1, dk2, dk3, kc, nu, cnst, cl1, cl2, cl3;
   int filter, acf;
-  uint64_t s0, s1;        // state after seeding
-  uint64_t row_step[4];   // A^n1: one row of draws
+  uint32_t s0, s1;        // state after seeding
+  uint32_t row_step[4];   // A^n1: one row of draws
   float2* spec;           // [n3][n2][n1h]
 };
 
@@ -83,54 +84,69 @@ __device__ __forceinline__ float axis_k(int t, int n, float dk) {
   return __fmul_rn(static_cast<float>(t <= n / 2 ? t : n - t), dk);
 }
 
+// One warp per run of rows along x in the planes k and n3 - k, whose
+// amplitudes are the same: two generators, one amplitude. Lane l takes the
+// points i = l + 32 t. Bound: instruction issue (two modular matrix steps,
+// two outputs and two sine-cosine pairs per amplitude). The generator's
+// products in 64-bit arithmetic and an amplitude per point took 1.20 ms on
+// the 514^3 grid.
 __global__ void __launch_bounds__(256) fim_spectrum_kernel(const SpecArgs A) {
   __shared__ uint32_t sp[kPowWords];
   for (int i = threadIdx.x; i < kPowWords; i += blockDim.x) sp[i] = g_fim_pow[i];
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long rows = static_cast<long long>(A.n2) * A.n3;
-  const long long r0 = warp * kRowsPerWarp;
-  if (r0 >= rows) return;
-  // State at the first draw of this lane in row r0: A^(r0 n1) then A^(l + 1).
-  State st{A.s0, A.s1};
-  const unsigned long long skip = static_cast<unsigned long long>(r0) * A.n1;
-  for (int b = 0; b < kJumpBits; ++b)
-    if ((skip >> b) & 1ull) st = apply(c_jump[b], st);
-  st = apply(c_lane[lane], st);
-  const float pi2 = 2.0f;
-  for (long long r = r0; r < r0 + kRowsPerWarp && r < rows; ++r) {
-    const int k = static_cast<int>(r / A.n2);
-    const int j = static_cast<int>(r - static_cast<long long>(k) * A.n2);
-    const float ky = axis_k(j, A.n2, A.dk2), kz = axis_k(k, A.n3, A.dk3);
-    const float kyy = __fmul_rn(ky, ky), kzz = __fmul_rn(kz, kz);
-    const float ay = __fmul_rn(ky, A.cl2), az = __fmul_rn(kz, A.cl3);
-    const float ayy = __fmul_rn(ay, ay), azz = __fmul_rn(az, az);
-    State s = st;
-    float2* out = A.spec + r * A.n1h;
+  const int runs = (A.n2 + kRowsPerWarp - 1) / kRowsPerWarp;  // runs of rows per plane
+  const int k = static_cast<int>(warp / runs);
+  if (k > A.n3 / 2) return;
+  const int j0 = static_cast<int>(warp - static_cast<long long>(k) * runs) * kRowsPerWarp;
+  const int km = k == 0 ? 0 : A.n3 - k;  // the mirrored plane
+  const bool two = km != k;
+  // State at the first draw of this lane in row (j0, k): A^(row n1), A^(l + 1).
+  auto first = [&](int plane) {
+    State st{A.s0, A.s1};
+    const unsigned long long skip = (static_cast<unsigned long long>(plane) * A.n2 + j0) * A.n1;
+    for (int b = 0; b < kJumpBits; ++b)
+      if ((skip >> b) & 1ull) st = apply(c_jump[b], st);
+    return apply(c_lane[lane], st);
+  };
+  State sa = first(k), sb = two ? first(km) : sa;
+  const float kz = axis_k(k, A.n3, A.dk3), kzz = __fmul_rn(kz, kz);
+  const float az = __fmul_rn(kz, A.cl3), azz = __fmul_rn(az, az);
+  const uint32_t step[4] = {c_step[0], c_step[1], c_step[2], c_step[3]};
+  // cos and sin of 2 pi u, times the amplitude
+  auto wave = [&](const State& s, float amp) {
+    const uint32_t x = s.r0;
+    const uint32_t y = mulmod3(sp[x & 2047u], sp[kPow0 + ((x >> 11) & 2047u)], sp[kPow0 + kPow1 + (x >> 22)]);
+    const float u = to_u01(x == 0 ? 0u : y);
+    float sn, cs;
+    sincospif(__fmul_rn(u, 2.0f), &sn, &cs);
+    return make_float2(__fmul_rn(cs, amp), __fmul_rn(sn, amp));
+  };
+  for (int j = j0; j < j0 + kRowsPerWarp && j < A.n2; ++j) {
+    const float ky = axis_k(j, A.n2, A.dk2), kyy = __fmul_rn(ky, ky);
+    const float ay = __fmul_rn(ky, A.cl2), ayy = __fmul_rn(ay, ay);
+    State a = sa, b = sb;
+    float2* out_a = A.spec + (static_cast<long long>(k) * A.n2 + j) * A.n1h;
+    float2* out_b = A.spec + (static_cast<long long>(km) * A.n2 + j) * A.n1h;
     for (int i = lane; i < A.n1h; i += 32) {
-      const uint32_t x = static_cast<uint32_t>(s.r0);
-      const uint32_t y = x == 0 ? 0u
-                                : mulmod3(sp[x & 2047u], sp[kPow0 + ((x >> 11) & 2047u)], sp[kPow0 + kPow1 + (x >> 22)]);
-      const float u = to_u01(y);
       const float kx = __fmul_rn(static_cast<float>(i), A.dk1);  // i <= n1/2 on the half grid
-      const float kr = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(kx, kx), kyy), kzz));
-      const float butter = (A.filter && kr > A.kc) ? 0.0f : 1.0f;
-      const float ax = __fmul_rn(kx, A.cl1);
-      const float kr2 = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(ax, ax), ayy), azz));
-      float fv;
-      if (A.acf == 0)
-        fv = __fdiv_rn(1.0f, powf(__fadd_rn(1.0f, __fmul_rn(kr2, kr2)), A.nu));
-      else
-        fv = expf(__fmul_rn(-0.25f, __fmul_rn(kr2, kr2)));
-      const float amp = __fmul_rn(__fsqrt_rn(__fmul_rn(A.cnst, fv)), butter);
-      const float h = __fmul_rn(__fmul_rn(u, pi2), kPiF);
-      float sn, cs;
-      sincosf(h, &sn, &cs);
-      out[i] = make_float2(__fmul_rn(cs, amp), __fmul_rn(sn, amp));
-      s = apply(c_step, s);
+      float amp = 0.0f;
+      if (!(A.filter && __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(kx, kx), kyy), kzz)) > A.kc)) {
+        const float ax = __fmul_rn(kx, A.cl1);
+        const float q = __fadd_rn(__fadd_rn(__fmul_rn(ax, ax), ayy), azz);
+        const float fv = A.acf == 0 ? __fdiv_rn(1.0f, powf(__fadd_rn(1.0f, q), A.nu)) : expf(__fmul_rn(-0.25f, q));
+        amp = __fsqrt_rn(__fmul_rn(A.cnst, fv));
+      }
+      out_a[i] = wave(a, amp);
+      a = apply(step, a);
+      if (two) {
+        out_b[i] = wave(b, amp);
+        b = apply(step, b);
+      }
     }
-    st = apply(A.row_step, st);
+    sa = apply(A.row_step, sa);
+    if (two) sb = apply(A.row_step, sb);
   }
 }
 
@@ -182,57 +198,59 @@ __global__ void fim_clear_imag_kernel(float2* spec, int n1h, long long rows, int
   spec[r * n1h + i].y = 0.0f;
 }
 
-// Scaling of the transform's real output, with one statistics record per
-// block (count, mean, M2 of the scaled values, FP64). A block covers
-// kScaleThreads * kScaleRun values as kScaleRun / 4 coalesced float4 sweeps;
-// each thread sums its values about its first one before the warp and block
-// merges (a fixed order, so the records are deterministic).
-constexpr int kScaleRun = 16;
-constexpr int kScaleThreads = 256;
+// Statistics of the transform's real output times `scaling` (FP64, one record
+// per block, merged in record order). The values themselves are scaled where
+// they are next read (mapping, or rescale and taper): writing them back here
+// cost 0.13 ms of 0.23 on the 514^3 grid. Blocks stride over pieces of
+// kStatThreads * 16 values as four coalesced float4 sweeps; each thread sums
+// about its first value in a fixed order, so the records are deterministic.
+constexpr int kStatRun = 16;
+constexpr int kStatThreads = 256;
+constexpr int kStatBlocks = 148 * 8;
 
-__global__ void __launch_bounds__(kScaleThreads) fim_scale_kernel(float* f, long long n, float scaling, Moments* rec) {
-  __shared__ Moments s_warp[kScaleThreads / 32];
-  const long long base = static_cast<long long>(blockIdx.x) * kScaleThreads * kScaleRun;
-  double cnt = 0.0, s1 = 0.0, s2 = 0.0, shift = 0.0;
-  bool have = false;
-  auto take = [&](float v) {
-    if (!have) {
-      shift = v;
-      have = true;
-    }
-    const double d = static_cast<double>(v) - shift;
-    s1 += d;
-    s2 = fma(d, d, s2);
-    cnt += 1.0;
+__global__ void __launch_bounds__(kStatThreads) fim_stats_kernel(const float* __restrict__ f, long long n, float scaling,
+                                                                 Moments* rec) {
+  __shared__ Moments s_warp[kStatThreads / 32];
+  double s1[4] = {0.0, 0.0, 0.0, 0.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};
+  long long count = 0;
+  const double shift = __fmul_rn(f[min(n - 1, (static_cast<long long>(blockIdx.x) * kStatThreads + threadIdx.x) * 4)], scaling);
+  auto take = [&](float v, int c) {
+    const double d = static_cast<double>(__fmul_rn(v, scaling)) - shift;
+    s1[c] += d;
+    s2[c] = fma(d, d, s2[c]);
   };
+  const long long piece = static_cast<long long>(kStatThreads) * kStatRun;
+  for (long long base = blockIdx.x * piece; base < n; base += gridDim.x * piece) {
+    float4 v[kStatRun / 4];
 #pragma unroll
-  for (int q = 0; q < kScaleRun / 4; ++q) {
-    const long long p = base + (static_cast<long long>(q) * kScaleThreads + threadIdx.x) * 4;
-    if (p + 4 <= n) {
-      float4 v = *reinterpret_cast<const float4*>(f + p);
-      v.x = __fmul_rn(v.x, scaling);
-      v.y = __fmul_rn(v.y, scaling);
-      v.z = __fmul_rn(v.z, scaling);
-      v.w = __fmul_rn(v.w, scaling);
-      *reinterpret_cast<float4*>(f + p) = v;
-      take(v.x);
-      take(v.y);
-      take(v.z);
-      take(v.w);
-    } else {
-      for (long long e = p; e < n && e < p + 4; ++e) {
-        const float v = __fmul_rn(f[e], scaling);
-        f[e] = v;
-        take(v);
+    for (int q = 0; q < kStatRun / 4; ++q) {
+      const long long p = base + (static_cast<long long>(q) * kStatThreads + threadIdx.x) * 4;
+      if (p + 4 <= n) v[q] = __ldg(reinterpret_cast<const float4*>(f + p));
+    }
+#pragma unroll
+    for (int q = 0; q < kStatRun / 4; ++q) {
+      const long long p = base + (static_cast<long long>(q) * kStatThreads + threadIdx.x) * 4;
+      if (p + 4 <= n) {
+        take(v[q].x, 0);
+        take(v[q].y, 1);
+        take(v[q].z, 2);
+        take(v[q].w, 3);
+        count += 4;
+      } else {
+        for (long long e = p; e < n && e < p + 4; ++e) {
+          take(f[e], 0);
+          ++count;
+        }
       }
     }
   }
-  Moments mo = warp_moments(moments_from_shifted(cnt, shift, s1, s2));
+  Moments mo = warp_moments(moments_from_shifted(static_cast<double>(count), shift, (s1[0] + s1[1]) + (s1[2] + s1[3]),
+                                                 (s2[0] + s2[1]) + (s2[2] + s2[3])));
   if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = mo;
   __syncthreads();
   if (threadIdx.x == 0) {
     Moments b = s_warp[0];
-    for (int w = 1; w < kScaleThreads / 32; ++w) b = moments_merge(b, s_warp[w]);
+    for (int w = 1; w < kStatThreads / 32; ++w) b = moments_merge(b, s_warp[w]);
     rec[blockIdx.x] = b;
   }
 }
@@ -242,6 +260,7 @@ struct MapArgs {
   float dh;
   float o1, o2, o3;     // off_axis
   const float* delta;   // internal field, x fastest
+  float scaling;        // of delta's values (1: they are final)
   // structured external grid (x null): fs - 1 and extents, step ds
   int f1, f2, f3, e1, e2;
   float ds;
@@ -250,40 +269,55 @@ struct MapArgs {
   long long n;
 };
 
-// Nearest internal node of one external point: NINT of (P / dh + 3) - 1 in
-// the reference's 1-based index space of delta(0:n1, 0:n2, 0:n3), 0 = halo.
-__device__ __forceinline__ float map_value(const MapArgs& A, float px, float py, float pz) {
-  const float fi = __fsub_rn(__fadd_rn(__fdiv_rn(px, A.dh), 3.0f), 1.0f);
-  const float fj = __fsub_rn(__fadd_rn(__fdiv_rn(py, A.dh), 3.0f), 1.0f);
-  const float fk = __fsub_rn(__fadd_rn(__fdiv_rn(pz, A.dh), 3.0f), 1.0f);
-  if (!(fi >= 1.0f && fi < static_cast<float>(A.n1 + 1) && fj >= 1.0f && fj < static_cast<float>(A.n2 + 1) &&
-        fk >= 1.0f && fk < static_cast<float>(A.n3 + 1)))
-    return 0.0f;
-  const int a = static_cast<int>(roundf(fi)) - 1, b = static_cast<int>(roundf(fj)) - 1;
-  int c = static_cast<int>(roundf(fk)) - 1;
-  if (a == 0 || b == 0) return 0.0f;  // halo below x and y: zero (no neighbour)
-  if (c == 0) c = A.n3;               // halo below z: the last plane (periodic)
-  return A.delta[(a - 1) + static_cast<long long>(A.n1) * ((b - 1) + static_cast<long long>(A.n2) * (c - 1))];
+// Nearest internal node along one axis of n points of an external coordinate:
+// NINT of (p / dh + 3) - 1 in the reference's 1-based index space of
+// delta(0:n), 0 = halo; -1 outside.
+__device__ __forceinline__ int axis_node(float p, float dh, int n) {
+  const float f = __fsub_rn(__fadd_rn(__fdiv_rn(p, dh), 3.0f), 1.0f);
+  if (!(f >= 1.0f && f < static_cast<float>(n + 1))) return -1;
+  return static_cast<int>(roundf(f)) - 1;
+}
+// The value at nodes (a, b, c): zero outside and in the halo below x and y
+// (no neighbour), the last plane in the halo below z (periodic).
+__device__ __forceinline__ float node_value(const MapArgs& A, int a, int b, int c) {
+  if (a <= 0 || b <= 0 || c < 0) return 0.0f;
+  if (c == 0) c = A.n3;
+  return __fmul_rn(A.delta[(a - 1) + static_cast<long long>(A.n1) * ((b - 1) + static_cast<long long>(A.n2) * (c - 1))],
+                   A.scaling);
 }
 
 // Point sets: one thread per point.
 __global__ void fim_map_points_kernel(const MapArgs A) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long p = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; p < A.n; p += stride)
-    A.field[p] = map_value(A, __fsub_rn(A.x[p], A.o1), __fsub_rn(A.y[p], A.o2), __fsub_rn(A.z[p], A.o3));
+    A.field[p] = node_value(A, axis_node(__fsub_rn(A.x[p], A.o1), A.dh, A.n1), axis_node(__fsub_rn(A.y[p], A.o2), A.dh, A.n2),
+                            axis_node(__fsub_rn(A.z[p], A.o3), A.dh, A.n3));
 }
 
-// Structured grids: blocks along x, rows (j, k) over blockIdx.y; each row's
-// y and z coordinates are computed once, x per thread.
-__global__ void fim_map_grid_kernel(const MapArgs A, int rows) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.e1) return;
-  const float px = __fsub_rn(__fmul_rn(static_cast<float>(A.f1 + i), A.ds), A.o1);
+// Structured grids: a block keeps the nodes of up to kMapRun points along x
+// per thread and strides over the rows (j, k). One row per block with every
+// coordinate mapped per point took 0.49 ms at 512^3 (2.2 TB/s).
+constexpr int kMapRun = 4;
+constexpr int kMapThreads = 128;
+__global__ void __launch_bounds__(kMapThreads) fim_map_grid_kernel(const MapArgs A, int rows) {
+  int a[kMapRun];
+  const int i0 = blockIdx.x * kMapThreads * kMapRun + threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kMapRun; ++q) {
+    const int i = i0 + q * kMapThreads;
+    a[q] = axis_node(__fsub_rn(__fmul_rn(static_cast<float>(A.f1 + i), A.ds), A.o1), A.dh, A.n1);
+  }
   for (int row = blockIdx.y; row < rows; row += gridDim.y) {
     const int k = row / A.e2, j = row - k * A.e2;
-    const float py = __fsub_rn(__fmul_rn(static_cast<float>(A.f2 + j), A.ds), A.o2);
-    const float pz = __fsub_rn(__fmul_rn(static_cast<float>(A.f3 + k), A.ds), A.o3);
-    A.field[static_cast<long long>(row) * A.e1 + i] = map_value(A, px, py, pz);
+    const int b = axis_node(__fsub_rn(__fmul_rn(static_cast<float>(A.f2 + j), A.ds), A.o2), A.dh, A.n2);
+    const int c = axis_node(__fsub_rn(__fmul_rn(static_cast<float>(A.f3 + k), A.ds), A.o3), A.dh, A.n3);
+    float* out = A.field + static_cast<long long>(row) * A.e1;
+    float v[kMapRun];
+#pragma unroll
+    for (int q = 0; q < kMapRun; ++q) v[q] = i0 + q * kMapThreads < A.e1 ? node_value(A, a[q], b, c) : 0.0f;
+#pragma unroll
+    for (int q = 0; q < kMapRun; ++q)
+      if (i0 + q * kMapThreads < A.e1) out[i0 + q * kMapThreads] = v[q];
   }
 }
 
@@ -392,18 +426,21 @@ cudaError_t ensure_fim_tables() {
   static const std::vector<uint32_t> pw = device_pow_tables();
   e = cudaMemcpyToSymbol(g_fim_pow, pw.data(), sizeof(uint32_t) * pw.size());
   if (e != cudaSuccess) return e;
-  uint64_t jump[kJumpBits][4], lane[32][4], step[4];
+  uint32_t jump[kJumpBits][4], lane[32][4], step[4];
+  auto put = [](uint32_t* to, const Mat& m) {
+    for (int q = 0; q < 4; ++q) to[q] = static_cast<uint32_t>(m.v[q]);
+  };
   Mat p = kStepMat;
   for (int b = 0; b < kJumpBits; ++b) {
-    std::memcpy(jump[b], p.v, sizeof(p.v));
+    put(jump[b], p);
     p = mat_mul(p, p);
   }
   Mat q = kStepMat;
   for (int l = 0; l < 32; ++l) {
-    std::memcpy(lane[l], q.v, sizeof(q.v));
+    put(lane[l], q);
     q = mat_mul(q, kStepMat);
   }
-  std::memcpy(step, mat_pow(kStepMat, 32).v, sizeof(step));
+  put(step, mat_pow(kStepMat, 32));
   if ((e = cudaMemcpyToSymbol(c_jump, jump, sizeof(jump))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_lane, lane, sizeof(lane))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_step, step, sizeof(step))) != cudaSuccess) return e;
@@ -454,7 +491,7 @@ FimLayout fim_layout(const FimGrid& g, int npoi) {
   L.n1h = g.npts[0] / 2 + 1;
   L.rows = static_cast<long long>(g.npts[1]) * g.npts[2];
   L.real = static_cast<long long>(g.npts[0]) * L.rows;
-  L.nrec = (L.real + kScaleThreads * kScaleRun - 1) / (kScaleThreads * kScaleRun);
+  L.nrec = std::min<long long>(kStatBlocks, (L.real + kStatThreads * kStatRun - 1) / (kStatThreads * kStatRun));
   size_t off = 0;
   L.off_spec = off;
   off = align256(off + sizeof(float2) * static_cast<size_t>(L.n1h * L.rows));
@@ -528,11 +565,12 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   A.acf = in.acf;
   Yarn2 y;
   y.seed(in.seed);
-  A.s0 = y.r0, A.s1 = y.r1;
-  std::memcpy(A.row_step, mat_pow(kStepMat, static_cast<unsigned long long>(n1)).v, sizeof(A.row_step));
+  A.s0 = static_cast<uint32_t>(y.r0), A.s1 = static_cast<uint32_t>(y.r1);
+  const Mat row = mat_pow(kStepMat, static_cast<unsigned long long>(n1));
+  for (int q = 0; q < 4; ++q) A.row_step[q] = static_cast<uint32_t>(row.v[q]);
   A.spec = spec;
   cudaEventRecord(ev[0], st);
-  const long long warps = (L.rows + kRowsPerWarp - 1) / kRowsPerWarp;
+  const long long warps = static_cast<long long>((n2 + kRowsPerWarp - 1) / kRowsPerWarp) * (n3 / 2 + 1);
   fim_spectrum_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st>>>(A);
   if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_spectrum_kernel", e);
   cudaEventRecord(ev[1], st);
@@ -597,8 +635,8 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   const float dhn = in.ndim == 2 ? in.dh * in.dh : (in.dh * in.dh) * in.dh;
   const float scaling = 1.0f / std::sqrt(((static_cast<float>(n1) * static_cast<float>(n2)) * static_cast<float>(n3)) *
                                          dhn);
-  fim_scale_kernel<<<static_cast<unsigned>(L.nrec), kScaleThreads, 0, st>>>(real, L.real, scaling, rec);
-  if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_scale_kernel", e);
+  fim_stats_kernel<<<static_cast<unsigned>(L.nrec), kStatThreads, 0, st>>>(real, L.real, scaling, rec);
+  if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_stats_kernel", e);
   if ((e = launch_stats_records(rec, L.nrec, d_out, st)) != cudaSuccess) return failed("statistics", e);
   float mv[2];
   if ((e = cudaMemcpyAsync(mv, d_out, sizeof(mv), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
@@ -610,8 +648,11 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   stats[3] = mv[0];
   // 5. rescale and taper on the internal grid.
   std::vector<float> pt;
+  float pending = scaling;  // scaling not yet applied to the internal field
   if (in.rescale == 1 || in.npoi > 0) {
     FinalizeArgs fa{};
+    fa.prescale = scaling;
+    pending = 1.0f;
     if (in.rescale == 1) {
       fa.rescale = 1;
       fa.scaling = in.sigma / stats[2];
@@ -642,6 +683,7 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   M.dh = in.dh;
   M.o1 = g.off_axis[0], M.o2 = g.off_axis[1], M.o3 = g.off_axis[2];
   M.delta = real;
+  M.scaling = pending;
   M.field = d_field;
   if (in.structured) {
     M.f1 = in.fs[0] - 1, M.f2 = in.fs[1] - 1, M.f3 = in.fs[2] - 1;
@@ -654,8 +696,9 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   }
   if (in.structured) {
     const int rows = M.e2 * (in.fe[2] - in.fs[2] + 1);
-    const dim3 grid((M.e1 + 127) / 128, static_cast<unsigned>(std::min(rows, 65535)));
-    fim_map_grid_kernel<<<grid, 128, 0, st>>>(M, rows);
+    const unsigned gx = static_cast<unsigned>((M.e1 + kMapThreads * kMapRun - 1) / (kMapThreads * kMapRun));
+    const dim3 grid(gx, static_cast<unsigned>(std::min<long long>(rows, std::max(1u, 148u * 16u / gx))));
+    fim_map_grid_kernel<<<grid, kMapThreads, 0, st>>>(M, rows);
   } else {
     fim_map_points_kernel<<<blocks_for(M.n, 256), 256, 0, st>>>(M);
   }

@@ -278,6 +278,7 @@ cudaError_t launch_stats_records(const StatRecord* d_rec, long long count, float
 // Structured fields (d_x null) take coordinates (i + fs - 2) dh from the
 // index; point sets read d_x, d_y, d_z.
 struct FinalizeArgs {
+  float prescale;  // first factor of the values (0: none)
   int rescale;
   float scaling, mean;  // field * scaling - mean
   const float* d_poi;

@@ -150,6 +150,7 @@ __global__ void finalize_kernel(float* f, long long n, const FinalizeArgs a) {
   const long long plane = static_cast<long long>(a.n0) * a.n1;
   for (long long p = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += stride) {
     float v = f[p];
+    if (a.prescale != 0.0f) v = __fmul_rn(v, a.prescale);
     if (a.rescale) v = __fsub_rn(__fmul_rn(v, a.scaling), a.mean);
     if (a.npoi > 0) {
       float x, y, z;

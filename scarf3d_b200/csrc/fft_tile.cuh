@@ -234,19 +234,84 @@ __device__ __forceinline__ void stage(const FftPlan& f, int s, const float4* __r
     for (int t = 0; t < R; ++t) out(base + t * m, p, t, v[t]);
   }
 }
+// The last stage forwards, a product with hat[position] and the first stage
+// backwards (e^{-i}) in registers: a butterfly of the last stage holds what its
+// inverse needs.
+template <int R, int NP, class In, class Out>
+__device__ __forceinline__ void product(const FftPlan& f, const float4* __restrict__ hat, In in, Out out) {
+  for (int it = threadIdx.x; it < f.n / R * NP; it += blockDim.x) {
+    const int p = it & (NP - 1), base = it / NP * R;
+    C2 v[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = in(base + t, p);
+    Dft<R>::run(v);
+#pragma unroll
+    for (int t = 0; t < R; ++t) {
+      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(hat + base + t));
+      const C2 y = cmul(v[t], x.x, x.y);
+      v[t] = C2{y.im, y.re};  // the e^{-i} transform is the e^{+i} one with the parts exchanged
+    }
+    Dft<R>::run(v);
+#pragma unroll
+    for (int t = 0; t < R; ++t) out(base + t, p, t, C2{v[t].im, v[t].re});
+  }
+}
+// A stage of the e^{-i} transform by decimation in time: stage s undone.
+template <int R, int NP, class In, class Out>
+__device__ __forceinline__ void back(const FftPlan& f, int s, const float4* __restrict__ tw, In in, Out out) {
+  const int m = f.m[s], len = m * R;
+  const float inv_m = f.inv_m[s];
+  for (int it = threadIdx.x; it < f.n / R * NP; it += blockDim.x) {
+    const int p = it & (NP - 1), g = it / NP;
+    const int blk = static_cast<int>((static_cast<float>(g) + 0.5f) * inv_m);
+    const int q = g - blk * m, base = blk * len + q;
+    C2 v[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) {
+      const C2 x = in(base + t * m, p);
+      v[t] = C2{x.im, x.re};
+    }
+    const float4* w = tw + (f.n - len) + q;
+#pragma unroll
+    for (int t = 1; t < R; ++t, w += m) {
+      // conj(w) x with the parts exchanged is w times the exchanged x
+      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(w));
+      v[t] = cmul(v[t], x.x, x.y);
+    }
+    Dft<R>::run(v);
+#pragma unroll
+    for (int t = 0; t < R; ++t) out(base + t * m, p, t, C2{v[t].im, v[t].re});
+  }
+}
+#define SCARF_FFT_RADICES(CALL, r) \
+  switch (r) {                     \
+    case 12: CALL(12); break;      \
+    case 10: CALL(10); break;      \
+    case 9: CALL(9); break;        \
+    case 8: CALL(8); break;        \
+    case 6: CALL(6); break;        \
+    case 5: CALL(5); break;        \
+    case 4: CALL(4); break;        \
+    case 3: CALL(3); break;        \
+    default: CALL(2); break;       \
+  }
 template <int NP, class In, class Out>
 __device__ __forceinline__ void stage_any(const FftPlan& f, int s, const float4* tw, In in, Out out) {
-  switch (f.r[s]) {
-    case 12: stage<12, NP>(f, s, tw, in, out); break;
-    case 10: stage<10, NP>(f, s, tw, in, out); break;
-    case 9: stage<9, NP>(f, s, tw, in, out); break;
-    case 8: stage<8, NP>(f, s, tw, in, out); break;
-    case 6: stage<6, NP>(f, s, tw, in, out); break;
-    case 5: stage<5, NP>(f, s, tw, in, out); break;
-    case 4: stage<4, NP>(f, s, tw, in, out); break;
-    case 3: stage<3, NP>(f, s, tw, in, out); break;
-    default: stage<2, NP>(f, s, tw, in, out); break;
-  }
+#define SCARF_FFT_CALL(R) stage<R, NP>(f, s, tw, in, out)
+  SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[s])
+#undef SCARF_FFT_CALL
+}
+template <int NP, class In, class Out>
+__device__ __forceinline__ void product_any(const FftPlan& f, const float4* hat, In in, Out out) {
+#define SCARF_FFT_CALL(R) product<R, NP>(f, hat, in, out)
+  SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[f.nst - 1])
+#undef SCARF_FFT_CALL
+}
+template <int NP, class In, class Out>
+__device__ __forceinline__ void back_any(const FftPlan& f, int s, const float4* tw, In in, Out out) {
+#define SCARF_FFT_CALL(R) back<R, NP>(f, s, tw, in, out)
+  SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[s])
+#undef SCARF_FFT_CALL
 }
 
 // Twiddle i < n of a plan: for each stage, [t - 1][q] for t = 1 .. r - 1 and

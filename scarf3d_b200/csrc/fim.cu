@@ -15,13 +15,12 @@
 //      place instead of mirroring (its exchange sends only one of two
 //      subarrays; see fim_symmetry_kernel).
 //   3. inverse transform (:1705-2315): c2c along z and y (FFTW_BACKWARD, no
-//      normalisation), then c2r along x, by cuFFT; the imaginary parts of the
-//      x bins 0 and n1/2, which a c2r transform does not use, are cleared
-//      before it so that every c2r implementation reads the same input.
-//   4. per-block statistics records of the values scaled by
-//      1 / sqrt(n1 n2 n3 dh^n) (:1019; the mean/variance of the internal grid,
-//      :1027-1036), merged in record order; the scaling itself is applied by
-//      the next step that reads the values.
+//      normalisation), then c2r along x (fim_fft.cu; cuFFT for axes too long
+//      for shared memory).
+//   4. scaling by 1 / sqrt(n1 n2 n3 dh^n) (:1019) and statistics records of the
+//      scaled values (the mean/variance of the internal grid, :1027-1036),
+//      merged in record order: in the c2r step, or after cuFFT's in a pass of
+//      their own that leaves the scaling to the next reader.
 //   5. rescale and taper on the internal grid (:1038-1070) in one pass.
 //   6. each external point takes the value of its nearest internal node
 //      (grid_mapping / order_points / interpolate, :1110-1699, 3086-3162),
@@ -483,15 +482,18 @@ void fim_grid(const FimInputs& in, FimGrid* g) {
 namespace {
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 struct FimLayout {
-  size_t off_spec, off_real, off_rec, off_poi, off_out, bytes;
+  size_t off_spec, off_real, off_rec, off_poi, off_out, off_tables, bytes;
   long long n1h, rows, real, nrec;
+  bool own;  // this library's transform; else cuFFT
+  FimFft fft;
 };
 FimLayout fim_layout(const FimGrid& g, int npoi) {
   FimLayout L{};
   L.n1h = g.npts[0] / 2 + 1;
   L.rows = static_cast<long long>(g.npts[1]) * g.npts[2];
   L.real = static_cast<long long>(g.npts[0]) * L.rows;
-  L.nrec = std::min<long long>(kStatBlocks, (L.real + kStatThreads * kStatRun - 1) / (kStatThreads * kStatRun));
+  L.own = fim_fft_plan(g.npts, g.npts[2] > 1, &L.fft);
+  L.nrec = L.own ? fim_fft_records(L.fft) : std::min<long long>(kStatBlocks, (L.real + kStatThreads * kStatRun - 1) / (kStatThreads * kStatRun));
   size_t off = 0;
   L.off_spec = off;
   off = align256(off + sizeof(float2) * static_cast<size_t>(L.n1h * L.rows));
@@ -503,6 +505,8 @@ FimLayout fim_layout(const FimGrid& g, int npoi) {
   off = align256(off + sizeof(float) * 3 * static_cast<size_t>(std::max(npoi, 1)));
   L.off_out = off;  // mean, variance
   off = align256(off + 2 * sizeof(float));
+  L.off_tables = off;
+  if (L.own) off = align256(off + L.fft.tables);
   L.bytes = off;
   return L;
 }
@@ -517,7 +521,6 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
     *what = w;
     return e;
   };
-  if (!load_cufft()) return failed("cuFFT (libcufft.so.11) could not be loaded", cudaErrorSharedObjectInitFailed);
   cudaError_t e = ensure_fim_tables();
   if (e != cudaSuccess) return failed("FIM generator tables", e);
   const int n1 = g.npts[0], n2 = g.npts[1], n3 = g.npts[2];
@@ -578,65 +581,76 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   fim_symmetry_kernel<<<static_cast<unsigned>((2 * L.rows + 255) / 256), 256, 0, st>>>(spec, n1, n2, n3);
   if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_symmetry_kernel", e);
   cudaEventRecord(ev[2], st);
-  // 3. inverse transform: c2c along z and y (x bins as the batch), the
-  // unused imaginary parts of x bins 0 and n1/2 cleared, c2r along x.
-  const int n1h = static_cast<int>(L.n1h);
-  const bool three = in.ndim == 3 && n3 > 1;
-  // The plans: this device's cached pair when the grid matches, else new
-  // ones (cached for the next call; on devices beyond the cache, freed on
-  // return).
-  int dev = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return failed("cudaGetDevice", e);
-  const unsigned long long ctx = current_context_id();
-  const bool cacheable = dev < kPlanDevices && ctx != 0;
-  FimPlans local;
-  FimPlans& P = cacheable ? g_fim_plans[dev] : local;
-  struct LocalGuard {
-    FimPlans* p;
-    ~LocalGuard() { destroy_plans(*p); }
-  } lg{&local};
-  if (cacheable && P.ctx != ctx) P = FimPlans();  // handles of a reset context are dropped
-  if (P.yz && !(P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.three == (three ? 1 : 0))) destroy_plans(P);
-  if (!P.yz) {
-    FimPlans fresh;
-    struct FreshGuard {
-      FimPlans* p;
-      bool keep = false;
-      ~FreshGuard() {
-        if (!keep) destroy_plans(*p);
-      }
-    } fg{&fresh};
-    int dims3[2] = {n3, n2}, dims2[1] = {n2};
-    int* dims = three ? dims3 : dims2;
-    const int rank = three ? 2 : 1;
-    if (g_cufft.plan_many(&fresh.yz, rank, dims, dims, n1h, 1, dims, n1h, 1, CUFFT_C2C, n1h) != CUFFT_SUCCESS)
-      return failed("cufftPlanMany (z, y)", cudaErrorUnknown);
-    int dx[1] = {n1}, ex[1] = {n1h}, ox[1] = {n1};
-    if (g_cufft.plan_many(&fresh.x, 1, dx, ex, 1, n1h, ox, 1, n1, CUFFT_C2R, static_cast<int>(L.rows)) !=
-        CUFFT_SUCCESS)
-      return failed("cufftPlanMany (x)", cudaErrorUnknown);
-    fresh.ctx = ctx;
-    fresh.n1 = n1, fresh.n2 = n2, fresh.n3 = n3, fresh.three = three ? 1 : 0;
-    P = fresh;
-    fg.keep = true;
-  }
-  const cufftHandle p_yz = P.yz, p_x = P.x;
-  {
-    if (g_cufft.set_stream(p_yz, st) != CUFFT_SUCCESS || g_cufft.set_stream(p_x, st) != CUFFT_SUCCESS)
-      return failed("cufftSetStream", cudaErrorUnknown);
-    cufftComplex* c = reinterpret_cast<cufftComplex*>(spec);
-    if (g_cufft.exec_c2c(p_yz, c, c, CUFFT_INVERSE) != CUFFT_SUCCESS) return failed("cufftExecC2C", cudaErrorUnknown);
-    fim_clear_imag_kernel<<<static_cast<unsigned>((2 * L.rows + 255) / 256), 256, 0, st>>>(spec, n1h, L.rows, n1 / 2);
-    if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_clear_imag_kernel", e);
-    if (g_cufft.exec_c2r(p_x, c, real) != CUFFT_SUCCESS) return failed("cufftExecC2R", cudaErrorUnknown);
-  }
-  cudaEventRecord(ev[3], st);
-  // 4. scaling 1 / sqrt(n1 n2 n3 dh^n) and statistics of the internal grid.
+  // 3. inverse transform, scaled by 1 / sqrt(n1 n2 n3 dh^n), and statistics of
+  // the internal grid.
   const float dhn = in.ndim == 2 ? in.dh * in.dh : (in.dh * in.dh) * in.dh;
   const float scaling = 1.0f / std::sqrt(((static_cast<float>(n1) * static_cast<float>(n2)) * static_cast<float>(n3)) *
                                          dhn);
-  fim_stats_kernel<<<static_cast<unsigned>(L.nrec), kStatThreads, 0, st>>>(real, L.real, scaling, rec);
-  if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_stats_kernel", e);
+  float pending = 1.0f;  // scaling not yet applied to the internal field
+  if (L.own) {
+    if ((e = launch_fim_fft(L.fft, spec, real, w + L.off_tables, scaling, rec, st)) != cudaSuccess)
+      return failed("FIM transform", e);
+    cudaEventRecord(ev[3], st);
+  } else {
+    // Axes beyond shared memory: cuFFT, c2c along z and y (x bins as the
+    // batch), the unused imaginary parts of x bins 0 and n1/2 cleared, c2r
+    // along x.
+    if (!load_cufft()) return failed("cuFFT (libcufft.so.11) could not be loaded", cudaErrorSharedObjectInitFailed);
+    pending = scaling;
+    const int n1h = static_cast<int>(L.n1h);
+    const bool three = in.ndim == 3 && n3 > 1;
+    // The plans: this device's cached pair when the grid matches, else new
+    // ones (cached for the next call; on devices beyond the cache, freed on
+    // return).
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return failed("cudaGetDevice", e);
+    const unsigned long long ctx = current_context_id();
+    const bool cacheable = dev < kPlanDevices && ctx != 0;
+    FimPlans local;
+    FimPlans& P = cacheable ? g_fim_plans[dev] : local;
+    struct LocalGuard {
+      FimPlans* p;
+      ~LocalGuard() { destroy_plans(*p); }
+    } lg{&local};
+    if (cacheable && P.ctx != ctx) P = FimPlans();  // handles of a reset context are dropped
+    if (P.yz && !(P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.three == (three ? 1 : 0))) destroy_plans(P);
+    if (!P.yz) {
+      FimPlans fresh;
+      struct FreshGuard {
+        FimPlans* p;
+        bool keep = false;
+        ~FreshGuard() {
+          if (!keep) destroy_plans(*p);
+        }
+      } fg{&fresh};
+      int dims3[2] = {n3, n2}, dims2[1] = {n2};
+      int* dims = three ? dims3 : dims2;
+      const int rank = three ? 2 : 1;
+      if (g_cufft.plan_many(&fresh.yz, rank, dims, dims, n1h, 1, dims, n1h, 1, CUFFT_C2C, n1h) != CUFFT_SUCCESS)
+        return failed("cufftPlanMany (z, y)", cudaErrorUnknown);
+      int dx[1] = {n1}, ex[1] = {n1h}, ox[1] = {n1};
+      if (g_cufft.plan_many(&fresh.x, 1, dx, ex, 1, n1h, ox, 1, n1, CUFFT_C2R, static_cast<int>(L.rows)) !=
+          CUFFT_SUCCESS)
+        return failed("cufftPlanMany (x)", cudaErrorUnknown);
+      fresh.ctx = ctx;
+      fresh.n1 = n1, fresh.n2 = n2, fresh.n3 = n3, fresh.three = three ? 1 : 0;
+      P = fresh;
+      fg.keep = true;
+    }
+    const cufftHandle p_yz = P.yz, p_x = P.x;
+    {
+      if (g_cufft.set_stream(p_yz, st) != CUFFT_SUCCESS || g_cufft.set_stream(p_x, st) != CUFFT_SUCCESS)
+        return failed("cufftSetStream", cudaErrorUnknown);
+      cufftComplex* c = reinterpret_cast<cufftComplex*>(spec);
+      if (g_cufft.exec_c2c(p_yz, c, c, CUFFT_INVERSE) != CUFFT_SUCCESS) return failed("cufftExecC2C", cudaErrorUnknown);
+      fim_clear_imag_kernel<<<static_cast<unsigned>((2 * L.rows + 255) / 256), 256, 0, st>>>(spec, n1h, L.rows, n1 / 2);
+      if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_clear_imag_kernel", e);
+      if (g_cufft.exec_c2r(p_x, c, real) != CUFFT_SUCCESS) return failed("cufftExecC2R", cudaErrorUnknown);
+    }
+    cudaEventRecord(ev[3], st);
+    fim_stats_kernel<<<static_cast<unsigned>(L.nrec), kStatThreads, 0, st>>>(real, L.real, scaling, rec);
+    if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_stats_kernel", e);
+  }
   if ((e = launch_stats_records(rec, L.nrec, d_out, st)) != cudaSuccess) return failed("statistics", e);
   float mv[2];
   if ((e = cudaMemcpyAsync(mv, d_out, sizeof(mv), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
@@ -648,10 +662,9 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   stats[3] = mv[0];
   // 5. rescale and taper on the internal grid.
   std::vector<float> pt;
-  float pending = scaling;  // scaling not yet applied to the internal field
   if (in.rescale == 1 || in.npoi > 0) {
     FinalizeArgs fa{};
-    fa.prescale = scaling;
+    if (pending != 1.0f) fa.prescale = pending;
     pending = 1.0f;
     if (in.rescale == 1) {
       fa.rescale = 1;

@@ -763,7 +763,10 @@ bool factor(int rest, int most, int depth, int* r, int* best, int* nbest) {
     }
   return *nbest > 0;
 }
+}  // namespace
+
 bool fft_plan(int n, FftPlan* f) {
+  if (n < 4) return false;
   int rest = n;
   for (int k : {2, 3, 5})
     while (rest % k == 0) rest /= k;
@@ -782,6 +785,8 @@ bool fft_plan(int n, FftPlan* f) {
 }
 
 constexpr size_t kSmemMax = 224 * 1024;  // dynamic; the kernels keep a little static shared memory
+
+namespace {
 
 // Launch shape of a transform kernel: two tile buffers where they fit, and
 // the block size that fills an SM's registers (kFftMaxThreads threads) with

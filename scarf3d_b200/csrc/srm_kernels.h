@@ -182,6 +182,8 @@ struct FftPlan {
   float inv_m[kMaxStages];
 };
 
+// False when n has a prime factor above 5 or fewer than two stages.
+bool fft_plan(int n, FftPlan* f);
 struct GridPlan {
   int ndim, nh, nent;
   int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly
@@ -268,10 +270,10 @@ size_t stats_partials_bytes(long long n);
 // results as the reference returns them) to d_out[0..1] (float).
 cudaError_t launch_field_stats(const float* d_field, long long n, double* d_partials, float* d_out,
                                cudaStream_t stream);
-// Merge `count` statistics records in record order (one block, fixed tree)
+// Merge `count` statistics records (overwritten) in record order, by fixed trees,
 // into the FP32 mean and unbiased variance at d_out[0..1], as
 // launch_field_stats reports them.
-cudaError_t launch_stats_records(const StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream);
+cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream);
 // Rescale (when rescale != 0, scarflib_srm.f90:897-912) and the taper of
 // every point of interest (scarflib_common.f90:881-994), in the reference's
 // order, in one pass over the field. d_poi: npoi x 3 floats.
@@ -310,6 +312,23 @@ struct FimGrid {
   float info0, info1;
 };
 void fim_grid(const FimInputs& in, FimGrid* g);
+// Inverse transform of the half spectrum (fim_fft.cu).
+struct FimAxis {
+  int n, blue;  // transform length (0: none); 1: Bluestein's form, over f.n points
+  FftPlan f;
+};
+struct FimFft {
+  int n[3];
+  FimAxis ax[3];  // x (length n1 / 2), y, z
+  size_t tables;  // bytes of the device tables
+};
+// False when an axis does not fit shared memory (cuFFT then transforms).
+bool fim_fft_plan(const int npts[3], bool three, FimFft* plan);
+long long fim_fft_records(const FimFft& plan);
+// spec [n3][n2][n1 / 2 + 1] (overwritten) -> real [n3][n2][n1], times scaling,
+// with fim_fft_records(plan) statistics records of the result.
+cudaError_t launch_fim_fft(const FimFft& plan, float2* spec, float* real, void* d_tables, float scaling, StatRecord* rec,
+                           cudaStream_t stream);
 size_t fim_workspace_bytes(const FimGrid& g, int npoi);
 // The whole FIM into the device field of the external points; stats as the
 // reference's info(1:8). d_work: fim_workspace_bytes, 256-byte aligned. On

@@ -110,14 +110,30 @@ __global__ void __launch_bounds__(1024) stats_finish(const double* part, int npa
 // FP32 mean in exact arithmetic.
 constexpr int kMergeThreads = 1024;
 
+// Many records first merge in groups of kGroup (a fixed tree), each group's
+// result left in its first record: one block alone took 52 us for 33 000.
+constexpr int kGroup = 256;
+__global__ void __launch_bounds__(kGroup) stats_records_group(Moments* rec, long long count) {
+  __shared__ Moments red[kGroup];
+  const long long r = static_cast<long long>(blockIdx.x) * kGroup + threadIdx.x;
+  red[threadIdx.x] = r < count ? rec[r] : Moments{0.0, 0.0, 0.0};
+  __syncthreads();
+  for (int o = 1; o < kGroup; o <<= 1) {
+    if (threadIdx.x % (2 * o) == 0) red[threadIdx.x] = moments_merge(red[threadIdx.x], red[threadIdx.x + o]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) rec[r] = red[0];
+}
+
+// Merges records 0, stride, 2 stride, ... (count of them).
 __global__ void __launch_bounds__(kMergeThreads) stats_records_merge(const Moments* __restrict__ rec, long long count,
-                                                                      float* out) {
+                                                                      int stride, float* out) {
   __shared__ Moments red[kMergeThreads];
   const long long per = (count + kMergeThreads - 1) / kMergeThreads;
   const long long r0 = static_cast<long long>(threadIdx.x) * per;
   const long long r1 = r0 + per < count ? r0 + per : count;
   Moments m{0.0, 0.0, 0.0};
-  for (long long r = r0; r < r1; ++r) m = moments_merge(m, rec[r]);
+  for (long long r = r0; r < r1; ++r) m = moments_merge(m, rec[r * stride]);
   red[threadIdx.x] = m;
   __syncthreads();
   for (int o = kMergeThreads / 2; o > 0; o >>= 1) {
@@ -207,8 +223,15 @@ cudaError_t launch_field_stats(const float* d_field, long long n, double* d_part
   return cudaGetLastError();
 }
 
-cudaError_t launch_stats_records(const StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream) {
-  stats_records_merge<<<1, kMergeThreads, 0, stream>>>(d_rec, count, d_out);
+cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream) {
+  int stride = 1;
+  if (count > 4 * kMergeThreads) {
+    const long long groups = (count + kGroup - 1) / kGroup;
+    stats_records_group<<<static_cast<unsigned>(groups), kGroup, 0, stream>>>(d_rec, count);
+    count = groups;
+    stride = kGroup;
+  }
+  stats_records_merge<<<1, kMergeThreads, 0, stream>>>(d_rec, count, stride, d_out);
   return cudaGetLastError();
 }
 

@@ -1,0 +1,53 @@
+"""The FIM's inverse transform over axis lengths of both forms (plain, and
+Bluestein's for prime factors above 5), even and odd half lengths, tiles that the
+x bins and rows do not fill, two-point axes, and axes beyond shared memory
+(cuFFT), through scarf_execute against the FP64 transform of the oracle.
+
+Tolerance: FP32 transforms of at most ~1 100 points, three axes of up to two
+transforms with ~11 levels each and ~6e-8 a level, a few 1e-7 in all; 2e-6."""
+import numpy as np
+import pytest
+
+import scarf3d_b200 as sb
+from conftest import rel_rms
+from oracle import fim
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+DS = 50.0
+
+
+def _run(internal, acf=0, **kw):
+    """A field whose internal grid has the given (even) axis lengths."""
+    nd = len(internal)
+    fe = [n - 1 for n in internal]
+    cl = [max(0.1 * n * DS, 2.5 * DS) for n in internal]
+    par = dict(ds=DS, acf=acf, cl=cl, sigma=0.05, hurst=0.4 if acf == 0 else 0.0, pad=0, **kw)
+    assert sb.fim_internal_grid(nd, [0.0] * nd, [(f - 1) * DS for f in fe], DS, cl)[0][:nd] == list(internal)
+    try:
+        sb.scarf_initialize(fs=[1] * nd, fe=fe, method=0, **par)
+        dev = torch.full((int(np.prod(fe)),), float("nan"), device="cuda")
+        _, stats = sb.scarf_execute(31, dev)
+    finally:
+        sb.scarf_finalize()
+    ref, info, _ = fim.execute_structured(fs=[1] * nd, fe=fe, seed=31, **par)
+    got = dev.cpu().numpy()
+    assert rel_rms(got, ref) <= 2e-6, rel_rms(got, ref)
+    assert abs(stats[2] / info[2] - 1) <= 1e-5 and abs(stats[3] - info[3]) <= 1e-5 * info[2]
+
+
+@pytest.mark.parametrize("internal", [
+    (48, 40, 36), (46, 58, 62), (8, 14, 22), (34, 4, 6), (4, 2, 26), (130, 50, 34), (258, 30, 24), (16, 514, 10),
+    (30, 8, 514)])
+def test_three_dimensions(internal):
+    _run(internal)
+
+
+@pytest.mark.parametrize("internal", [(514, 78), (64, 96), (94, 1028), (1026, 34), (1902, 50), (50, 1902)])
+def test_two_dimensions(internal):
+    _run(internal, acf=1)
+
+
+def test_rescaled():
+    _run((38, 46, 30), rescale=1)

@@ -794,16 +794,20 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     // workspace fits (also within the device-memory cap), unless a tensor-core
     // plan was tuned for this grid.
     GridPlan grid{};
-    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned && grid_make_plan(s.ndim, n, nh, &grid) &&
+    const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
+    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned &&
+                    grid_make_plan(s.ndim, n, nh, overlap ? kGridHostPassBytes : kGridPassBytes, &grid) &&
                     (!planned || grid_pays(grid, plan));
-    if (use_grid && (want_records(grid_stat_records(grid)) != SCARF_OK ||
-                     t_ctx->res.work.ensure(grid.bytes) != cudaSuccess)) {
+    auto grid_fits = [&] {
+      if (want_records(grid_stat_records(grid)) == SCARF_OK && t_ctx->res.work.ensure(grid.bytes) == cudaSuccess)
+        return true;
       (void)cudaGetLastError();
       (void)scarf::take_device_alloc_failure();
-      use_grid = false;
-    }
+      return false;
+    };
+    if (use_grid && !grid_fits())  // smaller passes, then the tensor-core form
+      use_grid = grid_make_plan(s.ndim, n, nh, 0, &grid) && grid_fits();
     if (use_grid) {
-      const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
       if (overlap) {
         rc = ensure_pass_resources(grid_passes(grid));
         if (rc) return rc;
@@ -825,7 +829,6 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
       // Without rescale or taper the field is final when the kernel stores
       // it: copy it out slab by slab while the kernel still runs.
       TcSlabSignal sig;
-      const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
       if (overlap) {
         tc_slab_layout(plan, t_ctx->cfg.overlap_items, &sig);
         rc = ensure_slab_resources(sig.nslabs);

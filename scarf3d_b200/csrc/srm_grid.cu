@@ -854,7 +854,7 @@ double window_beta(int n, int m) {
 
 }  // namespace
 
-bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
+bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPlan* P) {
   GridPlan p{};
   if (nh <= 0 || nh > kGridMaxHarmonics || n[0] <= 0 || n[1] <= 0 || n[2] <= 0) return false;
   p.ndim = ndim;
@@ -877,10 +877,12 @@ bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
   p.nkeys = (p.nbx + kSpan) * p.nby;
   p.nent = 2 * nh;
   const int nzp = (p.nz + 31) / 32 * 32;
-  // Planes per pass: T1 and T2 of a pass stay in L2 between the kernels.
+  // Planes per pass: about pass_bytes of T1 and T2, the planes shared out
+  // evenly (a last pass of a few planes costs as much as one of 32).
   const size_t per_z = sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * (p.my + (p.ny > 1 ? p.ny : 0));
-  int zc = static_cast<int>(std::max<size_t>(1, kGridPassBytes / (per_z * 32))) * 32;
-  p.zc = std::min(zc, nzp);
+  const long long most = std::max<long long>(32, static_cast<long long>(1.3 * static_cast<double>(pass_bytes) / per_z));
+  const long long want = (p.nz + most - 1) / most;
+  p.zc = static_cast<int>(std::min<long long>((p.nz + 32 * want - 1) / (32 * want) * 32, nzp));
   // E for as many passes as fit a bounded buffer.
   const size_t e_pass = sizeof(float2) * static_cast<size_t>(p.nent) * p.zc;
   const int passes = static_cast<int>(std::max<size_t>(1, kGridEBytes / e_pass));
@@ -919,10 +921,11 @@ bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* P) {
 }
 
 bool grid_pays(const GridPlan& p, const TcPlan& tc) {
-  const double cells = static_cast<double>(p.mx / 2) * p.my * p.nz, visits = p.ny > 1 ? 9.0 : 3.0;
-  const double grid = 90.0 + 1.35e-5 * cells + p.nh * (0.008 + 0.67e-5 * visits * p.nz);
+  const double cells = static_cast<double>(p.mx / 2) * p.my * p.nz, nh = p.nh;
+  const double grid = 93.0 + 1.0e-5 * cells + nh * (0.0045 + (p.ny > 1 ? 3.5e-5 : 0.8e-5) * p.nz);
   const double waves = std::ceil(static_cast<double>(tc.bix) * tc.bjx * tc.bn / 148.0);
-  return grid < 50.0 + waves * (20.0 + 0.0435 * p.nh);
+  const double flat = p.ny > 1 ? 0.0 : 3.0e-5 * static_cast<double>(p.nx) * p.nz;
+  return grid < 50.0 + flat + waves * (19.0 + 0.042 * nh) + 6.0e-6 * nh * (tc.n1 + tc.n2 + tc.n3);
 }
 
 int grid_passes(const GridPlan& p) { return (p.nz + p.zc - 1) / p.zc; }
@@ -1045,7 +1048,7 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
       grid_spread_kernel<1><<<gs, 32 * kSpreadWarps, sizeof(SpreadWarp) * kSpreadWarps, stream>>>(A, task_blocks, zoff, p.zc);
       grid_parts_kernel<1><<<gp, 32 * kB, 0, stream>>>(A, p.zc);
     }
-    const long long groups = planes / kZT;
+    const long long groups = (z1 - z0 + kZT - 1) / kZT;
     if (p.ny > 1) {
       const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * (p.mx / 2 + 1));
       grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * (p.mx / 2 + 1)), y.nbuf);

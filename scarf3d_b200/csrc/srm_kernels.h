@@ -171,7 +171,11 @@ cudaError_t tc_batch_launch(const TcBatchPlan& plan, void* d_work, cudaStream_t 
 
 // ---- gridded Fourier form of structured sums (srm_grid.cu) ----
 constexpr int kGridMaxHarmonics = 1 << 20;
-constexpr size_t kGridPassBytes = size_t(48) << 20;  // T1 and T2 of one pass
+// T1 and T2 of one pass. Passes that fit L2 (48-96 MB) gained nothing from it,
+// and each kernel of a small pass ends in a wave that fills part of the chip:
+// 512^3 x 20 000 2.20 ms at 48 MB, 1.99 at 128, 1.82 at 400, 1.69 at 1 500. Fields
+// whose planes leave for the host behind each pass take smaller ones.
+constexpr size_t kGridPassBytes = size_t(512) << 20, kGridHostPassBytes = size_t(72) << 20;
 constexpr size_t kGridEBytes = size_t(1) << 30;      // E of as many passes as fit
 // Stages of an FFT of length n: radix, distance between a butterfly's
 // elements and its reciprocal.
@@ -197,14 +201,14 @@ struct GridPlan {
 };
 // False when the form does not take the grid (an axis too long for a
 // transform in shared memory, no or too many harmonics).
-bool grid_make_plan(int ndim, const int n[3], int nh, GridPlan* plan);
+bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPlan* plan);
 // Whether the gridded sum is faster than a tensor-core plan, from fits (in us)
 // to measured device times. The contraction pays per wave of output tiles and
-// harmonic, the gridded sum per cell of its wavenumber grid, and per harmonic
-// and plane. Measured, gridded / tensor cores: 128^3 120 / 99 us at 500
-// harmonics, 127 / 126 at 1 000, 169 / 280 at 4 000; 400^3 1 104 / 926 at 1 000,
-// 1 160 / 1 582 at 2 000, 1 506 / 10 768 at 16 000; 24 x 24 x 1000 339 / 297 at
-// 4 000; 1 500 x 1 500 143 / 159 at 500, 573 / 1 250 at 16 000.
+// harmonic and for its tables, the gridded sum per cell of its wavenumber grid
+// and per harmonic and plane. Measured, gridded / tensor cores: 32 x 32 95 / 96 us at
+// 500 harmonics, 103 / 226 at 4 000; 128^3 132 / 169 at 2 000, 221 / 750 at
+// 16 000; 400^3 770 / 908 at 1 000, 992 / 11 121 at 16 000; 30 x 40 x 512 520 /
+// 773 at 16 000; 1 500 x 1 500 372 / 1 168 at 16 000.
 bool grid_pays(const GridPlan& p, const TcPlan& tc);
 int grid_passes(const GridPlan& p);
 // Planes [z0, z1) that a pass completes; whole contiguous pieces of the field.

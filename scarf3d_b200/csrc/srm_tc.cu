@@ -294,10 +294,72 @@ __device__ __forceinline__ double2 cmul(double2 x, double2 y) {
   return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
 }
 
-__device__ __forceinline__ double2 expi(double th) {
+// e^{i th} of a phase reduced in turns: exact reduction, and sincospi needs
+// none of its own.
+__device__ __forceinline__ double2 expi_turns(double th) {
+  const double t = th * 0.15915494309189533577;  // 1 / (2 pi)
   double s, c;
-  sincos(th, &s, &c);
+  sincospi(2.0 * (t - rint(t)), &s, &c);
   return make_double2(c, s);
+}
+// The factor tables of one harmonic's R and S rows: entry e of
+// {U_r (with the amplitude b - i a), V_r, U_s, V_s}.
+__device__ __forceinline__ double2 rs_factor(const TableJob& T, int e, int nur, int nus, double kr, double ks, double c,
+                                             double a, double b) {
+  const bool is_r = e < nur + 16;
+  const int f = is_r ? e : e - nur - 16, nu = is_r ? nur : nus;
+  const bool coarse = f < nu;
+  const double off = coarse ? (is_r ? T.off[T.ax_r] : T.off[T.ax_s]) : 0.0;
+  const double idx = coarse ? 16.0 * f : f - nu;
+  const double2 z = expi_turns((is_r ? kr : ks) * ((idx + off) * T.ds) + (is_r && coarse ? c : 0.0));
+  // (b - i a)(cos + i sin)
+  return is_r && coarse ? make_double2(b * z.x + a * z.y, b * z.y - a * z.x) : z;
+}
+// Entry idx of the R (is_r) or S row from the factor tables, and its place in
+// the image. Row tiles are powers of two wide.
+__device__ __forceinline__ void rs_entry(const TableJob& T, const double2* fac, int nur, int nus, int e, int nr, int h,
+                                         bool valid) {
+  const bool is_r = e < nr;
+  const int idx = is_r ? e : e - nr, tw = is_r ? T.ti : T.tj;
+  const int blk = idx >> (31 - __clz(tw)), t = idx & (tw - 1);
+  const double2* u = fac + (is_r ? 0 : nur + 16);
+  float2 out = make_float2(0.0f, 0.0f);
+  if (valid && idx < (is_r ? T.n1 : T.n2)) {
+    const double2 z = cmul(u[idx >> 4], u[(is_r ? nur : nus) + (idx & 15)]);
+    out = make_float2(static_cast<float>(z.x), static_cast<float>(z.y));
+  }
+  const int k = h / kStageHarm, hp = h - k * kStageHarm;
+  (is_r ? T.rimg : T.simg)[((static_cast<size_t>(blk) * T.stages + k) * kStageHarm + hp) * tw + t] = out;
+}
+// The same for four harmonics' column factors {U[4][nu], V[4][16]}.
+__device__ __forceinline__ void c_factor(const TableJob& T, int e, int nu, const double kc[4], double2* u4, double2* v4) {
+  const int u = e / (nu + 16), r = e - u * (nu + 16);
+  const double k = u == 0 ? kc[0] : u == 1 ? kc[1] : u == 2 ? kc[2] : kc[3];
+  const double2 z = expi_turns(k * ((r < nu ? 16.0 * r + T.off[T.ax_c] : static_cast<double>(r - nu)) * T.ds));
+  if (r < nu) u4[u * nu + r] = z;
+  else v4[u * 16 + (r - nu)] = z;
+}
+template <bool kBf16>
+__device__ __forceinline__ void c_entry(const TableJob& T, const double2* u4, const double2* v4, int nu, int nb, int row,
+                                        int k, int chunk, const bool valid[4]) {
+  const int col = nb * T.ntile_n + row;
+  const int part_rows = T.parts == 1 ? T.ntile_n : T.ntile_n >> 1;
+  const int part = row >= part_rows ? 1 : 0, prow = row - part * part_rows;
+  uint32_t hi[4], lo[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    float cs32 = 0.0f, sn32 = 0.0f;
+    if (valid[u] && col < T.n3) {
+      const double2 z = cmul(u4[u * nu + (col >> 4)], v4[u * 16 + (col & 15)]);
+      cs32 = static_cast<float>(z.x);
+      sn32 = static_cast<float>(z.y);
+    }
+    split_pair<kBf16>(cs32, sn32, hi[u], lo[u]);
+  }
+  uint8_t* base = T.cimg + ((static_cast<size_t>(nb) * T.stages + k) * T.parts + part) * (2u * part_rows * kRowBytes);
+  const uint32_t off = swz64(static_cast<uint32_t>(prow), static_cast<uint32_t>(chunk));
+  *reinterpret_cast<uint4*>(base + off) = *reinterpret_cast<const uint4*>(hi);
+  *reinterpret_cast<uint4*>(base + static_cast<size_t>(part_rows) * kRowBytes + off) = *reinterpret_cast<const uint4*>(lo);
 }
 
 // R and S images: one block per harmonic at a time (grid-strided),
@@ -307,50 +369,15 @@ __global__ void tc_build_rs_factored(const TableJob j0, const TableJob* jobs) {
   const TableJob& T = jobs ? jobs[blockIdx.y] : j0;
   const int nr = T.bi * T.ti, ns = T.bj * T.tj;  // image widths (padded)
   const int nur = (nr + 15) / 16, nus = (ns + 15) / 16;
-  double2* ur = fsh;
-  double2* vr = ur + nur;
-  double2* us = vr + 16;
-  double2* vs = us + nus;
-  const int nfac = nur + nus + 32;
-  const double offr = T.off[T.ax_r], offs = T.off[T.ax_s];
   for (int h = blockIdx.x; h < T.stages * kStageHarm; h += gridDim.x) {
     const bool valid = h < T.nh;
     double kv[3] = {0.0, 0.0, 0.0}, c = 0.0, a = 0.0, b = 0.0;
     if (valid) harmonic_k(T, h, kv, c, a, b);
     const double kr = kv[T.ax_r], ks = kv[T.ax_s];
     __syncthreads();  // the previous harmonic's entries are written
-    for (int e = threadIdx.x; e < nfac; e += blockDim.x) {
-      if (e < nur) {
-        ur[e] = expi(kr * ((16.0 * e + offr) * T.ds) + c);
-      } else if (e < nur + 16) {
-        vr[e - nur] = expi(kr * ((e - nur) * T.ds));
-      } else if (e < nur + 16 + nus) {
-        us[e - nur - 16] = expi(ks * ((16.0 * (e - nur - 16) + offs) * T.ds));
-      } else {
-        vs[e - nur - 16 - nus] = expi(ks * ((e - nur - 16 - nus) * T.ds));
-      }
-    }
+    for (int e = threadIdx.x; e < nur + nus + 32; e += blockDim.x) fsh[e] = rs_factor(T, e, nur, nus, kr, ks, c, a, b);
     __syncthreads();
-    const int k = h / kStageHarm, hp = h - k * kStageHarm;
-    for (int e = threadIdx.x; e < nr + ns; e += blockDim.x) {
-      const bool is_r = e < nr;
-      const int idx = is_r ? e : e - nr;
-      const int tw = is_r ? T.ti : T.tj;
-      const int blk = idx / tw, t = idx - blk * tw;
-      float2 out = make_float2(0.0f, 0.0f);
-      if (valid && idx < (is_r ? T.n1 : T.n2)) {
-        if (is_r) {
-          const double2 z = cmul(ur[idx >> 4], vr[idx & 15]);
-          // (b - i a)(cos + i sin)
-          out = make_float2(static_cast<float>(b * z.x + a * z.y), static_cast<float>(b * z.y - a * z.x));
-        } else {
-          const double2 z = cmul(us[idx >> 4], vs[idx & 15]);
-          out = make_float2(static_cast<float>(z.x), static_cast<float>(z.y));
-        }
-      }
-      const size_t q = ((static_cast<size_t>(blk) * T.stages + k) * kStageHarm + hp) * tw + t;
-      (is_r ? T.rimg : T.simg)[q] = out;
-    }
+    for (int e = threadIdx.x; e < nr + ns; e += blockDim.x) rs_entry(T, fsh, nur, nus, e, nr, h, valid);
   }
 }
 
@@ -364,8 +391,6 @@ __global__ void tc_build_c_factored(const TableJob j0, const TableJob* jobs) {
   const int nu = (ncol + 15) / 16;
   double2* u4 = fsh;          // [4][nu]
   double2* v4 = u4 + 4 * nu;  // [4][16]
-  const double offc = T.off[T.ax_c];
-  const int part_rows = T.ntile_n / T.parts;
   for (int j = blockIdx.x; j < T.stages * 4; j += gridDim.x) {
     const int k = j >> 2, chunk = j & 3;
     bool valid[4];
@@ -379,33 +404,11 @@ __global__ void tc_build_c_factored(const TableJob j0, const TableJob* jobs) {
       kc[u] = kv[T.ax_c];
     }
     __syncthreads();  // the previous chunk's entries are written
-    for (int e = threadIdx.x; e < 4 * (nu + 16); e += blockDim.x) {
-      const int u = e / (nu + 16), r = e - u * (nu + 16);
-      if (r < nu) u4[u * nu + r] = expi(kc[u] * ((16.0 * r + offc) * T.ds));
-      else v4[u * 16 + (r - nu)] = expi(kc[u] * ((r - nu) * T.ds));
-    }
+    for (int e = threadIdx.x; e < 4 * (nu + 16); e += blockDim.x) c_factor(T, e, nu, kc, u4, v4);
     __syncthreads();
-    for (int col = threadIdx.x; col < ncol; col += blockDim.x) {
-      const int nb = col / T.ntile_n, row = col - nb * T.ntile_n;
-      const int part = row / part_rows, prow = row - part * part_rows;
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float cs32 = 0.0f, sn32 = 0.0f;
-        if (valid[u] && col < T.n3) {
-          const double2 z = cmul(u4[u * nu + (col >> 4)], v4[u * 16 + (col & 15)]);
-          cs32 = static_cast<float>(z.x);
-          sn32 = static_cast<float>(z.y);
-        }
-        split_pair<kBf16>(cs32, sn32, hi[u], lo[u]);
-      }
-      uint8_t* base = T.cimg + ((static_cast<size_t>(nb) * T.stages + k) * T.parts + part) *
-                                   (2u * part_rows * kRowBytes);
-      const uint32_t off = swz64(static_cast<uint32_t>(prow), static_cast<uint32_t>(chunk));
-      *reinterpret_cast<uint4*>(base + off) = *reinterpret_cast<const uint4*>(hi);
-      *reinterpret_cast<uint4*>(base + static_cast<size_t>(part_rows) * kRowBytes + off) =
-          *reinterpret_cast<const uint4*>(lo);
-    }
+    for (int nb = 0; nb < T.bn; ++nb)
+      for (int row = threadIdx.x; row < T.ntile_n; row += blockDim.x)
+        c_entry<kBf16>(T, u4, v4, nu, nb, row, k, chunk, valid);
   }
 }
 
@@ -425,48 +428,16 @@ __global__ void __launch_bounds__(32 * kBuilderWarps) tc_build_rs_warps(const Ta
   const int nur = (nr + 15) / 16, nus = (ns + 15) / 16;
   const int nfac = nur + nus + 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2* ur = fsh + warp * nfac;
-  double2* vr = ur + nur;
-  double2* us = vr + 16;
-  double2* vs = us + nus;
-  const double offr = T.off[T.ax_r], offs = T.off[T.ax_s];
+  double2* fac = fsh + warp * nfac;
   for (int h = blockIdx.x * kBuilderWarps + warp; h < T.stages * kStageHarm; h += gridDim.x * kBuilderWarps) {
     const bool valid = h < T.nh;
     double kv[3] = {0.0, 0.0, 0.0}, c = 0.0, a = 0.0, b = 0.0;
     if (valid) harmonic_k(T, h, kv, c, a, b);
     const double kr = kv[T.ax_r], ks = kv[T.ax_s];
     __syncwarp();  // the previous harmonic's entries are written
-    for (int e = lane; e < nfac; e += 32) {
-      if (e < nur) {
-        ur[e] = expi(kr * ((16.0 * e + offr) * T.ds) + c);
-      } else if (e < nur + 16) {
-        vr[e - nur] = expi(kr * ((e - nur) * T.ds));
-      } else if (e < nur + 16 + nus) {
-        us[e - nur - 16] = expi(ks * ((16.0 * (e - nur - 16) + offs) * T.ds));
-      } else {
-        vs[e - nur - 16 - nus] = expi(ks * ((e - nur - 16 - nus) * T.ds));
-      }
-    }
+    for (int e = lane; e < nfac; e += 32) fac[e] = rs_factor(T, e, nur, nus, kr, ks, c, a, b);
     __syncwarp();
-    const int k = h / kStageHarm, hp = h - k * kStageHarm;
-    for (int e = lane; e < nr + ns; e += 32) {
-      const bool is_r = e < nr;
-      const int idx = is_r ? e : e - nr;
-      const int tw = is_r ? T.ti : T.tj;
-      const int blk = idx / tw, t = idx - blk * tw;
-      float2 out = make_float2(0.0f, 0.0f);
-      if (valid && idx < (is_r ? T.n1 : T.n2)) {
-        if (is_r) {
-          const double2 z = cmul(ur[idx >> 4], vr[idx & 15]);
-          out = make_float2(static_cast<float>(b * z.x + a * z.y), static_cast<float>(b * z.y - a * z.x));
-        } else {
-          const double2 z = cmul(us[idx >> 4], vs[idx & 15]);
-          out = make_float2(static_cast<float>(z.x), static_cast<float>(z.y));
-        }
-      }
-      const size_t q = ((static_cast<size_t>(blk) * T.stages + k) * kStageHarm + hp) * tw + t;
-      (is_r ? T.rimg : T.simg)[q] = out;
-    }
+    for (int e = lane; e < nr + ns; e += 32) rs_entry(T, fac, nur, nus, e, nr, h, valid);
   }
 }
 
@@ -479,8 +450,6 @@ __global__ void __launch_bounds__(32 * kBuilderWarps) tc_build_c_warps(const Tab
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double2* u4 = fsh + warp * 4 * (nu + 16);  // [4][nu]
   double2* v4 = u4 + 4 * nu;                 // [4][16]
-  const double offc = T.off[T.ax_c];
-  const int part_rows = T.ntile_n / T.parts;
   for (int j = blockIdx.x * kBuilderWarps + warp; j < T.stages * 4; j += gridDim.x * kBuilderWarps) {
     const int k = j >> 2, chunk = j & 3;
     bool valid[4];
@@ -494,33 +463,10 @@ __global__ void __launch_bounds__(32 * kBuilderWarps) tc_build_c_warps(const Tab
       kc[u] = kv[T.ax_c];
     }
     __syncwarp();  // the previous chunk's entries are written
-    for (int e = lane; e < 4 * (nu + 16); e += 32) {
-      const int u = e / (nu + 16), r = e - u * (nu + 16);
-      if (r < nu) u4[u * nu + r] = expi(kc[u] * ((16.0 * r + offc) * T.ds));
-      else v4[u * 16 + (r - nu)] = expi(kc[u] * ((r - nu) * T.ds));
-    }
+    for (int e = lane; e < 4 * (nu + 16); e += 32) c_factor(T, e, nu, kc, u4, v4);
     __syncwarp();
-    for (int col = lane; col < ncol; col += 32) {
-      const int nb = col / T.ntile_n, row = col - nb * T.ntile_n;
-      const int part = row / part_rows, prow = row - part * part_rows;
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float cs32 = 0.0f, sn32 = 0.0f;
-        if (valid[u] && col < T.n3) {
-          const double2 z = cmul(u4[u * nu + (col >> 4)], v4[u * 16 + (col & 15)]);
-          cs32 = static_cast<float>(z.x);
-          sn32 = static_cast<float>(z.y);
-        }
-        split_pair<kBf16>(cs32, sn32, hi[u], lo[u]);
-      }
-      uint8_t* base = T.cimg + ((static_cast<size_t>(nb) * T.stages + k) * T.parts + part) *
-                                   (2u * part_rows * kRowBytes);
-      const uint32_t off = swz64(static_cast<uint32_t>(prow), static_cast<uint32_t>(chunk));
-      *reinterpret_cast<uint4*>(base + off) = *reinterpret_cast<const uint4*>(hi);
-      *reinterpret_cast<uint4*>(base + static_cast<size_t>(part_rows) * kRowBytes + off) =
-          *reinterpret_cast<const uint4*>(lo);
-    }
+    for (int nb = 0; nb < T.bn; ++nb)
+      for (int row = lane; row < T.ntile_n; row += 32) c_entry<kBf16>(T, u4, v4, nu, nb, row, k, chunk, valid);
   }
 }
 

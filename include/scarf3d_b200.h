@@ -156,8 +156,8 @@ int scarf_set_tc_precision(int operand_type, int terms);
  * of 16, per GPU name and driver); the default plan is kept unless a
  * candidate beats it by 3 %. With scarf_set_tc_autotune(1), plans made afterwards
  * (scarf_srm_tc_workspace_bytes / scarf_srm_tc_structured, and
- * scarf_execute for fixed_columns = 1 tunings) follow the recorded choice
- * of their bucket; other buckets keep the default plans. Tuned plans compute
+ * scarf_execute's tensor-core form for fixed_columns = 1 tunings) follow the
+ * recorded choice of their bucket; other buckets keep the default plans. Tuned plans compute
  * the same sum; a different column axis changes how the per-axis factors
  * combine, so results may differ at the rounding level (within the
  * tensor-core tolerance). The tuning allocates its own device scratch. */

@@ -790,12 +790,12 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     const bool have_tuned = use_tc && nh > 0 && tc_tuned_choice(s.ndim, n, true, &tuned);
     const bool planned = have_tuned ? tc_make_plan(s.ndim, n, nh, &plan, tuned.tile_j, false, tuned.variant)
                                     : tc_make_plan(s.ndim, n, nh, &plan);
-    // The automatic form: the gridded sum where it is the faster and its
-    // workspace fits (also within the device-memory cap), unless a tensor-core
-    // plan was tuned for this grid.
+    // The automatic form: the gridded sum where it is faster than the
+    // tensor-core plan (tuned or not) and its workspace fits, also within the
+    // device-memory cap.
     GridPlan grid{};
     const bool overlap = t_ctx->cfg.overlap_items > 0 && !on_device && p.rescale != 1 && !tapering;
-    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 && !have_tuned &&
+    bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 &&
                     grid_make_plan(s.ndim, n, nh, overlap ? kGridHostPassBytes : kGridPassBytes, &grid) &&
                     (!planned || grid_pays(grid, plan));
     auto grid_fits = [&] {

@@ -534,55 +534,43 @@ __global__ void __launch_bounds__(32 * kB * KY) grid_parts_kernel(const GridArgs
 }
 
 // The transforms' blocks are persistent: a block takes tiles blockIdx.x,
-// blockIdx.x + gridDim.x, ... and has the next tile on its way (one bulk copy
-// into the other buffer) while it transforms the current one. Loaded by the
-// threads themselves, a tile's latency was 40 % of its time.
-struct TileRing {
-  unsigned char* buf;
-  uint64_t* bar;
-  uint32_t bytes;  // one tile
-  uint32_t pitch;  // between buffers
-  int nbuf;
-};
-__device__ __forceinline__ void tile_issue(const TileRing& R, int slot, const void* src) {
-  mbar_arrive_expect_tx(R.bar + slot, R.bytes);
-  bulk_g2s(R.buf + static_cast<size_t>(slot) * R.pitch, src, R.bytes, R.bar + slot);
+// blockIdx.x + gridDim.x, ... each by one bulk copy (loaded by the threads
+// themselves, a tile's latency was 40 % of its time) into one buffer: the
+// copies are covered by the SM's other blocks. A second buffer per block, for
+// the next tile, halves the blocks that fit, and the stages' barriers then
+// stand open (sums of 512^3 points x 20 000 harmonics 1 771 us with two
+// buffers, 1 661 with one; 1024 x 1024 x 100 x 10 000 1 549 and 1 305).
+__device__ __forceinline__ void tile_issue(unsigned char* buf, uint64_t* bar, const void* src, uint32_t bytes) {
+  mbar_arrive_expect_tx(bar, bytes);
+  bulk_g2s(buf, src, bytes, bar);
 }
 
 // Step 2: inverse FFT along cy of the planes of a tile (one cx), the ny
 // outputs kept.
-__global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridArgs A, int tiles, int nbuf) {
+__global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridArgs A, int tiles) {
   using namespace fft;
   constexpr int NP = kPairs;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_full[2];
+  __shared__ __align__(8) uint64_t s_full;
   const FftPlan& f = A.fy;
   const uint32_t bytes = static_cast<uint32_t>(A.my) * NP * 16;
-  const TileRing R{smem, s_full, bytes, bytes, nbuf};
   const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t1);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < nbuf; ++i) mbar_init(&s_full[i], 1);
+    mbar_init(&s_full, 1);
     fence_mbar_init();
-    for (int i = 0; i < nbuf; ++i) {
-      const long long t = blockIdx.x + static_cast<long long>(i) * gridDim.x;
-      if (t < tiles) tile_issue(R, i, base + static_cast<size_t>(t) * bytes);
-    }
+    if (static_cast<int>(blockIdx.x) < tiles) tile_issue(smem, &s_full, base + static_cast<size_t>(blockIdx.x) * bytes, bytes);
   }
   __syncthreads();
+  ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
   const int rl = f.r[f.nst - 1], hop = f.n / rl, row = (A.hx + 1) * NP;
   int n = 0;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
-    const int slot = n % nbuf;
-    const bool ok = mbar_wait_bounded(&s_full[slot], (n / nbuf) & 1, A.status);
+    const bool ok = mbar_wait_bounded(&s_full, n & 1, A.status);
     if (!__syncthreads_and(ok)) {
-      // Unwind: the copies in flight land before the block exits.
-      if (threadIdx.x == 0)
-        for (int i = 0; i < nbuf; ++i)
-          if (t + static_cast<long long>(i) * gridDim.x < tiles)
-            mbar_wait_drain(&s_full[(n + i) % nbuf], ((n + i) / nbuf) & 1);
+      // Unwind: the copy in flight lands before the block exits.
+      if (threadIdx.x == 0) mbar_wait_drain(&s_full, n & 1);
       return;
     }
-    ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem + static_cast<size_t>(slot) * bytes);
     const int g = t / (A.hx + 1), cx = t - g * (A.hx + 1);
     ulonglong2* dst = reinterpret_cast<ulonglong2*>(A.t2) + static_cast<size_t>(g) * A.ny * row + cx * NP;
     auto in = [&](int e, int p) {
@@ -602,10 +590,10 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridAr
     }
     stage_any<NP>(f, f.nst - 1, A.twy, in, gout);
     __syncthreads();
-    const long long next = t + static_cast<long long>(nbuf) * gridDim.x;
+    const long long next = t + static_cast<long long>(gridDim.x);
     if (threadIdx.x == 0 && next < tiles) {
       fence_proxy_async_smem();
-      tile_issue(R, slot, base + static_cast<size_t>(next) * bytes);
+      tile_issue(smem, &s_full, base + static_cast<size_t>(next) * bytes, bytes);
     }
   }
 }
@@ -615,28 +603,25 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridAr
 // length hx whose output m is (x[2 m], x[2 m + 1]); x rows leave through
 // shared memory, divided by both axes' window transforms.
 __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridArgs A, float* field, int zbeg, int nzc,
-                                                                    int tiles, int nbuf, Moments* stats) {
+                                                                    int tiles, Moments* stats) {
   using namespace fft;
   constexpr int NP = kPairs;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_full[2];
+  __shared__ __align__(8) uint64_t s_full;
   __shared__ Moments s_warp[kFftMaxThreads / 32];
   const FftPlan& f = A.fx;
   const uint32_t bytes = static_cast<uint32_t>(A.hx + 1) * NP * 16;
-  const TileRing R{smem, s_full, bytes, bytes, nbuf};
   const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t2);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < nbuf; ++i) mbar_init(&s_full[i], 1);
+    mbar_init(&s_full, 1);
     fence_mbar_init();
-    for (int i = 0; i < nbuf; ++i) {
-      const long long t = blockIdx.x + static_cast<long long>(i) * gridDim.x;
-      if (t < tiles) tile_issue(R, i, base + static_cast<size_t>(t) * bytes);
-    }
+    if (static_cast<int>(blockIdx.x) < tiles) tile_issue(smem, &s_full, base + static_cast<size_t>(blockIdx.x) * bytes, bytes);
   }
   __syncthreads();
   int pitch = (A.nx + 2) / 2 * 2;  // even for the paired stores; half of it odd: no bank conflicts
   if (pitch / 2 % 2 == 0) pitch += 2;
-  float* rows = reinterpret_cast<float*>(smem + static_cast<size_t>(nbuf) * bytes);
+  float* rows = reinterpret_cast<float*>(smem + bytes);
+  ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
   const int half = f.n / 2;
   const int rl = f.r[f.nst - 1], hop = f.n / rl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -644,16 +629,11 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
   double s1[2] = {0.0, 0.0}, s2[2] = {0.0, 0.0}, shift = 0.0;
   int count = 0, n = 0;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
-    const int slot = n % nbuf;
-    const bool ok = mbar_wait_bounded(&s_full[slot], (n / nbuf) & 1, A.status);
+    const bool ok = mbar_wait_bounded(&s_full, n & 1, A.status);
     if (!__syncthreads_and(ok)) {
-      if (threadIdx.x == 0)
-        for (int i = 0; i < nbuf; ++i)
-          if (t + static_cast<long long>(i) * gridDim.x < tiles)
-            mbar_wait_drain(&s_full[(n + i) % nbuf], ((n + i) / nbuf) & 1);
+      if (threadIdx.x == 0) mbar_wait_drain(&s_full, n & 1);
       return;
     }
-    ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem + static_cast<size_t>(slot) * bytes);
     const int g = t / A.ny, j = t - g * A.ny, z0 = g * kZT;
     for (int it = threadIdx.x; it < (half + 1) * NP; it += blockDim.x) {
       const int p = it & (NP - 1), k = it / NP;
@@ -691,10 +671,10 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
     __syncthreads();
     stage_any<NP>(f, f.nst - 1, A.twx, in, rout);
     __syncthreads();
-    const long long next = t + static_cast<long long>(nbuf) * gridDim.x;
+    const long long next = t + static_cast<long long>(gridDim.x);
     if (threadIdx.x == 0 && next < tiles) {
       fence_proxy_async_smem();
-      tile_issue(R, slot, base + static_cast<size_t>(next) * bytes);
+      tile_issue(smem, &s_full, base + static_cast<size_t>(next) * bytes, bytes);
     }
     // Rows of x: one warp per plane at a time, two values per lane where the
     // field's rows are 8-byte aligned. The next tile's rows are written after
@@ -788,17 +768,16 @@ constexpr size_t kSmemMax = 224 * 1024;  // dynamic; the kernels keep a little s
 
 namespace {
 
-// Launch shape of a transform kernel: two tile buffers where they fit, and
-// the block size that fills an SM's registers (kFftMaxThreads threads) with
-// the least idle threads in the stages' rounds.
+// Launch shape of a transform kernel: the block size that fills an SM's
+// registers (kFftMaxThreads threads) with the least idle threads in the
+// stages' rounds.
 struct FftShape {
-  int threads, blocks, nbuf;
+  int threads, blocks;
   size_t smem;
 };
 FftShape fft_shape(const FftPlan& f, size_t tile, size_t extra, long long tiles) {
   FftShape best{};
-  best.nbuf = 2 * tile + extra <= kSmemMax ? 2 : 1;
-  best.smem = best.nbuf * tile + extra;
+  best.smem = tile + extra;
   double best_cost = 1e30;
   for (int t = 64; t <= kFftMaxThreads; t += 32) {
     const int per_sm = static_cast<int>(std::min<size_t>(std::min<size_t>(kSmemMax / best.smem, kFftMaxThreads / t), 8));
@@ -1051,10 +1030,10 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
     const long long groups = (z1 - z0 + kZT - 1) / kZT;
     if (p.ny > 1) {
       const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * (p.mx / 2 + 1));
-      grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * (p.mx / 2 + 1)), y.nbuf);
+      grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * (p.mx / 2 + 1)));
     }
     const FftShape x = x_shape(p, z1 - z0);
-    grid_fft_x_kernel<<<x.blocks, x.threads, x.smem, stream>>>(A, d_field, z0, z1 - z0, x_tiles(p, z1 - z0), x.nbuf,
+    grid_fft_x_kernel<<<x.blocks, x.threads, x.smem, stream>>>(A, d_field, z0, z1 - z0, x_tiles(p, z1 - z0),
                                                                d_stats);
     if (d_stats) d_stats += x.blocks;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

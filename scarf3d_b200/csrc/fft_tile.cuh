@@ -236,9 +236,10 @@ __device__ __forceinline__ void stage(const FftPlan& f, int s, const float4* __r
 }
 // The last stage forwards, a product with hat[position] and the first stage
 // backwards (e^{-i}) in registers: a butterfly of the last stage holds what its
-// inverse needs.
-template <int R, int NP, class In, class Out>
-__device__ __forceinline__ void product(const FftPlan& f, const float4* __restrict__ hat, In in, Out out) {
+// inverse needs. first(base, p, v, y) sees the butterfly's first value before
+// the product and may change it after.
+template <int R, int NP, class In, class Out, class First>
+__device__ __forceinline__ void product(const FftPlan& f, const float4* __restrict__ hat, In in, Out out, First first) {
   for (int it = threadIdx.x; it < f.n / R * NP; it += blockDim.x) {
     const int p = it & (NP - 1), base = it / NP * R;
     C2 v[R];
@@ -248,7 +249,8 @@ __device__ __forceinline__ void product(const FftPlan& f, const float4* __restri
 #pragma unroll
     for (int t = 0; t < R; ++t) {
       const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(hat + base + t));
-      const C2 y = cmul(v[t], x.x, x.y);
+      C2 y = cmul(v[t], x.x, x.y);
+      if (t == 0) first(base, p, v[0], y);
       v[t] = C2{y.im, y.re};  // the e^{-i} transform is the e^{+i} one with the parts exchanged
     }
     Dft<R>::run(v);
@@ -301,9 +303,9 @@ __device__ __forceinline__ void stage_any(const FftPlan& f, int s, const float4*
   SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[s])
 #undef SCARF_FFT_CALL
 }
-template <int NP, class In, class Out>
-__device__ __forceinline__ void product_any(const FftPlan& f, const float4* hat, In in, Out out) {
-#define SCARF_FFT_CALL(R) product<R, NP>(f, hat, in, out)
+template <int NP, class In, class Out, class First>
+__device__ __forceinline__ void product_any(const FftPlan& f, const float4* hat, In in, Out out, First first) {
+#define SCARF_FFT_CALL(R) product<R, NP>(f, hat, in, out, first)
   SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[f.nst - 1])
 #undef SCARF_FFT_CALL
 }

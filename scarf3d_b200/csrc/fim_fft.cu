@@ -13,9 +13,22 @@
 // backwards are one step in registers. Lengths without larger prime factors take
 // a plain transform.
 //
-// Bound: shared-memory traffic of the stages (1 080 points take eight passes
-// over a 69 KB tile). 514^3: cuFFT's transforms took 4.2 ms (z 1.51, y 1.42, x
-// 1.26 with its preprocessing) and the statistics 0.11 more; these take 3.2.
+// N = q p with p prime and p - 1 without prime factors above 5 (514 = 2 x 257)
+// takes a shorter way. Indices n = p b + q m and k = (k mod q, k mod p) split the
+// transform into q-point ones over b and p-point ones over m without twiddles
+// (Good 1958, Thomas 1963), and the p-point ones are, with a primitive root g,
+// cyclic convolutions over the non-zero residues (Rader 1968):
+//   Y[g^-v] = y[0] + sum_u y[g^u] c_{v - u},  c_d = e^{2 pi i g^-d / p},
+// p - 1 points where Bluestein's form takes at least 2 p - 1. The tile's q (p - 1)
+// values run through one plan: the q-point stages, then the convolution in each
+// of q blocks; the q values of residue 0 are transformed apart, added to the
+// convolution through its constant term, and with that term's input they are the
+// outputs of residue 0.
+//
+// Bound: shared-memory traffic of the stages. 514^3: cuFFT's transforms took
+// 4.2 ms (z 1.51, y 1.42, x 1.26 with its preprocessing) and the statistics 0.11
+// more; Bluestein's form over 1 080 points (69 KB tiles) 3.2, Rader's over 512
+// (33 KB) 1.8. A q beyond 64 would make the serial q-point sums long: Bluestein.
 //
 // The c2r step stores the scaled field (1 / sqrt(n1 n2 n3 dh^n), :1019) and
 // records its statistics (:1027-1036), one record per block, as it goes.
@@ -35,7 +48,8 @@ using namespace fft;
 
 constexpr int kPairs = 4;               // transform pairs of a tile
 constexpr int kTile = 2 * kPairs;       // transforms of a tile
-// Blocks of at most 256 threads at 80 registers: three per SM at ~1 100 points.
+// Blocks of at most 256 threads at 80 registers: three per SM at ~1 100 points
+// (Bluestein's form).
 // With 112 registers (two) the transforms of the 514^3 grid took 3.9 ms, with 64
 // (spilling) 3.6, so 3.2.
 constexpr int kMaxThreads = 256, kSmThreads = 3 * kMaxThreads;
@@ -49,7 +63,15 @@ struct AxisTables {
   const float4* tw;     // {cos, cos, sin, sin}
   const float4* chirp;  // n entries, the same form
   const float4* hat;    // f.n entries
-  const int* rev;       // at e - t of the last stage
+  const int* rev;       // at e - t of the last stage (plain)
+  // Rader's form: input and output of each position, position of each input
+  // (q inputs of residue 0 at f.n .. ), outputs of residue 0, roots of the
+  // q-point transform.
+  const int* src;
+  const int* dst;
+  const int* place;
+  const int* zero;
+  const float4* roots;
   const float4* pack;   // e^{2 pi i k / n1}, k <= n1 / 4 (real axis)
 };
 
@@ -59,6 +81,11 @@ struct TableArgs {
   float4* chirp[3];
   float4* hat[3];
   int* rev[3];
+  int* src[3];
+  int* dst[3];
+  int* place[3];
+  int* zero[3];
+  float4* roots[3];
   float4* pack;
   int n1;
 };
@@ -74,6 +101,89 @@ __device__ __forceinline__ double chirp_turns(int n, int N) {
   return static_cast<double>(q) / (2.0 * N);
 }
 
+// b^e modulo p
+__device__ __forceinline__ int power_mod(int b, int e, int p) {
+  long long r = 1, x = b;
+  for (; e > 0; e >>= 1) {
+    if (e & 1) r = r * x % p;
+    x = x * x % p;
+  }
+  return static_cast<int>(r);
+}
+// Frequency at position pos of stages s0 .. s1 - 1, which transform `span` points.
+__device__ __forceinline__ int stage_frequency(const FftPlan& f, int s0, int s1, int span, int pos) {
+  int k = 0, w = 1;
+  for (int s = s0; s < s1; ++s) {
+    span /= f.r[s];
+    const int d = pos / span;
+    pos -= d * span;
+    k += d * w;
+    w *= f.r[s];
+  }
+  return k;
+}
+// Rader's form: the q-point stages see the q blocks only.
+__device__ double rader_twiddle(const FimAxis& X, int i) {
+  const FftPlan& f = X.f;
+  int at = i, len = f.n;
+  for (int s = 0; s < X.sq; ++s) {
+    const int count = len - f.m[s];
+    if (at < count) {
+      const int t = at / f.m[s], b = (at - t * f.m[s]) / (X.p - 1);
+      return static_cast<double>(b * (t + 1)) / (len / (X.p - 1));
+    }
+    at -= count;
+    len = f.m[s];
+  }
+  return twiddle_entry(f, i);
+}
+__device__ void rader_tables(const TableArgs& A, int a, int i, int lane) {
+  const FimAxis& X = A.ax[a];
+  const FftPlan& f = X.f;
+  const int len = X.p - 1;
+  if (lane == 0) {
+    if (i < f.n) {
+      const int j = i / len, u = i - j * len;
+      const int from = static_cast<int>((static_cast<long long>(X.p) * j + static_cast<long long>(X.q) * power_mod(X.root, u, X.p)) % X.n);
+      A.tw[a][i] = dup_root(rader_twiddle(X, i));
+      A.src[a][i] = from;
+      A.place[a][from] = i;
+      A.dst[a][i] = static_cast<int>((static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, j)) * X.cq +
+                                      static_cast<long long>(power_mod(X.root, len - u, X.p)) * X.cp) % X.n);
+    }
+    if (i < X.q) {
+      A.place[a][static_cast<long long>(X.p) * i % X.n] = f.n + i;
+      A.zero[a][i] = static_cast<int>(static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, i)) * X.cq % X.n);
+    }
+    if (i < X.q * X.q) {
+      const int j = i / X.q, b = i - j * X.q;
+      A.roots[a][i] = dup_root(static_cast<double>(b * stage_frequency(f, 0, X.sq, X.q, j) % X.q) / X.q);
+    }
+  }
+  if (i >= f.n) return;
+  // hat = (1 / (p - 1)) sum_d c_d e^{2 pi i d freq / (p - 1)}
+  const int freq = stage_frequency(f, X.sq, f.nst, len, i % len);
+  const int hop = power_mod(X.root, len - 32 % len, X.p);  // g^-32
+  long long gd = power_mod(X.root, (len - lane % len) % len, X.p);
+  double re = 0.0, im = 0.0;
+  for (int d = lane; d < len; d += 32) {
+    double s, c;
+    const double turns = static_cast<double>(gd) / X.p + static_cast<double>(static_cast<long long>(d) * freq % len) / len;
+    sincospi(2.0 * (turns - rint(turns)), &s, &c);
+    re += c;
+    im += s;
+    gd = gd * hop % X.p;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    re += __shfl_down_sync(0xffffffffu, re, o);
+    im += __shfl_down_sync(0xffffffffu, im, o);
+  }
+  if (lane == 0) {
+    const float x = static_cast<float>(re / len), y = static_cast<float>(im / len);
+    A.hat[a][i] = make_float4(x, x, y, y);
+  }
+}
+
 // blockIdx.y: axis; one warp per table index.
 __global__ void __launch_bounds__(128) fim_tables_kernel(const TableArgs A) {
   const int a = blockIdx.y, lane = threadIdx.x & 31;
@@ -81,14 +191,19 @@ __global__ void __launch_bounds__(128) fim_tables_kernel(const TableArgs A) {
   const FimAxis& X = A.ax[a];
   if (X.n == 0) return;  // axis not transformed
   const FftPlan& f = X.f;
+  if (lane == 0 && a == 0 && i <= X.n / 2) A.pack[i] = dup_root(static_cast<double>(i) / A.n1);
+  if (X.form == kFimRader) {
+    rader_tables(A, a, i, lane);
+    return;
+  }
+  const bool blue = X.form == kFimBluestein;
   if (lane == 0) {
     if (i < f.n) A.tw[a][i] = dup_root(twiddle_entry(f, i));
-    if (X.blue && i < X.n) A.chirp[a][i] = dup_root(chirp_turns(i, X.n));
+    if (blue && i < X.n) A.chirp[a][i] = dup_root(chirp_turns(i, X.n));
     const int r = f.r[f.nst - 1];
-    if (!X.blue && i < f.n / r) A.rev[a][i * r] = output_order(f, i);
-    if (a == 0 && i <= X.n / 2) A.pack[i] = dup_root(static_cast<double>(i) / A.n1);
+    if (!blue && i < f.n / r) A.rev[a][i * r] = output_order(f, i);
   }
-  if (!X.blue || i >= f.n) return;
+  if (!blue || i >= f.n) return;
   // hat[pos] = (1 / M) sum_m conj(c_m) e^{2 pi i m freq / M}, m = -(N-1) .. N-1
   const int r = f.r[f.nst - 1], g = i / r, t = i - g * r;
   const int freq = output_order(f, g) + t * (f.n / r);
@@ -123,9 +238,10 @@ __device__ __forceinline__ C2 times(C2 a, const float4* t) {
   return cmul(a, w.re, w.im);
 }
 
-// The tile's transforms. in(e, p) gives input e < X.n of pair p, out(e, p, v)
+// The tile's transforms. in(e, p) gives input e < X.n of pair p (kPlaced: the
+// inputs are in the tile, those of Rader's form where `place` says), out(e, p, v)
 // takes output e < X.n.
-template <class In, class Out>
+template <int kForm, bool kPlaced, class In, class Out>
 __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTables& T, ulonglong2* sh, In in, Out out) {
   const FftPlan& f = X.f;
   auto sin = [&](int e, int p) {
@@ -134,7 +250,7 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
   };
   auto sout = [&](int e, int p, int, C2 v) { sh[e * kPairs + p] = make_ulonglong2(v.re, v.im); };
   const int last = f.nst - 1, rl = f.r[last], hop = f.n / rl;
-  if (!X.blue) {
+  if constexpr (kForm == kFimPlain) {
     stage_any<kPairs>(f, 0, T.tw, in, sout);
     for (int s = 1; s < last; ++s) {
       __syncthreads();
@@ -143,38 +259,83 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
     __syncthreads();
     stage_any<kPairs>(f, last, T.tw, sin,
                       [&](int e, int p, int t, C2 v) { out(__ldg(T.rev + e - t) + t * hop, p, v); });
-    return;
-  }
-  auto bin = [&](int e, int p) {
-    if (e >= X.n) return C2{0ull, 0ull};
-    return times(in(e, p), T.chirp + e);
-  };
-  stage_any<kPairs>(f, 0, T.tw, bin, sout);
-  for (int s = 1; s < last; ++s) {
+  } else if constexpr (kForm == kFimRader) {
+    const int q = X.q;
+    auto first = [&](int e, int p) { return kPlaced ? sin(e, p) : in(__ldg(T.src + e), p); };
+    auto zero = [&](int b, int p) { return kPlaced ? sin(f.n + b, p) : in(b * X.p, p); };
+    // Residue 0: q-point transforms into slots f.n + q .. (the last threads,
+    // which have the fewest butterflies).
+    for (int it = blockDim.x - 1 - threadIdx.x; it < q * kPairs; it += blockDim.x) {
+      const int p = it & (kPairs - 1), j = it / kPairs;
+      C2 v = zero(0, p);
+      for (int b = 1; b < q; ++b) v = v + times(zero(b, p), T.roots + j * q + b);
+      sout(f.n + q + j, p, 0, v);
+    }
+    stage_any<kPairs>(f, 0, T.tw, first, sout);
+    for (int s = 1; s < last; ++s) {
+      __syncthreads();
+      stage_any<kPairs>(f, s, T.tw, sin, sout);
+    }
     __syncthreads();
-    stage_any<kPairs>(f, s, T.tw, sin, sout);
-  }
-  __syncthreads();
-  product_any<kPairs>(f, T.hat, sin, sout);
-  for (int s = last - 1; s > 0; --s) {
+    // A block's constant term: with residue 0's value it is the output of
+    // residue 0 (slots f.n ..), and that value joins its product.
+    auto constant = [&](int base, int p, C2 v, C2& y) {
+      const int j = static_cast<int>((static_cast<float>(base) + 0.5f) * X.inv_len);
+      if (j * (X.p - 1) != base) return;
+      const C2 z = sin(f.n + q + j, p);
+      sout(f.n + j, p, 0, z + v);
+      y = y + z;
+    };
+    auto put = [&](int e, int p, int, C2 v) { out(__ldg(T.dst + e), p, v); };
+    if (last == X.sq) {
+      product_any<kPairs>(f, T.hat, sin, put, constant);
+      __syncthreads();
+    } else {
+      product_any<kPairs>(f, T.hat, sin, sout, constant);
+      for (int s = last - 1; s > X.sq; --s) {
+        __syncthreads();
+        back_any<kPairs>(f, s, T.tw, sin, sout);
+      }
+      __syncthreads();
+      back_any<kPairs>(f, X.sq, T.tw, sin, put);
+    }
+    for (int it = blockDim.x - 1 - threadIdx.x; it < q * kPairs; it += blockDim.x) {
+      const int p = it & (kPairs - 1), j = it / kPairs;
+      out(__ldg(T.zero + j), p, sin(f.n + j, p));
+    }
+  } else {
+    auto bin = [&](int e, int p) {
+      if (e >= X.n) return C2{0ull, 0ull};
+      return times(in(e, p), T.chirp + e);
+    };
+    stage_any<kPairs>(f, 0, T.tw, bin, sout);
+    for (int s = 1; s < last; ++s) {
+      __syncthreads();
+      stage_any<kPairs>(f, s, T.tw, sin, sout);
+    }
     __syncthreads();
-    back_any<kPairs>(f, s, T.tw, sin, sout);
+    product_any<kPairs>(f, T.hat, sin, sout, [](int, int, C2, C2&) {});
+    for (int s = last - 1; s > 0; --s) {
+      __syncthreads();
+      back_any<kPairs>(f, s, T.tw, sin, sout);
+    }
+    __syncthreads();
+    back_any<kPairs>(f, 0, T.tw, sin, [&](int e, int p, int, C2 v) {
+      if (e < X.n) out(e, p, times(v, T.chirp + e));
+    });
   }
-  __syncthreads();
-  back_any<kPairs>(f, 0, T.tw, sin, [&](int e, int p, int, C2 v) {
-    if (e < X.n) out(e, p, times(v, T.chirp + e));
-  });
 }
 
 // c2c along z or y, in place: blockIdx.x selects eight neighbouring x bins,
 // blockIdx.y the row or plane.
+template <int kForm>
 __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_columns_kernel(const FimAxis X, const AxisTables T, float2* spec, int n1h,
                                                                   long long step, long long outer) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int i0 = blockIdx.x * kTile, left = n1h - i0;
   float2* base = spec + blockIdx.y * outer + i0;
   const bool wide = (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (step & 1) == 0;
-  transform_tile(
+  transform_tile<kForm, false>(
       X, T, reinterpret_cast<ulonglong2*>(smem),
       [&](int e, int p) {
         const float2* s = base + e * step + 2 * p;
@@ -200,6 +361,7 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_col
 
 // c2r along x: eight rows per tile, the n1 / 2 + 1 bins of each packed into a
 // complex transform of length n1 / 2 (only real parts of bins 0 and n1 / 2).
+template <int kForm>
 __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_rows_kernel(const FimAxis X, const AxisTables T, const float2* spec,
                                                                float* real, long long rows, float scaling, Moments* rec) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -216,19 +378,23 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
     if (2 * p + 1 < left) b = __ldg(src + static_cast<long long>(2 * p + 1) * (n + 1) + k);
     return C2{pack(a.x, b.x), pack(a.y, b.y)};
   };
+  auto place = [&](int k) {
+    if constexpr (kForm == kFimRader) return __ldg(T.place + k);
+    return k;
+  };
   for (int it = threadIdx.x; it < (half + 1) * kPairs; it += blockDim.x) {
     const int p = it & (kPairs - 1), k = it / kPairs;
     const C2 a = bin(k, p), b = bin(n - k, p);
     if (k == 0) {
-      sh[p] = make_ulonglong2(add(a.re, b.re), sub(a.re, b.re));
+      sh[place(0) * kPairs + p] = make_ulonglong2(add(a.re, b.re), sub(a.re, b.re));
     } else {
       // Bins 0 < k < n count twice (Hermitian): (A_k + conj A_{n-k}) +
       // i e^{2 pi i k / n1} (A_k - conj A_{n-k}).
       const C2 s = C2{add(a.re, b.re), sub(a.im, b.im)};
       const C2 u = times(C2{sub(a.re, b.re), add(a.im, b.im)}, T.pack + k);
       const C2 z = add_i(s, u);
-      sh[k * kPairs + p] = make_ulonglong2(z.re, z.im);
-      if (2 * k != n) sh[(n - k) * kPairs + p] = make_ulonglong2(add(s.re, u.im), sub(u.re, s.im));
+      sh[place(k) * kPairs + p] = make_ulonglong2(z.re, z.im);
+      if (2 * k != n) sh[place(n - k) * kPairs + p] = make_ulonglong2(add(s.re, u.im), sub(u.re, s.im));
     }
   }
   __syncthreads();
@@ -246,7 +412,7 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
     s2[1] = ::fma(g, g, s2[1]);
     count += 2;
   };
-  transform_tile(
+  transform_tile<kForm, true>(
       X, T, sh,
       [&](int e, int p) {
         const ulonglong2 v = sh[e * kPairs + p];
@@ -267,11 +433,85 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
 }
 
 // ------------------------------------------------------------------- plans --
+size_t axis_smem(const FimAxis& X) {
+  return sizeof(float2) * kTile * (static_cast<size_t>(X.f.n) + (X.form == kFimRader ? 2 * X.q : 0));
+}
+
+// Appends the radices of an n-point transform; false when there are none.
+bool append_radices(int n, FftPlan* f) {
+  if (n == 1) return true;
+  FftPlan g{};
+  const bool one = n <= 12 && n != 7 && n != 11;  // a single butterfly
+  if (one) {
+    g.nst = 1;
+    g.r[0] = n;
+  } else if (!fft_plan(n, &g)) {
+    return false;
+  }
+  if (f->nst + g.nst > FftPlan::kMaxStages) return false;
+  for (int s = 0; s < g.nst; ++s) f->r[f->nst++] = g.r[s];
+  return true;
+}
+
+constexpr int kMostBlocks = 64;  // q of Rader's form: q^2 roots, and serial q-point sums
+
+// n = q p with one prime p above 5, p - 1 without prime factors above 5.
+bool rader_axis(int n, FimAxis* X) {
+  int q = 1, p = n;
+  for (int k : {2, 3, 5})
+    while (p % k == 0) p /= k, q *= k;
+  if (p < 7 || q > kMostBlocks) return false;
+  for (int k = 7; k * k <= p; k += 2)
+    if (p % k == 0) return false;
+  FftPlan f{};
+  if (!append_radices(q, &f)) return false;
+  const int sq = f.nst;
+  // At least two stages: a barrier then separates a tile's reads from its writes.
+  if (!append_radices(p - 1, &f) || f.nst < 2) return false;
+  f.n = q * (p - 1);
+  int len = f.n;
+  for (int s = 0; s < f.nst; ++s) {
+    len /= f.r[s];
+    f.m[s] = len;
+    f.inv_m[s] = 1.0f / static_cast<float>(len);
+  }
+  X->f = f;
+  X->form = kFimRader;
+  X->q = q;
+  X->p = p;
+  X->sq = sq;
+  X->inv_len = 1.0f / static_cast<float>(p - 1);
+  auto power = [&](long long b, int e) {
+    long long r = 1;
+    for (b %= p; e > 0; e >>= 1, b = b * b % p)
+      if (e & 1) r = r * b % p;
+    return r;
+  };
+  // g is a primitive root when no g^((p - 1) / prime) is 1.
+  for (X->root = 2;; ++X->root) {
+    bool ok = true;
+    for (int k : {2, 3, 5})
+      if ((p - 1) % k == 0 && power(X->root, (p - 1) / k) == 1) ok = false;
+    if (ok) break;
+  }
+  X->cp = X->cq = 0;
+  for (int v = 0; v < n; v += q)
+    if (v % p == 1) X->cp = v;
+  for (int v = 0; v < n; v += p)
+    if (v % q == 1 % q) {
+      X->cq = v;
+      break;
+    }
+  return true;
+}
+
 bool make_axis(int n, FimAxis* X) {
+  *X = FimAxis{};
   X->n = n;
-  X->blue = 0;
-  if (fft_plan(n, &X->f)) return sizeof(float2) * kTile * static_cast<size_t>(n) <= kSmemMax;
-  X->blue = 1;
+  X->form = kFimPlain;
+  X->q = X->p = 1;
+  if (fft_plan(n, &X->f) || rader_axis(n, X)) return axis_smem(*X) <= kSmemMax;
+  X->form = kFimBluestein;
   const int lo = std::max(4, 2 * n - 1);
   double best = 0.0;
   int found = 0;
@@ -285,10 +525,8 @@ bool make_axis(int n, FimAxis* X) {
       X->f = f;
     }
   }
-  return found && sizeof(float2) * kTile * static_cast<size_t>(found) <= kSmemMax;
+  return found && axis_smem(*X) <= kSmemMax;
 }
-
-size_t axis_smem(const FimAxis& X) { return sizeof(float2) * kTile * static_cast<size_t>(X.f.n); }
 
 // The block size that fills an SM (kSmThreads) with the least idle threads.
 int axis_threads(const FimAxis& X) {
@@ -308,8 +546,33 @@ int axis_threads(const FimAxis& X) {
   return best;
 }
 
-size_t table_bytes(const FimAxis& X) {
-  return sizeof(float4) * (2 * static_cast<size_t>(X.f.n) + 2 * static_cast<size_t>(X.n) + 2) + sizeof(int) * static_cast<size_t>(X.f.n);
+// Lays the tables of an axis out from w; returns their bytes.
+size_t axis_tables(const FimAxis& X, int d, uint8_t* w, TableArgs* A) {
+  size_t at = 0;
+  auto take = [&](size_t count, size_t size) {
+    uint8_t* p = w + at;
+    at += (count * size + 15) / 16 * 16;
+    return p;
+  };
+  const size_t m = X.f.n, n = X.n, q = X.q;
+  A->tw[d] = reinterpret_cast<float4*>(take(m, sizeof(float4)));
+  if (X.form != kFimPlain) A->hat[d] = reinterpret_cast<float4*>(take(m, sizeof(float4)));
+  if (X.form == kFimPlain) A->rev[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
+  if (X.form == kFimBluestein) A->chirp[d] = reinterpret_cast<float4*>(take(n, sizeof(float4)));
+  if (X.form == kFimRader) {
+    A->roots[d] = reinterpret_cast<float4*>(take(q * q, sizeof(float4)));
+    A->src[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
+    A->dst[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
+    A->place[d] = reinterpret_cast<int*>(take(n, sizeof(int)));
+    A->zero[d] = reinterpret_cast<int*>(take(q, sizeof(int)));
+  }
+  if (d == 0) A->pack = reinterpret_cast<float4*>(take(n / 2 + 1, sizeof(float4)));
+  return (at + 255) / 256 * 256;
+}
+
+template <class F>
+cudaError_t most_smem(F* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
 }
 
 cudaError_t ensure_attributes() {
@@ -318,9 +581,12 @@ cudaError_t ensure_attributes() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  const int most = static_cast<int>(kSmemMax);
-  e = cudaFuncSetAttribute(fim_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(fim_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  e = most_smem(fim_columns_kernel<kFimPlain>);
+  if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimBluestein>);
+  if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimRader>);
+  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimPlain>);
+  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimBluestein>);
+  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimRader>);
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
   return e;
 }
@@ -337,8 +603,9 @@ bool fim_fft_plan(const int npts[3], bool three, FimFft* P) {
   for (int d = 1; d < 3; ++d)
     if (npts[d] > 65535) return false;
   P->tables = 0;
+  TableArgs A{};
   for (int d = 0; d < 3; ++d)
-    if (P->ax[d].n) P->tables += (table_bytes(P->ax[d]) + 255) / 256 * 256;
+    if (P->ax[d].n) P->tables += axis_tables(P->ax[d], d, nullptr, &A);
   return true;
 }
 
@@ -358,31 +625,40 @@ cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_t
     A.ax[d] = P.ax[d];
     const FimAxis& X = P.ax[d];
     if (!X.n) continue;
-    float4* q = reinterpret_cast<float4*>(w);
-    A.tw[d] = q;
-    A.hat[d] = q + X.f.n;
-    A.chirp[d] = A.hat[d] + X.f.n;
-    float4* pk = A.chirp[d] + X.n;
-    if (d == 0) A.pack = pk;
-    A.rev[d] = reinterpret_cast<int*>(pk + X.n + 2);
-    T[d] = AxisTables{A.tw[d], A.chirp[d], A.hat[d], A.rev[d], d == 0 ? A.pack : nullptr};
-    w += (table_bytes(X) + 255) / 256 * 256;
-    most = std::max(most, std::max(X.f.n, X.n + 1));
+    w += axis_tables(X, d, w, &A);
+    T[d] = AxisTables{A.tw[d], A.chirp[d], A.hat[d], A.rev[d], A.src[d], A.dst[d], A.place[d], A.zero[d], A.roots[d],
+                      d == 0 ? A.pack : nullptr};
+    most = std::max(most, std::max(X.f.n, std::max(X.n + 1, X.q * X.q)));
   }
   A.n1 = P.n[0];
   fim_tables_kernel<<<dim3((most + 3) / 4, 3), 128, 0, stream>>>(A);
   const int n1h = P.n[0] / 2 + 1;
   const unsigned tiles = static_cast<unsigned>((n1h + kTile - 1) / kTile);
   const long long row = n1h, plane = row * P.n[1];
-  if (P.ax[2].n)
-    fim_columns_kernel<<<dim3(tiles, P.n[1]), axis_threads(P.ax[2]), axis_smem(P.ax[2]), stream>>>(P.ax[2], T[2], spec, n1h,
-                                                                                                   plane, row);
-  if (P.ax[1].n)
-    fim_columns_kernel<<<dim3(tiles, P.n[2]), axis_threads(P.ax[1]), axis_smem(P.ax[1]), stream>>>(P.ax[1], T[1], spec, n1h,
-                                                                                                   row, plane);
+  auto columns = [&](const FimAxis& X, const AxisTables& t, int outer, long long step, long long hop) {
+    const dim3 grid(tiles, outer);
+    const int threads = axis_threads(X);
+    const size_t smem = axis_smem(X);
+    if (X.form == kFimPlain)
+      fim_columns_kernel<kFimPlain><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
+    else if (X.form == kFimRader)
+      fim_columns_kernel<kFimRader><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
+    else
+      fim_columns_kernel<kFimBluestein><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
+  };
+  if (P.ax[2].n) columns(P.ax[2], T[2], P.n[1], plane, row);
+  if (P.ax[1].n) columns(P.ax[1], T[1], P.n[2], row, plane);
   const long long rows = static_cast<long long>(P.n[1]) * P.n[2];
-  fim_rows_kernel<<<static_cast<unsigned>(fim_fft_records(P)), axis_threads(P.ax[0]), axis_smem(P.ax[0]), stream>>>(
-      P.ax[0], T[0], spec, real, rows, scaling, rec);
+  const unsigned blocks = static_cast<unsigned>(fim_fft_records(P));
+  const FimAxis& X = P.ax[0];
+  const int threads = axis_threads(X);
+  const size_t smem = axis_smem(X);
+  if (X.form == kFimPlain)
+    fim_rows_kernel<kFimPlain><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
+  else if (X.form == kFimRader)
+    fim_rows_kernel<kFimRader><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
+  else
+    fim_rows_kernel<kFimBluestein><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
   return cudaGetLastError();
 }
 

@@ -317,9 +317,15 @@ struct FimGrid {
 };
 void fim_grid(const FimInputs& in, FimGrid* g);
 // Inverse transform of the half spectrum (fim_fft.cu).
+enum FimForm { kFimPlain, kFimBluestein, kFimRader };
 struct FimAxis {
-  int n, blue;  // transform length (0: none); 1: Bluestein's form, over f.n points
+  int n, form;  // transform length (0: none); its form, over f.n points
   FftPlan f;
+  // Rader's form: n = q p, p prime; the first sq stages of f are the q-point
+  // transform's. root: a primitive root of p; cq, cp: 1 modulo q (p) and 0
+  // modulo p (q).
+  int q, p, sq, root, cq, cp;
+  float inv_len;  // 1 / (p - 1)
 };
 struct FimFft {
   int n[3];

@@ -1,5 +1,5 @@
-"""The FIM's inverse transform over axis lengths of both forms (plain, and
-Bluestein's for prime factors above 5), even and odd half lengths, tiles that the
+"""The FIM's inverse transform over axis lengths of its forms (plain, and
+Rader's or Bluestein's for prime factors above 5), even and odd half lengths, tiles that the
 x bins and rows do not fill, two-point axes, and axes beyond shared memory
 (cuFFT), through scarf_execute against the FP64 transform of the oracle.
 
@@ -51,3 +51,19 @@ def test_two_dimensions(internal):
 
 def test_rescaled():
     _run((38, 46, 30), rescale=1)
+
+
+@pytest.mark.parametrize("internal", [
+    # y and z: q = 2 to 54 blocks, p - 1 as one butterfly (7, 11, 13) and as
+    # several stages, one and more q-point stages; x: the halves 7 (too short for
+    # a plan of two stages), 17, 19, 31 (one block), 14, 28, 65, 257 and 541
+    (14, 22, 26), (34, 14, 84), (38, 66, 52), (62, 100, 34), (28, 140, 22), (56, 38, 76), (130, 202, 14),
+    (514, 26, 82), (1082, 8, 14)])
+def test_rader_form(internal):
+    _run(internal)
+
+
+@pytest.mark.parametrize("internal", [(44, 1026), (1538, 38), (26, 1082), (102, 420), (36, 462)])
+def test_rader_form_long(internal):
+    # 54 blocks of 19, halves of 769, two blocks of 541, 60 blocks of 7; 462 = 6 x 7 x 11 has two primes (Bluestein)
+    _run(internal)

@@ -12,11 +12,21 @@
 
 #include <cuda_runtime.h>
 
+#include "common.cuh"
 #include "srm_kernels.h"
 
 namespace scarf {
 
 namespace fft {
+
+// Asynchronous copies of a thread's own elements into shared memory.
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // A pair of FP32 values in one 64-bit register and sm_100's packed operations.
 using f2 = unsigned long long;

@@ -28,7 +28,8 @@
 // Bound: shared-memory traffic of the stages. 514^3: cuFFT's transforms took
 // 4.2 ms (z 1.51, y 1.42, x 1.26 with its preprocessing) and the statistics 0.11
 // more; Bluestein's form over 1 080 points (69 KB tiles) 3.2, Rader's over 512
-// (33 KB) 1.8. A q beyond 64 would make the serial q-point sums long: Bluestein.
+// (33 KB) 1.8, and 1.7 with inputs copied asynchronously into their slots (all
+// in flight at once) and rows stored in order. A q beyond 64 would make the serial q-point sums long: Bluestein.
 //
 // The c2r step stores the scaled field (1 / sqrt(n1 n2 n3 dh^n), :1019) and
 // records its statistics (:1027-1036), one record per block, as it goes.
@@ -64,14 +65,13 @@ struct AxisTables {
   const float4* chirp;  // n entries, the same form
   const float4* hat;    // f.n entries
   const int* rev;       // at e - t of the last stage (plain)
-  // Rader's form: input and output of each position, position of each input
-  // (q inputs of residue 0 at f.n .. ), outputs of residue 0, roots of the
-  // q-point transform.
-  const int* src;
+  // Rader's form: output of each position, position of each input (the q of
+  // residue 0 at f.n .. ), outputs of residue 0, roots of the q-point transform.
   const int* dst;
   const int* place;
   const int* zero;
   const float4* roots;
+  const int* from;      // slot of each output (real axis, plain and Rader's form)
   const float4* pack;   // e^{2 pi i k / n1}, k <= n1 / 4 (real axis)
 };
 
@@ -81,11 +81,11 @@ struct TableArgs {
   float4* chirp[3];
   float4* hat[3];
   int* rev[3];
-  int* src[3];
   int* dst[3];
   int* place[3];
   int* zero[3];
   float4* roots[3];
+  int* from;
   float4* pack;
   int n1;
 };
@@ -146,14 +146,17 @@ __device__ void rader_tables(const TableArgs& A, int a, int i, int lane) {
       const int j = i / len, u = i - j * len;
       const int from = static_cast<int>((static_cast<long long>(X.p) * j + static_cast<long long>(X.q) * power_mod(X.root, u, X.p)) % X.n);
       A.tw[a][i] = dup_root(rader_twiddle(X, i));
-      A.src[a][i] = from;
       A.place[a][from] = i;
-      A.dst[a][i] = static_cast<int>((static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, j)) * X.cq +
-                                      static_cast<long long>(power_mod(X.root, len - u, X.p)) * X.cp) % X.n);
+      const int to = static_cast<int>((static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, j)) * X.cq +
+                                       static_cast<long long>(power_mod(X.root, len - u, X.p)) * X.cp) % X.n);
+      A.dst[a][i] = to;
+      if (a == 0) A.from[to] = i;
     }
     if (i < X.q) {
       A.place[a][static_cast<long long>(X.p) * i % X.n] = f.n + i;
-      A.zero[a][i] = static_cast<int>(static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, i)) * X.cq % X.n);
+      const int to = static_cast<int>(static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, i)) * X.cq % X.n);
+      A.zero[a][i] = to;
+      if (a == 0) A.from[to] = f.n + i;
     }
     if (i < X.q * X.q) {
       const int j = i / X.q, b = i - j * X.q;
@@ -201,7 +204,12 @@ __global__ void __launch_bounds__(128) fim_tables_kernel(const TableArgs A) {
     if (i < f.n) A.tw[a][i] = dup_root(twiddle_entry(f, i));
     if (blue && i < X.n) A.chirp[a][i] = dup_root(chirp_turns(i, X.n));
     const int r = f.r[f.nst - 1];
-    if (!blue && i < f.n / r) A.rev[a][i * r] = output_order(f, i);
+    if (!blue && i < f.n / r) {
+      const int k = output_order(f, i);
+      A.rev[a][i * r] = k;
+      if (a == 0)
+        for (int t = 0; t < r; ++t) A.from[k + t * (f.n / r)] = i * r + t;
+    }
   }
   if (!blue || i >= f.n) return;
   // hat[pos] = (1 / M) sum_m conj(c_m) e^{2 pi i m freq / M}, m = -(N-1) .. N-1
@@ -238,40 +246,55 @@ __device__ __forceinline__ C2 times(C2 a, const float4* t) {
   return cmul(a, w.re, w.im);
 }
 
-// The tile's transforms. in(e, p) gives input e < X.n of pair p (kPlaced: the
-// inputs are in the tile, those of Rader's form where `place` says), out(e, p, v)
-// takes output e < X.n.
-template <int kForm, bool kPlaced, class In, class Out>
-__device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTables& T, ulonglong2* sh, In in, Out out) {
+// Slot of input e < X.n in a tile.
+template <int kForm>
+__device__ __forceinline__ int input_slot(const AxisTables& T, int e) {
+  if constexpr (kForm == kFimRader) return __ldg(T.place + e);
+  return e;
+}
+
+// The tile's transforms, its inputs in the tile's slots. Columns: inputs as
+// {re0, im0, re1, im1}, out(e, p, v) takes output e < X.n. Rows (kRows): outputs
+// stay in the slots that `from` gives, except for Bluestein's, whose last stage
+// has them in order. (Leaving from the last stage of the other forms, eight bytes
+// at a time in their order, the rows wrote six times their sectors.)
+template <int kForm, bool kRows, class Out>
+__device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTables& T, ulonglong2* sh, Out out) {
   const FftPlan& f = X.f;
   auto sin = [&](int e, int p) {
     const ulonglong2 v = sh[e * kPairs + p];
     return C2{v.x, v.y};
   };
   auto sout = [&](int e, int p, int, C2 v) { sh[e * kPairs + p] = make_ulonglong2(v.re, v.im); };
+  auto input = [&](int e, int p) {
+    if constexpr (kRows) return sin(e, p);
+    const float4 v = *reinterpret_cast<const float4*>(sh + e * kPairs + p);
+    return C2{pack(v.x, v.z), pack(v.y, v.w)};
+  };
   const int last = f.nst - 1, rl = f.r[last], hop = f.n / rl;
   if constexpr (kForm == kFimPlain) {
-    stage_any<kPairs>(f, 0, T.tw, in, sout);
+    stage_any<kPairs>(f, 0, T.tw, input, sout);
     for (int s = 1; s < last; ++s) {
       __syncthreads();
       stage_any<kPairs>(f, s, T.tw, sin, sout);
     }
     __syncthreads();
-    stage_any<kPairs>(f, last, T.tw, sin,
-                      [&](int e, int p, int t, C2 v) { out(__ldg(T.rev + e - t) + t * hop, p, v); });
+    if constexpr (kRows)
+      stage_any<kPairs>(f, last, T.tw, sin, sout);
+    else
+      stage_any<kPairs>(f, last, T.tw, sin,
+                        [&](int e, int p, int t, C2 v) { out(__ldg(T.rev + e - t) + t * hop, p, v); });
   } else if constexpr (kForm == kFimRader) {
     const int q = X.q;
-    auto first = [&](int e, int p) { return kPlaced ? sin(e, p) : in(__ldg(T.src + e), p); };
-    auto zero = [&](int b, int p) { return kPlaced ? sin(f.n + b, p) : in(b * X.p, p); };
     // Residue 0: q-point transforms into slots f.n + q .. (the last threads,
     // which have the fewest butterflies).
     for (int it = blockDim.x - 1 - threadIdx.x; it < q * kPairs; it += blockDim.x) {
       const int p = it & (kPairs - 1), j = it / kPairs;
-      C2 v = zero(0, p);
-      for (int b = 1; b < q; ++b) v = v + times(zero(b, p), T.roots + j * q + b);
+      C2 v = input(f.n, p);
+      for (int b = 1; b < q; ++b) v = v + times(input(f.n + b, p), T.roots + j * q + b);
       sout(f.n + q + j, p, 0, v);
     }
-    stage_any<kPairs>(f, 0, T.tw, first, sout);
+    stage_any<kPairs>(f, 0, T.tw, input, sout);
     for (int s = 1; s < last; ++s) {
       __syncthreads();
       stage_any<kPairs>(f, s, T.tw, sin, sout);
@@ -286,7 +309,12 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
       sout(f.n + j, p, 0, z + v);
       y = y + z;
     };
-    auto put = [&](int e, int p, int, C2 v) { out(__ldg(T.dst + e), p, v); };
+    auto put = [&](int e, int p, int t, C2 v) {
+      if constexpr (kRows)
+        sout(e, p, t, v);
+      else
+        out(__ldg(T.dst + e), p, v);
+    };
     if (last == X.sq) {
       product_any<kPairs>(f, T.hat, sin, put, constant);
       __syncthreads();
@@ -299,6 +327,7 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
       __syncthreads();
       back_any<kPairs>(f, X.sq, T.tw, sin, put);
     }
+    if constexpr (kRows) return;
     for (int it = blockDim.x - 1 - threadIdx.x; it < q * kPairs; it += blockDim.x) {
       const int p = it & (kPairs - 1), j = it / kPairs;
       out(__ldg(T.zero + j), p, sin(f.n + j, p));
@@ -306,7 +335,7 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
   } else {
     auto bin = [&](int e, int p) {
       if (e >= X.n) return C2{0ull, 0ull};
-      return times(in(e, p), T.chirp + e);
+      return times(input(e, p), T.chirp + e);
     };
     stage_any<kPairs>(f, 0, T.tw, bin, sout);
     for (int s = 1; s < last; ++s) {
@@ -335,28 +364,31 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_col
   const int i0 = blockIdx.x * kTile, left = n1h - i0;
   float2* base = spec + blockIdx.y * outer + i0;
   const bool wide = (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (step & 1) == 0;
-  transform_tile<kForm, false>(
-      X, T, reinterpret_cast<ulonglong2*>(smem),
-      [&](int e, int p) {
-        const float2* s = base + e * step + 2 * p;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (wide && 2 * p + 1 < left) {
-          v = *reinterpret_cast<const float4*>(s);
-        } else {
-          if (2 * p < left) v.x = s[0].x, v.y = s[0].y;
-          if (2 * p + 1 < left) v.z = s[1].x, v.w = s[1].y;
-        }
-        return C2{pack(v.x, v.z), pack(v.y, v.w)};
-      },
-      [&](int e, int p, C2 v) {
-        float2* d = base + e * step + 2 * p;
-        if (wide && 2 * p + 1 < left) {
-          *reinterpret_cast<float4*>(d) = make_float4(lo(v.re), lo(v.im), hi(v.re), hi(v.im));
-        } else {
-          if (2 * p < left) d[0] = make_float2(lo(v.re), lo(v.im));
-          if (2 * p + 1 < left) d[1] = make_float2(hi(v.re), hi(v.im));
-        }
-      });
+  ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
+  for (int it = threadIdx.x; it < X.n * kPairs; it += blockDim.x) {
+    const int p = it & (kPairs - 1), e = it / kPairs;
+    const float2* s = base + e * step + 2 * p;
+    float2* d = reinterpret_cast<float2*>(sh + input_slot<kForm>(T, e) * kPairs + p);
+    if (wide && 2 * p + 1 < left) {
+      cp_async16(d, s);
+    } else {
+      if (2 * p < left) cp_async8(d, s);
+      else d[0] = make_float2(0.0f, 0.0f);
+      if (2 * p + 1 < left) cp_async8(d + 1, s + 1);
+      else d[1] = make_float2(0.0f, 0.0f);
+    }
+  }
+  cp_async_wait();
+  __syncthreads();
+  transform_tile<kForm, false>(X, T, sh, [&](int e, int p, C2 v) {
+    float2* d = base + e * step + 2 * p;
+    if (wide && 2 * p + 1 < left) {
+      *reinterpret_cast<float4*>(d) = make_float4(lo(v.re), lo(v.im), hi(v.re), hi(v.im));
+    } else {
+      if (2 * p < left) d[0] = make_float2(lo(v.re), lo(v.im));
+      if (2 * p + 1 < left) d[1] = make_float2(hi(v.re), hi(v.im));
+    }
+  });
 }
 
 // c2r along x: eight rows per tile, the n1 / 2 + 1 bins of each packed into a
@@ -372,29 +404,35 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
   const float2* src = spec + r0 * (n + 1);
   float* dst = real + r0 * (2 * n);
   ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
-  auto bin = [&](int k, int p) {
-    float2 a = make_float2(0.0f, 0.0f), b = a;
-    if (2 * p < left) a = __ldg(src + static_cast<long long>(2 * p) * (n + 1) + k);
-    if (2 * p + 1 < left) b = __ldg(src + static_cast<long long>(2 * p + 1) * (n + 1) + k);
-    return C2{pack(a.x, b.x), pack(a.y, b.y)};
-  };
-  auto place = [&](int k) {
-    if constexpr (kForm == kFimRader) return __ldg(T.place + k);
-    return k;
-  };
+  // Bin n waits in the slot behind the others (Bluestein's form: an empty one).
+  const int spare = kForm == kFimRader ? X.f.n + 2 * X.q : n;
+  auto slot = [&](int k, int p) { return sh + (k == n ? spare : input_slot<kForm>(T, k)) * kPairs + p; };
+  for (int it = threadIdx.x; it < (n + 1) * kPairs; it += blockDim.x) {
+    const int p = it & (kPairs - 1), k = it / kPairs;
+    float2* d = reinterpret_cast<float2*>(slot(k, p));
+    const float2* s = src + static_cast<long long>(2 * p) * (n + 1) + k;
+    if (2 * p < left) cp_async8(d, s);
+    else d[0] = make_float2(0.0f, 0.0f);
+    if (2 * p + 1 < left) cp_async8(d + 1, s + n + 1);
+    else d[1] = make_float2(0.0f, 0.0f);
+  }
+  cp_async_wait();
+  __syncthreads();
   for (int it = threadIdx.x; it < (half + 1) * kPairs; it += blockDim.x) {
     const int p = it & (kPairs - 1), k = it / kPairs;
-    const C2 a = bin(k, p), b = bin(n - k, p);
+    ulonglong2 *pa = slot(k, p), *pb = slot(n - k, p);
+    const float4 x = *reinterpret_cast<const float4*>(pa), y = *reinterpret_cast<const float4*>(pb);
+    const C2 a = C2{pack(x.x, x.z), pack(x.y, x.w)}, b = C2{pack(y.x, y.z), pack(y.y, y.w)};
     if (k == 0) {
-      sh[place(0) * kPairs + p] = make_ulonglong2(add(a.re, b.re), sub(a.re, b.re));
+      *pa = make_ulonglong2(add(a.re, b.re), sub(a.re, b.re));
     } else {
       // Bins 0 < k < n count twice (Hermitian): (A_k + conj A_{n-k}) +
       // i e^{2 pi i k / n1} (A_k - conj A_{n-k}).
       const C2 s = C2{add(a.re, b.re), sub(a.im, b.im)};
       const C2 u = times(C2{sub(a.re, b.re), add(a.im, b.im)}, T.pack + k);
       const C2 z = add_i(s, u);
-      sh[place(k) * kPairs + p] = make_ulonglong2(z.re, z.im);
-      if (2 * k != n) sh[place(n - k) * kPairs + p] = make_ulonglong2(add(s.re, u.im), sub(u.re, s.im));
+      *pa = make_ulonglong2(z.re, z.im);
+      if (2 * k != n) *pb = make_ulonglong2(add(s.re, u.im), sub(u.re, s.im));
     }
   }
   __syncthreads();
@@ -412,16 +450,19 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
     s2[1] = ::fma(g, g, s2[1]);
     count += 2;
   };
-  transform_tile<kForm, true>(
-      X, T, sh,
-      [&](int e, int p) {
-        const ulonglong2 v = sh[e * kPairs + p];
-        return C2{v.x, v.y};
-      },
-      [&](int e, int p, C2 v) {
-        if (2 * p < left) put(2 * p, e, lo(v.re), lo(v.im));
-        if (2 * p + 1 < left) put(2 * p + 1, e, hi(v.re), hi(v.im));
-      });
+  auto store = [&](int e, int p, C2 v) {
+    if (2 * p < left) put(2 * p, e, lo(v.re), lo(v.im));
+    if (2 * p + 1 < left) put(2 * p + 1, e, hi(v.re), hi(v.im));
+  };
+  transform_tile<kForm, true>(X, T, sh, store);
+  if constexpr (kForm != kFimBluestein) {
+    __syncthreads();
+    for (int it = threadIdx.x; it < n * kPairs; it += blockDim.x) {
+      const int p = it & (kPairs - 1), e = it / kPairs;
+      const ulonglong2 v = sh[__ldg(T.from + e) * kPairs + p];
+      store(e, p, C2{v.x, v.y});
+    }
+  }
   const Moments m = warp_moments(moments_from_shifted(count, shift, s1[0] + s1[1], s2[0] + s2[1]));
   if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = m;
   __syncthreads();
@@ -434,7 +475,7 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_row
 
 // ------------------------------------------------------------------- plans --
 size_t axis_smem(const FimAxis& X) {
-  return sizeof(float2) * kTile * (static_cast<size_t>(X.f.n) + (X.form == kFimRader ? 2 * X.q : 0));
+  return sizeof(float2) * kTile * (static_cast<size_t>(X.f.n) + (X.form == kFimRader ? 2 * X.q : 0) + 1);
 }
 
 // Appends the radices of an n-point transform; false when there are none.
@@ -561,11 +602,11 @@ size_t axis_tables(const FimAxis& X, int d, uint8_t* w, TableArgs* A) {
   if (X.form == kFimBluestein) A->chirp[d] = reinterpret_cast<float4*>(take(n, sizeof(float4)));
   if (X.form == kFimRader) {
     A->roots[d] = reinterpret_cast<float4*>(take(q * q, sizeof(float4)));
-    A->src[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
     A->dst[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
     A->place[d] = reinterpret_cast<int*>(take(n, sizeof(int)));
     A->zero[d] = reinterpret_cast<int*>(take(q, sizeof(int)));
   }
+  if (d == 0 && X.form != kFimBluestein) A->from = reinterpret_cast<int*>(take(n, sizeof(int)));
   if (d == 0) A->pack = reinterpret_cast<float4*>(take(n / 2 + 1, sizeof(float4)));
   return (at + 255) / 256 * 256;
 }
@@ -626,8 +667,8 @@ cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_t
     const FimAxis& X = P.ax[d];
     if (!X.n) continue;
     w += axis_tables(X, d, w, &A);
-    T[d] = AxisTables{A.tw[d], A.chirp[d], A.hat[d], A.rev[d], A.src[d], A.dst[d], A.place[d], A.zero[d], A.roots[d],
-                      d == 0 ? A.pack : nullptr};
+    T[d] = AxisTables{A.tw[d], A.chirp[d], A.hat[d], A.rev[d], A.dst[d], A.place[d], A.zero[d], A.roots[d],
+                      d == 0 ? A.from : nullptr, d == 0 ? A.pack : nullptr};
     most = std::max(most, std::max(X.f.n, std::max(X.n + 1, X.q * X.q)));
   }
   A.n1 = P.n[0];

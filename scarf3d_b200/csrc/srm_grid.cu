@@ -379,14 +379,6 @@ struct SpreadWarp {
 constexpr int kSpreadWarps = 8;
 static_assert(sizeof(SpreadWarp) >= sizeof(float2) * kB * kB * 32, "the partial sums take the entries' place");
 
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 template <int KY>  // cells along y: kB, or 1 when only x is gridded
 struct BinSum {
   float2 acc[kB][KY];
@@ -416,14 +408,14 @@ __device__ __forceinline__ void sum_entries(const GridArgs& A, SpreadWarp& W, in
   const int ent = __shfl_sync(0xffffffffu, hi, rc) - (__shfl_sync(0xffffffffu, pre, rc) - (beg + lane));
   if (lane < n) {
     const float* w = A.weights + static_cast<size_t>(ent) * (2 * kSpan * kB);
-    cp_async16(&W.w[lane][0], w + rc / kSpan * kB);
-    cp_async16(&W.w[lane][kB], w + (kSpan + rc % kSpan) * kB);
+    fft::cp_async16(&W.w[lane][0], w + rc / kSpan * kB);
+    fft::cp_async16(&W.w[lane][kB], w + (kSpan + rc % kSpan) * kB);
   }
   for (int u = 0; u < n; ++u) {
     const int en = __shfl_sync(0xffffffffu, ent, u);
-    cp_async8(&W.e[u][lane], ez + static_cast<size_t>(en) * A.ez);
+    fft::cp_async8(&W.e[u][lane], ez + static_cast<size_t>(en) * A.ez);
   }
-  cp_async_wait();
+  fft::cp_async_wait();
   __syncwarp();
 #pragma unroll 2
   for (int u = 0; u < n; ++u) {

@@ -74,6 +74,12 @@ __device__ __forceinline__ C2 cmul(C2 a, f2 wr, f2 wi) {
 }
 __device__ __forceinline__ C2 scale(C2 a, f2 s) { return C2{mul(a.re, s), mul(a.im, s)}; }
 
+// A complex table entry in both halves.
+__device__ __forceinline__ C2 root(const float2* t) {
+  const float2 w = __ldg(t);
+  return C2{dup(w.x), dup(w.y)};
+}
+
 // Twiddles of the composite radices, evaluated by the compiler.
 constexpr double cos_series(double x) {
   double t = 1.0, s = 1.0;
@@ -213,12 +219,12 @@ struct Dft<12> : DftComposite<4, 3> {};
 // One stage of radix R by the whole block: reads through in(e, p), writes
 // through out(e, p, t, v) where t is the butterfly's output number. In place
 // when both address the tile: a butterfly writes where it read. tw: the
-// plan's twiddles (twiddle_entry) as {wr, wr, wi, wi}; neighbouring
+// plan's twiddles (twiddle_entry); neighbouring
 // butterflies read neighbouring entries (one table of e^{2 pi i k / n} read
 // with a stride took up to eight cache lines per load, and the load unit was
 // what bounded the stages).
 template <int R, int NP, class In, class Out>
-__device__ __forceinline__ void stage(const FftPlan& f, int s, const float4* __restrict__ tw, In in, Out out) {
+__device__ __forceinline__ void stage(const FftPlan& f, int s, const float2* __restrict__ tw, In in, Out out) {
   const int m = f.m[s];
   const int len = m * R;
   const float inv_m = f.inv_m[s];
@@ -233,11 +239,11 @@ __device__ __forceinline__ void stage(const FftPlan& f, int s, const float4* __r
     Dft<R>::run(v);
     if (m > 1) {
       // The stages before this one have n - len entries in all.
-      const float4* w = tw + (f.n - len) + q;
+      const float2* w = tw + (f.n - len) + q;
 #pragma unroll
       for (int t = 1; t < R; ++t, w += m) {
-        const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(w));
-        v[t] = cmul(v[t], x.x, x.y);
+        const C2 x = root(w);
+        v[t] = cmul(v[t], x.re, x.im);
       }
     }
 #pragma unroll
@@ -249,7 +255,7 @@ __device__ __forceinline__ void stage(const FftPlan& f, int s, const float4* __r
 // inverse needs. first(base, p, v, y) sees the butterfly's first value before
 // the product and may change it after.
 template <int R, int NP, class In, class Out, class First>
-__device__ __forceinline__ void product(const FftPlan& f, const float4* __restrict__ hat, In in, Out out, First first) {
+__device__ __forceinline__ void product(const FftPlan& f, const float2* __restrict__ hat, In in, Out out, First first) {
   for (int it = threadIdx.x; it < f.n / R * NP; it += blockDim.x) {
     const int p = it & (NP - 1), base = it / NP * R;
     C2 v[R];
@@ -258,8 +264,8 @@ __device__ __forceinline__ void product(const FftPlan& f, const float4* __restri
     Dft<R>::run(v);
 #pragma unroll
     for (int t = 0; t < R; ++t) {
-      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(hat + base + t));
-      C2 y = cmul(v[t], x.x, x.y);
+      const C2 x = root(hat + base + t);
+      C2 y = cmul(v[t], x.re, x.im);
       if (t == 0) first(base, p, v[0], y);
       v[t] = C2{y.im, y.re};  // the e^{-i} transform is the e^{+i} one with the parts exchanged
     }
@@ -270,7 +276,7 @@ __device__ __forceinline__ void product(const FftPlan& f, const float4* __restri
 }
 // A stage of the e^{-i} transform by decimation in time: stage s undone.
 template <int R, int NP, class In, class Out>
-__device__ __forceinline__ void back(const FftPlan& f, int s, const float4* __restrict__ tw, In in, Out out) {
+__device__ __forceinline__ void back(const FftPlan& f, int s, const float2* __restrict__ tw, In in, Out out) {
   const int m = f.m[s], len = m * R;
   const float inv_m = f.inv_m[s];
   for (int it = threadIdx.x; it < f.n / R * NP; it += blockDim.x) {
@@ -283,12 +289,12 @@ __device__ __forceinline__ void back(const FftPlan& f, int s, const float4* __re
       const C2 x = in(base + t * m, p);
       v[t] = C2{x.im, x.re};
     }
-    const float4* w = tw + (f.n - len) + q;
+    const float2* w = tw + (f.n - len) + q;
 #pragma unroll
     for (int t = 1; t < R; ++t, w += m) {
       // conj(w) x with the parts exchanged is w times the exchanged x
-      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(w));
-      v[t] = cmul(v[t], x.x, x.y);
+      const C2 x = root(w);
+      v[t] = cmul(v[t], x.re, x.im);
     }
     Dft<R>::run(v);
 #pragma unroll
@@ -308,19 +314,19 @@ __device__ __forceinline__ void back(const FftPlan& f, int s, const float4* __re
     default: CALL(2); break;       \
   }
 template <int NP, class In, class Out>
-__device__ __forceinline__ void stage_any(const FftPlan& f, int s, const float4* tw, In in, Out out) {
+__device__ __forceinline__ void stage_any(const FftPlan& f, int s, const float2* tw, In in, Out out) {
 #define SCARF_FFT_CALL(R) stage<R, NP>(f, s, tw, in, out)
   SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[s])
 #undef SCARF_FFT_CALL
 }
 template <int NP, class In, class Out, class First>
-__device__ __forceinline__ void product_any(const FftPlan& f, const float4* hat, In in, Out out, First first) {
+__device__ __forceinline__ void product_any(const FftPlan& f, const float2* hat, In in, Out out, First first) {
 #define SCARF_FFT_CALL(R) product<R, NP>(f, hat, in, out, first)
   SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[f.nst - 1])
 #undef SCARF_FFT_CALL
 }
 template <int NP, class In, class Out>
-__device__ __forceinline__ void back_any(const FftPlan& f, int s, const float4* tw, In in, Out out) {
+__device__ __forceinline__ void back_any(const FftPlan& f, int s, const float2* tw, In in, Out out) {
 #define SCARF_FFT_CALL(R) back<R, NP>(f, s, tw, in, out)
   SCARF_FFT_RADICES(SCARF_FFT_CALL, f.r[s])
 #undef SCARF_FFT_CALL

@@ -61,39 +61,39 @@ constexpr size_t kSmemMax = 224 * 1024;
 // (plain) the output order of the last stage's butterflies; for the real axis
 // the roots of its packing.
 struct AxisTables {
-  const float4* tw;     // {cos, cos, sin, sin}
-  const float4* chirp;  // n entries, the same form
-  const float4* hat;    // f.n entries
+  const float2* tw;     // {cos, sin}
+  const float2* chirp;  // n entries, the same form
+  const float2* hat;    // f.n entries
   const int* rev;       // at e - t of the last stage (plain)
   // Rader's form: output of each position, position of each input (the q of
   // residue 0 at f.n .. ), outputs of residue 0, roots of the q-point transform.
   const int* dst;
   const int* place;
   const int* zero;
-  const float4* roots;
+  const float2* roots;
   const int* from;      // slot of each output (real axis, plain and Rader's form)
-  const float4* pack;   // e^{2 pi i k / n1}, k <= n1 / 4 (real axis)
+  const float2* pack;   // e^{2 pi i k / n1}, k <= n1 / 4 (real axis)
 };
 
 struct TableArgs {
   FimAxis ax[3];
-  float4* tw[3];
-  float4* chirp[3];
-  float4* hat[3];
+  float2* tw[3];
+  float2* chirp[3];
+  float2* hat[3];
   int* rev[3];
   int* dst[3];
   int* place[3];
   int* zero[3];
-  float4* roots[3];
+  float2* roots[3];
   int* from;
-  float4* pack;
+  float2* pack;
   int n1;
 };
 
-__device__ __forceinline__ float4 dup_root(double turns) {
+__device__ __forceinline__ float2 table_root(double turns) {
   double s, c;
   sincospi(2.0 * (turns - rint(turns)), &s, &c);
-  return make_float4(static_cast<float>(c), static_cast<float>(c), static_cast<float>(s), static_cast<float>(s));
+  return make_float2(static_cast<float>(c), static_cast<float>(s));
 }
 // n^2 / (2 N) modulo 1, exactly reduced
 __device__ __forceinline__ double chirp_turns(int n, int N) {
@@ -145,7 +145,7 @@ __device__ void rader_tables(const TableArgs& A, int a, int i, int lane) {
     if (i < f.n) {
       const int j = i / len, u = i - j * len;
       const int from = static_cast<int>((static_cast<long long>(X.p) * j + static_cast<long long>(X.q) * power_mod(X.root, u, X.p)) % X.n);
-      A.tw[a][i] = dup_root(rader_twiddle(X, i));
+      A.tw[a][i] = table_root(rader_twiddle(X, i));
       A.place[a][from] = i;
       const int to = static_cast<int>((static_cast<long long>(stage_frequency(f, 0, X.sq, X.q, j)) * X.cq +
                                        static_cast<long long>(power_mod(X.root, len - u, X.p)) * X.cp) % X.n);
@@ -160,7 +160,7 @@ __device__ void rader_tables(const TableArgs& A, int a, int i, int lane) {
     }
     if (i < X.q * X.q) {
       const int j = i / X.q, b = i - j * X.q;
-      A.roots[a][i] = dup_root(static_cast<double>(b * stage_frequency(f, 0, X.sq, X.q, j) % X.q) / X.q);
+      A.roots[a][i] = table_root(static_cast<double>(b * stage_frequency(f, 0, X.sq, X.q, j) % X.q) / X.q);
     }
   }
   if (i >= f.n) return;
@@ -182,8 +182,7 @@ __device__ void rader_tables(const TableArgs& A, int a, int i, int lane) {
     im += __shfl_down_sync(0xffffffffu, im, o);
   }
   if (lane == 0) {
-    const float x = static_cast<float>(re / len), y = static_cast<float>(im / len);
-    A.hat[a][i] = make_float4(x, x, y, y);
+    A.hat[a][i] = make_float2(static_cast<float>(re / len), static_cast<float>(im / len));
   }
 }
 
@@ -194,15 +193,15 @@ __global__ void __launch_bounds__(128) fim_tables_kernel(const TableArgs A) {
   const FimAxis& X = A.ax[a];
   if (X.n == 0) return;  // axis not transformed
   const FftPlan& f = X.f;
-  if (lane == 0 && a == 0 && i <= X.n / 2) A.pack[i] = dup_root(static_cast<double>(i) / A.n1);
+  if (lane == 0 && a == 0 && i <= X.n / 2) A.pack[i] = table_root(static_cast<double>(i) / A.n1);
   if (X.form == kFimRader) {
     rader_tables(A, a, i, lane);
     return;
   }
   const bool blue = X.form == kFimBluestein;
   if (lane == 0) {
-    if (i < f.n) A.tw[a][i] = dup_root(twiddle_entry(f, i));
-    if (blue && i < X.n) A.chirp[a][i] = dup_root(chirp_turns(i, X.n));
+    if (i < f.n) A.tw[a][i] = table_root(twiddle_entry(f, i));
+    if (blue && i < X.n) A.chirp[a][i] = table_root(chirp_turns(i, X.n));
     const int r = f.r[f.nst - 1];
     if (!blue && i < f.n / r) {
       const int k = output_order(f, i);
@@ -232,17 +231,12 @@ __global__ void __launch_bounds__(128) fim_tables_kernel(const TableArgs A) {
     im += __shfl_down_sync(0xffffffffu, im, o);
   }
   if (lane == 0) {
-    const float x = static_cast<float>(re / f.n), y = static_cast<float>(im / f.n);
-    A.hat[a][i] = make_float4(x, x, y, y);
+    A.hat[a][i] = make_float2(static_cast<float>(re / f.n), static_cast<float>(im / f.n));
   }
 }
 
-__device__ __forceinline__ C2 load2(const float4* t) {
-  const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(t));
-  return C2{v.x, v.y};
-}
-__device__ __forceinline__ C2 times(C2 a, const float4* t) {
-  const C2 w = load2(t);
+__device__ __forceinline__ C2 times(C2 a, const float2* t) {
+  const C2 w = root(t);
   return cmul(a, w.re, w.im);
 }
 
@@ -596,18 +590,18 @@ size_t axis_tables(const FimAxis& X, int d, uint8_t* w, TableArgs* A) {
     return p;
   };
   const size_t m = X.f.n, n = X.n, q = X.q;
-  A->tw[d] = reinterpret_cast<float4*>(take(m, sizeof(float4)));
-  if (X.form != kFimPlain) A->hat[d] = reinterpret_cast<float4*>(take(m, sizeof(float4)));
+  A->tw[d] = reinterpret_cast<float2*>(take(m, sizeof(float2)));
+  if (X.form != kFimPlain) A->hat[d] = reinterpret_cast<float2*>(take(m, sizeof(float2)));
   if (X.form == kFimPlain) A->rev[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
-  if (X.form == kFimBluestein) A->chirp[d] = reinterpret_cast<float4*>(take(n, sizeof(float4)));
+  if (X.form == kFimBluestein) A->chirp[d] = reinterpret_cast<float2*>(take(n, sizeof(float2)));
   if (X.form == kFimRader) {
-    A->roots[d] = reinterpret_cast<float4*>(take(q * q, sizeof(float4)));
+    A->roots[d] = reinterpret_cast<float2*>(take(q * q, sizeof(float2)));
     A->dst[d] = reinterpret_cast<int*>(take(m, sizeof(int)));
     A->place[d] = reinterpret_cast<int*>(take(n, sizeof(int)));
     A->zero[d] = reinterpret_cast<int*>(take(q, sizeof(int)));
   }
   if (d == 0 && X.form != kFimBluestein) A->from = reinterpret_cast<int*>(take(n, sizeof(int)));
-  if (d == 0) A->pack = reinterpret_cast<float4*>(take(n / 2 + 1, sizeof(float4)));
+  if (d == 0) A->pack = reinterpret_cast<float2*>(take(n / 2 + 1, sizeof(float2)));
   return (at + 255) / 256 * 256;
 }
 

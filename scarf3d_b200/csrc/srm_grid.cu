@@ -85,11 +85,11 @@ struct GridArgs {
   int* ntasks;         // three counters: tasks, slots, bins with several parts
   int4* tasks;         // {bin, part, parts, slot} of the bins that blocks sum
   int4* multi;         // {bin, parts, slot, -} of those with several parts
-  // Twiddles as {cos, cos, sin, sin}: of the plans fx and fy, and
+  // Twiddles {cos, sin}: of the plans fx and fy, and
   // e^{2 pi i k / mx} for k <= hx / 2.
-  float4* twx;
-  float4* twy;
-  float4* twr;
+  float2* twx;
+  float2* twy;
+  float2* twr;
   int* revx;
   int* revy;
   int* status;         // error word of the bounded waits
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
   auto root = [&](double turns) {
     double s, c;
     sincospi(2.0 * turns, &s, &c);
-    return make_float4(static_cast<float>(c), static_cast<float>(c), static_cast<float>(s), static_cast<float>(s));
+    return make_float2(static_cast<float>(c), static_cast<float>(s));
   };
   if (t < A.hx) {
     A.twx[t] = root(fft::twiddle_entry(A.fx, static_cast<int>(t)));
@@ -634,9 +634,9 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
         sh[p] = make_ulonglong2(add(a.x, b.x), sub(a.x, b.x));
       } else {
         // P = A_k / 2, Q = conj(A_{n-k}) / 2: (P + Q) + i e^{2 pi i k / mx} (P - Q)
-        const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(A.twr + k));
+        const C2 w = fft::root(A.twr + k);
         const C2 s = scale(C2{add(a.x, b.x), sub(a.y, b.y)}, dup(0.5f));
-        const C2 u = cmul(scale(C2{sub(a.x, b.x), add(a.y, b.y)}, dup(0.5f)), w.x, w.y);
+        const C2 u = cmul(scale(C2{sub(a.x, b.x), add(a.y, b.y)}, dup(0.5f)), w.re, w.im);
         const C2 z = add_i(s, u);
         sh[k * NP + p] = make_ulonglong2(z.re, z.im);
         // index n - k: the conjugate of s - i u
@@ -885,7 +885,7 @@ bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPla
   p.off_t2 = p.ny > 1 ? p.off_partial : p.off_t1;
   p.off_tasks = take(sizeof(int4) * (p.maxtasks + p.maxslots));
   p.off_dc = take(sizeof(float) * (p.nx + 2 + p.ny));
-  p.off_tables = take(sizeof(float4) * (p.mx + p.my) + sizeof(int) * (p.mx + p.my));
+  p.off_tables = take(sizeof(float2) * (p.mx + p.my) + sizeof(int) * (p.mx + p.my));
   p.bytes = off;
   *P = p;
   return true;
@@ -984,7 +984,7 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.partial = reinterpret_cast<float2*>(w + p.off_partial);
   A.tasks = reinterpret_cast<int4*>(w + p.off_tasks);
   A.multi = A.tasks + p.maxtasks;
-  A.twx = reinterpret_cast<float4*>(w + p.off_tables);
+  A.twx = reinterpret_cast<float2*>(w + p.off_tables);
   A.twr = A.twx + p.mx / 2;
   A.twy = A.twr + p.mx / 2;
   A.revx = reinterpret_cast<int*>(A.twy + p.my);

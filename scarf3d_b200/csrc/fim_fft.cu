@@ -28,8 +28,9 @@
 // Bound: shared-memory traffic of the stages. 514^3: cuFFT's transforms took
 // 4.2 ms (z 1.51, y 1.42, x 1.26 with its preprocessing) and the statistics 0.11
 // more; Bluestein's form over 1 080 points (69 KB tiles) 3.2, Rader's over 512
-// (33 KB) 1.8, and 1.7 with inputs copied asynchronously into their slots (all
-// in flight at once) and rows stored in order. A q beyond 64 would make the serial q-point sums long: Bluestein.
+// (33 KB) 1.8, 1.7 with inputs copied asynchronously into their slots (all in
+// flight at once) and rows stored in order, 1.4 with tables of plain entries and
+// 1 024 threads per SM. A q beyond 64 would make the serial q-point sums long: Bluestein.
 //
 // The c2r step stores the scaled field (1 / sqrt(n1 n2 n3 dh^n), :1019) and
 // records its statistics (:1027-1036), one record per block, as it goes.
@@ -49,11 +50,13 @@ using namespace fft;
 
 constexpr int kPairs = 4;               // transform pairs of a tile
 constexpr int kTile = 2 * kPairs;       // transforms of a tile
-// Blocks of at most 256 threads at 80 registers: three per SM at ~1 100 points
-// (Bluestein's form).
-// With 112 registers (two) the transforms of the 514^3 grid took 3.9 ms, with 64
-// (spilling) 3.6, so 3.2.
-constexpr int kMaxThreads = 256, kSmThreads = 3 * kMaxThreads;
+// Threads of an SM and most of a block, by form: the stages wait for memory and
+// barriers, so threads count for more than spills. Transform of 514^3 points
+// (Rader's form) 1 675 us with 640 threads of 96 registers, 1 595 with 768 of 80,
+// 1 565 with 896 of 72 and 1 398 with 1 024 of 64; 256^3 (plain) 164, 161, 156,
+// 153; but 258^3 (Bluestein's, whose radices are larger) 341, 340, 347, 349.
+constexpr int sm_threads(int form) { return form == kFimBluestein ? 768 : 1024; }
+constexpr int most_threads(int) { return 256; }
 constexpr size_t kSmemMax = 224 * 1024;
 
 // Device tables of one axis: twiddles of its plan, then (Bluestein) the chirp
@@ -352,8 +355,8 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
 // c2c along z or y, in place: blockIdx.x selects eight neighbouring x bins,
 // blockIdx.y the row or plane.
 template <int kForm>
-__global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_columns_kernel(const FimAxis X, const AxisTables T, float2* spec, int n1h,
-                                                                  long long step, long long outer) {
+__global__ void __launch_bounds__(most_threads(kForm), sm_threads(kForm) / most_threads(kForm))
+    fim_columns_kernel(const FimAxis X, const AxisTables T, float2* spec, int n1h, long long step, long long outer) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int i0 = blockIdx.x * kTile, left = n1h - i0;
   float2* base = spec + blockIdx.y * outer + i0;
@@ -388,10 +391,11 @@ __global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_col
 // c2r along x: eight rows per tile, the n1 / 2 + 1 bins of each packed into a
 // complex transform of length n1 / 2 (only real parts of bins 0 and n1 / 2).
 template <int kForm>
-__global__ void __launch_bounds__(kMaxThreads, kSmThreads / kMaxThreads) fim_rows_kernel(const FimAxis X, const AxisTables T, const float2* spec,
-                                                               float* real, long long rows, float scaling, Moments* rec) {
+__global__ void __launch_bounds__(most_threads(kForm), sm_threads(kForm) / most_threads(kForm))
+    fim_rows_kernel(const FimAxis X, const AxisTables T, const float2* spec, float* real, long long rows, float scaling,
+                    Moments* rec) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ Moments s_warp[kMaxThreads / 32];
+  __shared__ Moments s_warp[most_threads(kForm) / 32];
   const int n = X.n, half = n / 2;
   const long long r0 = static_cast<long long>(blockIdx.x) * kTile;
   const int left = static_cast<int>(rows - r0 < kTile ? rows - r0 : kTile);
@@ -563,12 +567,12 @@ bool make_axis(int n, FimAxis* X) {
   return found && axis_smem(*X) <= kSmemMax;
 }
 
-// The block size that fills an SM (kSmThreads) with the least idle threads.
+// The block size that fills an SM (sm_threads) with the least idle threads.
 int axis_threads(const FimAxis& X) {
   int best = 128;
   double best_cost = 1e30;
-  for (int t = 64; t <= kMaxThreads; t += 32) {
-    const int blocks = static_cast<int>(std::min<size_t>(std::min<size_t>(kSmemMax / axis_smem(X), kSmThreads / t), 16));
+  for (int t = 64; t <= most_threads(X.form); t += 32) {
+    const int blocks = static_cast<int>(std::min<size_t>(std::min<size_t>(kSmemMax / axis_smem(X), sm_threads(X.form) / t), 16));
     if (blocks < 1) continue;
     double work = 0.0;
     for (int s = 0; s < X.f.nst; ++s) {

@@ -54,6 +54,8 @@ struct GridArgs {
   int mx, my, hx;      // transform lengths, hx = mx / 2
   int nx, ny, nz;      // logical extents: x, gridded second axis (1: none), z
   int sx, sy;          // index of the grid's middle: i' = i - sx, j' = j - sy
+  int ax;              // columns cx < ax that harmonics reach (T1 and T2 hold these)
+  int ylo, yhi, ya;    // cells cy < ylo and the last yhi of my that they reach, ya in all (T1's rows)
   int nbx, nby, nkeys; // cell bins along x and y; start-bin keys
   int nent;            // entries: a harmonic and possibly its mirror
   int nh;
@@ -79,8 +81,8 @@ struct GridArgs {
   // whichever parts these are.
   float2* e;           // [nent][ez]
   // A transform's tile (kZT planes) is one contiguous piece.
-  float2* t1;          // [zc / kZT][hx + 1][my][kZT]
-  float2* t2;          // [zc / kZT][ny][hx + 1][kZT]
+  float2* t1;          // [zc / kZT][ax][ya][kZT]
+  float2* t2;          // [zc / kZT][ny][ax][kZT]
   float2* partial;     // [slot][kB * kB][zc]
   int* ntasks;         // three counters: tasks, slots, bins with several parts
   int4* tasks;         // {bin, part, parts, slot} of the bins that blocks sum
@@ -434,12 +436,14 @@ __device__ __forceinline__ void sum_entries(const GridArgs& A, SpreadWarp& W, in
   }
 }
 
-// T1 cell (cx, cy), plane z of the pass.
-__device__ __forceinline__ size_t t1_index(const GridArgs& A, int cx, int cy, int z) {
+// T1 cell (cx, cy), plane z of the pass; shift: row_shift of the cell's bin.
+__device__ __forceinline__ size_t t1_index(const GridArgs& A, int cx, int cy, int shift, int z) {
   const int g = z / kZT;
-  // A single gridded axis goes straight to step 3, as [zc / kZT][ny = 1][hx + 1][kZT].
-  return ((static_cast<size_t>(g) * (A.hx + 1) + cx) * A.my + cy) * kZT + z % kZT;
+  // A single gridded axis goes straight to step 3, as [zc / kZT][ny = 1][ax][kZT].
+  return ((static_cast<size_t>(g) * A.ax + cx) * A.ya + (cy - shift)) * kZT + z % kZT;
 }
+// Cells minus rows of T1 in a row of bins (a bin is in one of the two pieces).
+__device__ __forceinline__ int row_shift(const GridArgs& A, int by) { return by * kB >= A.ylo ? A.my - A.ya : 0; }
 
 template <int KY>
 __global__ void __launch_bounds__(32 * kSpreadWarps) grid_spread_kernel(const GridArgs A, int task_blocks, int zoff, int zc) {
@@ -474,8 +478,8 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) grid_spread_kernel(const Gr
         const int cx = bx * kB + c / KY, cy = by * kB + c % KY;
         if (T.z > 1)
           A.partial[(static_cast<size_t>(T.w + T.y) * (kB * KY) + c) * zc + z] = v;
-        else if (cx <= A.hx && cy < A.my)
-          A.t1[t1_index(A, cx, cy, z)] = v;
+        else if (cx < A.ax && cy < A.my)
+          A.t1[t1_index(A, cx, cy, row_shift(A, by), z)] = v;
       }
       __syncthreads();
     }
@@ -483,19 +487,21 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) grid_spread_kernel(const Gr
   }
   const int bin = (blockIdx.x - task_blocks) * kSpreadWarps + warp;
   if (bin >= A.nbx * A.nby) return;
+  const int bx = bin / A.nby, by = bin - bx * A.nby;
+  if (by * kB >= A.ylo && by * kB < A.my - A.yhi) return;  // out of reach
   bin_ranges(A, bin, lane, &lo, &hi);
   const int total = __reduce_add_sync(0xffffffffu, hi - lo);
   if (total > kSparse) return;
   sum_entries(A, warps[warp], lane, lo, hi, 0, total, ez, S);
-  const int bx = bin / A.nby, by = bin - bx * A.nby;
+  const int shift = row_shift(A, by);
 #pragma unroll
   for (int i = 0; i < kB; ++i) {
     const int cx = bx * kB + i;
-    if (cx > A.hx) break;
+    if (cx >= A.ax) break;
 #pragma unroll
     for (int j = 0; j < KY; ++j) {
       const int cy = by * kB + j;
-      if (cy < A.my) A.t1[t1_index(A, cx, cy, z)] = S.acc[i][j];
+      if (cy < A.my) A.t1[t1_index(A, cx, cy, shift, z)] = S.acc[i][j];
     }
   }
 }
@@ -521,7 +527,7 @@ __global__ void __launch_bounds__(32 * kB * KY) grid_parts_kernel(const GridArgs
     }
     for (; q < T.y; ++q) v = cadd(v, p[q * hop]);
     const int cx = bx * kB + cell / KY, cy = by * kB + cell % KY;
-    if (cx <= A.hx && cy < A.my) A.t1[t1_index(A, cx, cy, z)] = v;
+    if (cx < A.ax && cy < A.my) A.t1[t1_index(A, cx, cy, row_shift(A, by), z)] = v;
   }
 }
 
@@ -545,16 +551,27 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridAr
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_full;
   const FftPlan& f = A.fy;
-  const uint32_t bytes = static_cast<uint32_t>(A.my) * NP * 16;
+  // Rows of the cells in reach, in two pieces; the gap between them is zero.
+  const uint32_t low = static_cast<uint32_t>(A.ylo) * NP * 16, bytes = static_cast<uint32_t>(A.ya) * NP * 16;
   const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t1);
+  auto issue = [&](int t) {
+    const unsigned char* src = base + static_cast<size_t>(t) * bytes;
+    mbar_arrive_expect_tx(&s_full, bytes);
+    bulk_g2s(smem, src, low, &s_full);
+    if (A.yhi) bulk_g2s(smem + static_cast<size_t>(A.my - A.yhi) * NP * 16, src + low, bytes - low, &s_full);
+  };
   if (threadIdx.x == 0) {
     mbar_init(&s_full, 1);
     fence_mbar_init();
-    if (static_cast<int>(blockIdx.x) < tiles) tile_issue(smem, &s_full, base + static_cast<size_t>(blockIdx.x) * bytes, bytes);
+    if (static_cast<int>(blockIdx.x) < tiles) issue(blockIdx.x);
   }
   __syncthreads();
   ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
-  const int rl = f.r[f.nst - 1], hop = f.n / rl, row = (A.hx + 1) * NP;
+  auto clear_gap = [&] {
+    for (int it = threadIdx.x; it < (A.my - A.ya) * NP; it += blockDim.x) sh[A.ylo * NP + it] = make_ulonglong2(0, 0);
+  };
+  clear_gap();
+  const int rl = f.r[f.nst - 1], hop = f.n / rl, row = A.ax * NP;
   int n = 0;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
     const bool ok = mbar_wait_bounded(&s_full, n & 1, A.status);
@@ -563,7 +580,7 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridAr
       if (threadIdx.x == 0) mbar_wait_drain(&s_full, n & 1);
       return;
     }
-    const int g = t / (A.hx + 1), cx = t - g * (A.hx + 1);
+    const int g = t / A.ax, cx = t - g * A.ax;
     ulonglong2* dst = reinterpret_cast<ulonglong2*>(A.t2) + static_cast<size_t>(g) * A.ny * row + cx * NP;
     auto in = [&](int e, int p) {
       const ulonglong2 v = sh[e * NP + p];
@@ -582,16 +599,17 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_y_kernel(const GridAr
     }
     stage_any<NP>(f, f.nst - 1, A.twy, in, gout);
     __syncthreads();
+    clear_gap();
     const long long next = t + static_cast<long long>(gridDim.x);
     if (threadIdx.x == 0 && next < tiles) {
       fence_proxy_async_smem();
-      tile_issue(smem, &s_full, base + static_cast<size_t>(next) * bytes, bytes);
+      issue(static_cast<int>(next));
     }
   }
 }
 
 // Step 3: inverse real FFT along cx of the planes of a tile (one j): the
-// hx + 1 inputs (real parts only at 0 and hx) as one complex transform of
+// hx + 1 inputs (real parts only at 0 and hx; zero from ax on) as one complex transform of
 // length hx whose output m is (x[2 m], x[2 m + 1]); x rows leave through
 // shared memory, divided by both axes' window transforms.
 __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridArgs A, float* field, int zbeg, int nzc,
@@ -602,7 +620,7 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
   __shared__ __align__(8) uint64_t s_full;
   __shared__ Moments s_warp[kFftMaxThreads / 32];
   const FftPlan& f = A.fx;
-  const uint32_t bytes = static_cast<uint32_t>(A.hx + 1) * NP * 16;
+  const uint32_t bytes = static_cast<uint32_t>(A.ax) * NP * 16;
   const unsigned char* base = reinterpret_cast<const unsigned char*>(A.t2);
   if (threadIdx.x == 0) {
     mbar_init(&s_full, 1);
@@ -612,7 +630,7 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
   __syncthreads();
   int pitch = (A.nx + 2) / 2 * 2;  // even for the paired stores; half of it odd: no bank conflicts
   if (pitch / 2 % 2 == 0) pitch += 2;
-  float* rows = reinterpret_cast<float*>(smem + bytes);
+  float* rows = reinterpret_cast<float*>(smem + static_cast<size_t>(A.hx + 1) * NP * 16);
   ulonglong2* sh = reinterpret_cast<ulonglong2*>(smem);
   const int half = f.n / 2;
   const int rl = f.r[f.nst - 1], hop = f.n / rl;
@@ -629,7 +647,8 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
     const int g = t / A.ny, j = t - g * A.ny, z0 = g * kZT;
     for (int it = threadIdx.x; it < (half + 1) * NP; it += blockDim.x) {
       const int p = it & (NP - 1), k = it / NP;
-      const ulonglong2 a = sh[k * NP + p], b = sh[(f.n - k) * NP + p];
+      const ulonglong2 none = make_ulonglong2(0, 0);
+      const ulonglong2 a = k < A.ax ? sh[k * NP + p] : none, b = f.n - k < A.ax ? sh[(f.n - k) * NP + p] : none;
       if (k == 0) {
         sh[p] = make_ulonglong2(add(a.x, b.x), sub(a.x, b.x));
       } else {
@@ -825,7 +844,15 @@ double window_beta(int n, int m) {
 
 }  // namespace
 
-bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPlan* P) {
+void grid_reach(const scarf_srm_params& p, const scarf_srm_setup& s, double reach[3]) {
+  for (int c = 0; c < 3; ++c) {
+    double q = 0.0;
+    for (int r = 0; r < s.ndim; ++r) q += std::pow(s.m[3 * r + c] / static_cast<double>(p.cl[r]), 2);
+    reach[c] = s.kc * std::sqrt(q) * p.ds / 6.28318530717958647692;
+  }
+}
+
+bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* P) {
   GridPlan p{};
   if (nh <= 0 || nh > kGridMaxHarmonics || n[0] <= 0 || n[1] <= 0 || n[2] <= 0) return false;
   p.ndim = ndim;
@@ -843,14 +870,25 @@ bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPla
   p.my = 1;
   if (p.ny > 1 && !(p.my = fft_length(p.ny, false, &p.fy))) return false;
   if ((p.ny > 1 && tile_y(p) > kSmemMax) || tile_x(p) + rows_x(p) > kSmemMax) return false;
-  p.nbx = (p.mx / 2 + kB) / kB;
+  // Cells that the harmonics' windows reach, with a cell to spare for FP32
+  // wavenumbers; all of them where the reach passes the half period.
+  p.ax = p.mx / 2 + 1;
+  p.ylo = p.my, p.yhi = 0;
+  if (reach) {
+    auto cells = [&](double turns, int m) { return turns < 0.5 ? static_cast<int>(turns * m + 0.5 * kW) + 3 : m; };
+    p.ax = std::min(p.ax, cells(reach[0], p.mx));
+    const int low = (cells(reach[p.ax_y], p.my) + kB - 1) / kB * kB;  // whole bins
+    if (p.ny > 1 && 2 * low < p.my) p.ylo = p.yhi = low;
+  }
+  p.ya = p.ylo + p.yhi;
+  p.nbx = (p.ax + kB - 1) / kB;
   p.nby = p.ny > 1 ? p.my / kB : 1;
   p.nkeys = (p.nbx + kSpan) * p.nby;
   p.nent = 2 * nh;
   const int nzp = (p.nz + 31) / 32 * 32;
   // Planes per pass: about pass_bytes of T1 and T2, the planes shared out
   // evenly (a last pass of a few planes costs as much as one of 32).
-  const size_t per_z = sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * (p.my + (p.ny > 1 ? p.ny : 0));
+  const size_t per_z = sizeof(float2) * static_cast<size_t>(p.ax) * (p.ya + (p.ny > 1 ? p.ny : 0));
   const long long most = std::max<long long>(32, static_cast<long long>(1.3 * static_cast<double>(pass_bytes) / per_z));
   const long long want = (p.nz + most - 1) / most;
   p.zc = static_cast<int>(std::min<long long>((p.nz + 32 * want - 1) / (32 * want) * 32, nzp));
@@ -876,11 +914,11 @@ bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPla
   p.off_bins = take(sizeof(int) * (p.nkeys + 2));
   p.off_weights = take(sizeof(float) * 2 * kSpan * kB * static_cast<size_t>(p.nent));
   p.off_e = take(sizeof(float2) * static_cast<size_t>(p.nent) * p.ez);
-  p.off_t1 = take(sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.my * p.zc);
+  p.off_t1 = take(sizeof(float2) * static_cast<size_t>(p.ax) * p.ya * p.zc);
   // T2 takes the place of the partial sums, which are in T1 by then; a single
   // gridded axis has no T2.
   const size_t partial = sizeof(float2) * static_cast<size_t>(p.maxslots) * kB * (p.ny > 1 ? kB : 1) * p.zc;
-  const size_t t2 = p.ny > 1 ? sizeof(float2) * static_cast<size_t>(p.mx / 2 + 1) * p.ny * p.zc : 0;
+  const size_t t2 = p.ny > 1 ? sizeof(float2) * static_cast<size_t>(p.ax) * p.ny * p.zc : 0;
   p.off_partial = take(std::max(partial, t2));
   p.off_t2 = p.ny > 1 ? p.off_partial : p.off_t1;
   p.off_tasks = take(sizeof(int4) * (p.maxtasks + p.maxslots));
@@ -952,6 +990,7 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.nx = p.nx, A.ny = p.ny, A.nz = p.nz;
   A.sx = p.nx / 4 * 2;  // even: outputs come in pairs
   A.sy = p.ny / 2;
+  A.ax = p.ax, A.ylo = p.ylo, A.yhi = p.yhi, A.ya = p.ya;
   A.nbx = p.nbx, A.nby = p.nby, A.nkeys = p.nkeys;
   A.nent = p.nent, A.nh = p.nh;
   A.ez = p.ez;
@@ -1021,8 +1060,8 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
     }
     const long long groups = (z1 - z0 + kZT - 1) / kZT;
     if (p.ny > 1) {
-      const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * (p.mx / 2 + 1));
-      grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * (p.mx / 2 + 1)));
+      const FftShape y = fft_shape(p.fy, tile_y(p), 0, groups * p.ax);
+      grid_fft_y_kernel<<<y.blocks, y.threads, y.smem, stream>>>(A, static_cast<int>(groups * p.ax));
     }
     const FftShape x = x_shape(p, z1 - z0);
     grid_fft_x_kernel<<<x.blocks, x.threads, x.smem, stream>>>(A, d_field, z0, z1 - z0, x_tiles(p, z1 - z0),

@@ -194,6 +194,7 @@ struct GridPlan {
   int ax_y, ax_z;      // their physical axes
   int mx, my;          // transform lengths
   FftPlan fx, fy;      // of length mx / 2 and my
+  int ax, ylo, yhi, ya;  // cells in reach: columns of x; rows of y (first, last, both)
   int nbx, nby, nkeys, maxtasks, maxslots;
   int zc, ez;          // planes per pass, per build of E
   size_t off_counts, off_keys, off_members, off_par, off_w, off_bins, off_weights, off_e, off_t1, off_t2, off_partial,
@@ -201,7 +202,11 @@ struct GridPlan {
 };
 // False when the form does not take the grid (an axis too long for a
 // transform in shared memory, no or too many harmonics).
-bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, GridPlan* plan);
+bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* plan);
+// The largest wavenumber along each axis (turns per grid step) of a harmonic
+// that the sampler keeps (u <= kc along the ellipsoid of the correlation
+// lengths). grid_make_plan without one (null) keeps every cell.
+void grid_reach(const scarf_srm_params& p, const scarf_srm_setup& s, double reach[3]);
 // Whether the gridded sum is faster than a tensor-core plan, from fits (in us)
 // to measured device times. The contraction pays per wave of output tiles and
 // harmonic and for its tables, the gridded sum per cell of its wavenumber grid

@@ -29,11 +29,11 @@ def _reset():
     sb.set_form(sb.FORM_AUTO)
 
 
-def _case(n, nharm, fs=None, acf=0, frac=0.1, angles=(0.0, 0.0, 0.0), ds=25.0, seed=77, dh=None):
+def _case(n, nharm, fs=None, acf=0, frac=0.1, angles=(0.0, 0.0, 0.0), ds=25.0, seed=77, dh=None, cl=None):
     fs = fs or [1] * len(n)
     fe = [s + v - 1 for s, v in zip(fs, n)]
     span = max(v - 1 for v in n) * ds
-    cl = [max(frac * span, 3 * ds)] * len(n)
+    cl = cl or [max(frac * span, 3 * ds)] * len(n)
     # the domain of the sampler: the largest span along every axis, so that
     # one-point axes do not make the sampling infeasible
     nc, fc = [0.0] * len(n), [span] * len(n)
@@ -92,3 +92,19 @@ def test_several_passes_and_reproducibility():
     sb.scarf_execute(77, pinned.numpy())
     assert np.array_equal(host, a.cpu().numpy()) and np.array_equal(pinned.numpy(), host)
     assert np.array_equal(sh[:4], sa[:4])
+
+
+@pytest.mark.parametrize("n,cl,angles", [
+    # correlation lengths that leave the harmonics few of the cells: along x,
+    # along y, both, neither; turned; two dimensions
+    ((96, 64, 40), (4000.0, 250.0, 250.0), (0.0, 0.0, 0.0)),
+    ((96, 64, 40), (250.0, 4000.0, 250.0), (0.0, 0.0, 0.0)),
+    ((120, 90, 33), (900.0, 700.0, 200.0), (0.0, 0.0, 0.0)),
+    ((48, 40, 36), (300.0, 300.0, 1500.0), (0.0, 0.0, 0.0)),
+    ((120, 90, 33), (900.0, 700.0, 200.0), (35.0, -20.0, 50.0)),
+    ((30, 200, 33), (300.0, 3000.0, 150.0), (-75.0, 0.0, 0.0)),
+    ((300, 140), (2500.0, 300.0), (0.0, 0.0, 0.0)),
+    ((140, 300), (300.0, 2500.0), (40.0, 0.0, 0.0)),
+])
+def test_reach_of_the_harmonics(n, cl, angles):
+    _case(n, 3000, cl=list(cl), angles=angles)

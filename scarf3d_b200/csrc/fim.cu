@@ -482,7 +482,7 @@ void fim_grid(const FimInputs& in, FimGrid* g) {
 namespace {
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 struct FimLayout {
-  size_t off_spec, off_real, off_rec, off_poi, off_out, off_tables, bytes;
+  size_t off_spec, off_real, off_rec, off_poi, off_tables, bytes;
   long long n1h, rows, real, nrec;
   bool own;  // this library's transform; else cuFFT
   FimFft fft;
@@ -503,8 +503,6 @@ FimLayout fim_layout(const FimGrid& g, int npoi) {
   off = align256(off + sizeof(StatRecord) * static_cast<size_t>(L.nrec));
   L.off_poi = off;
   off = align256(off + sizeof(float) * 3 * static_cast<size_t>(std::max(npoi, 1)));
-  L.off_out = off;  // mean, variance
-  off = align256(off + 2 * sizeof(float));
   L.off_tables = off;
   if (L.own) off = align256(off + L.fft.tables);
   L.bytes = off;
@@ -530,7 +528,6 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   float* real = reinterpret_cast<float*>(w + L.off_real);
   StatRecord* rec = reinterpret_cast<StatRecord*>(w + L.off_rec);
   float* d_poi = reinterpret_cast<float*>(w + L.off_poi);
-  float* d_out = reinterpret_cast<float*>(w + L.off_out);
 
   cudaEvent_t ev[5] = {};
   for (auto& x : ev)
@@ -651,15 +648,14 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
     fim_stats_kernel<<<static_cast<unsigned>(L.nrec), kStatThreads, 0, st>>>(real, L.real, scaling, rec);
     if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_stats_kernel", e);
   }
-  if ((e = launch_stats_records(rec, L.nrec, d_out, st)) != cudaSuccess) return failed("statistics", e);
-  float mv[2];
-  if ((e = cudaMemcpyAsync(mv, d_out, sizeof(mv), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-    return failed("statistics copy", e);
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return failed("FIM transform", e);
+  if ((e = launch_stats_records(rec, L.nrec, in.d_result, st)) != cudaSuccess) return failed("statistics", e);
   stats[0] = g.info0;
   stats[1] = g.info1;
-  stats[2] = std::sqrt(mv[1]);
-  stats[3] = mv[0];
+  // The statistics, once the stream has passed their kernel.
+  auto take_statistics = [&] {
+    stats[2] = std::sqrt(in.result[1]);
+    stats[3] = in.result[0];
+  };
   // 5. rescale and taper on the internal grid.
   std::vector<float> pt;
   if (in.rescale == 1 || in.npoi > 0) {
@@ -667,6 +663,8 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
     if (pending != 1.0f) fa.prescale = pending;
     pending = 1.0f;
     if (in.rescale == 1) {
+      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return failed("FIM transform", e);
+      take_statistics();
       fa.rescale = 1;
       fa.scaling = in.sigma / stats[2];
       fa.mean = stats[3];
@@ -718,6 +716,7 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
   if ((e = cudaGetLastError()) != cudaSuccess) return failed("fim_map kernels", e);
   cudaEventRecord(ev[4], st);
   if ((e = cudaEventSynchronize(ev[4])) != cudaSuccess) return failed("FIM mapping", e);
+  if (in.rescale != 1) take_statistics();
   float ms[4] = {0, 0, 0, 0};
   for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]);
   // info(5:8) of the reference's TIMING build: spectrum, symmetry, transform

@@ -188,6 +188,8 @@ struct Resources {
   cudaEvent_t evp = nullptr;  // the coordinates' upload on the copy stream
   std::vector<cudaEvent_t> pass_ev;    // end of each pass of the gridded form
   cudaStream_t copy_stream = nullptr;  // non-blocking: runs beside the legacy stream too
+  float* result = nullptr;             // mean, variance and status word of a call (host-mapped)
+  float* result_dev = nullptr;
   int* slab_flags = nullptr;           // host-mapped, written by the kernel
   int* slab_flags_dev = nullptr;
   int slab_cap = 0;
@@ -203,6 +205,8 @@ struct Resources {
       if (e) cudaEventDestroy(e);
       e = nullptr;
     }
+    if (result) cudaFreeHost(result);
+    result = result_dev = nullptr;
     if (slab_flags) cudaFreeHost(slab_flags);
     slab_flags = slab_flags_dev = nullptr;
     slab_cap = 0;
@@ -271,6 +275,13 @@ int ensure_resources() {
   }
   SCARF_CUDA(t_ctx->res.status.ensure(256));
   SCARF_CUDA(t_ctx->res.stats.ensure(stats_partials_bytes(0) + 256));
+  if (!t_ctx->res.result) {
+    void *h = nullptr, *d = nullptr;
+    SCARF_CUDA(cudaHostAlloc(&h, 4 * sizeof(float), cudaHostAllocMapped | cudaHostAllocPortable));
+    t_ctx->res.result = static_cast<float*>(h);
+    SCARF_CUDA(cudaHostGetDevicePointer(&d, h, 0));
+    t_ctx->res.result_dev = static_cast<float*>(d);
+  }
   if (!t_ctx->res.ev0) SCARF_CUDA(cudaEventCreate(&t_ctx->res.ev0));
   if (!t_ctx->res.ev1) SCARF_CUDA(cudaEventCreate(&t_ctx->res.ev1));
   if (!t_ctx->res.evk0) SCARF_CUDA(cudaEventCreate(&t_ctx->res.evk0));
@@ -678,6 +689,8 @@ int fim_execute_impl(int seed, float* field, float stats[8], int flags) {
     in.d_z = c + 2 * stride;
   }
   SCARF_CUDA(t_ctx->res.work.ensure(fim_workspace_bytes(g, in.npoi)));
+  in.d_result = t_ctx->res.result_dev;
+  in.result = t_ctx->res.result;
   const char* what = "";
   const cudaError_t e = fim_run(in, g, t_ctx->res.work.p, d_field, stats, st, &what);
   if (e != cudaSuccess) return fail(SCARF_ERR_CUDA, "FIM: %s: %s", what, cudaGetErrorString(e));
@@ -882,19 +895,21 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   // returns (var, mean) unchanged; std = sqrt(var) in FP32. The summation
   // kernel recorded per-tile moments as it stored the field; one small
   // kernel merges them (a field without harmonics takes the two FP64 passes
-  // instead). The sum's status word comes back with them in one
-  // synchronisation (after a failed sum the statistics are dropped).
-  double* d_part = static_cast<double*>(t_ctx->res.stats.p);
-  float* d_out = reinterpret_cast<float*>(static_cast<char*>(t_ctx->res.stats.p) + stats_partials_bytes(0));
+  // instead). It writes them and the sum's status word to host-mapped memory,
+  // read after one synchronisation (after a failed sum the statistics are
+  // dropped).
+  volatile float* result = t_ctx->res.result;
+  result[2] = 0.0f;
   if (d_rec)
-    SCARF_CUDA(launch_stats_records(d_rec, nrec, d_out, st));
+    SCARF_CUDA(launch_stats_records(d_rec, nrec, t_ctx->res.result_dev, st, d_status));
   else
-    SCARF_CUDA(launch_field_stats(d_field, npts, d_part, d_out, st));
-  float mv[2];
-  int dev_status = 0;
-  SCARF_CUDA(cudaMemcpyAsync(&dev_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
-  SCARF_CUDA(cudaMemcpyAsync(mv, d_out, sizeof(mv), cudaMemcpyDeviceToHost, st));
+    SCARF_CUDA(launch_field_stats(d_field, npts, static_cast<double*>(t_ctx->res.stats.p), t_ctx->res.result_dev, st));
+  const bool finalizing = p.rescale == 1 || tapering;
+  if (!copied_out && !finalizing) SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, st));
   SCARF_CUDA(cudaStreamSynchronize(st));
+  const float mv[2] = {result[0], result[1]}, word = result[2];
+  int dev_status;
+  std::memcpy(&dev_status, &word, sizeof(int));
   if (dev_status != 0)
     return fail(SCARF_ERR_DEVICE, "device pipeline reported status %d (bounded wait expired)", dev_status);
   if (nh > 0) collect_kernel_time();
@@ -905,7 +920,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
 
   // Rescale (:897-912) and taper (:920-925), in one pass over the field.
   std::vector<float> poi3;
-  if (p.rescale == 1 || tapering) {
+  if (finalizing) {
     FinalizeArgs fa{};
     if (p.rescale == 1) {
       fa.rescale = 1;
@@ -946,7 +961,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, t_ctx->res.copy_stream));
     SCARF_CUDA(cudaStreamSynchronize(t_ctx->res.copy_stream));
   } else {
-    SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, st));
+    if (finalizing) SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, st));
     if (!on_device) {
       rc = copy_field_out(field, d_field, npts, st);
       if (rc) return rc;

@@ -282,7 +282,9 @@ cudaError_t launch_field_stats(const float* d_field, long long n, double* d_part
 // Merge `count` statistics records (overwritten) in record order, by fixed trees,
 // into the FP32 mean and unbiased variance at d_out[0..1], as
 // launch_field_stats reports them.
-cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream);
+// With d_status, d_out[2] takes that word's bits.
+cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream,
+                                 const int* d_status = nullptr);
 // Rescale (when rescale != 0, scarflib_srm.f90:897-912) and the taper of
 // every point of interest (scarflib_common.f90:881-994), in the reference's
 // order, in one pass over the field. d_poi: npoi x 3 floats.
@@ -312,6 +314,8 @@ struct FimInputs {
   long long npts;
   const float* poi;  // host, npoi points of poi_stride floats
   int npoi, poi_stride;
+  float* d_result;               // mean and variance, host-mapped: device address
+  const volatile float* result;  // and host address
 };
 // Internal (FFT) grid: points per axis, offset of its first node, and the
 // reference's info(1:2) flags (scarflib_fim.f90:787-818).

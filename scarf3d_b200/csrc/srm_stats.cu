@@ -125,9 +125,11 @@ __global__ void __launch_bounds__(kGroup) stats_records_group(Moments* rec, long
   if (threadIdx.x == 0) rec[r] = red[0];
 }
 
-// Merges records 0, stride, 2 stride, ... (count of them).
+// Merges records 0, stride, 2 stride, ... (count of them) into out: mean,
+// variance and, given one, the status word. out may be host-mapped: two small
+// copies back after the kernel cost a call ~10 us.
 __global__ void __launch_bounds__(kMergeThreads) stats_records_merge(const Moments* __restrict__ rec, long long count,
-                                                                      int stride, float* out) {
+                                                                      int stride, const int* status, float* out) {
   __shared__ Moments red[kMergeThreads];
   const long long per = (count + kMergeThreads - 1) / kMergeThreads;
   const long long r0 = static_cast<long long>(threadIdx.x) * per;
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(kMergeThreads) stats_records_merge(const Momen
     const Moments t = red[0];
     out[0] = static_cast<float>(t.mean);
     out[1] = static_cast<float>(t.m2 / (t.n - 1.0));
+    if (status) out[2] = __int_as_float(*status);
   }
 }
 
@@ -223,7 +226,8 @@ cudaError_t launch_field_stats(const float* d_field, long long n, double* d_part
   return cudaGetLastError();
 }
 
-cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream) {
+cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_out, cudaStream_t stream,
+                                 const int* d_status) {
   int stride = 1;
   if (count > 4 * kMergeThreads) {
     const long long groups = (count + kGroup - 1) / kGroup;
@@ -231,7 +235,7 @@ cudaError_t launch_stats_records(StatRecord* d_rec, long long count, float* d_ou
     count = groups;
     stride = kGroup;
   }
-  stats_records_merge<<<1, kMergeThreads, 0, stream>>>(d_rec, count, stride, d_out);
+  stats_records_merge<<<1, kMergeThreads, 0, stream>>>(d_rec, count, stride, d_status, d_out);
   return cudaGetLastError();
 }
 

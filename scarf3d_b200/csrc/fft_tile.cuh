@@ -160,6 +160,30 @@ struct Dft<5> {
   }
 };
 template <>
+struct Dft<7> {
+  static __device__ __forceinline__ void run(C2* v) {
+    // cos and sin of 2 pi k / 7, k = 1, 2, 3
+    constexpr float c[3] = {0.62348980185873353053f, -0.22252093395631440429f, -0.90096886790241912624f};
+    constexpr float s[3] = {0.78183148246802980871f, 0.97492791218182360702f, 0.43388373911755812048f};
+    const C2 p[3] = {v[1] + v[6], v[2] + v[5], v[3] + v[4]}, d[3] = {v[1] - v[6], v[2] - v[5], v[3] - v[4]};
+    const C2 x0 = v[0];
+    v[0] = v[0] + (p[0] + (p[1] + p[2]));
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+      C2 m = x0, n = C2{0ull, 0ull};
+#pragma unroll
+      for (int t = 1; t <= 3; ++t) {
+        const int e = k * t % 7, at = (e <= 3 ? e : 7 - e) - 1;
+        const f2 cc = dup(c[at]), ss = dup(e <= 3 ? s[at] : -s[at]);
+        m = C2{fma(p[t - 1].re, cc, m.re), fma(p[t - 1].im, cc, m.im)};
+        n = t == 1 ? scale(d[0], ss) : C2{fma(d[t - 1].re, ss, n.re), fma(d[t - 1].im, ss, n.im)};
+      }
+      v[k] = add_i(m, n);
+      v[7 - k] = sub_i(m, n);
+    }
+  }
+};
+template <>
 struct Dft<8> {
   static __device__ __forceinline__ void run(C2* v) {
     constexpr float r = 0.70710678118654752440f;
@@ -307,6 +331,7 @@ __device__ __forceinline__ void back(const FftPlan& f, int s, const float2* __re
     case 10: CALL(10); break;      \
     case 9: CALL(9); break;        \
     case 8: CALL(8); break;        \
+    case 7: CALL(7); break;        \
     case 6: CALL(6); break;        \
     case 5: CALL(5); break;        \
     case 4: CALL(4); break;        \

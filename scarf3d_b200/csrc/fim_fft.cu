@@ -10,10 +10,10 @@
 // memory (fft_tile.cuh): decimation in frequency forwards, whose output order
 // the product with the transformed chirp and the decimation in time backwards
 // take as it is; the last stage forwards, the product and the first stage
-// backwards are one step in registers. Lengths without larger prime factors take
+// backwards are one step in registers. Lengths without prime factors above 7 take
 // a plain transform.
 //
-// N = q p with p prime and p - 1 without prime factors above 5 (514 = 2 x 257)
+// N = q p with p prime and p - 1 without prime factors above 7 (514 = 2 x 257)
 // takes a shorter way. Indices n = p b + q m and k = (k mod q, k mod p) split the
 // transform into q-point ones over b and p-point ones over m without twiddles
 // (Good 1958, Thomas 1963), and the p-point ones are, with a primitive root g,
@@ -30,7 +30,8 @@
 // more; Bluestein's form over 1 080 points (69 KB tiles) 3.2, Rader's over 512
 // (33 KB) 1.8, 1.7 with inputs copied asynchronously into their slots (all in
 // flight at once) and rows stored in order, 1.4 with tables of plain entries and
-// 1 024 threads per SM. A q beyond 64 would make the serial q-point sums long: Bluestein.
+// 1 024 threads per SM. Radix 7 puts 258 = 6 x 43 (43 - 1 = 6 x 7) there too:
+// 258^3 341 -> 208 us. A q beyond 64 would make the serial q-point sums long: Bluestein.
 //
 // The c2r step stores the scaled field (1 / sqrt(n1 n2 n3 dh^n), :1019) and
 // records its statistics (:1027-1036), one record per block, as it goes.
@@ -54,7 +55,8 @@ constexpr int kTile = 2 * kPairs;       // transforms of a tile
 // barriers, so threads count for more than spills. Transform of 514^3 points
 // (Rader's form) 1 675 us with 640 threads of 96 registers, 1 595 with 768 of 80,
 // 1 565 with 896 of 72 and 1 398 with 1 024 of 64; 256^3 (plain) 164, 161, 156,
-// 153; but 258^3 (Bluestein's, whose radices are larger) 341, 340, 347, 349.
+// 153; but 402 x 402 x 202 (Bluestein's along x and y, whose radices are larger)
+// 543, 518, 525, 541.
 constexpr int sm_threads(int form) { return form == kFimBluestein ? 768 : 1024; }
 constexpr int most_threads(int) { return 256; }
 constexpr size_t kSmemMax = 224 * 1024;
@@ -480,11 +482,11 @@ size_t axis_smem(const FimAxis& X) {
 bool append_radices(int n, FftPlan* f) {
   if (n == 1) return true;
   FftPlan g{};
-  const bool one = n <= 12 && n != 7 && n != 11;  // a single butterfly
+  const bool one = n <= 12 && n != 11;  // a single butterfly
   if (one) {
     g.nst = 1;
     g.r[0] = n;
-  } else if (!fft_plan(n, &g)) {
+  } else if (!fft_plan(n, &g, 7)) {
     return false;
   }
   if (f->nst + g.nst > FftPlan::kMaxStages) return false;
@@ -494,13 +496,13 @@ bool append_radices(int n, FftPlan* f) {
 
 constexpr int kMostBlocks = 64;  // q of Rader's form: q^2 roots, and serial q-point sums
 
-// n = q p with one prime p above 5, p - 1 without prime factors above 5.
+// n = q p with one prime p above 7, p - 1 without prime factors above 7.
 bool rader_axis(int n, FimAxis* X) {
   int q = 1, p = n;
-  for (int k : {2, 3, 5})
+  for (int k : {2, 3, 5, 7})
     while (p % k == 0) p /= k, q *= k;
-  if (p < 7 || q > kMostBlocks) return false;
-  for (int k = 7; k * k <= p; k += 2)
+  if (p < 11 || q > kMostBlocks) return false;
+  for (int k = 11; k * k <= p; k += 2)
     if (p % k == 0) return false;
   FftPlan f{};
   if (!append_radices(q, &f)) return false;
@@ -529,7 +531,7 @@ bool rader_axis(int n, FimAxis* X) {
   // g is a primitive root when no g^((p - 1) / prime) is 1.
   for (X->root = 2;; ++X->root) {
     bool ok = true;
-    for (int k : {2, 3, 5})
+    for (int k : {2, 3, 5, 7})
       if ((p - 1) % k == 0 && power(X->root, (p - 1) / k) == 1) ok = false;
     if (ok) break;
   }
@@ -549,7 +551,7 @@ bool make_axis(int n, FimAxis* X) {
   X->n = n;
   X->form = kFimPlain;
   X->q = X->p = 1;
-  if (fft_plan(n, &X->f) || rader_axis(n, X)) return axis_smem(*X) <= kSmemMax;
+  if (fft_plan(n, &X->f, 7) || rader_axis(n, X)) return axis_smem(*X) <= kSmemMax;
   X->form = kFimBluestein;
   const int lo = std::max(4, 2 * n - 1);
   double best = 0.0;

@@ -16,12 +16,12 @@
 // part), so only cx in [0, Mx/2] is kept; the parts of a harmonic's cells
 // outside that range fold back as the cells of a mirror entry (-w, conj E).
 // The work is ~1.5 x 2.25 cells per point through two FFT passes plus 81
-// multiply-adds per harmonic and plane, where the factorised contraction
+// multiply-adds per harmonic and plane (144 with the bins' margins), where the factorised contraction
 // (srm_tc.cu) takes 12 tensor operations per point and harmonic.
 //
-// Precision: phases in FP64, E, weights and FFTs in FP32; ~4e-7 of the
-// field's standard deviation against FP64 where the split-BF16 contraction
-// has ~5e-6. Summation order is fixed (sorted entries, fixed partial sums),
+// Precision: phases in FP64, E, weights and FFTs in FP32; 2.4e-7 to 1.1e-6 of
+// the field's standard deviation (rms) against FP64, where the split-BF16
+// contraction has ~5e-6. Summation order is fixed (sorted entries, fixed partial sums),
 // so a field is reproducible bit for bit.
 #include <cuda_runtime.h>
 
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(kFftMaxThreads) grid_fft_x_kernel(const GridAr
 }
 
 // ------------------------------------------------------------------- plans --
-// Stages of an FFT of length n (2, 3, 5-smooth): the fewest, with the
+// Stages of an FFT of length n (primes up to 7): the fewest, with the
 // smallest largest radix (registers) among those; descending radices.
 bool factor(int rest, int most, int depth, int* r, int* best, int* nbest) {
   if (rest == 1) {
@@ -747,7 +747,7 @@ bool factor(int rest, int most, int depth, int* r, int* best, int* nbest) {
     return true;
   }
   if (depth == FftPlan::kMaxStages) return false;
-  for (int k : {12, 10, 9, 8, 6, 5, 4, 3, 2})
+  for (int k : {12, 10, 9, 8, 7, 6, 5, 4, 3, 2})
     if (k <= most && rest % k == 0) {
       r[depth] = k;
       factor(rest / k, k, depth + 1, r, best, nbest);
@@ -756,11 +756,11 @@ bool factor(int rest, int most, int depth, int* r, int* best, int* nbest) {
 }
 }  // namespace
 
-bool fft_plan(int n, FftPlan* f) {
+bool fft_plan(int n, FftPlan* f, int most_prime) {
   if (n < 4) return false;
   int rest = n;
-  for (int k : {2, 3, 5})
-    while (rest % k == 0) rest /= k;
+  for (int k : {2, 3, 5, 7})
+    while (k <= most_prime && rest % k == 0) rest /= k;
   if (rest != 1) return false;
   int r[FftPlan::kMaxStages], nst = 0;
   f->n = n;

@@ -186,8 +186,9 @@ struct FftPlan {
   float inv_m[kMaxStages];
 };
 
-// False when n has a prime factor above 5 or fewer than two stages.
-bool fft_plan(int n, FftPlan* f);
+// False when n has a prime factor above most_prime (5 or 7) or fewer than two
+// stages.
+bool fft_plan(int n, FftPlan* f, int most_prime = 5);
 struct GridPlan {
   int ndim, nh, nent;
   int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly

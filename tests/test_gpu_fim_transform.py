@@ -67,3 +67,10 @@ def test_rader_form(internal):
 def test_rader_form_long(internal):
     # 54 blocks of 19, halves of 769, two blocks of 541, 60 blocks of 7; 462 = 6 x 7 x 11 has two primes (Bluestein)
     _run(internal)
+
+
+@pytest.mark.parametrize("internal", [
+    # radix 7: plain lengths (halves of 49, 35 and 21), p - 1 with a factor 7 (29, 43, 71, 113), 7 in q
+    (98, 42, 28), (70, 126, 14), (42, 58, 86), (58, 98, 142), (172, 28, 226), (154, 34, 20), (258, 14, 258)])
+def test_factors_of_seven(internal):
+    _run(internal)

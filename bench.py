@@ -887,7 +887,7 @@ def run_b200(args, w):
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(nh * 20),
                     "d2h_bytes_per_step": int(npts * 4 + 8), "ms_per_step": t_e2e / args.steps * 1e3,
                     "host_sampling_ms": float(np.mean(host_s)) * 1e3, "device_ms": float(np.mean(device_s)) * 1e3,
-                    "host_memory": "page-locked",
+                    "host_memory": "page-locked", "form": "automatic (gridded Fourier sum where it is the faster)",
                     "pageable": {"value": work_total / t_e2e_pageable, "unit": UNIT,
                                  "ms_per_step": t_e2e_pageable / args.steps * 1e3,
                                  "host_memory": "pageable (numpy, malloc'd)", "field_equals_pinned": pageable_ok}},

@@ -95,7 +95,7 @@ int scarf_set_device_memory_cap(size_t bytes);
 size_t scarf_device_memory_in_use(void);
 /* Frees the device buffers the library keeps between calls (they are
  * allocated again on demand), and the FIM's cuFFT plans of the current
- * device (kept between calls; their work areas are cuFFT's own allocations,
+ * device (made for axes too long for its own transforms, kept between calls; their work areas are cuFFT's own allocations,
  * outside the cap); waits for the library's device work first. */
 int scarf_release_device_memory(void);
 /* Self-test of the bounded waits inside every pipeline kernel: `blocks`
@@ -188,8 +188,8 @@ int scarf_srm_tc_autotune(const scarf_srm_setup *s, const int fs[3], const int n
 int scarf_fim_internal_grid(int ndim, const float nc[3], const float fc[3], float dh, const float cl[3], int pad,
                             int npts[3], float off_axis[3], float flags[2]);
 /* Device bytes the FIM workspace of that grid takes (spectrum, transform
- * output, statistics records, points of interest; cuFFT's own work area
- * comes on top). */
+ * output, statistics records, points of interest, transform tables; where an
+ * axis needs cuFFT, its own work area comes on top). */
 size_t scarf_fim_workspace_bytes(const int npts[3], int npoi);
 
 /* Status-returning scarf_execute (c_binding.c:138-143); stats[8] as the

@@ -584,9 +584,9 @@ def tc_plan_info(ndim: int, n, nh: int) -> dict:
 
 
 def set_output_overlap(items_per_slab: int = 1):
-    """scarf_execute: copy finished field slabs (about items_per_slab work
-    items each; 1 = default size) to the host while the kernel runs, or the
-    whole field afterwards (0)."""
+    """scarf_execute: copy finished passes of the gridded sum, or slabs of the
+    tensor-core form (about items_per_slab work items each; 1 = default size),
+    to the host while the rest is computed, or the whole field afterwards (0)."""
     check(lib.scarf_set_output_overlap(int(items_per_slab)))
 
 

@@ -102,11 +102,34 @@ struct GridArgs {
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 
 // ------------------------------------------------------------- preparation --
+// I0(2 sqrt(z)) = sum_k z^k / (k!)^2 for 0 <= z < 200 (beta <= 28): every term is
+// positive, so Horner's rule keeps full relative precision; the first term left
+// out is below 1e-13 of the sum. A branch-free third of CUDA's cyl_bessel_i0 and
+// the square root of its argument.
+constexpr int kBesselTerms = 38;
+struct BesselSeries {
+  double c[kBesselTerms];
+  constexpr BesselSeries() : c() {
+    double v = 1.0;
+    for (int k = 0; k < kBesselTerms; ++k) {
+      c[k] = v;
+      v /= static_cast<double>(k + 1) * (k + 1);
+    }
+  }
+};
+__device__ __forceinline__ double bessel_i0_of(double z) {
+  constexpr BesselSeries s{};
+  double v = s.c[kBesselTerms - 1];
+#pragma unroll
+  for (int k = kBesselTerms - 2; k >= 0; --k) v = fma(v, z, s.c[k]);
+  return v;
+}
+
 // Kaiser-Bessel weight at distance d (cells) from a harmonic's wavenumber.
 __device__ __forceinline__ float kb_weight(double d, double beta, double inv_i0) {
   const double x = d * (2.0 / kW);
   const double t = 1.0 - x * x;
-  return t <= 0.0 ? 0.0f : static_cast<float>(cyl_bessel_i0(beta * sqrt(t)) * inv_i0);
+  return t <= 0.0 ? 0.0f : static_cast<float>(bessel_i0_of(0.25 * beta * beta * t) * inv_i0);
 }
 
 // One thread per item: every harmonic's wavenumber in cells, its phase at

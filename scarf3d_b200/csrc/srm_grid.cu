@@ -138,11 +138,11 @@ __device__ __forceinline__ float kb_weight(double d, double beta, double inv_i0)
 __device__ __forceinline__ int first_cell(double c) { return static_cast<int>(ceil(c - 0.5 * kW)); }
 __device__ __forceinline__ int floor_bin(int c) { return (c >= 0 ? c : c - (kB - 1)) / kB; }
 
-__device__ float window_inverse(int n, int m, double beta) {
+__device__ float window_inverse(int n, int m, double beta, double inv_i0) {
   const double pi = 3.14159265358979323846;
   const double u = pi * kW * n / m;
   const double r = sqrt(beta * beta - u * u);
-  return static_cast<float>(cyl_bessel_i0(beta) * r / (kW * sinh(r)));
+  return static_cast<float>(r / (inv_i0 * kW * sinh(r)));
 }
 
 __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
@@ -219,12 +219,12 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
   }
   t -= A.my;
   if (t < A.nx) {
-    A.dcx[t] = window_inverse(static_cast<int>(t) - A.sx, A.mx, A.beta_x) * A.scaling;
+    A.dcx[t] = window_inverse(static_cast<int>(t) - A.sx, A.mx, A.beta_x, A.inv_i0_x) * A.scaling;
     return;
   }
   t -= A.nx;
   if (t < A.ny) {
-    A.dcy[t] = A.ny > 1 ? window_inverse(static_cast<int>(t) - A.sy, A.my, A.beta_y) : 1.0f;
+    A.dcy[t] = A.ny > 1 ? window_inverse(static_cast<int>(t) - A.sy, A.my, A.beta_y, A.inv_i0_y) : 1.0f;
     return;
   }
   t -= A.ny;
@@ -336,7 +336,16 @@ __global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z
   if (first) {
     const int lo = A.bin_start[key], hi = A.bin_start[key + 1];
     int before = 0;
-    for (int k = lo + lane; k < hi; k += 32) before += A.members[k] < e ? 1 : 0;
+    // Four members per load: bins near zero wavenumber hold thousands of
+    // entries, each counting all of them.
+    const int head = min((lo + 3) & ~3, hi), tail = head + ((hi - head) & ~3);
+    if (lo + lane < head) before += A.members[lo + lane] < e ? 1 : 0;
+    if (tail + lane < hi) before += A.members[tail + lane] < e ? 1 : 0;
+#pragma unroll 4
+    for (int k = head + 4 * lane; k < tail; k += 128) {
+      const int4 m = *reinterpret_cast<const int4*>(A.members + k);
+      before += (m.x < e ? 1 : 0) + (m.y < e ? 1 : 0) + (m.z < e ? 1 : 0) + (m.w < e ? 1 : 0);
+    }
     i = lo + __reduce_add_sync(0xffffffffu, before);
     if (lane == 0) A.place[e] = i;
   } else {

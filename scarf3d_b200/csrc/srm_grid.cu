@@ -181,9 +181,16 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
       s -= s >= A.my ? A.my : 0;
       return static_cast<uint32_t>(bx * A.nby + s / kB);
     };
+    // One atomic per bin and warp: thousands of entries share the bins near
+    // zero wavenumber (20 000 harmonics: 11 us with one each, 6 so).
     auto arrive = [&](uint32_t k) {
-      const bool none = static_cast<int>(k) >= A.nkeys;
-      return make_uint2(k, none ? 0u : static_cast<uint32_t>(atomicAdd(A.counts + k, 1)));
+      if (static_cast<int>(k) >= A.nkeys) return make_uint2(k, 0u);
+      const unsigned same = __match_any_sync(__activemask(), k);
+      const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+      int at = 0;
+      if (lane == leader) at = atomicAdd(A.counts + k, __popc(same));
+      at = __shfl_sync(same, at, leader);
+      return make_uint2(k, static_cast<uint32_t>(at + __popc(same & ((1u << lane) - 1u))));
     };
     A.keys[t] = arrive(key(cx, cy));
     // Mirror entry: cells below 0 or above hx, folded back.

@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "common.cuh"
@@ -617,18 +618,19 @@ cudaError_t most_smem(F* kernel) {
 }
 
 cudaError_t ensure_attributes() {
-  static bool done[64] = {};
+  static std::atomic<unsigned long long> done[64];  // context ids
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  const unsigned long long ctx = current_context_id();
+  if (dev >= 0 && dev < 64 && ctx != 0 && done[dev] == ctx) return cudaSuccess;
   e = most_smem(fim_columns_kernel<kFimPlain>);
   if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimBluestein>);
   if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimRader>);
   if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimPlain>);
   if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimBluestein>);
   if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimRader>);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = ctx;
   return e;
 }
 

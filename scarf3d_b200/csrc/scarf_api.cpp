@@ -813,7 +813,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
     grid_reach(p, s, reach);
     const double* bound = t_ctx->cfg.src.srng ? nullptr : reach;
     bool use_grid = t_ctx->cfg.form == SCARF_FORM_AUTO && nh > 0 &&
-                    grid_make_plan(s.ndim, n, nh, overlap ? kGridHostPassBytes : kGridPassBytes, bound, &grid) &&
+                    grid_make_plan(n, nh, overlap ? kGridHostPassBytes : kGridPassBytes, bound, &grid) &&
                     (!planned || grid_pays(grid, plan));
     auto grid_fits = [&] {
       if (want_records(grid_stat_records(grid)) == SCARF_OK && t_ctx->res.work.ensure(grid.bytes) == cudaSuccess)
@@ -823,7 +823,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
       return false;
     };
     if (use_grid && !grid_fits())  // smaller passes, then the tensor-core form
-      use_grid = grid_make_plan(s.ndim, n, nh, 0, bound, &grid) && grid_fits();
+      use_grid = grid_make_plan(n, nh, 0, bound, &grid) && grid_fits();
     if (use_grid) {
       if (overlap) {
         rc = ensure_pass_resources(grid_passes(grid));

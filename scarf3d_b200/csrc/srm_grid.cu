@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 
@@ -60,7 +61,6 @@ struct GridArgs {
   int nent;            // entries: a harmonic and possibly its mirror
   int nh;
   long long ez;        // z pitch of E
-  int maxtasks, maxslots;
   double beta_x, beta_y, inv_i0_x, inv_i0_y;
   double m[9], bar[3], ds;
   int fs[3];           // first index (1-based) of the axes x, y, z of the caller
@@ -891,10 +891,9 @@ void grid_reach(const scarf_srm_params& p, const scarf_srm_setup& s, double reac
   }
 }
 
-bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* P) {
+bool grid_make_plan(const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* P) {
   GridPlan p{};
   if (nh <= 0 || nh > kGridMaxHarmonics || n[0] <= 0 || n[1] <= 0 || n[2] <= 0) return false;
-  p.ndim = ndim;
   p.nh = nh;
   p.nx = n[0];
   // The second axis is transformed, the third summed exactly; a single plane
@@ -998,13 +997,14 @@ long long grid_stat_records(const GridPlan& p) {  // one per block of every pass
 }
 
 namespace {
-// Dynamic shared-memory limits, raised once per device.
+// Dynamic shared-memory limits, raised once per device context.
 cudaError_t ensure_grid_attributes() {
-  static bool done[64] = {};
+  static std::atomic<unsigned long long> done[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  const unsigned long long ctx = current_context_id();
+  if (dev >= 0 && dev < 64 && ctx != 0 && done[dev] == ctx) return cudaSuccess;
   const int most = static_cast<int>(kSmemMax);
   const int spread = static_cast<int>(sizeof(SpreadWarp) * kSpreadWarps);
   e = cudaFuncSetAttribute(grid_spread_kernel<kB>, cudaFuncAttributeMaxDynamicSharedMemorySize, spread);
@@ -1012,7 +1012,7 @@ cudaError_t ensure_grid_attributes() {
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(grid_fft_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(grid_fft_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = ctx;
   return e;
 }
 }  // namespace
@@ -1033,8 +1033,6 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.nbx = p.nbx, A.nby = p.nby, A.nkeys = p.nkeys;
   A.nent = p.nent, A.nh = p.nh;
   A.ez = p.ez;
-  A.maxtasks = p.maxtasks;
-  A.maxslots = p.maxslots;
   A.beta_x = window_beta(p.nx, p.mx);
   A.beta_y = window_beta(p.ny, p.my);
   A.inv_i0_x = 1.0 / std::cyl_bessel_i(0.0, A.beta_x);

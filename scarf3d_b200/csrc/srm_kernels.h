@@ -190,7 +190,7 @@ struct FftPlan {
 // stages.
 bool fft_plan(int n, FftPlan* f, int most_prime = 5);
 struct GridPlan {
-  int ndim, nh, nent;
+  int nh, nent;
   int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly
   int ax_y, ax_z;      // their physical axes
   int mx, my;          // transform lengths
@@ -203,7 +203,7 @@ struct GridPlan {
 };
 // False when the form does not take the grid (an axis too long for a
 // transform in shared memory, no or too many harmonics).
-bool grid_make_plan(int ndim, const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* plan);
+bool grid_make_plan(const int n[3], int nh, size_t pass_bytes, const double reach[3], GridPlan* plan);
 // The largest wavenumber along each axis (turns per grid step) of a harmonic
 // that the sampler keeps (u <= kc along the ellipsoid of the correlation
 // lengths). grid_make_plan without one (null) keeps every cell.

@@ -266,6 +266,47 @@ class CtxScope {
   scarf_ctx* prev_;
 };
 
+// Page-locked memory for the table rows that an execute samples and uploads.
+// One for all contexts, under g_mu (page-locking one per context cost every
+// first call): only the execute that holds g_mu writes or reads it, and that
+// execute's upload has ended when it returns (RowsUpload). The sampling entry
+// points, which do not take g_mu, fill their callers' tables.
+struct TableRows {
+  char* p = nullptr;
+  size_t bytes = 0;
+  // Null (and nothing kept) beyond kMost bytes or without page-locked memory.
+  static constexpr size_t kMost = size_t(64) << 20;
+  float* ensure(size_t need) {
+    if (need > bytes) {
+      release();
+      void* h = nullptr;
+      if (need > kMost || cudaHostAlloc(&h, need, cudaHostAllocPortable) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+      }
+      p = static_cast<char*>(h);
+      bytes = need;
+    }
+    return reinterpret_cast<float*>(p);
+  }
+  void release() {
+    if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
+    p = nullptr;
+    bytes = 0;
+  }
+};
+TableRows g_rows;
+
+// Waits, on a return before the execute's own synchronisation, for the upload
+// of the rows.
+struct RowsUpload {
+  cudaStream_t st;
+  bool pending = true;
+  ~RowsUpload() {
+    if (pending) cudaStreamSynchronize(st);
+  }
+};
+
 int ensure_resources() {
   int dev = 0;
   SCARF_CUDA(cudaGetDevice(&dev));
@@ -729,16 +770,15 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   const int threads = t_ctx->cfg.threads > 0 ? t_ctx->cfg.threads : host_threads();
   long long pairs = 0;
   const bool on_gpu = !t_ctx->cfg.src.srng && t_ctx->cfg.sampler != SCARF_SAMPLER_HOST;
+  // The table's rows: page-locked where there is room, else the vector's.
   std::vector<float> table;
-  const float* rows = nullptr;  // in memory of the device sampler's, or the table
-  int nh;
-  if (on_gpu) {
-    nh = srm_sample_field(p, s, nullptr, &rows, &pairs, st, nullptr);
-  } else {
-    table.resize(5 * static_cast<size_t>(p.nharm));
-    nh = srm_sample(p, s, &t_ctx->cfg.src, threads, table.data(), &pairs);
+  float* rows = g_rows.ensure(5 * sizeof(float) * static_cast<size_t>(std::max(p.nharm, 0)));
+  if (!rows) {
+    table.resize(5 * static_cast<size_t>(std::max(p.nharm, 0)));
     rows = table.data();
   }
+  const int nh = on_gpu ? srm_sample_field(p, s, rows, &pairs, st, nullptr)
+                        : srm_sample(p, s, &t_ctx->cfg.src, threads, rows, &pairs);
   if (nh == -2) return sampler_fail("device sampler");
   if (nh < 0)
     return fail(SCARF_ERR_ARG,
@@ -770,6 +810,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   SCARF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   if (nh > 0)
     SCARF_CUDA(cudaMemcpyAsync(d_table, rows, sizeof(float) * 5 * nh, cudaMemcpyHostToDevice, st));
+  RowsUpload rows_upload{st};
 
   const float* dx = nullptr;
   const float* dy = nullptr;
@@ -907,6 +948,7 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   const bool finalizing = p.rescale == 1 || tapering;
   if (!copied_out && !finalizing) SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, st));
   SCARF_CUDA(cudaStreamSynchronize(st));
+  rows_upload.pending = false;
   const float mv[2] = {result[0], result[1]}, word = result[2];
   int dev_status;
   std::memcpy(&dev_status, &word, sizeof(int));
@@ -1334,7 +1376,7 @@ int scarf_srm_sample_device(const scarf_srm_params* p, const scarf_srm_setup* s,
   if (!p || !s || !table) return fail(SCARF_ERR_ARG, "NULL argument");
   scarf::take_device_alloc_failure();
   long long used = 0, open = 0;
-  const int kept = srm_sample_field(*p, *s, table, nullptr, &used, stream, &open);
+  const int kept = srm_sample_field(*p, *s, table, &used, stream, &open);
   if (kept == -1)
     return fail(SCARF_ERR_ARG, "rejection sampling infeasible: acceptance rate %.3g < %.1g", acceptance_rate(*s),
                 kMinAcceptance);
@@ -1681,6 +1723,7 @@ int scarf_release_device_memory(void) {
   }
   scarf::release_sampler_device_memory();
   scarf::release_field_sampler_memory();
+  g_rows.release();
   scarf::release_fim_plans();
   return SCARF_OK;
 }

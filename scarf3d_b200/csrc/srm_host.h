@@ -87,11 +87,9 @@ double acceptance_rate(const scarf_srm_setup& s);
 int srm_sample_device(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
                       void* stream, long long* uncertain);
 // The same table (and counts) by the single-field form of the device scan
-// (srm_sample_field.cu); scarf_execute's sampler. With `staged`, table may be
-// null and the rows are wherever *staged says: memory of the sampler's own
-// (page-locked, usually), valid until its next call.
-int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, const float** staged,
-                     long long* pairs_used, void* stream, long long* uncertain);
+// (srm_sample_field.cu); scarf_execute's sampler.
+int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
+                     void* stream, long long* uncertain);
 void release_field_sampler_memory();
 // Host decision for a pair the device left open (glibc spectrum), and a
 // harmonic's table row from u and the three pairs drawn after it.

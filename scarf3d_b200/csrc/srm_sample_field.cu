@@ -227,10 +227,9 @@ struct FieldSampler {
   int device = -1;
   unsigned long long ctx = 0;
   Buf work;
-  char* host = nullptr;  // page-locked: header, words, draws, staged table rows
+  char* host = nullptr;  // page-locked: header, words, draws
   size_t host_bytes = 0;
-  std::vector<uint32_t> kept;    // candidates that became harmonics
-  std::vector<float> fallback;   // rows of the batched sampler for a caller without a table
+  std::vector<uint32_t> kept;  // candidates that became harmonics
 };
 FieldSampler g_field;
 
@@ -284,23 +283,11 @@ void release_field_sampler_memory() {
   if (g_field.host) cudaFreeHost(g_field.host);
   g_field.host = nullptr;
   g_field.host_bytes = 0;
-  g_field.fallback = std::vector<float>();
 }
 
-int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, const float** staged,
-                     long long* pairs_used, void* stream_handle, long long* uncertain) {
-  // The batched sampler (chained passes) into the caller's table, or into a
-  // buffer of this sampler's that stays until its next call.
-  auto batched = [&]() {
-    float* t = table;
-    if (!t) {
-      std::lock_guard<std::mutex> lk(g_field.mu);
-      g_field.fallback.resize(5 * static_cast<size_t>(p.nharm));
-      t = g_field.fallback.data();
-    }
-    if (staged) *staged = t;
-    return srm_sample_device(p, s, t, pairs_used, stream_handle, uncertain);
-  };
+int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
+                     void* stream_handle, long long* uncertain) {
+  auto batched = [&] { return srm_sample_device(p, s, table, pairs_used, stream_handle, uncertain); };
   const cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
   const double acc = acceptance_rate(s);
   if (acc < kMinAcceptance) return -1;
@@ -326,8 +313,7 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
   const size_t off_reject = sizeof(int) * (static_cast<size_t>(blocks) + 4) / 16 * 16 + 16;
   const size_t off_out = off_reject + sizeof(uint32_t) * kRejectBins;
   const size_t off_draws = 64 + sizeof(uint32_t) * static_cast<size_t>((room + 15) / 16 * 16);
-  const size_t off_rows = off_draws + sizeof(Draws8) * static_cast<size_t>(room);
-  const size_t host_need = off_rows + (staged ? 5 * sizeof(float) * static_cast<size_t>(p.nharm) : 0);
+  const size_t host_need = off_draws + sizeof(Draws8) * static_cast<size_t>(room);
   if (host_need > kMaxStaging) {
     lk.unlock();
     return batched();
@@ -385,7 +371,6 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
   }
   const uint32_t* words = reinterpret_cast<const uint32_t*>(S.host + 64);
   const Draws8* draws = reinterpret_cast<const Draws8*>(S.host + off_draws);
-  float* rows = staged ? reinterpret_cast<float*>(S.host + off_rows) : table;
   if (S.kept.size() < static_cast<size_t>(p.nharm)) S.kept.resize(p.nharm);
   uint32_t* kept_at = S.kept.data();
   // The walk, in stream order exactly as the serial loop consumes pairs:
@@ -424,10 +409,9 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
     const int r1 = std::min(kept, (b + 1) * kRowBlock);
     for (int r = b * kRowBlock; r < r1; ++r) {
       const float* d = draws[kept_at[r]].r;
-      sampler_row(d[0] * (s.kmax - s.kmin) + s.kmin, d + 2, s.ndim, p.cl, rows + 5 * static_cast<size_t>(r));
+      sampler_row(d[0] * (s.kmax - s.kmin) + s.kmin, d + 2, s.ndim, p.cl, table + 5 * static_cast<size_t>(r));
     }
   });
-  if (staged) *staged = rows;
   if (pairs_used) *pairs_used = pos;
   if (uncertain) *uncertain = open;
   return kept;

@@ -170,6 +170,13 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
       a = -a;
     }
     if (wy < 0.0) wy += 1.0;
+    // A rotation or a caller's draws may not be finite. No cell index comes
+    // from such a wavenumber or phase: the harmonic stands at zero wavenumber
+    // with a phase that is no number, so that every value of the field is none.
+    if (!(isfinite(k[0]) && isfinite(k[1]) && isfinite(k[2]) && isfinite(ph))) {
+      wx = wy = wz = 0.0;
+      ph = __longlong_as_double(0x7ff8000000000000ll);
+    }
     const double cx = wx * A.mx, cy = wy * A.my;
     A.par[t] = make_double4(ph - rint(ph), wz, a, b);
     A.w[t] = make_double2(cx, cy);
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(128) grid_prep_kernel(const GridArgs A) {
     // One atomic per bin and warp: thousands of entries share the bins near
     // zero wavenumber (20 000 harmonics: 11 us with one each, 6 so).
     auto arrive = [&](uint32_t k) {
-      if (static_cast<int>(k) >= A.nkeys) return make_uint2(k, 0u);
+      if (k >= static_cast<uint32_t>(A.nkeys)) return make_uint2(k, 0u);
       const unsigned same = __match_any_sync(__activemask(), k);
       const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
       int at = 0;
@@ -307,7 +314,7 @@ __global__ void __launch_bounds__(256) grid_bins_kernel(const GridArgs A, int sc
     const int e = blockIdx.x * 256 + threadIdx.x;
     if (e >= A.nent) return;
     const uint2 k = A.keys[e];
-    if (static_cast<int>(k.x) < A.nkeys) A.members[A.bin_start[k.x] + k.y] = e;
+    if (k.x < static_cast<uint32_t>(A.nkeys)) A.members[A.bin_start[k.x] + k.y] = e;
     return;
   }
   const int bin = (blockIdx.x - scatter_blocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -337,8 +344,8 @@ __global__ void __launch_bounds__(256) grid_bins_kernel(const GridArgs A, int sc
 __global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z0, int nzc, int first) {
   const int e = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (e >= A.nent) return;
-  const int key = static_cast<int>(A.keys[e].x);
-  if (key >= A.nkeys) return;  // no mirror
+  const uint32_t key = A.keys[e].x;
+  if (key >= static_cast<uint32_t>(A.nkeys)) return;  // no mirror
   int i;
   if (first) {
     const int lo = A.bin_start[key], hi = A.bin_start[key + 1];

@@ -45,6 +45,9 @@ constexpr double kOversample = 1.5;
 constexpr int kSparse = 32;       // entries of a bin that one warp sums
 constexpr int kPart = 256;        // entries that one block sums (32 per warp)
 constexpr int kScanThreads = 1024;
+constexpr int kDense = 2048;      // entries of a start bin ranked by a block, where blocks rank
+constexpr int kRankThreads = 1024;
+constexpr int kRankWords = 8192;  // bitmap words of a ranking block: 262 144 entry numbers at a time
 constexpr int kZT = 8;            // planes of a transform tile
 constexpr int kPairs = kZT / 2;
 constexpr int kFftMaxThreads = 512;
@@ -60,6 +63,7 @@ struct GridArgs {
   int nbx, nby, nkeys; // cell bins along x and y; start-bin keys
   int nent;            // entries: a harmonic and possibly its mirror
   int nh;
+  int ranked;          // bins of more than kDense entries are ranked by blocks
   long long ez;        // z pitch of E
   double beta_x, beta_y, inv_i0_x, inv_i0_y;
   double m[9], bar[3], ds;
@@ -84,7 +88,8 @@ struct GridArgs {
   float2* t1;          // [zc / kZT][ax][ya][kZT]
   float2* t2;          // [zc / kZT][ny][ax][kZT]
   float2* partial;     // [slot][kB * kB][zc]
-  int* ntasks;         // three counters: tasks, slots, bins with several parts
+  int* ntasks;         // four counters: tasks, slots, bins with several parts, dense start bins
+  int* dense;          // keys of the start bins that blocks rank
   int4* tasks;         // {bin, part, parts, slot} of the bins that blocks sum
   int4* multi;         // {bin, parts, slot, -} of those with several parts
   // Twiddles {cos, sin}: of the plans fx and fy, and
@@ -283,6 +288,7 @@ __global__ void __launch_bounds__(kScanThreads) grid_scan_kernel(const GridArgs 
     for (int u = 0; u < 4; ++u) {
       const int k = base + 4 * t + u;
       if (k <= A.nkeys) A.bin_start[k] = at;
+      if (A.ranked && v[u] > kDense) A.dense[atomicAdd(A.ntasks + 3, 1)] = k;
       at += v[u];
     }
     carry += all;
@@ -337,6 +343,61 @@ __global__ void __launch_bounds__(256) grid_bins_kernel(const GridArgs A, int sc
   for (int p = lane; p < parts; p += 32) A.tasks[task + p] = make_int4(bin, p, parts, slot);
 }
 
+// Places of the entries of dense start bins, one block per bin at a time: a
+// bitmap of the bin's entry numbers, whose set bits below an entry's are its
+// rank. Linear in the bin, where counting every member for each entry
+// (grid_entry_kernel) is quadratic. Bound: two passes over the members, one
+// block per bin.
+__global__ void __launch_bounds__(kRankThreads) grid_rank_kernel(const GridArgs A) {
+  __shared__ uint32_t s_bits[kRankWords];
+  __shared__ int s_before[kRankThreads], s_warp[kRankThreads / 32];
+  constexpr int kEach = kRankWords / kRankThreads;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int n = A.ntasks[3];
+  for (int d = blockIdx.x; d < n; d += gridDim.x) {
+    const int key = A.dense[d], lo = A.bin_start[key], hi = A.bin_start[key + 1];
+    int base = lo;
+    for (int e0 = 0; e0 < A.nent; e0 += 32 * kRankWords) {
+      for (int w = t; w < kRankWords; w += kRankThreads) s_bits[w] = 0u;
+      __syncthreads();
+      for (int i = lo + t; i < hi; i += kRankThreads) {
+        const uint32_t b = static_cast<uint32_t>(A.members[i] - e0);
+        if (b < 32u * kRankWords) atomicOr(s_bits + (b >> 5), 1u << (b & 31u));
+      }
+      __syncthreads();
+      // Set bits before each run of kEach words.
+      int mine = 0;
+#pragma unroll
+      for (int w = 0; w < kEach; ++w) mine += __popc(s_bits[t * kEach + w]);
+      int x = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_warp[warp] = x;
+      __syncthreads();
+      int before = x - mine, all = 0;
+      for (int w = 0; w < kRankThreads / 32; ++w) {
+        before += w < warp ? s_warp[w] : 0;
+        all += s_warp[w];
+      }
+      s_before[t] = before;
+      __syncthreads();
+      for (int i = lo + t; i < hi; i += kRankThreads) {
+        const int e = A.members[i];
+        const uint32_t b = static_cast<uint32_t>(e - e0);
+        if (b >= 32u * kRankWords) continue;
+        const int word = static_cast<int>(b >> 5);
+        int rank = s_before[word / kEach] + __popc(s_bits[word] & ((1u << (b & 31u)) - 1u));
+        for (int w = word / kEach * kEach; w < word; ++w) rank += __popc(s_bits[w]);
+        A.place[e] = base + rank;
+      }
+      base += all;
+      __syncthreads();  // the bitmap is read
+    }
+  }
+}
+
 // One warp per entry: its place among its bin's entries (ordered by entry
 // number: a fixed order makes every sum over a bin reproducible), its weights
 // aligned to bins, and E along z: FP64 phases, stepped by 32 planes with one
@@ -347,8 +408,8 @@ __global__ void __launch_bounds__(128) grid_entry_kernel(const GridArgs A, int z
   const uint32_t key = A.keys[e].x;
   if (key >= static_cast<uint32_t>(A.nkeys)) return;  // no mirror
   int i;
-  if (first) {
-    const int lo = A.bin_start[key], hi = A.bin_start[key + 1];
+  const int lo = A.bin_start[key], hi = A.bin_start[key + 1];
+  if (first && !(A.ranked && hi - lo > kDense)) {
     int before = 0;
     // Four members per load: bins near zero wavenumber hold thousands of
     // entries, each counting all of them.
@@ -951,9 +1012,9 @@ bool grid_make_plan(const int n[3], int nh, size_t pass_bytes, const double reac
     off = align256(off + bytes);
     return at;
   };
-  p.off_counts = take(sizeof(int) * (p.nkeys + 3));
+  p.off_counts = take(sizeof(int) * (p.nkeys + 4));
   p.off_keys = take(sizeof(uint2) * p.nent);
-  p.off_members = take(2 * sizeof(int) * p.nent);
+  p.off_members = take(2 * sizeof(int) * p.nent + sizeof(int) * (p.nent / kDense + 1));
   p.off_par = take(sizeof(double4) * nh);
   p.off_w = take(sizeof(double2) * nh);
   p.off_bins = take(sizeof(int) * (p.nkeys + 2));
@@ -1057,6 +1118,8 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
   A.keys = reinterpret_cast<uint2*>(w + p.off_keys);
   A.members = reinterpret_cast<int*>(w + p.off_members);
   A.place = A.members + p.nent;
+  A.dense = A.place + p.nent;
+  A.ranked = p.nh > kGridCountedHarmonics ? 1 : 0;
   A.par = reinterpret_cast<double4*>(w + p.off_par);
   A.w = reinterpret_cast<double2*>(w + p.off_w);
   A.bin_start = reinterpret_cast<int*>(w + p.off_bins);
@@ -1077,12 +1140,13 @@ cudaError_t launch_grid_structured(const scarf_srm_setup& s, const int fs[3], fl
 
   const long long items = static_cast<long long>(p.nh) + 2 * (p.mx + p.my) + p.nx + p.ny;
   // Entry counts and the task counters behind them.
-  if ((e = cudaMemsetAsync(A.counts, 0, sizeof(int) * (p.nkeys + 3), stream)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(A.counts, 0, sizeof(int) * (p.nkeys + 4), stream)) != cudaSuccess) return e;
   grid_prep_kernel<<<static_cast<unsigned>((items + 127) / 128), 128, 0, stream>>>(A);
   grid_scan_kernel<<<1, kScanThreads, 0, stream>>>(A);
   const int nbins = p.nbx * p.nby;
   const int scatter = (p.nent + 255) / 256;
   grid_bins_kernel<<<scatter + (nbins + 7) / 8, 256, 0, stream>>>(A, scatter);
+  if (A.ranked) grid_rank_kernel<<<148, kRankThreads, 0, stream>>>(A);
   const int task_blocks = std::min(p.maxtasks, 148 * 4);
   for (int pass = 0; pass < grid_passes(p); ++pass) {
     int z0, z1;

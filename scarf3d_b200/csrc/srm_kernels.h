@@ -171,6 +171,14 @@ cudaError_t tc_batch_launch(const TcBatchPlan& plan, void* d_work, cudaStream_t 
 
 // ---- gridded Fourier form of structured sums (srm_grid.cu) ----
 constexpr int kGridMaxHarmonics = 1 << 20;
+// Beyond this many harmonics, blocks rank the entries of dense start bins (one
+// launch more); below, each entry counts its bin's members, which is quadratic
+// in a bin. Counted / ranked, 64 x 64 points, long correlation lengths (nearly
+// all harmonics in a few bins): 121 / 106 us at 10 000, 226 / 140 at 20 000,
+// 878 / 257 at 50 000, 11 497 / 1 017 at 200 000, 280 / 6.6 ms at 1 000 000.
+// Short ones, 128^3: 119 / 123 us at 5 000, 143 / 147 at 10 000, 199 / 206 at
+// 20 000, 379 / 374 at 50 000.
+constexpr int kGridCountedHarmonics = 1 << 14;
 // T1 and T2 of one pass. Passes that fit L2 (48-96 MB) gained nothing from it,
 // and each kernel of a small pass ends in a wave that fills part of the chip:
 // 512^3 x 20 000 2.20 ms at 48 MB, 1.99 at 128, 1.82 at 400, 1.69 at 1 500. Fields

@@ -324,9 +324,10 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
     S.host = nullptr;
     S.host_bytes = 0;
     void* h = nullptr;
-    if (cudaHostAlloc(&h, host_need, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return -2;
+    const size_t bytes = (host_need + (size_t(1) << 20) - 1) >> 20 << 20;  // whole megabytes: few reallocations
+    if (cudaHostAlloc(&h, bytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return -2;
     S.host = static_cast<char*>(h);
-    S.host_bytes = host_need;
+    S.host_bytes = bytes;
   }
   void* dev_host = nullptr;
   if (cudaHostGetDevicePointer(&dev_host, S.host, 0) != cudaSuccess) return -2;

@@ -1,0 +1,63 @@
+"""Fields into ordinary (pageable) host arrays, through the page-locked ring:
+bit for bit the device field, for sizes around a slot's and a piece's edges,
+in contexts that take turns, after the library's buffers were given back."""
+import numpy as np
+import pytest
+
+import scarf3d_b200 as sb
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _reset():
+    yield
+    sb.scarf_finalize()
+    sb.set_nharm(10000)
+    sb.set_form(sb.FORM_AUTO)
+
+
+def _init(n, method, nharm=2000):
+    sb.set_nharm(nharm)
+    span = [max(v - 1, 1) * 50.0 for v in n]
+    sb.scarf_initialize(fs=[1] * len(n), fe=list(n), ds=50.0, acf=0, cl=[0.1 * max(span)] * len(n), sigma=0.05,
+                        hurst=0.3, method=method, nc=[0.0] * len(n), fc=[max(span)] * len(n))
+
+
+def _both(n, seed=5):
+    dev, _ = sb.scarf_execute(seed, torch.full((int(np.prod(n)),), float("nan"), device="cuda"))
+    host, _ = sb.scarf_execute(seed, np.full(int(np.prod(n)), np.nan, np.float32))
+    assert np.array_equal(host, dev.cpu().numpy())
+
+
+# 2^18 points are 1 MB: a field just below, at and above a slot of one thread's
+# copy; four slots; slots of several pieces with and without a last partial one;
+# beyond the size whose quarters are slots
+@pytest.mark.parametrize("n", [
+    (511, 513), (512, 512), (513, 512), (1024, 1025), (1201, 800), (64, 64, 64), (127, 129, 65), (203, 151, 97),
+    (256, 256, 128), (257, 255, 129), (320, 288, 100)])
+@pytest.mark.parametrize("method,form", [(1, sb.FORM_AUTO), (1, sb.FORM_TC), (0, sb.FORM_AUTO)])
+def test_host_field_is_the_device_field(n, method, form):
+    sb.set_form(form)
+    _init(n, method)
+    _both(n)
+
+
+def test_contexts_take_turns():
+    sizes = [(64, 64, 64), (300, 200), (256, 200, 160), (40, 30, 20)]
+    ctxs = [sb.Context() for _ in sizes]
+    try:
+        for turn in range(3):
+            for i, (c, n) in enumerate(zip(ctxs, sizes)):
+                with c:
+                    if turn == 0:
+                        _init(n, i % 2)
+                    _both(n, seed=turn + 1)
+            if turn == 1:
+                sb.release_device_memory()
+    finally:
+        for c in ctxs:
+            with c:
+                sb.scarf_finalize()
+            c.close()

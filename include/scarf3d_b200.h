@@ -94,7 +94,8 @@ int scarf_set_device_memory_cap(size_t bytes);
 /* Device bytes the library holds now. */
 size_t scarf_device_memory_in_use(void);
 /* Frees the device buffers the library keeps between calls (they are
- * allocated again on demand), and the FIM's cuFFT plans of the current
+ * allocated again on demand), the page-locked buffers that its contexts share
+ * (table rows; the ring through which fields reach ordinary host arrays), and the FIM's cuFFT plans of the current
  * device (made for axes too long for its own transforms, kept between calls; their work areas are cuFFT's own allocations,
  * outside the cap); waits for the library's device work first. */
 int scarf_release_device_memory(void);

@@ -193,14 +193,8 @@ struct Resources {
   int* slab_flags = nullptr;           // host-mapped, written by the kernel
   int* slab_flags_dev = nullptr;
   int slab_cap = 0;
-  // Page-locked bounce ring for pageable host fields (kBounceSlots slots).
-  char* bounce = nullptr;
-  size_t bounce_slot = 0;
-  cudaEvent_t bounce_ev[4] = {};
+  cudaEvent_t bounce_ev[4] = {};  // a copy into each slot of the bounce ring
   void release() {
-    if (bounce) cudaFreeHost(bounce);
-    bounce = nullptr;
-    bounce_slot = 0;
     for (auto& e : bounce_ev) {
       if (e) cudaEventDestroy(e);
       e = nullptr;
@@ -374,9 +368,16 @@ inline void cpu_relax() {
 // while the next slots are in flight.
 constexpr int kBounceSlots = 4;
 constexpr size_t kBounceSlotCap = size_t(16) << 20;
-// Slots of the gridded form's copies: page-locking costs ~0.8 ms per MB, once per
-// context, and slots of this size keep the copy engine busy.
-constexpr size_t kPassSlotCap = size_t(6) << 20;
+// Slots of the gridded form's copies: a quarter of the field, so that no copy
+// waits for a slot, up to 8 MB; beyond, 6 MB. Calls with pageable fields, quarter /
+// 6 MB slots: 128^3 (8 MB) 0.66 / 0.77 ms, 203 x 151 x 97 and its like no
+// difference, 439 x 45 x 416 (31 MB) 0.94 / 1.6 ms; 8 / 6 MB slots:
+// 320 x 288 x 200 (70 MB) 2.7 / 2.1 ms, 300 x 200 x 300 (69 MB) 2.2 / 1.8.
+constexpr size_t kPassSlotCap = size_t(6) << 20, kQuarterSlotCap = size_t(8) << 20;
+size_t pass_slot(size_t field_bytes) {
+  const size_t quarter = (field_bytes + kBounceSlots - 1) / kBounceSlots;
+  return quarter <= kQuarterSlotCap ? std::max<size_t>(quarter, 1 << 20) : kPassSlotCap;
+}
 
 bool is_pageable(const void* p) {
   cudaPointerAttributes a{};
@@ -387,16 +388,33 @@ bool is_pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
-int ensure_bounce(size_t slot_bytes) {
-  slot_bytes = (slot_bytes + 4095) / 4096 * 4096;
-  if (t_ctx->res.bounce && t_ctx->res.bounce_slot >= slot_bytes) return SCARF_OK;
-  if (t_ctx->res.bounce) cudaFreeHost(t_ctx->res.bounce);
-  t_ctx->res.bounce = nullptr;
-  t_ctx->res.bounce_slot = 0;
-  void* h = nullptr;
-  SCARF_CUDA(cudaHostAlloc(&h, slot_bytes * kBounceSlots, cudaHostAllocDefault));
-  t_ctx->res.bounce = static_cast<char*>(h);
-  t_ctx->res.bounce_slot = slot_bytes;
+// The ring's memory: one for all contexts, under g_mu (page-locking takes ~1 ms
+// per MB, which one per context cost each context's first call: 128^3 points
+// into malloc'd memory 25 ms). Every copy through it has been emptied when the
+// call that issued it returns (BounceCopier), and its size is bounded by
+// kBounceSlots * kBounceSlotCap. A call lays its own slots out in it.
+struct BounceRing {
+  char* p = nullptr;
+  size_t bytes = 0;
+  void release() {
+    if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
+    p = nullptr;
+    bytes = 0;
+  }
+};
+BounceRing g_bounce;
+
+// Room for kBounceSlots slots; *slot_bytes comes back rounded to pages.
+int ensure_bounce(size_t* slot_bytes) {
+  *slot_bytes = (*slot_bytes + 4095) / 4096 * 4096;
+  const size_t need = *slot_bytes * kBounceSlots;
+  if (g_bounce.bytes < need) {
+    g_bounce.release();
+    void* h = nullptr;
+    SCARF_CUDA(cudaHostAlloc(&h, need, cudaHostAllocPortable));
+    g_bounce.p = static_cast<char*>(h);
+    g_bounce.bytes = need;
+  }
   for (auto& e : t_ctx->res.bounce_ev)
     if (!e) SCARF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return SCARF_OK;
@@ -407,10 +425,10 @@ int ensure_bounce(size_t slot_bytes) {
 // issue first completes the copy that last used its slot.
 class BounceCopier {
  public:
-  explicit BounceCopier(cudaStream_t cs) : cs_(cs) {}
+  BounceCopier(cudaStream_t cs, size_t slot_bytes) : cs_(cs), slot_(slot_bytes) {}
   ~BounceCopier() { finish(); }
   int issue(char* dst, size_t dpitch, const char* src, size_t spitch, size_t width, size_t height) {
-    const size_t cap = t_ctx->res.bounce_slot;
+    const size_t cap = slot_;
     const size_t rows_per = std::max<size_t>(1, cap / std::max<size_t>(width, 1));
     if (width > cap) {  // one row longer than a slot: split the row
       for (size_t r = 0; r < height; ++r)
@@ -461,7 +479,7 @@ class BounceCopier {
     next_ = (next_ + 1) % kBounceSlots;
     int rc = complete(slot);
     if (rc) return rc;
-    char* buf = t_ctx->res.bounce + static_cast<size_t>(slot) * t_ctx->res.bounce_slot;
+    char* buf = g_bounce.p + slot * slot_;
     SCARF_CUDA(cudaMemcpy2DAsync(buf, width, src, spitch, width, height, cudaMemcpyDeviceToHost, cs_));
     SCARF_CUDA(cudaEventRecord(t_ctx->res.bounce_ev[slot], cs_));
     pend_[slot] = Pending{true, dst, dpitch, width, height};
@@ -472,7 +490,7 @@ class BounceCopier {
     if (!q.busy) return SCARF_OK;
     q.busy = false;
     SCARF_CUDA(cudaEventSynchronize(t_ctx->res.bounce_ev[slot]));
-    const char* buf = t_ctx->res.bounce + static_cast<size_t>(slot) * t_ctx->res.bounce_slot;
+    const char* buf = g_bounce.p + slot * slot_;
     // Up to a megabyte one thread copies at once: waking others takes longer
     // (316 KB 208 us a call in pieces, 170 in one; 1 MB 260 and 212).
     const size_t piece = q.width * q.height <= (size_t(1) << 20) ? size_t(1) << 20 : size_t(256) << 10;
@@ -485,6 +503,7 @@ class BounceCopier {
     return SCARF_OK;
   }
   cudaStream_t cs_;
+  size_t slot_;
   int next_ = 0;
   Pending pend_[kBounceSlots];
 };
@@ -492,13 +511,15 @@ class BounceCopier {
 int copy_slabs_out(const TcPlan& plan, const TcSlabSignal& sig, const float* d_field, float* field,
                    cudaStream_t st) {
   const bool bounce = is_pageable(field);
+  size_t slot = 0;
   if (bounce) {
     const TcSlab e0 = tc_slab_extent(plan, sig, 0);
     const size_t slab_bytes = static_cast<size_t>(e0.y1 - e0.y0) * plan.n1 * (e0.z1 - e0.z0) * sizeof(float);
-    const int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(slab_bytes, 1 << 20)));
+    slot = std::min(kBounceSlotCap, std::max<size_t>(slab_bytes, 1 << 20));
+    const int rc = ensure_bounce(&slot);
     if (rc) return rc;
   }
-  BounceCopier bc(t_ctx->res.copy_stream);
+  BounceCopier bc(t_ctx->res.copy_stream, slot);
   volatile int* flags = t_ctx->res.slab_flags;
   const size_t plane = static_cast<size_t>(plan.n1) * plan.n2;
   bool idle = false;
@@ -548,12 +569,14 @@ int ensure_pass_resources(int passes) {
 int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
   const bool bounce = is_pageable(field);
   const size_t plane = sizeof(float) * static_cast<size_t>(plan.nx) * plan.ny;
+  size_t slot = 0;
   if (bounce) {
-    const int rc = ensure_bounce(std::min<size_t>(kPassSlotCap, std::max<size_t>(plane * plan.zc, 1 << 20)));
+    slot = pass_slot(plane * plan.nz);
+    const int rc = ensure_bounce(&slot);
     if (rc) return rc;
   }
   cudaStream_t cs = t_ctx->res.copy_stream;
-  BounceCopier bc(cs);
+  BounceCopier bc(cs, slot);
   for (int pass = 0; pass < grid_passes(plan); ++pass) {
     int z0, z1;
     grid_pass_planes(plan, pass, &z0, &z1);
@@ -565,7 +588,7 @@ int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
       SCARF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, cs));
       continue;
     }
-    const size_t row = t_ctx->res.bounce_slot;
+    const size_t row = slot;
     const size_t rows = bytes / row, rest = bytes - rows * row;
     int rc = SCARF_OK;
     if (rows) rc = bc.issue(dst, row, src, row, row, rows);
@@ -583,10 +606,10 @@ int copy_field_out(float* field, const float* d_field, long long npts, cudaStrea
     SCARF_CUDA(cudaMemcpyAsync(field, d_field, bytes, cudaMemcpyDeviceToHost, st));
     return SCARF_OK;
   }
-  int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(bytes / kBounceSlots, 1 << 20)));
+  size_t row = std::min(kBounceSlotCap, std::max<size_t>(bytes / kBounceSlots, 1 << 20));
+  int rc = ensure_bounce(&row);
   if (rc) return rc;
-  BounceCopier bc(st);
-  const size_t row = t_ctx->res.bounce_slot;
+  BounceCopier bc(st, row);
   const size_t rows = bytes / row, rest = bytes - rows * row;
   char* dst = reinterpret_cast<char*>(field);
   const char* src = reinterpret_cast<const char*>(d_field);
@@ -1729,6 +1752,7 @@ int scarf_release_device_memory(void) {
   scarf::release_sampler_device_memory();
   scarf::release_field_sampler_memory();
   g_rows.release();
+  g_bounce.release();
   scarf::release_fim_plans();
   return SCARF_OK;
 }

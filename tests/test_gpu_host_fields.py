@@ -1,6 +1,10 @@
 """Fields into ordinary (pageable) host arrays, through the page-locked ring:
 bit for bit the device field, for sizes around a slot's and a piece's edges,
-in contexts that take turns, after the library's buffers were given back."""
+in contexts that take turns (the ring is one for all), after the ring was given
+back; and fresh contexts do not page-lock a ring of their own."""
+import statistics
+import time
+
 import numpy as np
 import pytest
 
@@ -44,7 +48,7 @@ def test_host_field_is_the_device_field(n, method, form):
     _both(n)
 
 
-def test_contexts_take_turns():
+def test_contexts_take_turns_with_the_ring():
     sizes = [(64, 64, 64), (300, 200), (256, 200, 160), (40, 30, 20)]
     ctxs = [sb.Context() for _ in sizes]
     try:
@@ -61,3 +65,20 @@ def test_contexts_take_turns():
             with c:
                 sb.scarf_finalize()
             c.close()
+
+
+def test_fresh_contexts_do_not_page_lock_a_ring():
+    n, times = (128, 128, 128), []
+    for _ in range(9):
+        c = sb.Context()
+        with c:
+            _init(n, 1, nharm=5000)
+            field = np.zeros(int(np.prod(n)), np.float32)
+            t = time.perf_counter()
+            sb.scarf_execute(3, field)
+            times.append(time.perf_counter() - t)
+            sb.scarf_finalize()
+        c.close()
+    # Page-locking a ring takes ~1 ms per MB and the field's is 8 MB or more
+    # (16 to 25 ms a call measured); with the ring in place a call takes 2 ms.
+    assert statistics.median(times[1:]) < 6e-3

@@ -559,6 +559,7 @@ bool make_axis(int n, FimAxis* X) {
   int found = 0;
   for (int m = lo; m <= lo + lo / 4 + 16; ++m) {
     FftPlan f;
+    if (found && static_cast<double>(m) * (fft_least_stages(m) + 2) >= best) break;
     if (!fft_plan(m, &f)) continue;
     const double cost = static_cast<double>(m) * (f.nst + 2);
     if (!found || cost < best) {

@@ -197,6 +197,8 @@ struct FftPlan {
 // False when n has a prime factor above most_prime (5 or 7) or fewer than two
 // stages.
 bool fft_plan(int n, FftPlan* f, int most_prime = 5);
+// No plan of that length or a longer one has fewer stages.
+int fft_least_stages(int n);
 struct GridPlan {
   int nh, nent;
   int nx, ny, nz;      // x; the transformed second axis (1: none); the axis summed exactly

@@ -492,8 +492,12 @@ class BounceCopier {
     SCARF_CUDA(cudaEventSynchronize(t_ctx->res.bounce_ev[slot]));
     const char* buf = g_bounce.p + slot * slot_;
     // Up to a megabyte one thread copies at once: waking others takes longer
-    // (316 KB 208 us a call in pieces, 170 in one; 1 MB 260 and 212).
-    const size_t piece = q.width * q.height <= (size_t(1) << 20) ? size_t(1) << 20 : size_t(256) << 10;
+    // (316 KB 208 us a call in pieces, 170 in one; 1 MB 260 and 212). Then
+    // pieces of 512 KB (copies of 8, 10 and 16 MB fields through slots of a
+    // quarter: 0.31, 0.25 and 0.35 ms; of 256 KB 0.42, 0.53, 0.63), beyond 4 MB
+    // of 256 KB (6 MB slots, 320 x 288 x 200: 2.14 ms a call; of 512 KB 2.33).
+    const size_t bytes = q.width * q.height;
+    const size_t piece = bytes <= (size_t(1) << 20) ? size_t(1) << 20 : size_t(bytes <= (size_t(4) << 20) ? 512 : 256) << 10;
     const size_t per_row = (q.width + piece - 1) / piece;
     const Pending w = q;
     parallel_tasks(static_cast<int>(per_row * w.height), host_threads(), [&](int t) {

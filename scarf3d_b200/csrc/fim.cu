@@ -493,7 +493,7 @@ void fim_grid(const FimInputs& in, FimGrid* g) {
 namespace {
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 struct FimLayout {
-  size_t off_spec, off_real, off_rec, off_poi, off_tables, bytes;
+  size_t off_spec, off_real, off_rec, off_poi, bytes;
   long long n1h, rows, real, nrec;
   bool own;  // this library's transform; else cuFFT
   FimFft fft;
@@ -514,14 +514,16 @@ FimLayout fim_layout(const FimGrid& g, int npoi) {
   off = align256(off + sizeof(StatRecord) * static_cast<size_t>(L.nrec));
   L.off_poi = off;
   off = align256(off + sizeof(float) * 3 * static_cast<size_t>(std::max(npoi, 1)));
-  L.off_tables = off;
-  if (L.own) off = align256(off + L.fft.tables);
   L.bytes = off;
   return L;
 }
 }  // namespace
 
-size_t fim_workspace_bytes(const FimGrid& g, int npoi) { return fim_layout(g, npoi).bytes; }
+size_t fim_workspace_bytes(const FimGrid& g, int npoi, size_t* tables) {
+  const FimLayout L = fim_layout(g, npoi);
+  *tables = L.own ? align256(L.fft.tables) : 0;
+  return L.bytes;
+}
 
 cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* d_field, float stats[8],
                     cudaStream_t st, const char** what) {
@@ -600,7 +602,7 @@ cudaError_t fim_run(const FimInputs& in, const FimGrid& g, void* d_work, float* 
                                          dhn);
   float pending = 1.0f;  // scaling not yet applied to the internal field
   if (L.own) {
-    if ((e = launch_fim_fft(L.fft, spec, real, w + L.off_tables, scaling, rec, st)) != cudaSuccess)
+    if ((e = launch_fim_fft(L.fft, spec, real, in.d_tables, in.tables_ready, scaling, rec, st)) != cudaSuccess)
       return failed("FIM transform", e);
     cudaEventRecord(ev[3], st);
   } else {

@@ -657,8 +657,8 @@ long long fim_fft_records(const FimFft& P) {
   return (static_cast<long long>(P.n[1]) * P.n[2] + kTile - 1) / kTile;
 }
 
-cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_tables, float scaling, StatRecord* rec,
-                           cudaStream_t stream) {
+cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_tables, bool tables_ready, float scaling,
+                           StatRecord* rec, cudaStream_t stream) {
   cudaError_t e = ensure_attributes();
   if (e != cudaSuccess) return e;
   TableArgs A{};
@@ -675,7 +675,7 @@ cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_t
     most = std::max(most, std::max(X.f.n, std::max(X.n + 1, X.q * X.q)));
   }
   A.n1 = P.n[0];
-  fim_tables_kernel<<<dim3((most + 3) / 4, 3), 128, 0, stream>>>(A);
+  if (!tables_ready) fim_tables_kernel<<<dim3((most + 3) / 4, 3), 128, 0, stream>>>(A);
   const int n1h = P.n[0] / 2 + 1;
   const unsigned tiles = static_cast<unsigned>((n1h + kTile - 1) / kTile);
   const long long row = n1h, plane = row * P.n[1];

@@ -184,6 +184,11 @@ struct DeviceBuf {
 struct Resources {
   int device = -1;
   DeviceBuf status, stats, table, field, coords, work, slab_cnt, statrec, poi;
+  // Tables of the FIM's transforms: they depend on the internal grid's lengths
+  // alone and stay for the next call with the same (making them took 4 to 30 us
+  // of every call, most for axes with large prime factors).
+  DeviceBuf fim_tables;
+  int fim_tables_of[3] = {0, 0, 0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr, evs = nullptr;
   cudaEvent_t evp = nullptr;  // the coordinates' upload on the copy stream
   std::vector<cudaEvent_t> pass_ev;    // end of each pass of the gridded form
@@ -222,6 +227,8 @@ struct Resources {
     field.release();
     coords.release();
     work.release();
+    fim_tables.release();
+    std::fill_n(fim_tables_of, 3, 0);
     statrec.release();
     poi.release();
     if (ev0) cudaEventDestroy(ev0);
@@ -761,12 +768,19 @@ int fim_execute_impl(int seed, float* field, float stats[8], int flags) {
     in.d_y = c + stride;
     in.d_z = c + 2 * stride;
   }
-  SCARF_CUDA(t_ctx->res.work.ensure(fim_workspace_bytes(g, in.npoi)));
+  Resources& R = t_ctx->res;
+  size_t tables = 0;
+  SCARF_CUDA(R.work.ensure(fim_workspace_bytes(g, in.npoi, &tables)));
+  in.tables_ready = tables > 0 && std::equal(g.npts, g.npts + 3, R.fim_tables_of);
+  std::fill_n(R.fim_tables_of, 3, 0);
+  SCARF_CUDA(R.fim_tables.ensure(tables));
+  in.d_tables = R.fim_tables.p;
   in.d_result = t_ctx->res.result_dev;
   in.result = t_ctx->res.result;
   const char* what = "";
   const cudaError_t e = fim_run(in, g, t_ctx->res.work.p, d_field, stats, st, &what);
   if (e != cudaSuccess) return fail(SCARF_ERR_CUDA, "FIM: %s: %s", what, cudaGetErrorString(e));
+  if (tables > 0) std::copy_n(g.npts, 3, R.fim_tables_of);
   if (!on_device) {
     const int rc = copy_field_out(field, d_field, npts, st);
     if (rc) return rc;
@@ -1834,7 +1848,9 @@ size_t scarf_fim_workspace_bytes(const int npts[3], int npoi) {
   if (!npts || npts[0] <= 0 || npts[1] <= 0 || npts[2] <= 0 || npoi < 0) return 0;
   FimGrid g{};
   for (int c = 0; c < 3; ++c) g.npts[c] = npts[c];
-  return fim_workspace_bytes(g, npoi);
+  size_t tables = 0;
+  const size_t work = fim_workspace_bytes(g, npoi, &tables);
+  return work + tables;
 }
 
 int scarf_set_direct_sincos(int mode) {

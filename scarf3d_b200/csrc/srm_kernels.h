@@ -325,6 +325,8 @@ struct FimInputs {
   long long npts;
   const float* poi;  // host, npoi points of poi_stride floats
   int npoi, poi_stride;
+  void* d_tables;     // of the transforms (fim_workspace_bytes)
+  bool tables_ready;  // filled by an earlier call for the same internal grid
   float* d_result;               // mean and variance, host-mapped: device address
   const volatile float* result;  // and host address
 };
@@ -357,9 +359,11 @@ bool fim_fft_plan(const int npts[3], bool three, FimFft* plan);
 long long fim_fft_records(const FimFft& plan);
 // spec [n3][n2][n1 / 2 + 1] (overwritten) -> real [n3][n2][n1], times scaling,
 // with fim_fft_records(plan) statistics records of the result.
-cudaError_t launch_fim_fft(const FimFft& plan, float2* spec, float* real, void* d_tables, float scaling, StatRecord* rec,
-                           cudaStream_t stream);
-size_t fim_workspace_bytes(const FimGrid& g, int npoi);
+// d_tables: plan.tables bytes, filled first unless a call with this plan did.
+cudaError_t launch_fim_fft(const FimFft& plan, float2* spec, float* real, void* d_tables, bool tables_ready, float scaling,
+                           StatRecord* rec, cudaStream_t stream);
+// Device bytes of a grid's workspace and of its transforms' tables (0: cuFFT).
+size_t fim_workspace_bytes(const FimGrid& g, int npoi, size_t* tables);
 // The whole FIM into the device field of the external points; stats as the
 // reference's info(1:8). d_work: fim_workspace_bytes, 256-byte aligned. On
 // failure *what names the failing step. Synchronises `st`.

@@ -613,25 +613,34 @@ size_t axis_tables(const FimAxis& X, int d, uint8_t* w, TableArgs* A) {
   return (at + 255) / 256 * 256;
 }
 
+// Raises a kernel's limit of dynamic shared memory, once per device context.
+// Only of the kernels that a call launches: raising the limits of all forms
+// loads all of them, ~2 ms of a process's first call.
 template <class F>
-cudaError_t most_smem(F* kernel) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
-}
-
-cudaError_t ensure_attributes() {
-  static std::atomic<unsigned long long> done[64];  // context ids
+cudaError_t most_smem(F* kernel, std::atomic<unsigned long long> (&done)[64]) {  // done: context ids
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long ctx = current_context_id();
   if (dev >= 0 && dev < 64 && ctx != 0 && done[dev] == ctx) return cudaSuccess;
-  e = most_smem(fim_columns_kernel<kFimPlain>);
-  if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimBluestein>);
-  if (e == cudaSuccess) e = most_smem(fim_columns_kernel<kFimRader>);
-  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimPlain>);
-  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimBluestein>);
-  if (e == cudaSuccess) e = most_smem(fim_rows_kernel<kFimRader>);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = ctx;
+  return e;
+}
+
+template <int kForm, class... Args>
+cudaError_t launch_columns(dim3 grid, const FimAxis& X, cudaStream_t stream, Args... args) {
+  static std::atomic<unsigned long long> done[64];
+  const cudaError_t e = most_smem(fim_columns_kernel<kForm>, done);
+  if (e == cudaSuccess) fim_columns_kernel<kForm><<<grid, axis_threads(X), axis_smem(X), stream>>>(X, args...);
+  return e;
+}
+
+template <int kForm, class... Args>
+cudaError_t launch_rows(unsigned blocks, const FimAxis& X, cudaStream_t stream, Args... args) {
+  static std::atomic<unsigned long long> done[64];
+  const cudaError_t e = most_smem(fim_rows_kernel<kForm>, done);
+  if (e == cudaSuccess) fim_rows_kernel<kForm><<<blocks, axis_threads(X), axis_smem(X), stream>>>(X, args...);
   return e;
 }
 
@@ -659,8 +668,6 @@ long long fim_fft_records(const FimFft& P) {
 
 cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_tables, bool tables_ready, float scaling,
                            StatRecord* rec, cudaStream_t stream) {
-  cudaError_t e = ensure_attributes();
-  if (e != cudaSuccess) return e;
   TableArgs A{};
   AxisTables T[3] = {};
   uint8_t* w = static_cast<uint8_t*>(d_tables);
@@ -681,29 +688,23 @@ cudaError_t launch_fim_fft(const FimFft& P, float2* spec, float* real, void* d_t
   const long long row = n1h, plane = row * P.n[1];
   auto columns = [&](const FimAxis& X, const AxisTables& t, int outer, long long step, long long hop) {
     const dim3 grid(tiles, outer);
-    const int threads = axis_threads(X);
-    const size_t smem = axis_smem(X);
-    if (X.form == kFimPlain)
-      fim_columns_kernel<kFimPlain><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
-    else if (X.form == kFimRader)
-      fim_columns_kernel<kFimRader><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
-    else
-      fim_columns_kernel<kFimBluestein><<<grid, threads, smem, stream>>>(X, t, spec, n1h, step, hop);
+    if (X.form == kFimPlain) return launch_columns<kFimPlain>(grid, X, stream, t, spec, n1h, step, hop);
+    if (X.form == kFimRader) return launch_columns<kFimRader>(grid, X, stream, t, spec, n1h, step, hop);
+    return launch_columns<kFimBluestein>(grid, X, stream, t, spec, n1h, step, hop);
   };
-  if (P.ax[2].n) columns(P.ax[2], T[2], P.n[1], plane, row);
-  if (P.ax[1].n) columns(P.ax[1], T[1], P.n[2], row, plane);
+  cudaError_t e = cudaSuccess;
+  if (P.ax[2].n && (e = columns(P.ax[2], T[2], P.n[1], plane, row)) != cudaSuccess) return e;
+  if (P.ax[1].n && (e = columns(P.ax[1], T[1], P.n[2], row, plane)) != cudaSuccess) return e;
   const long long rows = static_cast<long long>(P.n[1]) * P.n[2];
   const unsigned blocks = static_cast<unsigned>(fim_fft_records(P));
   const FimAxis& X = P.ax[0];
-  const int threads = axis_threads(X);
-  const size_t smem = axis_smem(X);
   if (X.form == kFimPlain)
-    fim_rows_kernel<kFimPlain><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
+    e = launch_rows<kFimPlain>(blocks, X, stream, T[0], spec, real, rows, scaling, rec);
   else if (X.form == kFimRader)
-    fim_rows_kernel<kFimRader><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
+    e = launch_rows<kFimRader>(blocks, X, stream, T[0], spec, real, rows, scaling, rec);
   else
-    fim_rows_kernel<kFimBluestein><<<blocks, threads, smem, stream>>>(X, T[0], spec, real, rows, scaling, rec);
-  return cudaGetLastError();
+    e = launch_rows<kFimBluestein>(blocks, X, stream, T[0], spec, real, rows, scaling, rec);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace scarf

@@ -193,8 +193,6 @@ struct Resources {
   cudaEvent_t evp = nullptr;  // the coordinates' upload on the copy stream
   std::vector<cudaEvent_t> pass_ev;    // end of each pass of the gridded form
   cudaStream_t copy_stream = nullptr;  // non-blocking: runs beside the legacy stream too
-  float* result = nullptr;             // mean, variance and status word of a call (host-mapped)
-  float* result_dev = nullptr;
   int* slab_flags = nullptr;           // host-mapped, written by the kernel
   int* slab_flags_dev = nullptr;
   int slab_cap = 0;
@@ -204,8 +202,6 @@ struct Resources {
       if (e) cudaEventDestroy(e);
       e = nullptr;
     }
-    if (result) cudaFreeHost(result);
-    result = result_dev = nullptr;
     if (slab_flags) cudaFreeHost(slab_flags);
     slab_flags = slab_flags_dev = nullptr;
     slab_cap = 0;
@@ -267,39 +263,48 @@ class CtxScope {
   scarf_ctx* prev_;
 };
 
-// Page-locked memory for the table rows that an execute samples and uploads.
-// One for all contexts, under g_mu (page-locking one per context cost every
-// first call): only the execute that holds g_mu writes or reads it, and that
-// execute's upload has ended when it returns (RowsUpload). The sampling entry
-// points, which do not take g_mu, fill their callers' tables.
-struct TableRows {
+// Page-locked, device-mapped memory of an execute: the words it reads back
+// (mean, variance and status word), then the table rows that it samples and
+// uploads. One for all contexts, under g_mu (a context's own cost its first
+// call ~1 ms): only the execute that holds g_mu uses it, and that execute's
+// upload has ended when it returns (RowsUpload). The sampling entry points,
+// which do not take g_mu, fill their callers' tables.
+struct HostStage {
   char* p = nullptr;
+  float* result_dev = nullptr;
   size_t bytes = 0;
-  // Null (and nothing kept) beyond kMost bytes or without page-locked memory.
+  static constexpr size_t kResult = 64, kMost = size_t(64) << 20;
+  // Room for the words, and for rows of up to kMost bytes if it can be had.
   // Whole megabytes: page-locking one takes as long as a few bytes (0.9 to 2.7
   // ms), and a count of harmonics that grows seldom page-locks again.
-  static constexpr size_t kMost = size_t(64) << 20;
-  float* ensure(size_t need) {
-    if (need > bytes) {
-      release();
-      void* h = nullptr;
-      need = (need + (size_t(1) << 20) - 1) >> 20 << 20;
-      if (need > kMost || cudaHostAlloc(&h, need, cudaHostAllocPortable) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return nullptr;
-      }
-      p = static_cast<char*>(h);
-      bytes = need;
+  cudaError_t ensure(size_t row_bytes) {
+    const size_t need = (kResult + (row_bytes <= kMost ? row_bytes : 0) + (size_t(1) << 20) - 1) >> 20 << 20;
+    if (need <= bytes) return cudaSuccess;
+    void *h = nullptr, *d = nullptr;
+    cudaError_t e = cudaHostAlloc(&h, need, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess && (e = cudaHostGetDevicePointer(&d, h, 0)) != cudaSuccess) cudaFreeHost(h);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      return bytes ? cudaSuccess : e;
     }
-    return reinterpret_cast<float*>(p);
+    release();
+    p = static_cast<char*>(h);
+    result_dev = static_cast<float*>(d);
+    bytes = need;
+    return cudaSuccess;
+  }
+  float* result() { return reinterpret_cast<float*>(p); }
+  float* rows(size_t row_bytes) {  // null: not enough room
+    return row_bytes + kResult <= bytes ? reinterpret_cast<float*>(p + kResult) : nullptr;
   }
   void release() {
     if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
     p = nullptr;
+    result_dev = nullptr;
     bytes = 0;
   }
 };
-TableRows g_rows;
+HostStage g_stage;
 
 // Waits, on a return before the execute's own synchronisation, for the upload
 // of the rows.
@@ -320,13 +325,6 @@ int ensure_resources() {
   }
   SCARF_CUDA(t_ctx->res.status.ensure(256));
   SCARF_CUDA(t_ctx->res.stats.ensure(stats_partials_bytes(0) + 256));
-  if (!t_ctx->res.result) {
-    void *h = nullptr, *d = nullptr;
-    SCARF_CUDA(cudaHostAlloc(&h, 4 * sizeof(float), cudaHostAllocMapped | cudaHostAllocPortable));
-    t_ctx->res.result = static_cast<float*>(h);
-    SCARF_CUDA(cudaHostGetDevicePointer(&d, h, 0));
-    t_ctx->res.result_dev = static_cast<float*>(d);
-  }
   if (!t_ctx->res.ev0) SCARF_CUDA(cudaEventCreate(&t_ctx->res.ev0));
   if (!t_ctx->res.ev1) SCARF_CUDA(cudaEventCreate(&t_ctx->res.ev1));
   if (!t_ctx->res.evk0) SCARF_CUDA(cudaEventCreate(&t_ctx->res.evk0));
@@ -775,8 +773,9 @@ int fim_execute_impl(int seed, float* field, float stats[8], int flags) {
   std::fill_n(R.fim_tables_of, 3, 0);
   SCARF_CUDA(R.fim_tables.ensure(tables));
   in.d_tables = R.fim_tables.p;
-  in.d_result = t_ctx->res.result_dev;
-  in.result = t_ctx->res.result;
+  SCARF_CUDA(g_stage.ensure(0));
+  in.d_result = g_stage.result_dev;
+  in.result = g_stage.result();
   const char* what = "";
   const cudaError_t e = fim_run(in, g, t_ctx->res.work.p, d_field, stats, st, &what);
   if (e != cudaSuccess) return fail(SCARF_ERR_CUDA, "FIM: %s: %s", what, cudaGetErrorString(e));
@@ -818,9 +817,11 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   const bool on_gpu = !t_ctx->cfg.src.srng && t_ctx->cfg.sampler != SCARF_SAMPLER_HOST;
   // The table's rows: page-locked where there is room, else the vector's.
   std::vector<float> table;
-  float* rows = g_rows.ensure(5 * sizeof(float) * static_cast<size_t>(std::max(p.nharm, 0)));
+  const size_t row_bytes = 5 * sizeof(float) * static_cast<size_t>(std::max(p.nharm, 0));
+  SCARF_CUDA(g_stage.ensure(row_bytes));
+  float* rows = g_stage.rows(row_bytes);
   if (!rows) {
-    table.resize(5 * static_cast<size_t>(std::max(p.nharm, 0)));
+    table.resize(row_bytes / sizeof(float));
     rows = table.data();
   }
   const int nh = on_gpu ? srm_sample_field(p, s, rows, &pairs, st, nullptr)
@@ -985,12 +986,12 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
   // instead). It writes them and the sum's status word to host-mapped memory,
   // read after one synchronisation (after a failed sum the statistics are
   // dropped).
-  volatile float* result = t_ctx->res.result;
+  volatile float* result = g_stage.result();
   result[2] = 0.0f;
   if (d_rec)
-    SCARF_CUDA(launch_stats_records(d_rec, nrec, t_ctx->res.result_dev, st, d_status));
+    SCARF_CUDA(launch_stats_records(d_rec, nrec, g_stage.result_dev, st, d_status));
   else
-    SCARF_CUDA(launch_field_stats(d_field, npts, static_cast<double*>(t_ctx->res.stats.p), t_ctx->res.result_dev, st));
+    SCARF_CUDA(launch_field_stats(d_field, npts, static_cast<double*>(t_ctx->res.stats.p), g_stage.result_dev, st));
   const bool finalizing = p.rescale == 1 || tapering;
   if (!copied_out && !finalizing) SCARF_CUDA(cudaEventRecord(t_ctx->res.ev1, st));
   SCARF_CUDA(cudaStreamSynchronize(st));
@@ -1769,7 +1770,7 @@ int scarf_release_device_memory(void) {
   }
   scarf::release_sampler_device_memory();
   scarf::release_field_sampler_memory();
-  g_rows.release();
+  g_stage.release();
   g_bounce.release();
   scarf::release_fim_plans();
   return SCARF_OK;

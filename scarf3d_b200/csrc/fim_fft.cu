@@ -59,7 +59,11 @@ constexpr int kTile = 2 * kPairs;       // transforms of a tile
 // 153; but 402 x 402 x 202 (Bluestein's along x and y, whose radices are larger)
 // 543, 518, 525, 541.
 constexpr int sm_threads(int form) { return form == kFimBluestein ? 768 : 1024; }
-constexpr int most_threads(int) { return 256; }
+// A block takes 256 threads, more (up to an SM's) only where the tiles are too
+// few, or too large, for blocks of 256 to fill the SMs: 78 x 1407 points, six
+// tiles of Bluestein's form, 132 us a call with 256 and 126 with more.
+constexpr int most_threads(int form) { return sm_threads(form); }
+constexpr int kUsualThreads = 256;
 constexpr size_t kSmemMax = 224 * 1024;
 
 // Device tables of one axis: twiddles of its plan, then (Bluestein) the chirp
@@ -358,7 +362,7 @@ __device__ __forceinline__ void transform_tile(const FimAxis& X, const AxisTable
 // c2c along z or y, in place: blockIdx.x selects eight neighbouring x bins,
 // blockIdx.y the row or plane.
 template <int kForm>
-__global__ void __launch_bounds__(most_threads(kForm), sm_threads(kForm) / most_threads(kForm))
+__global__ void __launch_bounds__(most_threads(kForm), 1)
     fim_columns_kernel(const FimAxis X, const AxisTables T, float2* spec, int n1h, long long step, long long outer) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int i0 = blockIdx.x * kTile, left = n1h - i0;
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(most_threads(kForm), sm_threads(kForm) / most_
 // c2r along x: eight rows per tile, the n1 / 2 + 1 bins of each packed into a
 // complex transform of length n1 / 2 (only real parts of bins 0 and n1 / 2).
 template <int kForm>
-__global__ void __launch_bounds__(most_threads(kForm), sm_threads(kForm) / most_threads(kForm))
+__global__ void __launch_bounds__(most_threads(kForm), 1)
     fim_rows_kernel(const FimAxis X, const AxisTables T, const float2* spec, float* real, long long rows, float scaling,
                     Moments* rec) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -571,19 +575,23 @@ bool make_axis(int n, FimAxis* X) {
   return found && axis_smem(*X) <= kSmemMax;
 }
 
-// The block size that fills an SM (sm_threads) with the least idle threads.
-int axis_threads(const FimAxis& X) {
+// The block size that fills an SM (sm_threads) with the least idle threads;
+// beyond kUsualThreads only where such blocks leave half of it empty.
+int axis_threads(const FimAxis& X, long long tiles) {
   int best = 128;
   double best_cost = 1e30;
+  const int fit = static_cast<int>(std::min<size_t>(kSmemMax / axis_smem(X), 16));  // blocks of an SM
+  const int share = static_cast<int>(std::min<long long>((tiles + 147) / 148, 16));  // tiles of an SM
   for (int t = 64; t <= most_threads(X.form); t += 32) {
-    const int blocks = static_cast<int>(std::min<size_t>(std::min<size_t>(kSmemMax / axis_smem(X), sm_threads(X.form) / t), 16));
+    if (t > kUsualThreads && 2 * best * std::min(share, fit) > sm_threads(X.form)) break;
+    const int blocks = std::min(fit, sm_threads(X.form) / t);
     if (blocks < 1) continue;
     double work = 0.0;
     for (int s = 0; s < X.f.nst; ++s) {
       const int items = X.f.n / X.f.r[s] * kPairs;
       work += static_cast<double>((items + t - 1) / t) * t / items;
     }
-    const double cost = work / (blocks * t);
+    const double cost = work / (std::min(blocks, share) * t);
     if (cost < best_cost) best_cost = cost, best = t;
   }
   return best;
@@ -632,7 +640,8 @@ template <int kForm, class... Args>
 cudaError_t launch_columns(dim3 grid, const FimAxis& X, cudaStream_t stream, Args... args) {
   static std::atomic<unsigned long long> done[64];
   const cudaError_t e = most_smem(fim_columns_kernel<kForm>, done);
-  if (e == cudaSuccess) fim_columns_kernel<kForm><<<grid, axis_threads(X), axis_smem(X), stream>>>(X, args...);
+  const int threads = axis_threads(X, static_cast<long long>(grid.x) * grid.y);
+  if (e == cudaSuccess) fim_columns_kernel<kForm><<<grid, threads, axis_smem(X), stream>>>(X, args...);
   return e;
 }
 
@@ -640,7 +649,7 @@ template <int kForm, class... Args>
 cudaError_t launch_rows(unsigned blocks, const FimAxis& X, cudaStream_t stream, Args... args) {
   static std::atomic<unsigned long long> done[64];
   const cudaError_t e = most_smem(fim_rows_kernel<kForm>, done);
-  if (e == cudaSuccess) fim_rows_kernel<kForm><<<blocks, axis_threads(X), axis_smem(X), stream>>>(X, args...);
+  if (e == cudaSuccess) fim_rows_kernel<kForm><<<blocks, axis_threads(X, blocks), axis_smem(X), stream>>>(X, args...);
   return e;
 }
 

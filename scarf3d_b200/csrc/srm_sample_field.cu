@@ -285,16 +285,13 @@ void release_field_sampler_memory() {
   g_field.host_bytes = 0;
 }
 
-int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
-                     void* stream_handle, long long* uncertain) {
+namespace {
+// One scan of `want` pairs and its walk; kMorePairs when they ran out.
+constexpr int kMorePairs = -3;
+int sample_pairs(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
+                 void* stream_handle, long long* uncertain, double acc, double want) {
   auto batched = [&] { return srm_sample_device(p, s, table, pairs_used, stream_handle, uncertain); };
   const cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
-  const double acc = acceptance_rate(s);
-  if (acc < kMinAcceptance) return -1;
-  // Enough pairs for every harmonic at the expected acceptance, with the
-  // batched sampler's margin; fields that need more, or that a test caps, take
-  // its chained passes.
-  const double want = p.nharm * (1.0 / acc + 3.0) * 1.1 + 4096.0;
   if (want > kMaxPairs || device_sampler_pass_cap() > 0) return batched();
   const long long pairs = static_cast<long long>(want);
   std::unique_lock<std::mutex> lk(g_field.mu);
@@ -398,10 +395,7 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
       pos = q + 4;
     }
   }
-  if (l < p.nharm) {  // the pairs ran out
-    lk.unlock();
-    return batched();
-  }
+  if (l < p.nharm) return kMorePairs;
   // Table rows (host libm, ~85 ns each) on the worker pool. Rows started while
   // the walk runs, by workers waiting for it, measured slower: the waiting
   // threads take the processor time of the others.
@@ -416,6 +410,25 @@ int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float*
   if (pairs_used) *pairs_used = pos;
   if (uncertain) *uncertain = open;
   return kept;
+}
+
+}  // namespace
+
+int srm_sample_field(const scarf_srm_params& p, const scarf_srm_setup& s, float* table, long long* pairs_used,
+                     void* stream_handle, long long* uncertain) {
+  const double acc = acceptance_rate(s);
+  if (acc < kMinAcceptance) return -1;
+  // Enough pairs for every harmonic at the expected acceptance, with the
+  // batched sampler's margin. Few harmonics of a rare acceptance now and then
+  // need more: then twice as many are scanned, from the first (the batched
+  // sampler's passes after a scan in vain took longer than they alone: 100
+  // harmonics of one pair in 1 100 318 -> 360 us, 67 so). Fields of very many
+  // pairs, or that a test caps, take the batched sampler's chained passes.
+  double want = p.nharm * (1.0 / acc + 3.0) * 1.1 + 4096.0;
+  for (;; want *= 2.0) {
+    const int rc = sample_pairs(p, s, table, pairs_used, stream_handle, uncertain, acc, want);
+    if (rc != kMorePairs) return rc;
+  }
 }
 
 }  // namespace scarf

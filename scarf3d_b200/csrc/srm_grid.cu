@@ -1004,13 +1004,16 @@ bool grid_make_plan(const int n[3], int nh, size_t pass_bytes, const double reac
   p.nkeys = (p.nbx + kSpan) * p.nby;
   p.nent = 2 * nh;
   const int nzp = (p.nz + 31) / 32 * 32;
-  // Planes per pass: about pass_bytes of T1 and T2, the planes shared out
-  // evenly (a last pass of a few planes costs as much as one of 32).
+  // Planes per pass: about pass_bytes of T1 and T2 and at most kGridEBytes of E,
+  // in as few passes as that takes, of equal multiples of 32 planes (the last
+  // may be shorter: 200 planes in two passes are 128 and 72).
   const size_t per_z = sizeof(float2) * static_cast<size_t>(p.ax) * (p.ya + (p.ny > 1 ? p.ny : 0));
-  const long long most = std::max<long long>(32, static_cast<long long>(1.3 * static_cast<double>(pass_bytes) / per_z));
+  const long long cells_most = static_cast<long long>(1.3 * static_cast<double>(pass_bytes) / per_z);
+  const long long e_most = static_cast<long long>(kGridEBytes / (sizeof(float2) * static_cast<size_t>(p.nent)));
+  const long long most = std::max<long long>(32, std::min(cells_most, e_most));
   const long long want = (p.nz + most - 1) / most;
   p.zc = static_cast<int>(std::min<long long>((p.nz + 32 * want - 1) / (32 * want) * 32, nzp));
-  // E for as many passes as fit a bounded buffer.
+  // E for as many passes as fit its buffer.
   const size_t e_pass = sizeof(float2) * static_cast<size_t>(p.nent) * p.zc;
   const int passes = static_cast<int>(std::max<size_t>(1, kGridEBytes / e_pass));
   p.ez = static_cast<int>(std::min<long long>(static_cast<long long>(passes) * p.zc, (nzp + p.zc - 1) / p.zc * p.zc));

@@ -904,10 +904,13 @@ int execute_impl(int seed, float* field, float stats[8], int flags) {
                     grid_make_plan(n, nh, overlap ? kGridHostPassBytes : kGridPassBytes, bound, &grid) &&
                     (!planned || grid_pays(grid, plan));
     auto grid_fits = [&] {
-      if (want_records(grid_stat_records(grid)) == SCARF_OK && t_ctx->res.work.ensure(grid.bytes) == cudaSuccess)
-        return true;
+      if (t_ctx->res.statrec.ensure(sizeof(StatRecord) * static_cast<size_t>(grid_stat_records(grid))) == cudaSuccess &&
+          t_ctx->res.work.ensure(grid.bytes) == cudaSuccess)
+        return want_records(grid_stat_records(grid)) == SCARF_OK;
       (void)cudaGetLastError();
       (void)scarf::take_device_alloc_failure();
+      // The other form's records may be fewer: a cap that holds them holds no more.
+      t_ctx->res.statrec.release();
       return false;
     };
     if (use_grid && !grid_fits())  // smaller passes, then the tensor-core form

@@ -373,29 +373,27 @@ int sample_pairs(const scarf_srm_params& p, const scarf_srm_setup& s, float* tab
   uint32_t* kept_at = S.kept.data();
   // The walk, in stream order exactly as the serial loop consumes pairs:
   // reject until an accepted pair, then one pair of angles, then (for a kept
-  // harmonic) two pairs for a and b.
+  // harmonic) two pairs for a and b. Bound: mispredicted branches. 10 000
+  // harmonics of one pair in 20 take 48 us in one loop without a branch on the
+  // cut, 67 in a loop over candidates inside one over harmonics with one.
   long long open = 0;
   uint32_t pos = 0;
   int kept = 0, l = 0;
-  for (int ei = 0; l < p.nharm; ++l, ++ei) {
-    uint32_t w = 0;
-    for (; ei < head.total; ++ei) {
-      w = words[ei];
-      if ((w & (kAboveCut - 1)) < pos) continue;
-      if (!(w & kUndecided)) break;
+  const int total = head.total, nharm = p.nharm;
+  for (int ei = 0; ei < total && l < nharm; ++ei) {
+    const uint32_t w = words[ei], q = w & (kAboveCut - 1);
+    if (q < pos) continue;
+    if (w & kUndecided) {
       ++open;
-      if (sampler_host_accept(s, p.acf, draws[ei].r[0], draws[ei].r[1])) break;
+      if (!sampler_host_accept(s, p.acf, draws[ei].r[0], draws[ei].r[1])) continue;
     }
-    if (ei == head.total) break;
-    const uint32_t q = w & (kAboveCut - 1);
-    if (w & kAboveCut) {
-      pos = q + 2;
-    } else {
-      kept_at[kept++] = static_cast<uint32_t>(ei);
-      pos = q + 4;
-    }
+    const uint32_t keep = w & kAboveCut ? 0u : 1u;
+    kept_at[kept] = static_cast<uint32_t>(ei);
+    kept += static_cast<int>(keep);
+    pos = q + 2 + 2 * keep;
+    ++l;
   }
-  if (l < p.nharm) return kMorePairs;
+  if (l < nharm) return kMorePairs;
   // Table rows (host libm, ~85 ns each) on the worker pool. Rows started while
   // the walk runs, by workers waiting for it, measured slower: the waiting
   // threads take the processor time of the others.

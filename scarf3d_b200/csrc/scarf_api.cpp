@@ -373,6 +373,11 @@ inline void cpu_relax() {
 // while the next slots are in flight.
 constexpr int kBounceSlots = 4;
 constexpr size_t kBounceSlotCap = size_t(16) << 20;
+// Slots move on through six places where a copy takes more than the four that
+// are in flight: the link writes memory that the host's caches have let go
+// (320 x 288 x 200: 2.18 ms a call with four places, 1.93 with six; three
+// contexts in turn with four each 2.12).
+constexpr int kBouncePlaces = 6;
 // Slots of the gridded form's copies: a quarter of the field, so that no copy
 // waits for a slot, up to 8 MB; beyond, 6 MB. Calls with pageable fields, quarter /
 // 6 MB slots: 128^3 (8 MB) 0.66 / 0.77 ms, 203 x 151 x 97 and its like no
@@ -397,10 +402,11 @@ bool is_pageable(const void* p) {
 // per MB, which one per context cost each context's first call: 128^3 points
 // into malloc'd memory 25 ms). Every copy through it has been emptied when the
 // call that issued it returns (BounceCopier), and its size is bounded by
-// kBounceSlots * kBounceSlotCap. A call lays its own slots out in it.
+// kBounceSlots * kBounceSlotCap. A call lays its own places out in it.
 struct BounceRing {
   char* p = nullptr;
   size_t bytes = 0;
+  unsigned turn = 0;  // places used so far
   void release() {
     if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
     p = nullptr;
@@ -409,10 +415,18 @@ struct BounceRing {
 };
 BounceRing g_bounce;
 
-// Room for kBounceSlots slots; *slot_bytes comes back rounded to pages.
-int ensure_bounce(size_t* slot_bytes) {
-  *slot_bytes = (*slot_bytes + 4095) / 4096 * 4096;
-  const size_t need = *slot_bytes * kBounceSlots;
+struct BounceSlots {
+  size_t bytes = 0;  // of a slot, whole pages
+  int places = 0;
+};
+
+// Slots of slot_bytes for a copy of field_bytes.
+int ensure_bounce(size_t slot_bytes, size_t field_bytes, BounceSlots* b) {
+  b->bytes = (slot_bytes + 4095) / 4096 * 4096;
+  b->places = kBounceSlots;
+  if (field_bytes > kBounceSlots * b->bytes)
+    b->places = static_cast<int>(std::min<size_t>(kBouncePlaces, kBounceSlots * kBounceSlotCap / b->bytes));
+  const size_t need = b->places * b->bytes;
   if (g_bounce.bytes < need) {
     g_bounce.release();
     void* h = nullptr;
@@ -430,7 +444,7 @@ int ensure_bounce(size_t* slot_bytes) {
 // issue first completes the copy that last used its slot.
 class BounceCopier {
  public:
-  BounceCopier(cudaStream_t cs, size_t slot_bytes) : cs_(cs), slot_(slot_bytes) {}
+  BounceCopier(cudaStream_t cs, const BounceSlots& slots) : cs_(cs), slot_(slots.bytes), places_(slots.places) {}
   ~BounceCopier() { finish(); }
   int issue(char* dst, size_t dpitch, const char* src, size_t spitch, size_t width, size_t height) {
     const size_t cap = slot_;
@@ -476,6 +490,7 @@ class BounceCopier {
  private:
   struct Pending {
     bool busy = false;
+    const char* buf = nullptr;
     char* dst = nullptr;
     size_t dpitch = 0, width = 0, height = 0;
   };
@@ -484,10 +499,10 @@ class BounceCopier {
     next_ = (next_ + 1) % kBounceSlots;
     int rc = complete(slot);
     if (rc) return rc;
-    char* buf = g_bounce.p + slot * slot_;
+    char* buf = g_bounce.p + (g_bounce.turn++ % places_) * slot_;
     SCARF_CUDA(cudaMemcpy2DAsync(buf, width, src, spitch, width, height, cudaMemcpyDeviceToHost, cs_));
     SCARF_CUDA(cudaEventRecord(t_ctx->res.bounce_ev[slot], cs_));
-    pend_[slot] = Pending{true, dst, dpitch, width, height};
+    pend_[slot] = Pending{true, buf, dst, dpitch, width, height};
     return SCARF_OK;
   }
   int complete(int slot) {
@@ -495,24 +510,23 @@ class BounceCopier {
     if (!q.busy) return SCARF_OK;
     q.busy = false;
     SCARF_CUDA(cudaEventSynchronize(t_ctx->res.bounce_ev[slot]));
-    const char* buf = g_bounce.p + slot * slot_;
-    // Up to a megabyte one thread copies at once: waking others takes longer
-    // (316 KB 208 us a call in pieces, 170 in one; 1 MB 260 and 212). Then
-    // pieces of 512 KB (copies of 8, 10 and 16 MB fields through slots of a
-    // quarter: 0.31, 0.25 and 0.35 ms; of 256 KB 0.42, 0.53, 0.63), beyond 4 MB
+    // Slots of a megabyte are emptied by one thread: waking others takes longer
+    // (316 KB 208 us a call in pieces, 170 in one; 1 MB 260 and 212). Slots of
+    // up to 4 MB in pieces of 512 KB (copies of 8, 10 and 16 MB fields through
+    // quarters: 0.31, 0.25 and 0.35 ms; of 256 KB 0.42, 0.53, 0.63), larger ones
     // of 256 KB (6 MB slots, 320 x 288 x 200: 2.14 ms a call; of 512 KB 2.33).
-    const size_t bytes = q.width * q.height;
-    const size_t piece = bytes <= (size_t(1) << 20) ? size_t(1) << 20 : size_t(bytes <= (size_t(4) << 20) ? 512 : 256) << 10;
+    const size_t piece = size_t(slot_ <= (size_t(1) << 20) ? 1024 : slot_ <= (size_t(4) << 20) ? 512 : 256) << 10;
     const size_t per_row = (q.width + piece - 1) / piece;
     const Pending w = q;
     parallel_tasks(static_cast<int>(per_row * w.height), host_threads(), [&](int t) {
       const size_t r = static_cast<size_t>(t) / per_row, o = (static_cast<size_t>(t) % per_row) * piece;
-      std::memcpy(w.dst + r * w.dpitch + o, buf + r * w.width + o, std::min(piece, w.width - o));
+      std::memcpy(w.dst + r * w.dpitch + o, w.buf + r * w.width + o, std::min(piece, w.width - o));
     });
     return SCARF_OK;
   }
   cudaStream_t cs_;
   size_t slot_;
+  unsigned places_;
   int next_ = 0;
   Pending pend_[kBounceSlots];
 };
@@ -520,15 +534,15 @@ class BounceCopier {
 int copy_slabs_out(const TcPlan& plan, const TcSlabSignal& sig, const float* d_field, float* field,
                    cudaStream_t st) {
   const bool bounce = is_pageable(field);
-  size_t slot = 0;
+  BounceSlots slots;
   if (bounce) {
     const TcSlab e0 = tc_slab_extent(plan, sig, 0);
     const size_t slab_bytes = static_cast<size_t>(e0.y1 - e0.y0) * plan.n1 * (e0.z1 - e0.z0) * sizeof(float);
-    slot = std::min(kBounceSlotCap, std::max<size_t>(slab_bytes, 1 << 20));
-    const int rc = ensure_bounce(&slot);
+    const size_t all = sizeof(float) * static_cast<size_t>(plan.n1) * plan.n2 * plan.n3;
+    const int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(slab_bytes, 1 << 20)), all, &slots);
     if (rc) return rc;
   }
-  BounceCopier bc(t_ctx->res.copy_stream, slot);
+  BounceCopier bc(t_ctx->res.copy_stream, slots);
   volatile int* flags = t_ctx->res.slab_flags;
   const size_t plane = static_cast<size_t>(plan.n1) * plan.n2;
   bool idle = false;
@@ -578,14 +592,13 @@ int ensure_pass_resources(int passes) {
 int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
   const bool bounce = is_pageable(field);
   const size_t plane = sizeof(float) * static_cast<size_t>(plan.nx) * plan.ny;
-  size_t slot = 0;
+  BounceSlots slots;
   if (bounce) {
-    slot = pass_slot(plane * plan.nz);
-    const int rc = ensure_bounce(&slot);
+    const int rc = ensure_bounce(pass_slot(plane * plan.nz), plane * plan.nz, &slots);
     if (rc) return rc;
   }
   cudaStream_t cs = t_ctx->res.copy_stream;
-  BounceCopier bc(cs, slot);
+  BounceCopier bc(cs, slots);
   for (int pass = 0; pass < grid_passes(plan); ++pass) {
     int z0, z1;
     grid_pass_planes(plan, pass, &z0, &z1);
@@ -597,7 +610,7 @@ int copy_passes_out(const GridPlan& plan, const float* d_field, float* field) {
       SCARF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, cs));
       continue;
     }
-    const size_t row = slot;
+    const size_t row = slots.bytes;
     const size_t rows = bytes / row, rest = bytes - rows * row;
     int rc = SCARF_OK;
     if (rows) rc = bc.issue(dst, row, src, row, row, rows);
@@ -615,10 +628,11 @@ int copy_field_out(float* field, const float* d_field, long long npts, cudaStrea
     SCARF_CUDA(cudaMemcpyAsync(field, d_field, bytes, cudaMemcpyDeviceToHost, st));
     return SCARF_OK;
   }
-  size_t row = std::min(kBounceSlotCap, std::max<size_t>(bytes / kBounceSlots, 1 << 20));
-  int rc = ensure_bounce(&row);
+  BounceSlots slots;
+  int rc = ensure_bounce(std::min(kBounceSlotCap, std::max<size_t>(bytes / kBounceSlots, 1 << 20)), bytes, &slots);
   if (rc) return rc;
-  BounceCopier bc(st, row);
+  BounceCopier bc(st, slots);
+  const size_t row = slots.bytes;
   const size_t rows = bytes / row, rest = bytes - rows * row;
   char* dst = reinterpret_cast<char*>(field);
   const char* src = reinterpret_cast<const char*>(d_field);

@@ -92,7 +92,7 @@ __device__ __forceinline__ float axis_k(int t, int n, float dk) {
 // and two sine-cosine pairs per amplitude). On the 514^3 grid: 1.20 ms with the
 // generator's products in 64-bit arithmetic and an amplitude per point, 0.49
 // with 32-bit products and shared amplitudes, 0.45 with this recurrence for
-// the matrix step.
+// the matrix step, 0.47 with phases and wavenumbers rounded as the reference's.
 __global__ void __launch_bounds__(256) fim_spectrum_kernel(const SpecArgs A) {
   __shared__ uint32_t sp[kPowWords];
   for (int i = threadIdx.x; i < kPowWords; i += blockDim.x) sp[i] = g_fim_pow[i];

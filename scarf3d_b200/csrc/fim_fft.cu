@@ -53,7 +53,8 @@ using namespace fft;
 constexpr int kPairs = 4;               // transform pairs of a tile
 constexpr int kTile = 2 * kPairs;       // transforms of a tile
 // Threads of an SM and most of a block, by form: the stages wait for memory and
-// barriers, so threads count for more than spills. Transform of 514^3 points
+// barriers, so threads count for more than spills (64 registers: 170 to 310 bytes
+// a thread). Transform of 514^3 points
 // (Rader's form) 1 675 us with 640 threads of 96 registers, 1 595 with 768 of 80,
 // 1 565 with 896 of 72 and 1 398 with 1 024 of 64; 256^3 (plain) 164, 161, 156,
 // 153; but 402 x 402 x 202 (Bluestein's along x and y, whose radices are larger)

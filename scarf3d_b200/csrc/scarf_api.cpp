@@ -298,7 +298,8 @@ struct HostStage {
     return row_bytes + kResult <= bytes ? reinterpret_cast<float*>(p + kResult) : nullptr;
   }
   void release() {
-    if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
+    // A call that failed may have left a kernel that writes the words.
+    if (p && (cudaDeviceSynchronize() != cudaSuccess || cudaFreeHost(p) != cudaSuccess)) (void)cudaGetLastError();
     p = nullptr;
     result_dev = nullptr;
     bytes = 0;
